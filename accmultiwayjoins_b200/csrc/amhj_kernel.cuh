@@ -37,7 +37,7 @@ struct ProbeLaunch {
 // a pusher adds the task's share before publishing it and the warp that takes
 // the task inherits it, so busy == 0 means no work is left anywhere.
 __device__ __forceinline__ bool ws_push(const ProbePlan &P, const WsQueue &Q, const int32_t *vals, uint32_t s,
-                                        uint32_t sz, uint8_t depth, uint16_t qid, uint32_t w) {
+                                        uint32_t sz, uint8_t depth, uint16_t qid, uint32_t w, uint8_t m8) {
     ProbeState *st = Q.st;
     if (ld_volatile_u32(&st->q_tail) >= P.task_cap) return false;
     atomicAdd(&st->busy, 1u);
@@ -52,7 +52,7 @@ __device__ __forceinline__ bool ws_push(const ProbePlan &P, const WsQueue &Q, co
     t->aux = 0;
     t->sz = sz;
     t->depth = depth;
-    t->m8 = 0;
+    t->m8 = m8;
     t->qid = qid;
     t->w = w;
     __threadfence();
@@ -64,22 +64,26 @@ __device__ __forceinline__ bool ws_push(const ProbePlan &P, const WsQueue &Q, co
 // Split rule shared by every mode so a DRO residual replay truncates exactly
 // where the main pass did: a contiguous range longer than twice the task
 // size keeps one task's worth; the rest becomes two tasks (pushed only when
-// `push` is set).  `vals` points at the entry's column in the frontier.
+// `push` is set).  `vals` points at the entry's column in the frontier.  A
+// range of cached suffix tuples (m8 = FIB_FLAG) splits the same way: it can
+// be as long as the whole cache, and one warp left alone with it set the
+// time of the launch (a Zipf(1.0) chain of 1.3M-row relations: main pass
+// 6.2 ms).
 template <int MODE, bool WS>
 __device__ __forceinline__ uint32_t maybe_split(const ProbePlan &P, const WsQueue &Q, const LevelDesc &lv,
                                                 const int32_t *vals, uint32_t s, uint32_t sz, int depth,
-                                                uint16_t qid, uint32_t w) {
+                                                uint16_t qid, uint32_t w, uint8_t m8) {
     if (!WS || lv.layout == AMJ_LAYOUT_CUCKOO) return sz;
     const uint32_t chunk = P.task_chunk;
     if (sz <= 2 * chunk) return sz;
     const uint32_t rem = sz - chunk, half = rem / 2;
     if (MODE == PM_RESIDUAL) return chunk;
     // push the tail first so a failure leaves a contiguous kept range
-    if (!ws_push(P, Q, vals, s + chunk + half, rem - half, (uint8_t)depth, qid, w)) {
+    if (!ws_push(P, Q, vals, s + chunk + half, rem - half, (uint8_t)depth, qid, w, m8)) {
         if (P.dro) report_error(Q.status, (unsigned)-AMJ_EOVERFLOW, SITE_WS_QUEUE, sz);
         return sz;
     }
-    if (!ws_push(P, Q, vals, s + chunk, half, (uint8_t)depth, qid, w)) {
+    if (!ws_push(P, Q, vals, s + chunk, half, (uint8_t)depth, qid, w, m8)) {
         if (P.dro) report_error(Q.status, (unsigned)-AMJ_EOVERFLOW, SITE_WS_QUEUE, sz);
         return chunk + half;
     }
@@ -224,7 +228,7 @@ __device__ __forceinline__ void load_probe_batch(const ProbePlan &P, const WsQue
     uint8_t m8 = 0;
     if (valid) {
         sz = level_lookup(P.lv[0], [&](int a) { return F.vals[a * 32 + lane]; }, s, aux, m8);
-        sz = maybe_split<MODE, WS>(P, Q, P.lv[0], F.vals + lane, s, sz, 0, qid, 1u);
+        sz = maybe_split<MODE, WS>(P, Q, P.lv[0], F.vals + lane, s, sz, 0, qid, 1u, 0);
     }
     F.s[lane] = s;
     F.aux[lane] = aux;
@@ -259,7 +263,7 @@ __device__ __forceinline__ int load_task(const ProbePlan &P, const WsQueue &Q, c
     if (lane < P.k) F.vals[lane * 32] = t.vals[lane];
     __syncwarp();
     if (lane == 0) {
-        const uint32_t sz = maybe_split<MODE, WS>(P, Q, P.lv[td], F.vals, t.s, t.sz, td, t.qid, t.w);
+        const uint32_t sz = maybe_split<MODE, WS>(P, Q, P.lv[td], F.vals, t.s, t.sz, td, t.qid, t.w, t.m8);
         F.s[0] = t.s;
         F.aux[0] = t.aux;
         F.m8[0] = t.m8;
@@ -495,8 +499,8 @@ __device__ __forceinline__ void probe_step(const ProbePlan &P, const WsQueue &Q,
             m8 = FIB_FLAG;
         } else {
             sz = level_lookup(nl, [&](int a) { return C.vals[a * 32 + idx]; }, s, aux, m8);
-            sz = maybe_split<MODE, WS>(P, Q, nl, C.vals + idx, s, sz, nd, qid, wt);
         }
+        sz = maybe_split<MODE, WS>(P, Q, nl, C.vals + idx, s, sz, nd, qid, wt, fi >= 0 ? FIB_FLAG : (uint8_t)0);
         C.s[idx] = s;
         C.aux[idx] = aux;
         C.m8[idx] = m8;

@@ -526,6 +526,27 @@ def test_amhj_fib_materialized_and_other_layouts(layout):
             assert got.stats["fib_rows_served"] > 0
 
 
+@pytest.mark.parametrize("dup", [63, 64, 65, 97, 1000])
+@pytest.mark.parametrize("materialize", [False, True])
+def test_amhj_fib_served_ranges_split(dup, materialize):
+    """Cached suffix ranges shorter than, equal to and longer than twice the
+    task size (32): the longer ones are shared as tasks of cached tuples."""
+    key = np.arange(4, dtype=np.int32)
+    n = 4 * dup
+    rels = [([data.uniform(500, 0, 50, 1), data.uniform(500, 0, 8, 2)], [0, 1]),
+            ([data.uniform(200, 0, 8, 3), data.uniform(200, 0, 6, 4)], [1, 2]),
+            ([np.repeat(key, dup), np.arange(n, dtype=np.int32)], [2, 3]),
+            ([np.arange(n, dtype=np.int32), data.uniform(n, 0, 1 << 20, 5)], [3, 4])]
+    cnt, chk, cols = O.mhj(rels, tuples=True)
+    with Context(0, task_chunk=32) as ctx:
+        got = ctx.amhj("NORMAL", rels_on(ctx, rels), ws=1, fib=1, materialize=materialize)
+        assert (got.count, got.checksum) == (cnt, chk)
+        assert got.stats["fib_rows_served"] > 0
+        assert (got.stats["tasks_pushed"] > 0) == (dup > 64)
+        if materialize:
+            assert np.array_equal(sorted_rows(got.columns), sorted_rows(cols))
+
+
 def test_amhj_fib_star_and_out_of_core():
     """A star join with a shared key (every level keyed on attribute 0) is
     cacheable below level 1; the cache also serves every slice of an
