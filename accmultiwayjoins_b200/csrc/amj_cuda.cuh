@@ -86,6 +86,41 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
+// Up to 32 E values sorted by one warp in registers: value i of the
+// sorted sequence ends in register i % E of lane i / E.  The values may start in
+// any lanes and registers.  A bitonic network: a stage whose partner distance
+// j is E or more exchanges registers between lanes (shuffles), a shorter one
+// within a lane.
+template <int E>
+__device__ __forceinline__ void warp_bitonic_sort(int32_t (&x)[E], uint32_t lane) {
+#pragma unroll
+    for (uint32_t k = 2; k <= 32u * E; k <<= 1)
+#pragma unroll
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            if (j >= (uint32_t)E) {
+                const uint32_t lj = j / E;
+                const bool lower = (lane & lj) == 0;
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    const bool up = ((lane * E + e) & k) == 0;
+                    const int32_t y = __shfl_xor_sync(AMJ_FULL_MASK, x[e], lj);
+                    x[e] = (lower == up) ? min(x[e], y) : max(x[e], y);
+                }
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    const int p = e ^ (int)j;
+                    if (p > e) {
+                        const bool up = ((lane * E + e) & k) == 0;
+                        const int32_t a = x[e], b = x[p];
+                        x[e] = up ? min(a, b) : max(a, b);
+                        x[p] = up ? max(a, b) : min(a, b);
+                    }
+                }
+            }
+        }
+}
+
 __device__ __forceinline__ uint32_t ld_volatile_u32(const uint32_t *p) {
     return *(const volatile uint32_t *)p;
 }

@@ -65,7 +65,8 @@ struct TriArgs {
     const int32_t *inv;
     const uint64_t *wedge;        // (b << 32 | entry) of this slice's entries, sorted by b
     const uint64_t *moff;         // matrix mode: first word of every vertex a's matrix
-    uint32_t *mtx;                // matrix mode: row x of a's matrix has bit y when (a, x, y) is a triangle
+    uint32_t *mtx;                // matrix mode: a's matrix, bit (x, y) for every triangle (a, x, y)
+    const uint16_t *pid;          // matrix mode: every level-1 entry's place in its list by vertex id
     const int32_t *src1;          // level-0 value of every level-1 entry of R
     uint32_t rank_base;           // first rank of the per-warp bitmap
     uint32_t rank_bits;           // ranks the bitmap covers
@@ -408,8 +409,9 @@ __device__ __forceinline__ uint32_t tr_bit(const uint32_t *bm, int32_t c, uint32
 }
 
 // MODE 0: count and checksum; 1: also write the tuples; 2 (matrix mode):
-// record every triangle (a, x, y) as bit y - ta of row x - ta of a's matrix
-// (ta = the start of T(a) in level 1; rows have ceil(d+(a) / 32) words).
+// record every triangle (a, b, c) as bit c of row b of a's matrix, both at
+// their places among a's children by vertex id (A.pid; rows have
+// ceil(d+(a) / 32) words).
 template <int MODE, bool WIDE>
 __global__ __launch_bounds__(TR_THREADS, 3) void lftj_tri_wedge_kernel(const __grid_constant__ TriArgs A) {
     constexpr bool WRITE = MODE == 1;
@@ -427,7 +429,7 @@ __global__ __launch_bounds__(TR_THREADS, 3) void lftj_tri_wedge_kernel(const __g
     int32_t elo = 0, ehi = 0;  // ids of this lane's edge (a, b) in increasing order
     uint64_t eh = 0;           // hash prefix of elo
     uint64_t rowbase = 0;      // matrix mode: first word of this edge's row
-    uint32_t ta32 = 0;         // matrix mode: start of T(a) in level 1
+    auto set_bit = [&](uint64_t rb, uint32_t pc) { atomicOr(&A.mtx[rb + (pc >> 5)], 1u << (pc & 31)); };
     // the first n queued hits, one per lane: the triangle (c, lo, hi) in
     // increasing id order (x, y, z), hashed from the prefix of x
     auto flush = [&](uint32_t n) {
@@ -529,8 +531,7 @@ __global__ __launch_bounds__(TR_THREADS, 3) void lftj_tri_wedge_kernel(const __g
             child_range(A.T, a, ta, te);
             ts = (uint64_t)idx + 1;
             if (MATRIX) {
-                rowbase = A.moff[a] + ((uint64_t)idx - ta) * ((te - ta + 31) / 32);
-                ta32 = (uint32_t)ta;
+                rowbase = A.moff[a] + A.pid[idx] * ((te - ta + 31) / 32);
             } else {
                 const RankId ra = A.hid[a], rb = A.hid[b];
                 const bool alo = ra.id < rb.id;
@@ -582,7 +583,6 @@ __global__ __launch_bounds__(TR_THREADS, 3) void lftj_tri_wedge_kernel(const __g
                 const uint64_t wts = __shfl_sync(AMJ_FULL_MASK, ts, l);
                 const uint64_t wtl = __shfl_sync(AMJ_FULL_MASK, tl, l);
                 const uint64_t lrb = __shfl_sync(AMJ_FULL_MASK, rowbase, l);
-                const uint32_t lta = __shfl_sync(AMJ_FULL_MASK, ta32, l);
                 for (uint64_t k0 = wts; k0 < wtl; k0 += 32) {
                     const uint64_t k = k0 + lane;
                     bool hit = false;
@@ -592,10 +592,7 @@ __global__ __launch_bounds__(TR_THREADS, 3) void lftj_tri_wedge_kernel(const __g
                         hit = nl && (low_smem ? tr_sorted_find(W.low, nl, c) : tr_sorted_find(bl, nl, c));
                     }
                     if (MATRIX) {
-                        if (hit) {
-                            const uint32_t col = (uint32_t)k - lta;
-                            atomicOr(&A.mtx[lrb + (col >> 5)], 1u << (col & 31));
-                        }
+                        if (hit) set_bit(lrb, A.pid[k]);
                         continue;
                     }
                     const unsigned m = __ballot_sync(AMJ_FULL_MASK, hit);
@@ -663,13 +660,12 @@ __global__ __launch_bounds__(TR_THREADS, 3) void lftj_tri_wedge_kernel(const __g
 #pragma unroll
                     for (int u = 0; u < TR_UNROLL; u++) {
                         const uint64_t orb = __shfl_sync(AMJ_FULL_MASK, rowbase, own[u]);
-                        const uint32_t ota = __shfl_sync(AMJ_FULL_MASK, ta32, own[u]);
-#pragma unroll
-                        for (int t = 0; t < 4; t++)
-                            if ((bits >> (4 * u + t)) & 1u) {
-                                const uint32_t col = 4 * qi[u] + t - ota;
-                                atomicOr(&A.mtx[orb + (col >> 5)], 1u << (col & 31));
-                            }
+                        if (!((bits >> (4 * u)) & 15u)) continue;
+                        const ushort4 pc = reinterpret_cast<const ushort4 *>(A.pid)[qi[u]];
+                        if ((bits >> (4 * u)) & 1u) set_bit(orb, pc.x);
+                        if ((bits >> (4 * u + 1)) & 1u) set_bit(orb, pc.y);
+                        if ((bits >> (4 * u + 2)) & 1u) set_bit(orb, pc.z);
+                        if ((bits >> (4 * u + 3)) & 1u) set_bit(orb, pc.w);
                     }
                     continue;
                 }
@@ -712,12 +708,13 @@ __global__ void matrix_words_kernel(const int32_t *__restrict__ data0, const uin
     }
 }
 
-// The triangle matrices of a degree-ranked trie R (ranks 0..nv-1): row x of
-// vertex a's matrix has bit y for every triangle (a, x, y), x and y counted
-// from the start of T(a).  *moff gets the first word of each matrix; the
+// The triangle matrices of a degree-ranked trie R (ranks 0..nv-1): for every
+// triangle (a, b, c) row b of vertex a's matrix has bit c, b and c (in rank
+// order) at their places among a's children by vertex id (pid, one entry a
+// level-1 entry and TRIE_LEVEL1_PAD spare ones).  *moff gets the first word of each matrix; the
 // matrices need *words 32-bit words.  Fails with AMJ_ENOMEM beyond max_words.
-int lftj_tri_matrices(amj_ctx *ctx, const Trie2 &R, const uint64_t *wedge, uint64_t nv, uint32_t rank_bits,
-                      uint64_t max_words, DBuf<uint64_t> *moff, uint32_t **mtx, uint64_t *words) {
+int lftj_tri_matrices(amj_ctx *ctx, const Trie2 &R, const uint64_t *wedge, const uint16_t *pid, uint64_t nv,
+                      uint32_t rank_bits, uint64_t max_words, DBuf<uint64_t> *moff, uint32_t **mtx, uint64_t *words) {
     AMJ_TRY(moff->alloc(ctx, nv + 1));
     AMJ_CUDA_TRY(cudaMemsetAsync(moff->p, 0, (nv + 1) * sizeof(uint64_t), ctx->stream));
     if (R.len0) {
@@ -764,6 +761,7 @@ int lftj_tri_matrices(amj_ctx *ctx, const Trie2 &R, const uint64_t *wedge, uint6
     A.wedge = wedge;
     A.src1 = R.src1.p;
     A.moff = moff->p;
+    A.pid = pid;
     A.mtx = *mtx;
     A.cursor_r = cursor.p;
     uint32_t bits = TR_BITS;

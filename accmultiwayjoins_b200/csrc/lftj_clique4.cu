@@ -20,6 +20,7 @@
 #include "lftj_common.cuh"
 
 #include <algorithm>
+#include <cstddef>
 
 namespace amj {
 
@@ -224,29 +225,48 @@ struct C4Counters {
 // One 4-clique pass over the trie T of the edge relation: count and checksum,
 // and the tuples when `out` is given (out_cap rows).
 // ---- 4-cliques from triangle matrices (degree-ranked copy) ----
-// Over the degree-ranked copy every 4-clique a < x < y < z (ranks) is a
-// triangle (x, y, z) inside N+(a).  The wedge kernel in matrix mode records
-// the triangles (a, x, y) as bits: row x - ta of a's matrix holds bit y - ta
-// (ta = the start of T(a), so rows and columns are positions in N+(a)).
-// Then the 4-cliques through (a, x, y) are the set bits of row x AND row y:
-// persistent warps claim 32 level-1 entries (a, x) at a time, and for each
-// one walk the bits y of row x; each AND is one word per lane (rows have at
-// most 32 words: this path takes out-degrees up to 1024).  Found 4-cliques
-// go to a per-warp queue of (entry lane, y, z) and are mapped to ids, sorted,
-// hashed and written 32 at a time.
+// Over the degree-ranked copy every 4-clique has one vertex a of the lowest
+// rank, and is a triangle inside N+(a).  The wedge kernel in matrix mode
+// records the triangles through a as bits of a's matrix, whose rows and
+// columns are a's children by vertex id; c4m_mirror_kernel then makes row x
+// hold bit y for every y > x adjacent to x.  The 4-cliques through (a, x) are
+// the adjacent pairs y < z among the bits of row x.
+// Numbering by id (not by rank) lists x < y < z in the order of the result
+// tuple, into which only a has to be put at its place pa: the tuple hash of
+// (x, y), with a when it comes before z, is one prefix for all z, so a tuple
+// costs one hash step (a before z) or two (a last) and no sorting.
+// Persistent warps claim 32 level-1 entries (a, x) at a time.  The bits of
+// row x become a list; 32 values y of it (their prefixes in shared memory)
+// meet 32 values z at a time: each lane takes one z and collects its adjacency
+// to the 32 y as a mask (a word of row y a step, the same for neighbouring
+// lanes).  On the skewed R-MAT graphs over half of the pairs are adjacent
+// (55 % at scales 18 and 19), so the masks are dense; their bits go to a list
+// of at most 1024 pairs, which the lanes hash (and write) 32 at a time.
+// Measured, R-MAT scale 20 (12 G 4-cliques): 53 ms; each lane hashing its own
+// mask's bits (18 of 32 lanes active) 70 ms; three or five blocks per SM
+// instead of four 57 and 58 ms.  The kernel is bound by the integer pipe (two
+// 64-bit mixes a tuple) and the issue slots.  R-MAT scale 22 (94 G
+// 4-cliques): 337 ms, against 802 ms for the form in rank order, which
+// ANDed whole rows, queued their bits, and sorted and hashed every tuple in
+// three steps.
 constexpr int C4M_THREADS = 256;
 constexpr int C4M_WARPS = C4M_THREADS / 32;
-constexpr int C4M_QCAP = 1024;   // queued 4-cliques per warp (ring; one step adds at most 1024)
 constexpr uint32_t C4M_MAX_DEG = 1024;
-// per warp: the queue, then the bits y of the current row x
-constexpr size_t C4M_WARP_WORDS = C4M_QCAP + C4M_MAX_DEG / 2;
-constexpr size_t C4M_SMEM = (size_t)C4M_WARPS * C4M_WARP_WORDS * 4;
+
+struct C4MWarp {
+    uint64_t p[2][32];                // prefixes of the 32 y in progress, with a and without
+    int2 z[32];                       // the 32 z: id, and byte offset in p of its prefixes
+    int32_t yid[32];
+    uint16_t ylist[C4M_MAX_DEG + 8];  // the bits of row x, then zeros
+    uint16_t q[32 * 32 + 32];         // adjacent pairs: slot of y << 3 | lane of z << 11
+};
+static_assert(sizeof(C4MWarp) % 16 == 0 && offsetof(C4MWarp, ylist) % 16 == 0, "ylist is read 16 bytes at a time");
 
 struct C4MArgs {
     const int32_t *src1;     // rank a of every level-1 entry
-    const int32_t *id1;      // vertex id of every level-1 value
     const int32_t *inv;      // rank -> vertex id
-    const uint64_t *h1;      // first tuple-hash step of every vertex id
+    const int32_t *sid;      // every child list of level 1 by vertex id
+    const uint16_t *pa;      // place of a's id among its children's
     TrieRef T;
     const uint64_t *moff;    // first matrix word of every rank
     const uint32_t *mtx;
@@ -257,125 +277,146 @@ struct C4MArgs {
 };
 
 template <bool WRITE>
-__global__ __launch_bounds__(C4M_THREADS) void lftj_clique4_matrix_kernel(const __grid_constant__ C4MArgs A) {
-    extern __shared__ uint32_t c4m_smem[];
+__global__ __launch_bounds__(C4M_THREADS, 4) void lftj_clique4_matrix_kernel(const __grid_constant__ C4MArgs A) {
+    __shared__ C4MWarp smem[C4M_WARPS];
     const int lane = threadIdx.x & 31;
-    uint32_t *q = c4m_smem + (threadIdx.x >> 5) * C4M_WARP_WORDS;
-    uint16_t *ylist = reinterpret_cast<uint16_t *>(q + C4M_QCAP);
+    C4MWarp &S = smem[threadIdx.x >> 5];
     unsigned long long cnt = 0, chk = 0;
-    uint32_t qh = 0, qn = 0;
-    int32_t ida = 0, idx_ = 0;   // ids of this lane's entry (a, x)
-    uint32_t ta32 = 0;           // start of T(a)
-    // the first n queued 4-cliques, one per lane: (z << 15) | (y << 5) | lane of (a, x)
-    auto flush = [&](uint32_t n) {
-        __syncwarp();
-        const bool mine = (uint32_t)lane < n;
-        const uint32_t e = mine ? q[(qh + lane) & (C4M_QCAP - 1)] : 0u;
-        const int l = (int)(e & 31u);
-        const int32_t a = __shfl_sync(AMJ_FULL_MASK, ida, l);
-        const int32_t x = __shfl_sync(AMJ_FULL_MASK, idx_, l);
-        const uint32_t t0 = __shfl_sync(AMJ_FULL_MASK, ta32, l);
-        __syncwarp();
-        int32_t v[4] = {a, x, 0, 0};
-        if (mine) {
-            v[2] = A.id1[t0 + ((e >> 5) & 1023u)];
-            v[3] = A.id1[t0 + (e >> 15)];
-        }
-        // the tuple in increasing order (sorting network of four)
-        int32_t t;
-        if (v[0] > v[1]) { t = v[0]; v[0] = v[1]; v[1] = t; }
-        if (v[2] > v[3]) { t = v[2]; v[2] = v[3]; v[3] = t; }
-        if (v[0] > v[2]) { t = v[0]; v[0] = v[2]; v[2] = t; }
-        if (v[1] > v[3]) { t = v[1]; v[1] = v[3]; v[3] = t; }
-        if (v[1] > v[2]) { t = v[1]; v[1] = v[2]; v[2] = t; }
-        if (WRITE) {
-            unsigned long long at = 0;
-            if (lane == 0) at = atomicAdd(A.out_cursor, (unsigned long long)n);
-            at = __shfl_sync(AMJ_FULL_MASK, at, 0);
-            if (mine && at + lane < A.out_cap)
-                for (int i = 0; i < 4; i++) A.out[i][at + lane] = v[i];
-        }
-        if (mine) {
-            cnt++;
-            // the first step from the per-id table: one load instead of a mix
-            chk += amj_hash_step(amj_hash_step(amj_hash_step(A.h1[v[0]], v[1]), v[2]), v[3]);
-        }
-        qh = (qh + n) & (C4M_QCAP - 1);
-        qn -= n;
-    };
     while (true) {
         unsigned long long at = 0;
         if (lane == 0) at = atomicAdd(A.cursor, 32ull);
         at = __shfl_sync(AMJ_FULL_MASK, at, 0);
         if (at >= A.n) break;
         const uint64_t j = at + lane;
-        const bool valid = j < A.n;
-        uint32_t w = 0;
-        uint64_t rowbase = 0, mbase = 0;
-        if (valid) {
-            const int32_t a = A.src1[j];
-            uint64_t ta, te;
+        int32_t a = -1;
+        uint32_t deg = 0, row = 0;
+        uint64_t ta = 0, mbase = 0;
+        if (j < A.n) {
+            a = A.src1[j];
+            uint64_t te;
             child_range(A.T, a, ta, te);
-            w = (uint32_t)((te - ta + 31) / 32);
+            deg = (uint32_t)(te - ta);
+            row = (uint32_t)(j - ta);
             mbase = A.moff[a];
-            rowbase = mbase + (j - ta) * w;
-            ida = A.inv[a];
-            idx_ = A.id1[j];
-            ta32 = (uint32_t)ta;
         }
-        unsigned todo = __ballot_sync(AMJ_FULL_MASK, valid && w > 0);
+        // x needs two children after it
+        unsigned todo = __ballot_sync(AMJ_FULL_MASK, row + 2 < deg);
         while (todo) {
             const int l = __ffs(todo) - 1;
             todo &= todo - 1;
-            const uint32_t wl = __shfl_sync(AMJ_FULL_MASK, w, l);
-            const uint64_t rb = __shfl_sync(AMJ_FULL_MASK, rowbase, l);
-            const uint64_t mb = __shfl_sync(AMJ_FULL_MASK, mbase, l);
-            // row x, one word per lane; its bits y are the triangles (a, x, y)
-            const uint32_t rx = (uint32_t)lane < wl ? A.mtx[rb + lane] : 0u;
+            const uint32_t wl = (__shfl_sync(AMJ_FULL_MASK, deg, l) + 31) / 32;
+            const uint32_t x = __shfl_sync(AMJ_FULL_MASK, row, l);
+            const uint32_t *M = A.mtx + __shfl_sync(AMJ_FULL_MASK, mbase, l);
+            // the bits above x of row x, one word per lane
+            uint32_t rx = (uint32_t)lane < wl && (uint32_t)lane >= x / 32 ? M[x * wl + lane] : 0u;
+            if ((uint32_t)lane == x / 32) rx &= ~1u << (x & 31);
             const uint32_t nyl = __popc(rx);
             const uint32_t yincl = warp_inclusive_scan(nyl, lane);
             const uint32_t ny = __shfl_sync(AMJ_FULL_MASK, yincl, 31);
-            if (ny == 0) continue;
+            if (ny < 2) continue;
+            const int32_t al = __shfl_sync(AMJ_FULL_MASK, a, l);
+            const int32_t *sid = A.sid + __shfl_sync(AMJ_FULL_MASK, ta, l);
+            const int32_t ida = A.inv[al], xid = sid[x];
+            const uint32_t pa = A.pa[al];
+            __syncwarp();
             {
-                uint32_t p = yincl - nyl, m = rx;
+                uint32_t p = yincl, m = rx;
                 while (m) {
-                    const uint32_t b = __ffs(m) - 1;
-                    m &= m - 1;
-                    ylist[p++] = (uint16_t)(lane * 32 + b);
+                    const uint32_t b = 31 - __clz(m);
+                    m ^= 1u << b;
+                    S.ylist[--p] = (uint16_t)(lane * 32 + b);
                 }
+                if (lane < 8) S.ylist[ny + lane] = 0;
             }
             __syncwarp();
-            // 32 / wp bits y per step, wp lanes (one per word of row y) each
-            uint32_t wp = 1;
-            while (wp < wl) wp <<= 1;
-            const uint32_t G = 32 / wp, slot = (uint32_t)lane / wp, wd = (uint32_t)lane & (wp - 1);
-            const uint32_t rxw = __shfl_sync(AMJ_FULL_MASK, rx, (int)wd);
-            for (uint32_t b0 = 0; b0 < ny; b0 += G) {
-                const uint32_t yi = b0 + slot;
-                uint32_t c = 0, y = 0;
-                if (yi < ny) {
-                    y = ylist[yi];
-                    // z: bits of row x AND row y (row y holds bits above y only)
-                    if (wd < wl && wd >= y / 32) c = rxw & A.mtx[mb + (uint64_t)y * wl + wd];
+            // prefixes of x: e1 with a when it comes before x; e2 always with a
+            uint64_t e1 = amj_hash_step(AMJ_CHECKSUM_SEED, x < pa ? xid : ida), e2;
+            if (x < pa) e2 = amj_hash_step(e1, ida);
+            else e1 = e2 = amj_hash_step(e1, xid);
+            for (uint32_t y0 = 0; y0 + 1 < ny; y0 += 32) {
+                const uint32_t nb = min(32u, ny - y0);
+                if ((uint32_t)lane < nb) {
+                    // slot nb - 1 - i holds the prefixes of y i; where a
+                    // comes before x both hold a (e1 = e2 and y >= pa)
+                    const uint32_t y = S.ylist[y0 + lane];
+                    const int32_t yid = sid[y];
+                    const uint64_t p2 = amj_hash_step(e1, yid);
+                    S.p[1][nb - 1 - lane] = p2;
+                    S.p[0][nb - 1 - lane] = amj_hash_step(y < pa ? p2 : e2, y < pa ? ida : yid);
+                    if (WRITE) S.yid[nb - 1 - lane] = yid;
                 }
-                const uint32_t nh = __popc(c);
-                const uint32_t incl = warp_inclusive_scan(nh, lane);
-                const uint32_t tot = __shfl_sync(AMJ_FULL_MASK, incl, 31);
-                if (tot) {
-                    if (qn + tot > C4M_QCAP) flush(qn);   // make room (tot is at most 1024)
-                    uint32_t pos = qh + qn + incl - nh;
-                    while (c) {
-                        const uint32_t bz = __ffs(c) - 1;
-                        c &= c - 1;
-                        q[pos++ & (C4M_QCAP - 1)] = ((wd * 32 + bz) << 15) | (y << 5) | (uint32_t)l;
+                __syncwarp();
+                for (uint32_t z0 = y0; z0 < ny; z0 += 32) {
+                    const bool valid = z0 + lane < ny;
+                    const uint32_t z = valid ? S.ylist[z0 + lane] : 0u;
+                    // rows by 32-bit byte offsets from this lane's column of words
+                    const char *col = reinterpret_cast<const char *>(M + (z >> 5));
+                    const uint32_t sh = 31 - (z & 31);
+                    // bit nb - 1 - i of m: z is adjacent to y i
+                    uint32_t m = 0;
+                    for (uint32_t i = 0; i < nb; i += 8) {
+                        const uint4 y8 = *reinterpret_cast<const uint4 *>(S.ylist + y0 + i);
+                        const uint32_t yy[4] = {y8.x, y8.y, y8.z, y8.w};
+                        uint32_t w[8];
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            w[k] = *reinterpret_cast<const uint32_t *>(
+                                col + (size_t)(((yy[k / 2] >> (16 * (k & 1))) & 0xffffu) * (wl * 4)));
+#pragma unroll
+                        for (int k = 0; k < 8; k++) m = __funnelshift_l(w[k] << sh, m, 1);
                     }
-                    qn += tot;
-                    while (qn >= 32) flush(32);
+                    m >>= (0u - nb) & 7u;   // the zeros after the list
+                    if (z0 == y0) m &= (uint32_t)lane ? ~0u << (nb > (uint32_t)lane ? nb - lane : 0u) : 0u;   // y before z
+                    if (!valid) m = 0;
+                    const uint32_t nh = __popc(m);
+                    const uint32_t incl = warp_inclusive_scan(nh, lane);
+                    uint32_t qn = __shfl_sync(AMJ_FULL_MASK, incl, 31);
+                    if (!qn) continue;
+                    if (lane == 0) cnt += qn;
+                    // a comes after z where z < pa: prefixes without a
+                    S.z[lane] = make_int2(sid[z], z < pa ? (int)sizeof(S.p[0]) : 0);
+                    {
+                        uint16_t *qp = S.q + (incl - nh);
+                        while (m) {
+                            const uint32_t b = 31 - __clz(m);
+                            m ^= 1u << b;
+                            *qp++ = (uint16_t)((uint32_t)lane << 11 | b << 3);
+                        }
+                    }
+                    unsigned long long pos = 0;
+                    if (WRITE) {
+                        if (lane == 0) pos = atomicAdd(A.out_cursor, (unsigned long long)qn);
+                        pos = __shfl_sync(AMJ_FULL_MASK, pos, 0) + lane;
+                    }
+                    __syncwarp();
+#pragma unroll 2
+                    for (uint32_t i = lane; i < qn; i += 32) {
+                        const uint32_t e = S.q[i];
+                        const int2 zz = *reinterpret_cast<const int2 *>(reinterpret_cast<const char *>(S.z) + (e >> 8));
+                        uint64_t h = amj_hash_step(*reinterpret_cast<const uint64_t *>(
+                                                       reinterpret_cast<const char *>(S.p) + zz.y + (e & 0xffu)),
+                                                   zz.x);
+                        if (zz.y) h = amj_hash_step(h, ida);
+                        chk += h;
+                        if (WRITE) {
+                            int32_t v[4] = {ida, xid, S.yid[(e & 0xffu) >> 3], zz.x};   // a to its place
+#pragma unroll
+                            for (int k = 0; k < 3; k++)
+                                if (v[k] > v[k + 1]) {
+                                    const int32_t t = v[k];
+                                    v[k] = v[k + 1];
+                                    v[k + 1] = t;
+                                }
+                            if (pos < A.out_cap)
+                                for (int k = 0; k < 4; k++) A.out[k][pos] = v[k];
+                            pos += 32;
+                        }
+                    }
+                    __syncwarp();
                 }
+                __syncwarp();
             }
-            __syncwarp();
         }
-        if (qn) flush(qn);
     }
     cnt = warp_sum(cnt);
     chk = warp_sum(chk);
@@ -385,14 +426,112 @@ __global__ __launch_bounds__(C4M_THREADS) void lftj_clique4_matrix_kernel(const 
     }
 }
 
-__global__ void level1_ids_kernel(const int32_t *__restrict__ data1, uint64_t n, const int32_t *__restrict__ inv,
-                                  int32_t *__restrict__ id1) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        id1[i] = inv[data1[i]];
+// Transpose of a 32 x 32 bit block, row r in lane r.
+__device__ __forceinline__ uint32_t warp_transpose32(uint32_t v, uint32_t lane) {
+    uint32_t mask = 0x0000ffffu;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        const uint32_t o = __shfl_xor_sync(AMJ_FULL_MASK, v, d);
+        // lanes with bit d clear take the other lane's low columns into their high ones
+        v = (lane & d) ? ((v & ~mask) | ((o & ~mask) >> d)) : ((v & mask) | ((o & mask) << d));
+        mask ^= mask << (d >> 1);
+    }
+    return v;
 }
 
-int lftj_tri_matrices(amj_ctx *ctx, const Trie2 &R, const uint64_t *wedge, uint64_t nv, uint32_t rank_bits,
-                      uint64_t max_words, DBuf<uint64_t> *moff, uint32_t **mtx, uint64_t *words);
+// The wedge kernel leaves the edge between the children at places x < y as
+// bit y of row x or as bit x of row y, whichever ranks lower: afterwards every
+// row x has its bits y > x (bits below x are not read).  One warp a block row
+// of 32 rows: block (i, k) takes in the transpose of block (k, i).
+__global__ __launch_bounds__(256) void c4m_mirror_kernel(const TrieRef T, const int32_t *__restrict__ src1, uint64_t n,
+                                                        const uint64_t *__restrict__ moff, uint32_t *mtx) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
+        const uint64_t j = base + lane;
+        uint32_t deg = 0, row = 1;
+        uint64_t mb = 0;
+        if (j < n) {
+            const int32_t a = src1[j];
+            uint64_t ta, te;
+            child_range(T, a, ta, te);
+            deg = (uint32_t)(te - ta);
+            row = (uint32_t)(j - ta);
+            mb = moff[a];
+        }
+        unsigned todo = __ballot_sync(AMJ_FULL_MASK, (row & 31) == 0 && row + 1 < deg);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t d = __shfl_sync(AMJ_FULL_MASK, deg, l), r0 = __shfl_sync(AMJ_FULL_MASK, row, l);
+            const uint32_t w = (d + 31) / 32, i = r0 / 32;
+            uint32_t *M = mtx + __shfl_sync(AMJ_FULL_MASK, mb, l);
+            for (uint32_t k = i; k < w; k++) {
+                const uint32_t lo = 32 * k + lane < d ? M[(32 * k + lane) * w + i] : 0u;
+                const uint32_t t = warp_transpose32(lo, lane);
+                if (r0 + lane < d && t) M[(r0 + lane) * w + k] |= t;
+            }
+        }
+    }
+}
+
+// Child lists of up to 32 E entries: their vertex ids in increasing order
+// (sid), every entry's place in that order (pid), the place of a's own id.
+template <int E>
+__device__ __forceinline__ uint32_t c4m_order_row(const int32_t *__restrict__ data1, const int32_t *__restrict__ inv,
+                                                  int32_t *sid, uint16_t *__restrict__ pid, uint64_t s, uint32_t len,
+                                                  int32_t ida, uint32_t lane) {
+    int32_t x[E];
+#pragma unroll
+    for (int e = 0; e < E; e++) {
+        const uint32_t i = e * 32u + lane;
+        x[e] = i < len ? inv[data1[s + i]] : INT32_MAX;
+    }
+    uint32_t below = 0;
+#pragma unroll
+    for (int e = 0; e < E; e++) below += (e * 32u + lane < len && x[e] < ida) ? 1u : 0u;
+    warp_bitonic_sort<E>(x, lane);
+#pragma unroll
+    for (int e = 0; e < E; e++)
+        if (lane * E + e < len) sid[s + lane * E + e] = x[e];
+    __syncwarp();
+    for (uint32_t i = lane; i < len; i += 32) {
+        const int32_t id = inv[data1[s + i]];
+        uint32_t lo = 0, hi = len;
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (sid[s + mid] < id) lo = mid + 1;
+            else hi = mid;
+        }
+        pid[s + i] = (uint16_t)lo;
+    }
+    return warp_sum(below);
+}
+
+__global__ __launch_bounds__(256, 4) void c4m_order_kernel(const TrieRef T, uint64_t nv, const int32_t *__restrict__ inv,
+                                                          int32_t *sid, uint16_t *__restrict__ pid,
+                                                          uint16_t *__restrict__ pa) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t v = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < nv; v += warps) {
+        uint64_t s, e;
+        child_range(T, (int32_t)v, s, e);
+        const uint32_t len = (uint32_t)(e - s);
+        if (!len) continue;
+        const int32_t ida = inv[v];
+        uint32_t below;
+        if (len <= 32) below = c4m_order_row<1>(T.data1, inv, sid, pid, s, len, ida, lane);
+        else if (len <= 64) below = c4m_order_row<2>(T.data1, inv, sid, pid, s, len, ida, lane);
+        else if (len <= 128) below = c4m_order_row<4>(T.data1, inv, sid, pid, s, len, ida, lane);
+        else if (len <= 256) below = c4m_order_row<8>(T.data1, inv, sid, pid, s, len, ida, lane);
+        else if (len <= 512) below = c4m_order_row<16>(T.data1, inv, sid, pid, s, len, ida, lane);
+        else below = c4m_order_row<32>(T.data1, inv, sid, pid, s, len, ida, lane);
+        if (lane == 0) pa[v] = (uint16_t)below;
+    }
+}
+
+int lftj_tri_matrices(amj_ctx *ctx, const Trie2 &R, const uint64_t *wedge, const uint16_t *pid, uint64_t nv,
+                      uint32_t rank_bits, uint64_t max_words, DBuf<uint64_t> *moff, uint32_t **mtx, uint64_t *words);
 
 // Largest child list of the trie (its longest out-neighbour list).
 static int trie_max_children(amj_ctx *ctx, const Trie2 &T, uint64_t *maxc) {
@@ -416,19 +555,13 @@ static int trie_max_children(amj_ctx *ctx, const Trie2 &T, uint64_t *maxc) {
 struct C4Matrix {
     DBuf<uint64_t> moff;
     uint32_t *mtx = nullptr;   // the context's matrix buffer
-    DBuf<int32_t> id1;
-    DBuf<uint64_t> h1;         // amj_hash_step(AMJ_CHECKSUM_SEED, id) of every vertex id
+    DBuf<int32_t> sid;         // every child list by vertex id
+    DBuf<uint16_t> pa;         // place of each rank's own id among its children's
 };
-
-// the first step of the tuple hash of every vertex id in [0, nv)
-__global__ void id_hash_kernel(uint64_t nv, uint64_t *__restrict__ h1) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nv; i += (uint64_t)gridDim.x * blockDim.x)
-        h1[i] = amj_hash_step(AMJ_CHECKSUM_SEED, (int32_t)i);
-}
 
 // Whether the matrix path takes the degree-ranked trie T (every out-degree at
 // most 1024, the matrices within half the free device memory), and if so the
-// triangle matrices and the ids of level 1.
+// child lists by id and the triangle matrices.
 int lftj_clique4_matrix_prepare(amj_ctx *ctx, const Trie2 &T, const int32_t *inv, const uint64_t *wedge, uint64_t nv,
                                 uint32_t rank_bits, C4Matrix **out) {
     *out = nullptr;
@@ -441,29 +574,27 @@ int lftj_clique4_matrix_prepare(amj_ctx *ctx, const Trie2 &T, const int32_t *inv
     uint64_t words = 0;
     // at most half the free memory, or the buffer the context already holds
     const uint64_t max_words = std::max<uint64_t>(fr / 2 / 4, ctx->c4_mtx_words);
-    int rc = lftj_tri_matrices(ctx, T, wedge, nv, rank_bits, max_words, &m->moff, &m->mtx, &words);
-    if (rc == AMJ_ENOMEM) {   // the matrices do not fit: not this path
-        delete m;
-        return AMJ_OK;
-    }
-    if (rc == AMJ_OK) rc = m->id1.alloc(ctx, T.len1 ? T.len1 : 1);
+    DBuf<uint16_t> pid;   // read in aligned groups of four, past the last entry
+    int rc = m->sid.alloc(ctx, T.len1 ? T.len1 : 1);
+    if (rc == AMJ_OK) rc = m->pa.alloc(ctx, nv ? nv : 1);
+    if (rc == AMJ_OK) rc = pid.alloc(ctx, T.len1 + TRIE_LEVEL1_PAD);
     if (rc == AMJ_OK && T.len1) {
         note_launch(ctx);
-        level1_ids_kernel<<<(unsigned)std::min<uint64_t>((T.len1 + 255) / 256, (uint64_t)ctx->num_sms * 16), 256, 0,
-                            ctx->stream>>>(T.data1.p, T.len1, inv, m->id1.p);
-        if (cudaGetLastError() != cudaSuccess) rc = fail(AMJ_ECUDA, "LFTJ 4-clique: level-1 ids");
+        c4m_order_kernel<<<(unsigned)std::min<uint64_t>((nv * 32 + 255) / 256, (uint64_t)ctx->num_sms * 16), 256, 0,
+                           ctx->stream>>>(trie_ref(T), nv, inv, m->sid.p, pid.p, m->pa.p);
+        if (cudaGetLastError() != cudaSuccess) rc = fail(AMJ_ECUDA, "LFTJ 4-clique: child lists by id");
     }
-    // vertex ids are the ranks' images, all below nv
-    if (rc == AMJ_OK) rc = m->h1.alloc(ctx, nv ? nv : 1);
-    if (rc == AMJ_OK && nv) {
+    if (rc == AMJ_OK)
+        rc = lftj_tri_matrices(ctx, T, wedge, pid.p, nv, rank_bits, max_words, &m->moff, &m->mtx, &words);
+    if (rc == AMJ_OK && T.len1) {
         note_launch(ctx);
-        id_hash_kernel<<<(unsigned)std::min<uint64_t>((nv + 255) / 256, (uint64_t)ctx->num_sms * 16), 256, 0,
-                         ctx->stream>>>(nv, m->h1.p);
-        if (cudaGetLastError() != cudaSuccess) rc = fail(AMJ_ECUDA, "LFTJ 4-clique: id hashes");
+        c4m_mirror_kernel<<<(unsigned)std::min<uint64_t>((T.len1 + 255) / 256, (uint64_t)ctx->num_sms * 16), 256, 0,
+                            ctx->stream>>>(trie_ref(T), T.src1.p, T.len1, m->moff.p, m->mtx);
+        if (cudaGetLastError() != cudaSuccess) rc = fail(AMJ_ECUDA, "LFTJ 4-clique: mirrored matrices");
     }
     if (rc != AMJ_OK) {
         delete m;
-        return rc;
+        return rc == AMJ_ENOMEM ? AMJ_OK : rc;   // the matrices do not fit: not this path
     }
     *out = m;
     return AMJ_OK;
@@ -484,9 +615,9 @@ int lftj_clique4_matrix(amj_ctx *ctx, const Trie2 &T, const int32_t *inv, const 
     const bool write = out != nullptr;
     C4MArgs A{};
     A.src1 = T.src1.p;
-    A.id1 = m->id1.p;
     A.inv = inv;
-    A.h1 = m->h1.p;
+    A.sid = m->sid.p;
+    A.pa = m->pa.p;
     A.T = trie_ref(T);
     A.moff = m->moff.p;
     A.mtx = m->mtx;
@@ -500,13 +631,12 @@ int lftj_clique4_matrix(amj_ctx *ctx, const Trie2 &T, const int32_t *inv, const 
         A.out_cap = out_cap;
     }
     auto kern = write ? lftj_clique4_matrix_kernel<true> : lftj_clique4_matrix_kernel<false>;
-    AMJ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C4M_SMEM));
     int per_sm = 0;
-    AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C4M_THREADS, C4M_SMEM));
+    AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C4M_THREADS, 0));
     if (per_sm < 1) per_sm = 1;
     AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[0], ctx->stream));
     note_launch(ctx);
-    kern<<<(unsigned)(ctx->num_sms * per_sm), C4M_THREADS, C4M_SMEM, ctx->stream>>>(A);
+    kern<<<(unsigned)(ctx->num_sms * per_sm), C4M_THREADS, 0, ctx->stream>>>(A);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[1], ctx->stream));
     C4Counters h;

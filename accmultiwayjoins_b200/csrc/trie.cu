@@ -289,41 +289,6 @@ __device__ __forceinline__ uint32_t rk_distinct(const int32_t *x, uint32_t len, 
     return u;
 }
 
-// A row of up to 32 E values sorted by one warp in registers: value i of the
-// sorted row ends in register i % E of lane i / E.  The values may start in
-// any lanes and registers.  A bitonic network: a stage whose partner distance
-// j is E or more exchanges registers between lanes (shuffles), a shorter one
-// within a lane.
-template <int E>
-__device__ __forceinline__ void rk_warp_bitonic(int32_t (&x)[E], uint32_t lane) {
-#pragma unroll
-    for (uint32_t k = 2; k <= 32u * E; k <<= 1)
-#pragma unroll
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            if (j >= (uint32_t)E) {
-                const uint32_t lj = j / E;
-                const bool lower = (lane & lj) == 0;
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const bool up = ((lane * E + e) & k) == 0;
-                    const int32_t y = __shfl_xor_sync(AMJ_FULL_MASK, x[e], lj);
-                    x[e] = (lower == up) ? min(x[e], y) : max(x[e], y);
-                }
-            } else {
-#pragma unroll
-                for (int e = 0; e < E; e++) {
-                    const int p = e ^ (int)j;
-                    if (p > e) {
-                        const bool up = ((lane * E + e) & k) == 0;
-                        const int32_t a = x[e], b = x[p];
-                        x[e] = up ? min(a, b) : max(a, b);
-                        x[p] = up ? max(a, b) : min(a, b);
-                    }
-                }
-            }
-        }
-}
-
 // row v = data1[s, s + len), 32 (E / 2) < len <= 32 E: sorted in place, its
 // level-0 value into src1, its number of distinct values into uniq[v]
 template <int E>
@@ -336,7 +301,7 @@ __device__ __forceinline__ void rk_warp_row(int32_t *__restrict__ data1, int32_t
         const uint32_t i = e * 32u + lane;   // coalesced loads; the network fixes the order
         x[e] = i < len ? data1[s + i] : INT32_MAX;
     }
-    rk_warp_bitonic<E>(x, lane);
+    warp_bitonic_sort<E>(x, lane);
     const int32_t prev = __shfl_up_sync(AMJ_FULL_MASK, x[E - 1], 1);
     uint32_t u = 0;
 #pragma unroll

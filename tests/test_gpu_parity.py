@@ -1246,3 +1246,33 @@ def test_sharded_join_shares_sum_to_the_query(ctx):
         got = (sum(c for c, _ in parts) & M64, sum(h for _, h in parts) & M64)
         assert got == want, op
         assert all(c > 0 for c, _ in parts)
+
+
+@pytest.mark.parametrize("n,p", [(4, 1.0), (5, 1.0), (33, 0.7), (34, 1.0), (65, 0.6), (130, 0.5), (258, 0.5), (514, 0.4),
+                                 (1025, 0.35)])
+def test_clique4_matrix_order_by_ids(n, p):
+    """4-cliques by the triangle matrices where the degree order and the id
+    order have nothing to do with each other (the place of the lowest-ranked
+    vertex varies from first to last), at row lengths around the word, warp
+    and sort-network sizes up to the path's longest row."""
+    rng = np.random.default_rng(n)
+    u, v = np.triu_indices(n, 1)
+    keep = rng.random(len(u)) < p
+    keep |= u == 0   # the first vertex is adjacent to all
+    ids = rng.permutation(3 * n).astype(np.int32)[:n]
+    s, d = ids[u[keep]], ids[v[keep]]
+    s, d = np.minimum(s, d), np.maximum(s, d)
+    order = rng.permutation(len(s))
+    s, d = s[order], d[order]
+    with Context(0) as ctx:
+        e = ctx.relation([s, d], [0, 1])
+        got = ctx.lftj([e], clique4=True)
+        lists = ctx.lftj([e], clique4=True, clique4_lists=True)
+        assert (got.count, got.checksum) == (lists.count, lists.checksum)
+        if n <= 130:
+            assert (got.count, got.checksum) == O.four_clique(s, d)
+            m = ctx.lftj([e], clique4=True, materialize=True)
+            a = sorted_rows(m.columns)
+            assert (m.count, m.checksum) == (got.count, got.checksum)
+            assert np.all(a[:, :-1] < a[:, 1:]) and len(np.unique(a, axis=0)) == len(a) == got.count
+            assert data.checksum(m.columns) == got.checksum
