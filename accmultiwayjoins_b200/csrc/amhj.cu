@@ -125,6 +125,9 @@ int compile_plan(int query_type, amj_rel *const *rels, int nrels, int flags, Hos
 
 struct ExecScratch {
     std::map<IndexKey, HashIndex> indexes;
+    DBuf<char> index_block;      // memory of the indexes built together
+    cudaEvent_t end = nullptr;   // to be recorded behind the last launch, when a pass knows it is the last
+    bool ended = false;
     DBuf<ProbeState> st;
     DBuf<Task> tasks;
     DBuf<unsigned int> ready;
@@ -191,6 +194,23 @@ static int launch_probe(amj_ctx *ctx, const ProbeLaunch &PL, int mode, bool ws) 
     return AMJ_OK;
 }
 
+// The probe state, the status block and (work sharing) the task queue, for the
+// passes that use them: the flat kernels take none of it.
+static int ensure_state(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws) {
+    if (!X.st.p) {
+        AMJ_TRY(X.st.alloc(ctx, 1));
+        AMJ_TRY(status_reset(ctx));
+    }
+    if (ws && !X.tasks.p) {
+        AMJ_TRY(X.tasks.alloc(ctx, PL.P.task_cap));
+        AMJ_TRY(X.ready.alloc(ctx, PL.P.task_cap));
+    }
+    PL.st = X.st.p;
+    PL.tasks = X.tasks.p;
+    PL.task_ready = X.ready.p;
+    return AMJ_OK;
+}
+
 static int reset_state(amj_ctx *ctx, ProbeState *st, unsigned int *ready, uint32_t task_cap) {
     AMJ_CUDA_TRY(cudaMemsetAsync(st, 0, sizeof(ProbeState), ctx->stream));
     if (ready) AMJ_CUDA_TRY(cudaMemsetAsync(ready, 0, (size_t)task_cap * sizeof(unsigned int), ctx->stream));
@@ -200,8 +220,9 @@ static int reset_state(amj_ctx *ctx, ProbeState *st, unsigned int *ready, uint32
 // read the probe state back after the last launch; adds that launch's
 // kernel time to *kslot when given
 static int read_state(amj_ctx *ctx, const ProbeState *d, ProbeState *h, const char *what, double *kslot = nullptr) {
-    AMJ_CUDA_TRY(cudaMemcpyAsync(h, d, sizeof(ProbeState), cudaMemcpyDeviceToHost, ctx->stream));
+    AMJ_CUDA_TRY(cudaMemcpyAsync(ctx->h_small, d, sizeof(ProbeState), cudaMemcpyDeviceToHost, ctx->stream));
     AMJ_TRY(status_check(ctx, what));
+    std::memcpy(h, ctx->h_small, sizeof(ProbeState));
     if (kslot) *kslot += event_ms(ctx->kev[0], ctx->kev[1]);
     return AMJ_OK;
 }
@@ -267,11 +288,6 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
         unsigned long long count, checksum;
         unsigned int nover, pad;
     };
-    DBuf<Ctr> ctr;
-    DBuf<uint32_t> over;
-    AMJ_TRY(ctr.alloc(ctx, 1));
-    AMJ_TRY(over.alloc(ctx, rows ? rows : 1));
-    AMJ_CUDA_TRY(cudaMemsetAsync(ctr.p, 0, sizeof(Ctr), ctx->stream));
     const unsigned g = (unsigned)std::min<uint64_t>((rows + 255) / 256, (uint64_t)ctx->num_sms * 8);
     CanonPlan S{};
     int canon = star_canon(P, S);
@@ -280,37 +296,39 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
         canon = chain_canon(P, S);
         chain = canon > 0;
     }
-    DBuf<BucketHead> heads;
     uint32_t maxnb = 0;
-    if (canon) {
-        size_t tot = 0;
-        for (int c = 0; c < canon; c++) {
-            tot += S.nb[c];
-            maxnb = std::max(maxnb, S.nb[c]);
-        }
-        // the heads (32 B a bucket, up to four times the levels' columns)
-        // are built only while they take at most an eighth of the device's
-        // memory; otherwise a star takes the general kernel and a chain the
-        // DFS kernel
-        if (tot * sizeof(BucketHead) > ctx->device_mem / 8) {
-            if (chain) return run_passes(ctx, PL, X, ws, false, false, row_lo, row_hi, pr, res, false);
-            canon = 0;
-        } else {
-            AMJ_TRY(heads.alloc(ctx, tot));
-            // the heads are read by 256-bit loads, which need 32-byte alignment
-            if (reinterpret_cast<uintptr_t>(heads.p) % alignof(BucketHead) != 0) {
-                if (chain) return run_passes(ctx, PL, X, ws, false, false, row_lo, row_hi, pr, res, false);
-                canon = 0;
-            }
-        }
+    size_t nheads = 0;
+    for (int c = 0; c < canon; c++) {
+        nheads += S.nb[c];
+        maxnb = std::max(maxnb, S.nb[c]);
     }
+    // the heads (32 B a bucket, up to four times the levels' columns) are
+    // built only while they take at most an eighth of the device's memory;
+    // otherwise a star takes the general kernel and a chain the DFS kernel
+    if (nheads * sizeof(BucketHead) > ctx->device_mem / 8) {
+        if (chain) return run_passes(ctx, PL, X, ws, false, false, row_lo, row_hi, pr, res, false);
+        canon = 0;
+        nheads = 0;
+    }
+    // one block: the heads (read by 256-bit loads, which need 32-byte
+    // alignment), the counters, the list of rows left for the DFS kernel
+    DBuf<char> work;
+    AMJ_TRY(work.alloc(ctx, nheads * sizeof(BucketHead) + 256 + std::max<uint64_t>(rows, 1) * sizeof(uint32_t)));
+    if (reinterpret_cast<uintptr_t>(work.p) % alignof(BucketHead) != 0 && canon) {
+        if (chain) return run_passes(ctx, PL, X, ws, false, false, row_lo, row_hi, pr, res, false);
+        canon = 0;
+    }
+    BucketHead *heads = reinterpret_cast<BucketHead *>(work.p);
+    Ctr *ctr = reinterpret_cast<Ctr *>(heads + nheads);
+    uint32_t *over = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(ctr) + 256);
+    AMJ_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(Ctr), ctx->stream));
     AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[0], ctx->stream));
     if (canon) {
         HeadOut H{};
         size_t at = 0;
         for (int c = 0; c < canon; c++) {
-            H.p[c] = heads.p + at;
-            S.head[c] = heads.p + at;
+            H.p[c] = heads + at;
+            S.head[c] = heads + at;
             at += S.nb[c];
         }
         const unsigned gx = (unsigned)std::min<uint64_t>((maxnb + 255) / 256, (uint64_t)ctx->num_sms * 4);
@@ -321,28 +339,29 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     note_launch(ctx);
     if (chain) {
         switch (canon) {
-        case 1: amhj_chain_canon_kernel<1><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-        case 2: amhj_chain_canon_kernel<2><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-        case 3: amhj_chain_canon_kernel<3><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-        case 4: amhj_chain_canon_kernel<4><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-        case 5: amhj_chain_canon_kernel<5><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-        default: amhj_chain_canon_kernel<6><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover);
+        case 1: amhj_chain_canon_kernel<1><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+        case 2: amhj_chain_canon_kernel<2><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+        case 3: amhj_chain_canon_kernel<3><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+        case 4: amhj_chain_canon_kernel<4><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+        case 5: amhj_chain_canon_kernel<5><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+        default: amhj_chain_canon_kernel<6><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover);
         }
     } else switch (canon) {
-    case 1: amhj_star_canon_kernel<1><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-    case 2: amhj_star_canon_kernel<2><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-    case 3: amhj_star_canon_kernel<3><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-    case 4: amhj_star_canon_kernel<4><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover); break;
-    default: amhj_star_kernel<<<g ? g : 1, 256, 0, ctx->stream>>>(P, &ctr.p->count, &ctr.p->checksum, over.p, &ctr.p->nover);
+    case 1: amhj_star_canon_kernel<1><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+    case 2: amhj_star_canon_kernel<2><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+    case 3: amhj_star_canon_kernel<3><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+    case 4: amhj_star_canon_kernel<4><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
+    default: amhj_star_kernel<<<g ? g : 1, 256, 0, ctx->stream>>>(P, &ctr->count, &ctr->checksum, over, &ctr->nover);
     }
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[1], ctx->stream));
+    if (X.end) AMJ_CUDA_TRY(cudaEventRecord(X.end, ctx->stream));
     Ctr h{};
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&h, ctr.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    AMJ_TRY(read_back(ctx, &h, ctr, sizeof(h)));
     res->kernel_ms[0] += event_ms(ctx->kev[0], ctx->kev[1]);
     pr->count = h.count;
     pr->checksum = h.checksum;
+    X.ended = X.end && h.nover == 0;
     if (h.nover == 0) return AMJ_OK;
     // the listed rows, gathered into a probe relation of their own
     std::vector<DBuf<int32_t>> cols(P.probe_ncols);
@@ -356,21 +375,13 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     AMJ_CUDA_TRY(cudaMemcpyAsync(dcp.p, cp, sizeof(cp), cudaMemcpyHostToDevice, ctx->stream));
     note_launch(ctx);
     star_gather_kernel<<<(unsigned)std::min<uint64_t>((h.nover + 255) / 256, (uint64_t)ctx->num_sms * 8), 256, 0,
-                         ctx->stream>>>(P, over.p, h.nover, dcp.p);
+                         ctx->stream>>>(P, over, h.nover, dcp.p);
     AMJ_CUDA_TRY(cudaGetLastError());
     ProbeLaunch sub = PL;
     for (int c = 0; c < P.probe_ncols; c++) sub.P.probe_col[c] = cp[c];
     // The listed rows are the heavy ones, and gathered they sit in few warps'
     // row chunks: join them with work sharing whatever the query's ws, so
     // their frontiers spread over all warps (the same result).
-    if (!ws) {
-        if (!X.tasks.p) {
-            AMJ_TRY(X.tasks.alloc(ctx, P.task_cap));
-            AMJ_TRY(X.ready.alloc(ctx, P.task_cap));
-        }
-        sub.tasks = X.tasks.p;
-        sub.task_ready = X.ready.p;
-    }
     PassResult rest;
     AMJ_TRY(run_passes(ctx, sub, X, true, false, false, 0, h.nover, &rest, res, false));
     pr->count += rest.count;
@@ -380,7 +391,7 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
 
 // Materialised star plan (dro=0): per-row tuple counts, a scan, exact
 // allocation, and one flat write pass (amhj_star.cuh).
-static int run_star_write(amj_ctx *ctx, ProbeLaunch &PL, uint64_t row_lo, uint64_t row_hi, PassResult *pr,
+static int run_star_write(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, uint64_t row_lo, uint64_t row_hi, PassResult *pr,
                           amj_result *res) {
     PL.P.row_lo = row_lo;
     PL.P.row_hi = row_hi;
@@ -397,8 +408,7 @@ static int run_star_write(amj_ctx *ctx, ProbeLaunch &PL, uint64_t row_lo, uint64
     AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[1], ctx->stream));
     AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)off.p, (uint64_t *)off.p, rows, (uint64_t *)off.p + rows));
     unsigned long long total = 0;
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&total, off.p + rows, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    AMJ_TRY(read_back(ctx, &total, off.p + rows, sizeof(total)));
     res->kernel_ms[0] += event_ms(ctx->kev[0], ctx->kev[1]);
     AMJ_TRY(alloc_cols(ctx, P.k, total, pr->cols));
     for (int a = 0; a < P.k; a++) P.out[a] = pr->cols[a];
@@ -410,8 +420,9 @@ static int run_star_write(amj_ctx *ctx, ProbeLaunch &PL, uint64_t row_lo, uint64
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[3], ctx->stream));
     unsigned long long h[2] = {0, 0};
-    AMJ_CUDA_TRY(cudaMemcpyAsync(h, ctr.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    if (X.end) AMJ_CUDA_TRY(cudaEventRecord(X.end, ctx->stream));
+    AMJ_TRY(read_back(ctx, h, ctr.p, sizeof(h)));
+    X.ended = X.end != nullptr;
     res->kernel_ms[1] += event_ms(ctx->kev[2], ctx->kev[3]);
     if (h[0] != total) return fail(AMJ_ECUDA, "AMHJ: star write pass disagrees with its row counts");
     pr->count = total;
@@ -428,7 +439,8 @@ static int run_passes(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws, bo
     if (!materialize && allow_flat && (star_eligible(PL.P) || chain_canon(PL.P, chain_shape)))
         return run_flat_count(ctx, PL, X, ws, row_lo, row_hi, pr, res);
     if (materialize && !dro && allow_flat && star_eligible(PL.P))
-        return run_star_write(ctx, PL, row_lo, row_hi, pr, res);
+        return run_star_write(ctx, PL, X, row_lo, row_hi, pr, res);
+    AMJ_TRY(ensure_state(ctx, PL, X, ws));
     ProbePlan &P = PL.P;
     P.row_lo = row_lo;
     P.row_hi = row_hi;
@@ -453,8 +465,7 @@ static int run_passes(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws, bo
         AMJ_CUDA_TRY(cudaGetLastError());
         AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)l0.p, (uint64_t *)l0.p, rows, (uint64_t *)l0.p + rows));
         unsigned long long total = 0;
-        AMJ_CUDA_TRY(cudaMemcpyAsync(&total, l0.p + rows, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
-        AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        AMJ_TRY(read_back(ctx, &total, l0.p + rows, sizeof(total)));
         nchunks = (total + L0_CHUNK - 1) / L0_CHUNK;
         if (nchunks > 0xffffffffull) return fail(AMJ_EUNSUPPORTED, "AMHJ: more than 2^37 level-0 candidates in one slice");
         P.lbs = 1;
@@ -1081,6 +1092,9 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
     ExecScratch X;
     // ---- build phase
     std::vector<const HashIndex *> lvix(hp.L);
+    BucketSpec specs[AMJ_MAX_BUILD_TABLES] = {};   // built together below
+    static_assert(AMJ_MAX_BUILD_TABLES <= BUCKET_BUILD_MAX, "the indexes of a query are built by one call");
+    int nspecs = 0;
     for (int l = 0; l < hp.L; l++) {
         const LevelSpec &ls = hp.lv[l];
         IndexKey key{ls.rel, {-1, -1, -1, -1}, ls.ncols, ls.key_mode, layout};
@@ -1094,7 +1108,15 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
             }
         }
         auto it = X.indexes.find(key);
-        if (it == X.indexes.end()) {
+        if (it == X.indexes.end() && layout == AMJ_LAYOUT_BUCKET && ls.rel->n <= BUCKET_COUNT_MAX) {
+            it = X.indexes.emplace(key, HashIndex()).first;
+            BucketSpec &sp = specs[nspecs++];
+            for (int c = 0; c < ls.ncols; c++) sp.cols[c] = ls.rel->d_cols[ls.src_col[c]];
+            sp.ncols = ls.ncols;
+            sp.n = ls.rel->n;
+            sp.key_mode = ls.key_mode;
+            sp.out = &it->second;
+        } else if (it == X.indexes.end()) {
             HashIndex ix;
             const int32_t *cols[4];
             for (int c = 0; c < ls.ncols; c++) cols[c] = ls.rel->d_cols[ls.src_col[c]];
@@ -1111,6 +1133,7 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         }
         lvix[l] = &it->second;
     }
+    AMJ_TRY(build_bucket_indexes(ctx, specs, nspecs, &X.index_block));
     AMJ_CUDA_TRY(cudaEventRecord(e1, ctx->stream));
 
     // ---- probe plan
@@ -1121,16 +1144,7 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
     for (int l = 0; l < hp.L; l++) fill_level(hp.lv[l], *lvix[l], &P.lv[l]);
     plan_inline(P);
     P.sort_out = sort_out ? 1 : 0;
-    AMJ_TRY(X.st.alloc(ctx, 1));
-    PL.st = X.st.p;
     PL.status = ctx->d_status;
-    if (use_ws) {
-        AMJ_TRY(X.tasks.alloc(ctx, P.task_cap));
-        AMJ_TRY(X.ready.alloc(ctx, P.task_cap));
-        PL.tasks = X.tasks.p;
-        PL.task_ready = X.ready.p;
-    }
-    AMJ_TRY(status_reset(ctx));
     if (fib && !dro && hp.L >= 3) AMJ_TRY(build_fib(ctx, hp, lvix, PL, X, out));
 
     int rc = AMJ_OK;
@@ -1193,6 +1207,7 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         }
     } else {
         PassResult pr;
+        X.end = e2;
         rc = run_passes(ctx, PL, X, use_ws, dro != 0, materialize, 0, hp.probe->n, &pr, out, !(flags & AMJ_F_FRONTIER));
         if (rc == AMJ_OK) {
             out->count = pr.count;
@@ -1210,8 +1225,10 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         amj_result_release(out);
         return rc;
     }
-    AMJ_CUDA_TRY(cudaEventRecord(e2, ctx->stream));
-    AMJ_CUDA_TRY(cudaEventSynchronize(e2));
+    if (!X.ended) {
+        AMJ_CUDA_TRY(cudaEventRecord(e2, ctx->stream));
+        AMJ_CUDA_TRY(cudaEventSynchronize(e2));
+    }
     out->build_ms = event_ms(e0, e1);
     out->probe_ms = event_ms(e1, e2);
     out->total_ms = event_ms(e0, e2);

@@ -164,6 +164,7 @@ struct amj_ctx {
     size_t l2_bytes = 0;
     amj::DevStatus *d_status = nullptr;    // device status block
     amj::DevStatus *h_status = nullptr;    // pinned host mirror
+    void *h_small = nullptr;               // pinned bounce buffer of read_back (READ_BACK_MAX bytes)
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaStream_t side_stream[2] = {nullptr, nullptr};   // ooc copy / prefetch streams
     unsigned long long launches = 0;                     // kernels launched through this context
@@ -228,6 +229,12 @@ struct DBuf {
     T *detach() { T *q = p; p = nullptr; n = 0; return q; }
     ~DBuf() { release(); }
 };
+
+// Copy a small result (at most READ_BACK_MAX bytes) to the host and wait for
+// the context stream: through the context's pinned buffer, since a copy to
+// pageable memory is staged by the driver and returns later.
+constexpr size_t READ_BACK_MAX = 4096;
+int read_back(amj_ctx *ctx, void *dst, const void *d_src, size_t bytes);
 
 // Clear the device status block (enqueued on the context stream).
 int status_reset(amj_ctx *ctx);

@@ -35,7 +35,22 @@ struct HashIndex {
     DBuf<uint32_t> buc_ptrs;       // bucket layout: buckets+1 offsets
     DBuf<int32_t> cols[4];         // bucket layout: columns in bucket order
     DBuf<int2> slots;              // open addressing / cuckoo
+    DBuf<char> block;              // memory of buc_ptrs and cols where a counting build laid them out together
 };
+
+// One index of build_bucket_indexes.
+struct BucketSpec {
+    const int32_t *cols[4];
+    int ncols;
+    uint64_t n;
+    int key_mode;
+    HashIndex *out;
+};
+constexpr uint64_t BUCKET_COUNT_MAX = 1ull << 23;   // rows of an index that the counting build takes
+constexpr int BUCKET_BUILD_MAX = 8;                 // indexes of one build_bucket_indexes call
+// Bucket indexes of up to BUCKET_COUNT_MAX rows each, all built by one set of
+// launches in one block of memory, which `block` owns.
+int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<char> *block);
 
 int build_hash_index(amj_ctx *ctx, const int32_t *const *d_cols, int ncols, uint64_t n, int layout,
                      int key_mode, float load_factor, HashIndex *out);

@@ -17,6 +17,8 @@
 // eviction chain bounded in length; a key can appear at most 8 times.
 #include "hash_build_kernels.cuh"
 
+#include <algorithm>
+
 namespace amj {
 
 __global__ void pack_pairs_kernel(const int32_t *__restrict__ c0, const int32_t *__restrict__ c1, uint64_t n,
@@ -126,97 +128,148 @@ static unsigned grid_for(amj_ctx *ctx, uint64_t n, int threads = 256) {
 }
 
 // ---- counting build (the operator's indexes up to BUCKET_COUNT_MAX rows) ----
-// One count pass over the rows' buckets, a scan, and one scatter pass that
-// claims each row's slot with an atomic on its bucket's cursor: three
-// kernels instead of the radix sort's passes, which are launch-bound at
-// these sizes.  The lanes of a warp that fall in one bucket share one atomic
-// (a hot key costs one atomic per warp, not per row).  Rows keep no order
-// inside a bucket, as in the reference's build (shared-memory atomics); every
-// probe path reads a bucket as a set.
-constexpr uint64_t BUCKET_COUNT_MAX = 1ull << 23;
-
-struct BucketCols {
+// One pass counts the rows of every bucket and keeps each row's place in its
+// bucket (the value its atomic returned), a scan turns the counts into bucket
+// starts, and one pass moves every row to start + place: no radix sort, whose
+// passes are launch-bound at these sizes, and no atomics in the second pass.
+// The lanes of a warp that fall in one bucket share one atomic (a hot key
+// costs one atomic per warp, not per row).  Rows keep no order inside a
+// bucket, as in the reference's build (shared-memory atomics); every probe
+// path reads a bucket as a set.
+// All indexes of a query are built together: their buckets lie end to end in
+// one array, so one scan gives positions in shared columns, and a query has
+// one memset and four launches whatever its levels.  Built one by one (a
+// memset, a count, three scan launches, a copy of the starts and a scatter
+// with atomics a level) the 3-way chain of 1M rows took 144 us for its two
+// indexes, now 81 us, and the 4-way star of 1M / 200K / 100K / 10K rows 216 us,
+// now 67 us; the 10K-row chain, all launches, 154 us and 58 us.
+struct BucketJob {
     const int32_t *in[4];
-    int32_t *out[4];
     int ncols;
     int key_mode;
     uint32_t mask;
+    uint32_t n;
+    uint32_t base;   // first bucket in the shared counts
+    uint32_t row0;   // first row in the shared places
 };
 
-__device__ __forceinline__ uint32_t row_bucket(const BucketCols &C, uint64_t i) {
-    const uint32_t k = C.key_mode == KEY_PAIR ? hash_pair(C.in[0][i], C.in[1][i]) : (uint32_t)C.in[0][i];
-    return k & C.mask;
+struct BucketJobs {
+    BucketJob j[BUCKET_BUILD_MAX];
+    uint32_t *counts;   // counts, after the scan the starts
+    uint32_t *place;
+    int32_t *out[4];
+};
+
+__device__ __forceinline__ uint32_t row_bucket(const BucketJob &J, uint32_t i) {
+    const uint32_t k = J.key_mode == KEY_PAIR ? hash_pair(J.in[0][i], J.in[1][i]) : (uint32_t)J.in[0][i];
+    return J.base + (k & J.mask);
 }
 
-__global__ void bucket_count_kernel(const BucketCols C, uint64_t n, uint32_t *__restrict__ counts) {
+__global__ void bucket_count_kernel(const __grid_constant__ BucketJobs A) {
+    const BucketJob &J = A.j[blockIdx.y];
     const int lane = threadIdx.x & 31;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        const uint64_t i = base + lane;
-        const bool valid = i < n;
-        const uint32_t b = valid ? row_bucket(C, i) : 0xffffffffu;
-        const unsigned peers = __match_any_sync(AMJ_FULL_MASK, b);
-        if (valid && (peers & lanemask_lt()) == 0) atomicAdd(&counts[b], (uint32_t)__popc(peers));
-    }
-}
-
-__global__ void bucket_scatter_kernel(const BucketCols C, uint64_t n, uint32_t *__restrict__ cursor) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < n; base += stride) {
-        const uint64_t i = base + lane;
-        const bool valid = i < n;
-        const uint32_t b = valid ? row_bucket(C, i) : 0xffffffffu;
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < J.n; base += stride) {
+        const uint32_t i = base + lane;
+        const bool valid = i < J.n;
+        const uint32_t b = valid ? row_bucket(J, i) : 0xffffffffu;
         const unsigned peers = __match_any_sync(AMJ_FULL_MASK, b);
         const int leader = __ffs(peers) - 1;
         uint32_t at = 0;
-        if (valid && lane == leader) at = atomicAdd(&cursor[b], (uint32_t)__popc(peers));
+        if (valid && lane == leader) at = atomicAdd(&A.counts[b], (uint32_t)__popc(peers));
         at = __shfl_sync(AMJ_FULL_MASK, at, leader);
-        if (valid) {
-            const uint32_t pos = at + __popc(peers & lanemask_lt());
-            for (int c = 0; c < C.ncols; c++) C.out[c][pos] = C.in[c][i];
-        }
+        if (valid) A.place[J.row0 + i] = at + __popc(peers & lanemask_lt());
     }
 }
 
-static int build_bucket_counting(amj_ctx *ctx, const int32_t *const *d_cols, int ncols, uint64_t n, int key_mode,
-                                 uint64_t B, HashIndex *out) {
-    BucketCols C{};
-    for (int c = 0; c < ncols; c++) {
-        C.in[c] = d_cols[c];
-        C.out[c] = out->cols[c].p;
+__global__ void bucket_scatter_kernel(const __grid_constant__ BucketJobs A) {
+    const BucketJob &J = A.j[blockIdx.y];
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += stride) {
+        const uint32_t pos = A.counts[row_bucket(J, i)] + A.place[J.row0 + i];
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+            if (c < J.ncols) A.out[c][pos] = J.in[c][i];
     }
-    C.ncols = ncols;
-    C.key_mode = key_mode;
-    C.mask = out->mask;
-    AMJ_CUDA_TRY(cudaMemsetAsync(out->buc_ptrs.p, 0, (B + 1) * sizeof(uint32_t), ctx->stream));
+}
+
+int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<char> *block) {
+    if (count <= 0) return AMJ_OK;
+    if (count > BUCKET_BUILD_MAX) return fail(AMJ_EINVAL, "bucket indexes: too many at once");
+    uint64_t rows = 0, buckets = 0, nmax = 0;
+    int ncols = 1;
+    BucketJobs A{};
+    for (int t = 0; t < count; t++) {
+        const BucketSpec &sp = specs[t];
+        if (sp.n > BUCKET_COUNT_MAX || sp.ncols < 1 || sp.ncols > 4) return fail(AMJ_EINVAL, "bucket indexes: bad index");
+        const uint64_t B = sp.n ? floor_pow2(sp.n) : 1;
+        BucketJob &J = A.j[t];
+        for (int c = 0; c < sp.ncols; c++) J.in[c] = sp.cols[c];
+        J.ncols = sp.ncols;
+        J.key_mode = sp.key_mode;
+        J.mask = (uint32_t)(B - 1);
+        J.n = (uint32_t)sp.n;
+        J.base = (uint32_t)buckets;
+        J.row0 = (uint32_t)rows;
+        rows += sp.n;
+        buckets += B;
+        nmax = std::max(nmax, sp.n);
+        ncols = std::max(ncols, sp.ncols);
+    }
+    auto round = [](uint64_t b) { return (b + 255) / 256 * 256; };
+    const uint64_t ptr_bytes = round((buckets + 1) * sizeof(uint32_t));
+    const uint64_t col_bytes = round(std::max<uint64_t>(rows, 1) * sizeof(int32_t));
+    AMJ_TRY(block->alloc(ctx, ptr_bytes + ncols * col_bytes));
+    DBuf<uint32_t> place;
+    AMJ_TRY(place.alloc(ctx, rows));
+    A.counts = reinterpret_cast<uint32_t *>(block->p);
+    A.place = place.p;
+    for (int c = 0; c < ncols; c++) A.out[c] = reinterpret_cast<int32_t *>(block->p + ptr_bytes + c * col_bytes);
+    for (int t = 0; t < count; t++) {
+        // views of the block: no context, so they free nothing
+        HashIndex &ix = *specs[t].out;
+        ix.layout = AMJ_LAYOUT_BUCKET;
+        ix.key_mode = specs[t].key_mode;
+        ix.n = specs[t].n;
+        ix.ncols = specs[t].ncols;
+        ix.mask = A.j[t].mask;
+        ix.buc_ptrs.p = A.counts + A.j[t].base;
+        ix.buc_ptrs.n = (uint64_t)A.j[t].mask + 2;
+        for (int c = 0; c < specs[t].ncols; c++) {
+            ix.cols[c].p = A.out[c];
+            ix.cols[c].n = specs[t].n;
+        }
+    }
+    AMJ_CUDA_TRY(cudaMemsetAsync(A.counts, 0, (buckets + 1) * sizeof(uint32_t), ctx->stream));
+    if (!rows) return AMJ_OK;
+    const dim3 grid(grid_for(ctx, nmax), count);
     note_launch(ctx);
-    bucket_count_kernel<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(C, n, out->buc_ptrs.p);
+    bucket_count_kernel<<<grid, 256, 0, ctx->stream>>>(A);
     AMJ_CUDA_TRY(cudaGetLastError());
-    AMJ_TRY(scan_exclusive_u32(ctx, out->buc_ptrs.p, out->buc_ptrs.p, B + 1, nullptr));
-    DBuf<uint32_t> cursor;
-    AMJ_TRY(cursor.alloc(ctx, B));
-    AMJ_CUDA_TRY(cudaMemcpyAsync(cursor.p, out->buc_ptrs.p, B * sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                                 ctx->stream));
+    AMJ_TRY(scan_exclusive_u32(ctx, A.counts, A.counts, buckets + 1, nullptr));
     note_launch(ctx);
-    bucket_scatter_kernel<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(C, n, cursor.p);
+    bucket_scatter_kernel<<<grid, 256, 0, ctx->stream>>>(A);
     AMJ_CUDA_TRY(cudaGetLastError());
     return AMJ_OK;
 }
 
 static int build_bucket(amj_ctx *ctx, const int32_t *const *d_cols, int ncols, uint64_t n, int key_mode,
                         HashIndex *out) {
-    const uint64_t B = n ? floor_pow2(n) : 1;
+    if (n <= BUCKET_COUNT_MAX) {
+        BucketSpec sp{};
+        for (int c = 0; c < ncols; c++) sp.cols[c] = d_cols[c];
+        sp.ncols = ncols;
+        sp.n = n;
+        sp.key_mode = key_mode;
+        sp.out = out;
+        return build_bucket_indexes(ctx, &sp, 1, &out->block);
+    }
+    const uint64_t B = floor_pow2(n);
     if (B > (1ull << 31)) return fail(AMJ_EINVAL, "bucket index: too many rows");
     const int bits = log2_exact(B);
     out->mask = (uint32_t)(B - 1);
     AMJ_TRY(out->buc_ptrs.alloc(ctx, B + 1));
     for (int c = 0; c < ncols; c++) AMJ_TRY(out->cols[c].alloc(ctx, n ? n : 1));
-    if (n == 0) {
-        AMJ_CUDA_TRY(cudaMemsetAsync(out->buc_ptrs.p, 0, (B + 1) * sizeof(uint32_t), ctx->stream));
-        return AMJ_OK;
-    }
-    if (n <= BUCKET_COUNT_MAX) return build_bucket_counting(ctx, d_cols, ncols, n, key_mode, B, out);
     DBuf<uint64_t> a, b;
     AMJ_TRY(a.alloc(ctx, n));
     AMJ_TRY(b.alloc(ctx, n));

@@ -5,7 +5,8 @@
 // LFTJ-GPU/multi_partitioning.cuh:174-193).
 //
 // Scan: reduce-then-scan over 4096-element tiles (1024 threads x 4 items),
-// recursing on the tile sums.  No inter-block waiting.
+// recursing on the tile sums; up to SCAN_SELF_TILES tiles each block sums the
+// totals before its tile itself.  No inter-block waiting.
 //
 // Radix sort: per pass an up-sweep (per-tile digit histogram, digit-major),
 // a scan of the histogram, and a down-sweep that ranks each item stably
@@ -34,6 +35,13 @@ static int scan_exclusive_impl(amj_ctx *ctx, const T *in, T *out, uint64_t n, T 
     note_launch(ctx);
     scan_reduce_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(in, n, partial.p);
     AMJ_CUDA_TRY(cudaGetLastError());
+    if (tiles <= SCAN_SELF_TILES) {
+        // up to 16M elements: two launches instead of three
+        note_launch(ctx);
+        scan_tiles_self_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(in, out, n, partial.p, d_total);
+        AMJ_CUDA_TRY(cudaGetLastError());
+        return AMJ_OK;
+    }
     AMJ_TRY(scan_exclusive_impl<T>(ctx, partial.p, partial.p, tiles, nullptr));
     note_launch(ctx);
     scan_tiles_kernel<T><<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(in, out, n, partial.p, d_total);

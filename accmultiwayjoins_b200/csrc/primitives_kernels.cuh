@@ -83,6 +83,52 @@ __global__ __launch_bounds__(SCAN_THREADS) void scan_tiles_kernel(const T *in, T
     if (d_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *d_total = off + total;
 }
 
+// As scan_tiles_kernel, with the tile's offset summed here from the totals of
+// the tiles before it instead of a scan of the totals in a launch of its own
+// (each block reads at most SCAN_SELF_TILES totals, one L2 line per 16 or 32).
+constexpr uint64_t SCAN_SELF_TILES = 4096;
+
+template <typename T>
+__global__ __launch_bounds__(SCAN_THREADS) void scan_tiles_self_kernel(const T *in, T *out, uint64_t n,
+                                                                        const T *__restrict__ totals, T *d_total) {
+    __shared__ T tile[SCAN_TILE];
+    __shared__ T wsum[33];
+    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
+    T before = 0;
+    for (uint32_t i = threadIdx.x; i < blockIdx.x; i += SCAN_THREADS) before += totals[i];
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; k++) {
+        const int j = k * SCAN_THREADS + threadIdx.x;
+        const uint64_t i = base + j;
+        tile[j] = i < n ? in[i] : T(0);
+    }
+    T off;
+    block_exclusive_scan(before, wsum, off);
+    __syncthreads();
+    T v[SCAN_IPT];
+    T s = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; k++) {
+        v[k] = tile[threadIdx.x * SCAN_IPT + k];
+        s += v[k];
+    }
+    T total;
+    T run = off + block_exclusive_scan(s, wsum, total);
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; k++) {
+        tile[threadIdx.x * SCAN_IPT + k] = run;
+        run += v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; k++) {
+        const int j = k * SCAN_THREADS + threadIdx.x;
+        const uint64_t i = base + j;
+        if (i < n) out[i] = tile[j];
+    }
+    if (d_total && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *d_total = off + total;
+}
+
 // ------------------------------------------------------------ radix sort --
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;

@@ -47,6 +47,14 @@ void dev_free(amj_ctx *ctx, void *p) {
     if (p) (void)cudaFreeAsync(p, ctx->stream);
 }
 
+int read_back(amj_ctx *ctx, void *dst, const void *d_src, size_t bytes) {
+    if (bytes > READ_BACK_MAX) return fail(AMJ_EINVAL, "read_back: too large");
+    AMJ_CUDA_TRY(cudaMemcpyAsync(ctx->h_small, d_src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(dst, ctx->h_small, bytes);
+    return AMJ_OK;
+}
+
 int status_reset(amj_ctx *ctx) {
     AMJ_CUDA_TRY(cudaMemsetAsync(ctx->d_status, 0, sizeof(DevStatus), ctx->stream));
     return AMJ_OK;
@@ -153,6 +161,7 @@ extern "C" int amj_ctx_create(int device, const amj_opts *opts, amj_ctx **out) {
         if (cudaEventCreate(&c->ev[i]) != cudaSuccess || cudaEventCreate(&c->kev[i]) != cudaSuccess) rc = AMJ_ECUDA;
     if (rc == AMJ_OK && cudaMalloc((void **)&c->d_status, sizeof(DevStatus)) != cudaSuccess) rc = AMJ_ENOMEM;
     if (rc == AMJ_OK && cudaMallocHost((void **)&c->h_status, sizeof(DevStatus)) != cudaSuccess) rc = AMJ_ENOMEM;
+    if (rc == AMJ_OK && cudaMallocHost(&c->h_small, READ_BACK_MAX) != cudaSuccess) rc = AMJ_ENOMEM;
     if (rc == AMJ_OK && cudaMemset(c->d_status, 0, sizeof(DevStatus)) != cudaSuccess) rc = AMJ_ECUDA;
     if (rc != AMJ_OK) {
         (void)cudaGetLastError();
@@ -183,6 +192,7 @@ extern "C" void amj_ctx_destroy(amj_ctx *c) {
         if (c->side_stream[i]) (void)cudaStreamDestroy(c->side_stream[i]);
     if (c->d_status) (void)cudaFree(c->d_status);
     if (c->h_status) (void)cudaFreeHost(c->h_status);
+    if (c->h_small) (void)cudaFreeHost(c->h_small);
     if (c->c4_mtx) (void)cudaFree(c->c4_mtx);
     amj::pinned_cache_release(c);
     if (c->own_stream && c->stream) (void)cudaStreamDestroy(c->stream);
