@@ -16,11 +16,14 @@
 //  probe   level-0 candidate counts of every query's probe rows, one prefix
 //          array over all of them, units of 1024 level-0 candidates per query,
 //          and amhj_batch_kernel over the whole unit space plus the shared
-//          work-sharing queue.  Counts and checksums land in per-query slots.
+//          work-sharing queue.  Triangle queries have units and a kernel of
+//          their own (amhj_tri.cuh).  Counts and checksums land in per-query
+//          slots.
 //
 // Sizes are known on the host once the queries are submitted, so the whole
 // device sequence needs no host round trip and can be captured.
 #include "amhj_batch.h"
+#include "amhj_tri.cuh"
 
 #include <algorithm>
 #include <cstring>
@@ -137,40 +140,67 @@ __global__ void batch_l0_sizes_kernel(const ProbePlan *__restrict__ plans, const
             continue;
         }
         const uint32_t q = find_last_le(qrow, nq, r);
-        sizes[r] = l0_size_of(plans[q], r - qrow[q]);
+        const ProbePlan &P = plans[q];
+        const uint64_t i = r - qrow[q];
+        if (P.tri) {
+            uint32_t s;
+            bool by_a;
+            sizes[r] = tri_side(P, tri_col(P, 0)[i], tri_col(P, 1)[i], s, by_a);
+        } else {
+            sizes[r] = l0_size_of(P, i);
+        }
     }
 }
 
-// unit_base[q] = sum over queries before q of ceil(level-0 candidates / L0_CHUNK); one block
-__global__ void batch_units_kernel(const unsigned long long *__restrict__ l0, const unsigned long long *__restrict__ qrow,
-                                   uint32_t nq, unsigned long long *__restrict__ unit_base) {
-    __shared__ unsigned long long wsum[32];
-    __shared__ unsigned long long carry;
+// First unit of every query: unit_base[q] counts the units of L0_CHUNK level-0
+// candidates of the queries before q (none for a triangle query), tri_base[q]
+// the units of TRI_CHUNK candidates of the triangle queries before q.
+// units[0] = all units; one block
+__global__ void batch_units_kernel(const ProbePlan *__restrict__ plans, const unsigned long long *__restrict__ l0,
+                                   const unsigned long long *__restrict__ qrow, uint32_t nq,
+                                   unsigned long long *__restrict__ unit_base, unsigned long long *__restrict__ tri_base,
+                                   unsigned long long *__restrict__ units) {
+    __shared__ unsigned long long wsum[2][32];
+    __shared__ unsigned long long carry[2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if (threadIdx.x == 0) carry = 0;
+    if (threadIdx.x < 2) carry[threadIdx.x] = 0;
     __syncthreads();
     for (uint32_t b0 = 0; b0 < nq; b0 += blockDim.x) {
         const uint32_t q = b0 + threadIdx.x;
-        unsigned long long u = 0;
+        unsigned long long u = 0, t = 0;
         if (q < nq) {
             const unsigned long long c = l0[qrow[q + 1]] - l0[qrow[q]];
-            u = (c + L0_CHUNK - 1) / L0_CHUNK;
+            if (plans[q].tri) t = (c + TRI_CHUNK - 1) / TRI_CHUNK;
+            else u = (c + L0_CHUNK - 1) / L0_CHUNK;
         }
-        const unsigned long long incl = warp_inclusive_scan(u, lane);
-        if (lane == 31) wsum[warp] = incl;
+        const unsigned long long uincl = warp_inclusive_scan(u, lane), tincl = warp_inclusive_scan(t, lane);
+        if (lane == 31) {
+            wsum[0][warp] = uincl;
+            wsum[1][warp] = tincl;
+        }
         __syncthreads();
-        unsigned long long off = carry;
-        for (int w = 0; w < warp; w++) off += wsum[w];
-        if (q < nq) unit_base[q] = off + incl - u;
+        unsigned long long uoff = carry[0], toff = carry[1];
+        for (int w = 0; w < warp; w++) {
+            uoff += wsum[0][w];
+            toff += wsum[1][w];
+        }
+        if (q < nq) {
+            unit_base[q] = uoff + uincl - u;
+            tri_base[q] = toff + tincl - t;
+        }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned long long t = 0;
-            for (int w = 0; w < nw; w++) t += wsum[w];
-            carry += t;
+        if (threadIdx.x < 2) {
+            unsigned long long x = 0;
+            for (int w = 0; w < nw; w++) x += wsum[threadIdx.x][w];
+            carry[threadIdx.x] += x;
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) unit_base[nq] = carry;
+    if (threadIdx.x == 0) {
+        unit_base[nq] = carry[0];
+        tri_base[nq] = carry[1];
+        units[0] = carry[0] + carry[1];
+    }
 }
 
 __global__ void batch_reset_kernel(ProbeState *st, unsigned int warps) {
@@ -217,6 +247,14 @@ struct amj_batch {
     DBuf<int2> gslots;
     DBuf<ProbePlan> plans;
     DBuf<unsigned long long> qrow, sizes, l0, unit_base, q_count, q_checksum;
+    // triangle queries (amhj_tri.cuh): first units, [0] unit counter and [1]
+    // units of the whole batch, and the heads of their pair indexes
+    DBuf<unsigned long long> tri_base, tri_ctr, tri_first;
+    DBuf<TriHeadJob> tri_jobs;
+    DBuf<BucketHead> tri_heads;
+    uint32_t ntri = 0, ntri_jobs = 0;
+    uint64_t ntri_heads = 0;
+    unsigned tri_grid = 0;
     DBuf<ProbeState> st;
     DBuf<Task> tasks;
     DBuf<unsigned int> ready;
@@ -256,6 +294,11 @@ struct amj_batch {
         sizes.release();
         l0.release();
         unit_base.release();
+        tri_base.release();
+        tri_ctr.release();
+        tri_first.release();
+        tri_jobs.release();
+        tri_heads.release();
         q_count.release();
         q_checksum.release();
         st.release();
@@ -434,6 +477,8 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     AMJ_TRY(ensure(ctx, b->sizes, b->probe_rows + 1));
     AMJ_TRY(ensure(ctx, b->l0, b->probe_rows + 1));
     AMJ_TRY(ensure(ctx, b->unit_base, nq + 1));
+    AMJ_TRY(ensure(ctx, b->tri_base, nq + 1));
+    AMJ_TRY(ensure(ctx, b->tri_ctr, 2));
     AMJ_TRY(ensure(ctx, b->q_count, nq));
     AMJ_TRY(ensure(ctx, b->q_checksum, nq));
     AMJ_TRY(ensure(ctx, b->plans, nq));
@@ -443,6 +488,7 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     po.task_chunk = o.task_chunk;
     std::vector<ProbePlan> hplans(nq);
     uint32_t max_warp_bytes = 0;
+    b->ntri = 0;
     const int32_t *gc[4] = {b->gcols[0].p, b->gcols[1].p, b->gcols[2].p, b->gcols[3].p};
     for (uint32_t q = 0; q < nq; q++) {
         const HostPlan &hp = b->qs[q].hp;
@@ -465,7 +511,47 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
                 fill_level_desc(hp.lv[l], J.layout, J.key_mode, J.mask, nullptr, gc, b->gslots.p + J.base, &P.lv[l]);
         }
         plan_inline(P);
-        max_warp_bytes = std::max(max_warp_bytes, P.warp_bytes);
+        // the triangle over one edge relation, both levels in bucket indexes
+        P.tri = b->qs[q].qt == AMJ_QUERY_TRI && hp.L == 2 && P.inl[1] && P.lv[0].key_mode == KEY_SINGLE &&
+                P.lv[0].layout == AMJ_LAYOUT_BUCKET && P.lv[1].layout == AMJ_LAYOUT_BUCKET;
+        if (P.tri) b->ntri++;
+        else max_warp_bytes = std::max(max_warp_bytes, P.warp_bytes);
+    }
+    // the pair indexes of the triangle queries get bucket heads (32 B a bucket)
+    // while these take at most an eighth of the device's memory; a server's
+    // lanes, which admit requests by batch_estimate_bytes, go without
+    b->ntri_jobs = 0;
+    b->ntri_heads = 0;
+    if (b->ntri && !ctx->iprov) {
+        uint64_t total = 0;
+        std::map<int, uint64_t> first_of;   // job -> first head
+        std::vector<TriHeadJob> hj;
+        std::vector<unsigned long long> first;
+        for (uint32_t q = 0; q < nq; q++) {
+            if (!hplans[q].tri) continue;
+            const int job = where[level_job[q][1]];
+            if (!first_of.emplace(job, total).second) continue;
+            const LevelDesc &lv = hplans[q].lv[1];
+            hj.push_back(TriHeadJob{lv.buc_ptrs, lv.col[0], lv.col[1], total});
+            first.push_back(total);
+            total += (uint64_t)lv.mask + 1;
+        }
+        if (total * sizeof(BucketHead) <= ctx->device_mem / 8) {
+            AMJ_TRY(ensure(ctx, b->tri_heads, total));
+            AMJ_TRY(ensure(ctx, b->tri_jobs, hj.size()));
+            AMJ_TRY(ensure(ctx, b->tri_first, first.size()));
+            if (reinterpret_cast<uintptr_t>(b->tri_heads.p) % alignof(BucketHead) == 0) {
+                AMJ_CUDA_TRY(cudaMemcpyAsync(b->tri_jobs.p, hj.data(), hj.size() * sizeof(TriHeadJob),
+                                             cudaMemcpyHostToDevice, ctx->stream));
+                AMJ_CUDA_TRY(cudaMemcpyAsync(b->tri_first.p, first.data(), first.size() * sizeof(unsigned long long),
+                                             cudaMemcpyHostToDevice, ctx->stream));
+                AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));   // the host arrays end here
+                b->ntri_jobs = (uint32_t)hj.size();
+                b->ntri_heads = total;
+                for (uint32_t q = 0; q < nq; q++)
+                    if (hplans[q].tri) hplans[q].tri_heads = b->tri_heads.p + first_of[where[level_job[q][1]]];
+            }
+        }
     }
     AMJ_CUDA_TRY(cudaMemcpyAsync(b->plans.p, hplans.data(), nq * sizeof(ProbePlan), cudaMemcpyHostToDevice,
                                  ctx->stream));
@@ -480,7 +566,7 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     b->smem = (size_t)(b->block / 32) * b->warp_stride;
     if (b->smem > (size_t)ctx->max_smem_optin) return fail(AMJ_EUNSUPPORTED, "batch: frontier exceeds shared memory");
     b->weighted = false;
-    for (const ProbePlan &P : hplans) b->weighted |= P.has_inl != 0;
+    for (const ProbePlan &P : hplans) b->weighted |= P.has_inl != 0 && !P.tri;
     if (b->weighted) {
         if (b->block == 128) AMJ_TRY((batch_kernel_setup<128, true>(ctx, b->smem, &b->grid)));
         else if (b->block == 256) AMJ_TRY((batch_kernel_setup<256, true>(ctx, b->smem, &b->grid)));
@@ -490,7 +576,13 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
         else if (b->block == 256) AMJ_TRY((batch_kernel_setup<256, false>(ctx, b->smem, &b->grid)));
         else AMJ_TRY((batch_kernel_setup<512, false>(ctx, b->smem, &b->grid)));
     }
-    if (o.grid_blocks > 0 && (unsigned)o.grid_blocks < b->grid) b->grid = (unsigned)o.grid_blocks;
+    int tri_per_sm = 0;
+    AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tri_per_sm, batch_tri_kernel, TRI_THREADS, 0));
+    b->tri_grid = (unsigned)(ctx->num_sms * std::max(tri_per_sm, 1));
+    if (o.grid_blocks > 0) {
+        b->grid = std::min(b->grid, (unsigned)o.grid_blocks);
+        b->tri_grid = std::min(b->tri_grid, (unsigned)o.grid_blocks);
+    }
     const size_t hbytes = (2 * (size_t)nq + 1) * sizeof(unsigned long long) + sizeof(ProbeState);
     if (b->h_out_bytes < hbytes) {
         // pinned memory is kept across runs: freeing it synchronises the device
@@ -549,6 +641,13 @@ static int batch_record(amj_batch *b, bool capturing) {
             b->d_jobs.p, b->d_job_rb.p, njobs, b->bucket_rows, b->oa_rows, b->gslots.p, ctx->d_status);
         AMJ_CUDA_TRY(cudaGetLastError());
     }
+    if (b->ntri_heads) {
+        note_launch(ctx);
+        batch_tri_heads_kernel<<<batch_grid_for(ctx, b->ntri_heads), 256, 0, s>>>(b->tri_jobs.p, b->tri_first.p,
+                                                                                  b->ntri_jobs, b->ntri_heads,
+                                                                                  b->tri_heads.p);
+        AMJ_CUDA_TRY(cudaGetLastError());
+    }
     AMJ_TRY(mark(b->ev[1], s, capturing));
     // ---- probe
     note_launch(ctx);
@@ -557,7 +656,9 @@ static int batch_record(amj_batch *b, bool capturing) {
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)b->sizes.p, (uint64_t *)b->l0.p, b->probe_rows + 1, nullptr));
     note_launch(ctx);
-    batch_units_kernel<<<1, 1024, 0, s>>>(b->l0.p, b->qrow.p, nq, b->unit_base.p);
+    AMJ_CUDA_TRY(cudaMemsetAsync(b->tri_ctr.p, 0, 2 * sizeof(unsigned long long), s));
+    batch_units_kernel<<<1, 1024, 0, s>>>(b->plans.p, b->l0.p, b->qrow.p, nq, b->unit_base.p, b->tri_base.p,
+                                          b->tri_ctr.p + 1);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_CUDA_TRY(cudaMemsetAsync(b->ready.p, 0, (size_t)b->task_cap * sizeof(unsigned int), s));
     AMJ_CUDA_TRY(cudaMemsetAsync(b->q_count.p, 0, nq * sizeof(unsigned long long), s));
@@ -565,6 +666,18 @@ static int batch_record(amj_batch *b, bool capturing) {
     note_launch(ctx);
     batch_reset_kernel<<<1, 32, 0, s>>>(b->st.p, b->grid * (b->block / 32));
     AMJ_CUDA_TRY(cudaGetLastError());
+    if (b->ntri) {
+        TriLaunch T{};
+        T.plans = b->plans.p;
+        T.tri_base = b->tri_base.p;
+        T.next = b->tri_ctr.p;
+        T.q_count = b->q_count.p;
+        T.q_checksum = b->q_checksum.p;
+        T.nq = nq;
+        note_launch(ctx);
+        batch_tri_kernel<<<b->tri_grid, TRI_THREADS, 0, s>>>(T);
+        AMJ_CUDA_TRY(cudaGetLastError());
+    }
     BatchLaunch L;
     std::memset(&L, 0, sizeof(L));
     L.plans = b->plans.p;
@@ -644,7 +757,7 @@ int batch_launch(amj_batch *b, const amj_batch_opts &o) {
     unsigned long long *h = b->h_out;
     AMJ_CUDA_TRY(cudaMemcpyAsync(h, b->q_count.p, nq * 8, cudaMemcpyDeviceToHost, ctx->stream));
     AMJ_CUDA_TRY(cudaMemcpyAsync(h + nq, b->q_checksum.p, nq * 8, cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaMemcpyAsync(h + 2 * nq, b->unit_base.p + nq, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    AMJ_CUDA_TRY(cudaMemcpyAsync(h + 2 * nq, b->tri_ctr.p + 1, 8, cudaMemcpyDeviceToHost, ctx->stream));
     AMJ_CUDA_TRY(cudaMemcpyAsync(h + 2 * nq + 1, b->st.p, sizeof(ProbeState), cudaMemcpyDeviceToHost, ctx->stream));
     AMJ_CUDA_TRY(cudaEventRecord(b->done_ev, ctx->stream));
     return AMJ_OK;

@@ -39,11 +39,30 @@ struct LevelDesc {
     int8_t attr[4];
 };
 
+// The head of a bucket: its bounds and its first rows in one sector, so that
+// looking up a short bucket is one load (the flat star, chain and triangle
+// kernels).
+constexpr int HEAD_ROWS = 3;
+
+struct __align__(32) BucketHead {
+    uint32_t s, e;                      // the bucket's rows [s, e)
+    int32_t kp[2 * HEAD_ROWS];     // its first rows' (column 0, column 1), 0 past e
+};
+static_assert(sizeof(BucketHead) == 32, "a bucket head is one sector");
+
+// one 256-bit load of a head (32-byte aligned), through the read-only path
+__device__ __forceinline__ void load_head(const BucketHead *p, uint32_t (&w)[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+        : "l"(p));
+}
+
 struct alignas(16) ProbePlan {
     uint64_t row_lo, row_hi;            // probe rows handled by this launch
     const int32_t *probe_col[AMJ_MAX_COLS];
     int8_t probe_attr[AMJ_MAX_COLS];
-    int8_t probe_ncols, L, k, pad0;
+    int8_t probe_ncols, L, k;
+    int8_t tri;                         // batched: a triangle query joined by batch_tri_kernel
     LevelDesc lv[AMJ_MAX_BUILD_TABLES];
     // Inline filters: a level that binds nothing and is looked up by the
     // pair of its columns (C(0,2) of the triangle, D/E/F of the 4-clique) is
@@ -84,6 +103,7 @@ struct alignas(16) ProbePlan {
     uint32_t fib_mask;
     uint32_t fib_suffix_attrs;             // attributes the cached tuples provide
     int32_t fib_level;                     // -1: off
+    const BucketHead *tri_heads;           // tri: heads of the pair index (null: not built)
 };
 static_assert(sizeof(ProbePlan) % 16 == 0, "plans are copied as 16-byte words");
 

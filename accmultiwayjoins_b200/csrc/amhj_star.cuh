@@ -134,22 +134,14 @@ __global__ __launch_bounds__(256) void amhj_star_kernel(const __grid_constant__ 
 // distinct line a warp's load touches: the general kernel makes four per
 // level (two bucket bounds, a key, a payload).  Before the probe every bucket
 // of a level gets a 32-byte head, one sector: its bounds and its first
-// STAR_HEAD_ROWS rows (key, payload), read by one 256-bit load.  Dimension
+// HEAD_ROWS rows (key, payload), read by one 256-bit load.  Dimension
 // buckets hold one or two rows (keys unique, floorPow2(rows) buckets), so a
 // lookup is that one load.  A row whose buckets all hold at most
-// STAR_HEAD_ROWS rows, one of them with the key, is one tuple, hashed from
+// HEAD_ROWS rows, one of them with the key, is one tuple, hashed from
 // the keys' shared prefix.  Other rows count their matches per level from
 // the bounds and enumerate the product (an odometer over the levels, the
 // last fastest); products above STAR_MAX_PRODUCT are listed for the DFS
 // kernel as above.
-constexpr int STAR_HEAD_ROWS = 3;
-
-struct __align__(32) BucketHead {
-    uint32_t s, e;                      // the bucket's rows [s, e)
-    int32_t kp[2 * STAR_HEAD_ROWS];     // its first rows' (key, payload), 0 past e
-};
-static_assert(sizeof(BucketHead) == 32, "a bucket head is one sector");
-
 // A star (star_canon) or chain (chain_canon) plan with its levels in key
 // order: star level c is keyed by attribute c, chain level d by d + 1.
 struct CanonPlan {
@@ -201,20 +193,13 @@ __global__ void bucket_heads_kernel(const __grid_constant__ CanonPlan S, const _
         o.s = bp[h];
         o.e = bp[h + 1];
 #pragma unroll
-        for (int i = 0; i < STAR_HEAD_ROWS; i++) {
+        for (int i = 0; i < HEAD_ROWS; i++) {
             const bool in = o.s + i < o.e;
             o.kp[2 * i] = in ? S.key[c][o.s + i] : 0;
             o.kp[2 * i + 1] = in ? S.pay[c][o.s + i] : 0;
         }
         H.p[c][h] = o;
     }
-}
-
-// one 256-bit load of a head (32-byte aligned), through the read-only path
-__device__ __forceinline__ void load_head(const BucketHead *p, uint32_t (&w)[8]) {
-    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-        : "l"(p));
 }
 
 template <int L>
@@ -238,12 +223,12 @@ __global__ __launch_bounds__(256, 4) void amhj_star_canon_kernel(const __grid_co
             uint32_t nm = 0;
             int32_t p = 0;
 #pragma unroll
-            for (int i = 0; i < STAR_HEAD_ROWS; i++) {
+            for (int i = 0; i < HEAD_ROWS; i++) {
                 const bool m = (uint32_t)i < n && (int32_t)w[c][2 + 2 * i] == k[c];
                 nm += m ? 1u : 0u;
                 p = m ? (int32_t)w[c][3 + 2 * i] : p;
             }
-            one &= (n <= (uint32_t)STAR_HEAD_ROWS) & (nm == 1u);
+            one &= (n <= (uint32_t)HEAD_ROWS) & (nm == 1u);
             pay[c] = p;
         }
         uint64_t hk = AMJ_CHECKSUM_SEED;
@@ -359,7 +344,7 @@ __device__ __forceinline__ bool chain_walk(const CanonPlan &S, int32_t key, uint
     budget -= n;
     for (uint32_t i = 0; i < n; i++) {
         int32_t k, v;
-        if (i < (uint32_t)STAR_HEAD_ROWS) {
+        if (i < (uint32_t)HEAD_ROWS) {
             k = (int32_t)(i == 0 ? w[2] : (i == 1 ? w[4] : w[6]));
             v = (int32_t)(i == 0 ? w[3] : (i == 1 ? w[5] : w[7]));
         } else {

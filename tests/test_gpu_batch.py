@@ -168,3 +168,41 @@ def test_batch_rejects_what_it_does_not_run():
         assert e.value.status == L.AMJ_EINVAL
         r = b.run()
         assert (r.counts[0], r.checksums[0]) == O.mhj(data.chain_relations(100, 50, 2, seed=1))
+
+
+def tri_edges(kind, n, seed):
+    """Edge relations where one side's lists are much longer than the other's."""
+    rng = np.random.default_rng(seed)
+    if kind == "empty":
+        return np.zeros(0, np.int32), np.zeros(0, np.int32)
+    if kind == "hub_source":      # the hubs are first: long lists of a
+        s, d = data.rmat(9, n, 0.57, 0.19, 0.19, seed)
+    elif kind == "hub_target":    # the hubs are last: long lists of b
+        s, d = data.rmat(9, n, 0.57, 0.19, 0.19, seed)
+        s, d = 1000 - d, 1000 - s
+    elif kind == "bag":           # any direction, self-loops, repeated rows, negative ids
+        s = rng.integers(-20, 20, n).astype(np.int32)
+        d = rng.integers(-20, 20, n).astype(np.int32)
+    else:                         # sparse ids far above the bucket count, and few buckets hit
+        s = (rng.integers(0, 60, n) * 65536 + 7).astype(np.int32)
+        d = (rng.integers(0, 60, n) * 65536 + 7).astype(np.int32)
+    return np.ascontiguousarray(s, np.int32), np.ascontiguousarray(d, np.int32)
+
+
+@pytest.mark.parametrize("kind", ["empty", "hub_source", "hub_target", "bag", "sparse"])
+@pytest.mark.parametrize("n", [1, 31, 33, 700, 5000])
+def test_batch_triangle_queries(kind, n):
+    """Triangle queries beside another one: the candidates of each edge come
+    from the shorter list, repeated rows multiply, eager and replayed."""
+    edges = [tri_edges(kind, n, s) for s in (1, 2)]
+    want = [O.triangle(s, d) for s, d in edges]
+    star = [([data.uniform(100, 0, 50, 1)], [0]), ([data.permutation(50, 2), data.uniform(50, 0, 9, 3)], [0, 1])]
+    with Context(0) as ctx, ctx.batch() as b:
+        for s, d in edges:
+            b.submit("TRI", [ctx.relation([s, d], [0, 1])])
+        b.submit("NORMAL", [ctx.relation(c, a) for c, a in star])
+        want.append(O.mhj(star) if len(star) > 2 else (100, None))
+        for graph in (False, True, True):
+            r = b.run(use_graph=graph)
+            assert list(zip(r.counts, r.checksums))[:2] == want[:2]
+            assert r.counts[2] == 100
