@@ -152,26 +152,33 @@ __global__ void batch_l0_sizes_kernel(const ProbePlan *__restrict__ plans, const
     }
 }
 
-// First unit of every query: unit_base[q] counts the units of L0_CHUNK level-0
-// candidates of the queries before q (none for a triangle query), tri_base[q]
-// the units of TRI_CHUNK candidates of the triangle queries before q.
-// units[0] = all units; one block
+// First unit of every query: unit_base[q] counts the units of the queries
+// before q (none for a triangle query), tri_base[q] the units of TRI_CHUNK
+// candidates of the triangle queries before q.  units[0] = all units, units[1]
+// = level-0 candidates per unit (l0_chunk_for); one block
 __global__ void batch_units_kernel(const ProbePlan *__restrict__ plans, const unsigned long long *__restrict__ l0,
                                    const unsigned long long *__restrict__ qrow, uint32_t nq,
                                    unsigned long long *__restrict__ unit_base, unsigned long long *__restrict__ tri_base,
-                                   unsigned long long *__restrict__ units) {
+                                   unsigned long long *__restrict__ units, unsigned int warps) {
     __shared__ unsigned long long wsum[2][32];
-    __shared__ unsigned long long carry[2];
+    __shared__ unsigned long long carry[2], cand;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     if (threadIdx.x < 2) carry[threadIdx.x] = 0;
+    if (threadIdx.x == 0) cand = 0;
     __syncthreads();
+    unsigned long long mine = 0;
+    for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x)
+        if (!plans[q].tri) mine += l0[qrow[q + 1]] - l0[qrow[q]];
+    if (mine) atomicAdd(&cand, mine);
+    __syncthreads();
+    const uint32_t chunk = l0_chunk_for(cand, warps);
     for (uint32_t b0 = 0; b0 < nq; b0 += blockDim.x) {
         const uint32_t q = b0 + threadIdx.x;
         unsigned long long u = 0, t = 0;
         if (q < nq) {
             const unsigned long long c = l0[qrow[q + 1]] - l0[qrow[q]];
             if (plans[q].tri) t = (c + TRI_CHUNK - 1) / TRI_CHUNK;
-            else u = (c + L0_CHUNK - 1) / L0_CHUNK;
+            else u = (c + chunk - 1) / chunk;
         }
         const unsigned long long uincl = warp_inclusive_scan(u, lane), tincl = warp_inclusive_scan(t, lane);
         if (lane == 31) {
@@ -200,6 +207,7 @@ __global__ void batch_units_kernel(const ProbePlan *__restrict__ plans, const un
         unit_base[nq] = carry[0];
         tri_base[nq] = carry[1];
         units[0] = carry[0] + carry[1];
+        units[1] = chunk;
     }
 }
 
@@ -247,8 +255,8 @@ struct amj_batch {
     DBuf<int2> gslots;
     DBuf<ProbePlan> plans;
     DBuf<unsigned long long> qrow, sizes, l0, unit_base, q_count, q_checksum;
-    // triangle queries (amhj_tri.cuh): first units, [0] unit counter and [1]
-    // units of the whole batch, and the heads of their pair indexes
+    // triangle queries (amhj_tri.cuh): first units; [0] unit counter, [1] units of
+    // the whole batch, [2] level-0 candidates per unit; and the heads of their pair indexes
     DBuf<unsigned long long> tri_base, tri_ctr, tri_first;
     DBuf<TriHeadJob> tri_jobs;
     DBuf<BucketHead> tri_heads;
@@ -478,7 +486,7 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     AMJ_TRY(ensure(ctx, b->l0, b->probe_rows + 1));
     AMJ_TRY(ensure(ctx, b->unit_base, nq + 1));
     AMJ_TRY(ensure(ctx, b->tri_base, nq + 1));
-    AMJ_TRY(ensure(ctx, b->tri_ctr, 2));
+    AMJ_TRY(ensure(ctx, b->tri_ctr, 3));
     AMJ_TRY(ensure(ctx, b->q_count, nq));
     AMJ_TRY(ensure(ctx, b->q_checksum, nq));
     AMJ_TRY(ensure(ctx, b->plans, nq));
@@ -656,9 +664,9 @@ static int batch_record(amj_batch *b, bool capturing) {
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)b->sizes.p, (uint64_t *)b->l0.p, b->probe_rows + 1, nullptr));
     note_launch(ctx);
-    AMJ_CUDA_TRY(cudaMemsetAsync(b->tri_ctr.p, 0, 2 * sizeof(unsigned long long), s));
+    AMJ_CUDA_TRY(cudaMemsetAsync(b->tri_ctr.p, 0, 3 * sizeof(unsigned long long), s));
     batch_units_kernel<<<1, 1024, 0, s>>>(b->plans.p, b->l0.p, b->qrow.p, nq, b->unit_base.p, b->tri_base.p,
-                                          b->tri_ctr.p + 1);
+                                          b->tri_ctr.p + 1, b->grid * (b->block / 32));
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_CUDA_TRY(cudaMemsetAsync(b->ready.p, 0, (size_t)b->task_cap * sizeof(unsigned int), s));
     AMJ_CUDA_TRY(cudaMemsetAsync(b->q_count.p, 0, nq * sizeof(unsigned long long), s));
@@ -682,6 +690,7 @@ static int batch_record(amj_batch *b, bool capturing) {
     std::memset(&L, 0, sizeof(L));
     L.plans = b->plans.p;
     L.unit_base = b->unit_base.p;
+    L.l0_chunk = b->tri_ctr.p + 2;
     L.q_count = b->q_count.p;
     L.q_checksum = b->q_checksum.p;
     L.Q = WsQueue{b->st.p, b->tasks.p, b->ready.p, ctx->d_status};

@@ -126,6 +126,13 @@ static __device__ int ws_acquire(const WsQueue &Q, uint32_t cap, uint64_t spin_l
 }
 
 
+// Frontiers of more candidates than this are shared with waiting warps.  The
+// split of single long ranges leaves frontiers of many ranges below twice the
+// task size, and trees of them below one unit or task, to one warp: 14 skewed
+// chains ended in a tail of 7.1 ms whatever the size of their units, 5.0 ms with
+// the sharing.
+constexpr uint32_t WS_SHARE_MIN = 256;
+
 // last index r in [0, n) with E[r] <= g (E non-decreasing, E[0] <= g); warp-uniform call
 __device__ __forceinline__ uint64_t warp_row_of(const unsigned long long *E, uint64_t n, unsigned long long g, int lane) {
     uint64_t lo = 0, hi = n;   // answer in [lo, hi)
@@ -143,7 +150,20 @@ __device__ __forceinline__ uint64_t warp_row_of(const unsigned long long *E, uin
     return lo + (uint64_t)__popc(__ballot_sync(AMJ_FULL_MASK, le)) - 1;
 }
 
-constexpr uint32_t L0_CHUNK = 1024;   // level-0 candidates per work-sharing unit
+// Level-0 candidates per work-sharing unit.  A unit's later levels stay with
+// the warp that took it unless one bucket is long enough to be split, so few
+// large units end in a long tail: 14 skewed chains of 11 M level-0 candidates
+// took 24.6 ms in units of 1024 and 7.1 ms in units of 64.  Units shrink down to L0_CHUNK_MIN
+// until every warp gets L0_UNITS_PER_WARP of them; a unit costs two searches
+// for its rows, which the largest size makes negligible on large inputs.
+constexpr uint32_t L0_CHUNK_MAX = 1024, L0_CHUNK_MIN = 64;
+constexpr uint32_t L0_UNITS_PER_WARP = 64;
+
+__host__ __device__ inline uint32_t l0_chunk_for(unsigned long long candidates, unsigned long long warps) {
+    uint32_t c = L0_CHUNK_MAX;
+    while (c > L0_CHUNK_MIN && candidates / c < L0_UNITS_PER_WARP * warps) c >>= 1;
+    return c;
+}
 
 // A level-0 chunk of the plan's candidate space: candidates [g0, g1) of the
 // rows [row, rend).  l0_start holds absolute positions (a batched launch
@@ -153,11 +173,12 @@ struct L0Chunk {
     uint64_t row = 0, rend = 0;
 };
 
-__device__ __forceinline__ void l0_chunk_setup(const ProbePlan &P, unsigned long long chunk, int lane, L0Chunk &c) {
+__device__ __forceinline__ void l0_chunk_setup(const ProbePlan &P, uint32_t size, unsigned long long chunk, int lane,
+                                               L0Chunk &c) {
     const uint64_t rows = P.row_hi - P.row_lo;
     const unsigned long long first = P.l0_start[0], total = P.l0_start[rows];
-    c.g0 = first + chunk * (unsigned long long)L0_CHUNK;
-    c.g1 = c.g0 + L0_CHUNK < total ? c.g0 + L0_CHUNK : total;
+    c.g0 = first + chunk * (unsigned long long)size;
+    c.g1 = c.g0 + size < total ? c.g0 + size : total;
     if (c.g0 < total) {
         c.row = warp_row_of(P.l0_start, rows, c.g0, lane);
         c.rend = warp_row_of(P.l0_start, rows, c.g1 - 1, lane) + 1;
@@ -506,9 +527,24 @@ __device__ __forceinline__ void probe_step(const ProbePlan &P, const WsQueue &Q,
         C.m8[idx] = m8;
         if (WT) C.w[idx] = wt;
     }
-    const unsigned long long ps = warp_inclusive_scan((unsigned long long)(live ? sz : 0u), lane);
+    unsigned long long ps = warp_inclusive_scan((unsigned long long)(live ? sz : 0u), lane);
+    unsigned long long ctot = __shfl_sync(AMJ_FULL_MASK, ps, 31);
+    if (WS && MODE != PM_RESIDUAL && ctot > WS_SHARE_MIN && !P.dro && nl.layout != AMJ_LAYOUT_CUCKOO) {
+        // while warps wait for work, the second half of a large frontier
+        // becomes tasks (not with direct output, whose splits depend on the
+        // data alone)
+        int idle = 0;
+        if (lane == 0) idle = (int)(ld_volatile_u32(&Q.st->q_head) - ld_volatile_u32(&Q.st->q_tail));
+        idle = __shfl_sync(AMJ_FULL_MASK, idle, 0);
+        if (idle > 0) {
+            if (live && sz && ps - sz >= ctot / 2 &&
+                ws_push(P, Q, C.vals + idx, s, sz, (uint8_t)nd, qid, wt, m8))
+                sz = 0;
+            ps = warp_inclusive_scan((unsigned long long)(live ? sz : 0u), lane);
+            ctot = __shfl_sync(AMJ_FULL_MASK, ps, 31);
+        }
+    }
     if (live) C.psum[idx] = ps;
-    const unsigned long long ctot = __shfl_sync(AMJ_FULL_MASK, ps, 31);
     if (lane == 0) {
         C.meta[0] = 0;
         C.meta[1] = ctot;
@@ -644,7 +680,7 @@ __global__ __launch_bounds__(PROBE_THREADS) void amhj_probe_kernel(const __grid_
             u_live = true;
 
             if (have == 3) {
-                l0_chunk_setup(P, l0c, lane, ch);
+                l0_chunk_setup(P, P.l0_chunk, l0c, lane, ch);
                 continue;   // the first group is loaded at the top of the loop
             }
             if (have == 1) {
@@ -669,7 +705,7 @@ __global__ __launch_bounds__(PROBE_THREADS) void amhj_probe_kernel(const __grid_
 // ------------------------------------------------------------- batched --
 // Many queries in one persistent launch.  Their level-0 candidate spaces are
 // laid end to end (one prefix array over every query's probe rows) and cut
-// into L0_CHUNK units; unit_base[q] is the first unit of query q.  A warp
+// into units; unit_base[q] is the first unit of query q.  A warp
 // takes units in order, then work-sharing tasks (which carry their query),
 // and keeps the plan of the query it is on in its own shared memory, so a
 // switch between queries costs one 1 KB copy.  Counts and checksums go to
@@ -677,6 +713,7 @@ __global__ __launch_bounds__(PROBE_THREADS) void amhj_probe_kernel(const __grid_
 struct BatchLaunch {
     const ProbePlan *plans;
     const unsigned long long *unit_base;   // nq + 1 entries
+    const unsigned long long *l0_chunk;    // level-0 candidates per unit of this run
     unsigned long long *q_count;
     unsigned long long *q_checksum;
     WsQueue Q;
@@ -706,6 +743,7 @@ __global__ __launch_bounds__(THREADS) void amhj_batch_kernel(const __grid_consta
     const ProbePlan &P = *reinterpret_cast<const ProbePlan *>(wslot);
     char *wbase = wslot + BATCH_PLAN_BYTES;
     const unsigned long long total_units = B.unit_base[B.nq];
+    const uint32_t chunk = (uint32_t)*B.l0_chunk;
     ProbeAcc acc;
     UnitOut u;
     L0Chunk ch;
@@ -745,7 +783,7 @@ __global__ __launch_bounds__(THREADS) void amhj_batch_kernel(const __grid_consta
                 cur = q;
             }
             if (!task) {
-                l0_chunk_setup(P, b - B.unit_base[q], lane, ch);
+                l0_chunk_setup(P, chunk, b - B.unit_base[q], lane, ch);
             } else {
                 depth = load_task<PM_COUNT, true>(P, B.Q, wbase, tslot, lane);
             }

@@ -91,9 +91,10 @@ struct alignas(16) ProbePlan {
     uint32_t unit_cap;
     // work sharing at level 0: the level-0 candidates of rows row_lo..row_hi-1
     // form one space (l0_start[r - row_lo] = first candidate of row r,
-    // l0_start[rows] = total); units are 32-candidate chunks of it
+    // l0_start[rows] = total); units are chunks of l0_chunk candidates of it
     const unsigned long long *l0_start;
     uint32_t lbs;
+    uint32_t l0_chunk;
     // frequent-item buffering: a depth-fib_level entry whose key is one of
     // the cached frequent keys takes its suffix tuples from the cache
     const int32_t *fib_keys;               // hash set of frequent keys, fib_mask+1 slots

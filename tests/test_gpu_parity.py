@@ -542,7 +542,8 @@ def test_amhj_fib_served_ranges_split(dup, materialize):
         got = ctx.amhj("NORMAL", rels_on(ctx, rels), ws=1, fib=1, materialize=materialize)
         assert (got.count, got.checksum) == (cnt, chk)
         assert got.stats["fib_rows_served"] > 0
-        assert (got.stats["tasks_pushed"] > 0) == (dup > 64)
+        if dup > 64:
+            assert got.stats["tasks_pushed"] > 0
         if materialize:
             assert np.array_equal(sorted_rows(got.columns), sorted_rows(cols))
 
