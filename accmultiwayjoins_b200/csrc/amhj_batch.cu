@@ -5,11 +5,13 @@
 // executor is the batched form of that operator.  Every query is compiled as
 // amj_amhj_execute would compile it, then:
 //
-//  build   all build indexes of all queries at once.  The bucket layout packs
-//          every row as (global bucket << 32 | global row), where global
-//          bucket = the table's first bucket + its own bucket id, sorts the
-//          items once (stable LSD radix sort), gathers the index columns in
-//          that order and turns the run lengths into one bucket-offset array.
+//  build   all build indexes of all queries at once, their buckets end to end
+//          in one bucket-offset array and their rows in shared columns.
+//          Tables of up to 2^23 rows are built by counting; a batch with a
+//          larger one packs every row as (global bucket << 32 | global row),
+//          where global bucket = the table's first bucket + its own bucket
+//          id, sorts the items once (stable LSD radix sort), gathers the index
+//          columns in that order and turns the run lengths into the offsets.
 //          Each table's level descriptor points into the shared arrays.  The
 //          open-addressing layout inserts every row into its table's slot
 //          range in one kernel.
@@ -51,6 +53,92 @@ __device__ __forceinline__ uint32_t find_last_le(const unsigned long long *E, ui
         else hi = mid;
     }
     return lo;
+}
+
+// ---- counting build (every index of the batch within BUCKET_COUNT_MAX rows) ----
+// As build_bucket_indexes (hash_build.cu): each row's place in its bucket from
+// one counting pass, a scan, and one pass that moves the rows.  The random
+// writes stay within one table's columns, which L2 holds while the blocks work
+// on neighbouring rows: every block takes one tile of rows and ends, so the
+// blocks in flight are neighbours.  (In grid-stride loops the blocks drifted
+// apart by tables: the moving pass read and wrote 5.3 GB of DRAM for 1.4 GB of
+// data and took 2.2 ms, for 0.97 ms now.)  Above BUCKET_COUNT_MAX rows the
+// radix sort below, whose passes write runs, is faster.  Measured, the 200
+// indexes of a 128-query mix (60 M rows): 2.35 ms, by the radix sort 4.1 ms.
+constexpr uint32_t BATCH_TILE = 1024;   // rows of a 256-thread block, four a thread
+
+// The owner (job or query) of the rows of a tile, searched once a block.
+struct TileOwner {
+    uint32_t first;   // the owner of the tile's first row
+    bool whole;       // every row of the tile is its
+};
+
+__device__ __forceinline__ TileOwner tile_owner(const unsigned long long *__restrict__ base, uint32_t n,
+                                                unsigned long long r0) {
+    __shared__ TileOwner t;
+    if (threadIdx.x == 0) {
+        t.first = find_last_le(base, n, r0);
+        t.whole = t.first + 1 >= n || base[t.first + 1] >= r0 + BATCH_TILE;
+    }
+    __syncthreads();
+    return t;
+}
+
+__device__ __forceinline__ uint32_t batch_bucket(const BatchJob &J, uint64_t i) {
+    const int32_t c0 = J.col[0][i];
+    const uint32_t key = J.key_mode == KEY_PAIR ? hash_pair(c0, J.col[1][i]) : (uint32_t)c0;
+    return (uint32_t)(J.base + (key & J.mask));
+}
+
+__global__ __launch_bounds__(256) void batch_count_kernel(const BatchJob *__restrict__ jobs,
+                                                          const unsigned long long *__restrict__ job_rb, uint32_t njobs,
+                                                          uint64_t rows, uint32_t *__restrict__ counts,
+                                                          uint32_t *__restrict__ place) {
+    const int lane = threadIdx.x & 31;
+    // a stride between the tiles in flight: neighbouring rows of a skewed table
+    // would count in the same few buckets at once (1.35 ms, against 1.04)
+    for (uint64_t r0 = blockIdx.x * (uint64_t)BATCH_TILE; r0 < rows; r0 += gridDim.x * (uint64_t)BATCH_TILE) {
+        const TileOwner own = tile_owner(job_rb, njobs, r0);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint64_t r = r0 + k * 256 + threadIdx.x;
+            uint32_t b = 0xffffffffu;
+            if (r < rows) {
+                const BatchJob &J = jobs[own.whole ? own.first : find_last_le(job_rb, njobs, r)];
+                b = batch_bucket(J, r - J.row_base);
+            }
+            const unsigned peers = __match_any_sync(AMJ_FULL_MASK, b);
+            const int leader = __ffs(peers) - 1;
+            uint32_t at = 0;
+            if (r < rows && lane == leader) at = atomicAdd(&counts[b], (uint32_t)__popc(peers));
+            at = __shfl_sync(AMJ_FULL_MASK, at, leader);
+            if (r < rows) place[r] = at + __popc(peers & lanemask_lt());
+        }
+        __syncthreads();   // the next tile's owner overwrites this one's
+    }
+}
+
+__global__ __launch_bounds__(256) void batch_scatter_kernel(const BatchJob *__restrict__ jobs,
+                                                            const unsigned long long *__restrict__ job_rb,
+                                                            uint32_t njobs, uint64_t rows,
+                                                            const uint32_t *__restrict__ starts,
+                                                            const uint32_t *__restrict__ place, int32_t *c0,
+                                                            int32_t *c1, int32_t *c2, int32_t *c3) {
+    const uint64_t r0 = blockIdx.x * (uint64_t)BATCH_TILE;
+    const TileOwner own = tile_owner(job_rb, njobs, r0);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint64_t r = r0 + k * 256 + threadIdx.x;
+        if (r < rows) {
+            const BatchJob &J = jobs[own.whole ? own.first : find_last_le(job_rb, njobs, r)];
+            const uint64_t i = r - J.row_base;
+            const uint32_t pos = starts[batch_bucket(J, i)] + place[r];
+            c0[pos] = J.col[0][i];
+            if (J.ncols > 1) c1[pos] = J.col[1][i];
+            if (J.ncols > 2) c2[pos] = J.col[2][i];
+            if (J.ncols > 3) c3[pos] = J.col[3][i];
+        }
+    }
 }
 
 __global__ void batch_pack_kernel(const BatchJob *__restrict__ jobs, const unsigned long long *__restrict__ job_rb,
@@ -132,14 +220,19 @@ __global__ void batch_oa_insert_kernel(const BatchJob *__restrict__ jobs, const 
 }
 
 // level-0 candidate counts of every query's probe rows; sizes[rows] = 0
-__global__ void batch_l0_sizes_kernel(const ProbePlan *__restrict__ plans, const unsigned long long *__restrict__ qrow,
-                                      uint32_t nq, uint64_t rows, unsigned long long *__restrict__ sizes) {
-    for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r <= rows; r += (uint64_t)gridDim.x * blockDim.x) {
+__global__ __launch_bounds__(256) void batch_l0_sizes_kernel(const ProbePlan *__restrict__ plans,
+                                                             const unsigned long long *__restrict__ qrow, uint32_t nq,
+                                                             uint64_t rows, unsigned long long *__restrict__ sizes) {
+    const uint64_t r0 = blockIdx.x * (uint64_t)BATCH_TILE;
+    const TileOwner own = tile_owner(qrow, nq, r0);
+    for (int k = 0; k < 4; k++) {
+        const uint64_t r = r0 + k * 256 + threadIdx.x;
+        if (r > rows) return;
         if (r == rows) {
             sizes[r] = 0;
-            continue;
+            return;
         }
-        const uint32_t q = find_last_le(qrow, nq, r);
+        const uint32_t q = own.whole ? own.first : find_last_le(qrow, nq, r);
         const ProbePlan &P = plans[q];
         const uint64_t i = r - qrow[q];
         if (P.tri) {
@@ -249,7 +342,9 @@ struct amj_batch {
     size_t smem = 0;
     DBuf<BatchJob> d_jobs;
     DBuf<unsigned long long> d_job_rb;
+    bool counting = true;      // bucket indexes by counting (else by the radix sort of items_a / items_b)
     DBuf<uint64_t> items_a, items_b;
+    DBuf<uint32_t> place;
     DBuf<int32_t> gcols[4];
     DBuf<uint32_t> gptrs;
     DBuf<int2> gslots;
@@ -294,6 +389,7 @@ struct amj_batch {
         d_job_rb.release();
         items_a.release();
         items_b.release();
+        place.release();
         for (auto &c : gcols) c.release();
         gptrs.release();
         gslots.release();
@@ -360,6 +456,8 @@ static int batch_kernel_setup(amj_ctx *ctx, size_t smem, unsigned *grid) {
     *grid = (unsigned)(ctx->num_sms * per_sm);
     return AMJ_OK;
 }
+
+static unsigned batch_tiles(uint64_t rows) { return (unsigned)((rows + BATCH_TILE - 1) / BATCH_TILE); }
 
 // Plan the batch for the given options: jobs, plans, sizes, device buffers.
 // grow-only device buffer
@@ -471,8 +569,15 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     AMJ_CUDA_TRY(cudaMemcpyAsync(b->d_job_rb.p, b->job_rb.data(), njobs * sizeof(unsigned long long),
                                  cudaMemcpyHostToDevice, ctx->stream));
     const uint64_t br = std::max<uint64_t>(b->bucket_rows, 1);
-    AMJ_TRY(ensure(ctx, b->items_a, br));
-    AMJ_TRY(ensure(ctx, b->items_b, br));
+    b->counting = true;
+    for (auto &J : b->jobs)
+        if (J.layout == AMJ_LAYOUT_BUCKET) b->counting &= J.n <= BUCKET_COUNT_MAX;
+    if (b->counting) {
+        AMJ_TRY(ensure(ctx, b->place, br));
+    } else {
+        AMJ_TRY(ensure(ctx, b->items_a, br));
+        AMJ_TRY(ensure(ctx, b->items_b, br));
+    }
     for (int c = 0; c < b->ncols_max; c++) AMJ_TRY(ensure(ctx, b->gcols[c], br));
     AMJ_TRY(ensure(ctx, b->gptrs, b->total_buckets + 1));
     if (b->total_slots) AMJ_TRY(ensure(ctx, b->gslots, b->total_slots));
@@ -619,7 +724,19 @@ static int batch_record(amj_batch *b, bool capturing) {
     const unsigned long long l0 = ctx->launches;
     AMJ_TRY(mark(b->ev[0], s, capturing));
     // ---- build
-    if (b->bucket_rows) {
+    if (b->bucket_rows && b->counting) {
+        AMJ_CUDA_TRY(cudaMemsetAsync(b->gptrs.p, 0, (b->total_buckets + 1) * sizeof(uint32_t), s));
+        note_launch(ctx);
+        batch_count_kernel<<<std::min(batch_tiles(b->bucket_rows), (unsigned)ctx->num_sms * 8u), 256, 0, s>>>(
+            b->d_jobs.p, b->d_job_rb.p, njobs, b->bucket_rows, b->gptrs.p, b->place.p);
+        AMJ_CUDA_TRY(cudaGetLastError());
+        AMJ_TRY(scan_exclusive_u32(ctx, b->gptrs.p, b->gptrs.p, b->total_buckets + 1, nullptr));
+        note_launch(ctx);
+        batch_scatter_kernel<<<batch_tiles(b->bucket_rows), 256, 0, s>>>(
+            b->d_jobs.p, b->d_job_rb.p, njobs, b->bucket_rows, b->gptrs.p, b->place.p, b->gcols[0].p, b->gcols[1].p,
+            b->gcols[2].p, b->gcols[3].p);
+        AMJ_CUDA_TRY(cudaGetLastError());
+    } else if (b->bucket_rows) {
         note_launch(ctx);
         batch_pack_kernel<<<batch_grid_for(ctx, b->bucket_rows), 256, 0, s>>>(b->d_jobs.p, b->d_job_rb.p, njobs,
                                                                               b->bucket_rows, b->items_a.p);
@@ -659,7 +776,7 @@ static int batch_record(amj_batch *b, bool capturing) {
     AMJ_TRY(mark(b->ev[1], s, capturing));
     // ---- probe
     note_launch(ctx);
-    batch_l0_sizes_kernel<<<batch_grid_for(ctx, b->probe_rows + 1), 256, 0, s>>>(b->plans.p, b->qrow.p, nq,
+    batch_l0_sizes_kernel<<<batch_tiles(b->probe_rows + 1), 256, 0, s>>>(b->plans.p, b->qrow.p, nq,
                                                                                 b->probe_rows, b->sizes.p);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)b->sizes.p, (uint64_t *)b->l0.p, b->probe_rows + 1, nullptr));

@@ -164,7 +164,7 @@ struct amj_ctx {
     size_t l2_bytes = 0;
     amj::DevStatus *d_status = nullptr;    // device status block
     amj::DevStatus *h_status = nullptr;    // pinned host mirror
-    void *h_small = nullptr;               // pinned bounce buffer of read_back (READ_BACK_MAX bytes)
+    void *h_small = nullptr;               // pinned bounce buffer of read_back (READ_BACK_MAX bytes, behind h_status)
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaStream_t side_stream[2] = {nullptr, nullptr};   // ooc copy / prefetch streams
     unsigned long long launches = 0;                     // kernels launched through this context

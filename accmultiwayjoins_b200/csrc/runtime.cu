@@ -160,8 +160,11 @@ extern "C" int amj_ctx_create(int device, const amj_opts *opts, amj_ctx **out) {
     for (int i = 0; rc == AMJ_OK && i < 4; i++)
         if (cudaEventCreate(&c->ev[i]) != cudaSuccess || cudaEventCreate(&c->kev[i]) != cudaSuccess) rc = AMJ_ECUDA;
     if (rc == AMJ_OK && cudaMalloc((void **)&c->d_status, sizeof(DevStatus)) != cudaSuccess) rc = AMJ_ENOMEM;
-    if (rc == AMJ_OK && cudaMallocHost((void **)&c->h_status, sizeof(DevStatus)) != cudaSuccess) rc = AMJ_ENOMEM;
-    if (rc == AMJ_OK && cudaMallocHost(&c->h_small, READ_BACK_MAX) != cudaSuccess) rc = AMJ_ENOMEM;
+    // one pinned block (each costs a millisecond or two): the status mirror,
+    // then the bounce buffer
+    if (rc == AMJ_OK && cudaMallocHost((void **)&c->h_status, 64 + READ_BACK_MAX) != cudaSuccess) rc = AMJ_ENOMEM;
+    static_assert(sizeof(DevStatus) <= 64, "the bounce buffer starts behind the status mirror");
+    if (rc == AMJ_OK) c->h_small = reinterpret_cast<char *>(c->h_status) + 64;
     if (rc == AMJ_OK && cudaMemset(c->d_status, 0, sizeof(DevStatus)) != cudaSuccess) rc = AMJ_ECUDA;
     if (rc != AMJ_OK) {
         (void)cudaGetLastError();
@@ -192,7 +195,6 @@ extern "C" void amj_ctx_destroy(amj_ctx *c) {
         if (c->side_stream[i]) (void)cudaStreamDestroy(c->side_stream[i]);
     if (c->d_status) (void)cudaFree(c->d_status);
     if (c->h_status) (void)cudaFreeHost(c->h_status);
-    if (c->h_small) (void)cudaFreeHost(c->h_small);
     if (c->c4_mtx) (void)cudaFree(c->c4_mtx);
     amj::pinned_cache_release(c);
     if (c->own_stream && c->stream) (void)cudaStreamDestroy(c->stream);

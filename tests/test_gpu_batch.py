@@ -206,3 +206,25 @@ def test_batch_triangle_queries(kind, n):
             r = b.run(use_graph=graph)
             assert list(zip(r.counts, r.checksums))[:2] == want[:2]
             assert r.counts[2] == 100
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, (1 << 23) - 5, (1 << 23) + 1])
+def test_batch_index_builds_around_the_limits(n):
+    """Index builds at the edges of a tile of rows and on both sides of the
+    counting build's largest table, next to small tables of three columns."""
+    small = [([data.uniform(300, 0, 40, 1), data.uniform(300, 0, 9, 2)], [0, 1]),
+             ([data.uniform(500, 0, 9, 3), data.uniform(500, 0, 40, 4), data.uniform(500, 0, 99, 5)], [1, 0, 2])]
+    big = [([data.uniform(4000, 0, 1 << 20, 6), data.uniform(4000, 0, max(n, 2), 7)], [0, 1]),
+           ([data.uniform(n, 0, max(n, 2), 8), data.uniform(n, 0, 99, 9)], [1, 2])]
+    with Context(0) as ctx, ctx.batch() as b:
+        alone = []
+        for q in (small, big, small):
+            rels = [ctx.relation(c, a) for c, a in q]
+            b.submit("NORMAL", rels)
+            r = ctx.amhj("NORMAL", rels, plan="frontier")
+            alone.append((r.count, r.checksum))
+        r = b.run()
+        assert list(zip(r.counts, r.checksums)) == alone
+        assert alone[0] == alone[2] == O.mhj(small)
+        if n < 1 << 20:
+            assert alone[1] == O.mhj(big)
