@@ -27,7 +27,7 @@
 // served system runs the same stages again); amj_ctx_trim and the context's
 // destruction free them.  Rows are grouped by key hash on the device (input
 // tables stream through it in chunks; each part result is grouped before it
-// is copied back), so a part is a union of groups and the host scatters
+// is copied back), so a part is a run of groups and the host scatters
 // nothing up to 256 parts.  Part p+1 is copied to the device on one side
 // stream while part p is joined, and part p's grouped result goes back on
 // the other side stream while part p+1 is joined.
@@ -139,9 +139,8 @@ struct HostTable {
 // The rows a stage returns form the next stage's intermediate, which is
 // partitioned on the next key.  They are grouped on the device into
 // SUB_PARTS groups by that key's hash before they are copied back, so that
-// a part of the next stage (P <= SUB_PARTS parts, P a power of two) is the
-// union of the groups s with s & (P - 1) == p, and the host scatters
-// nothing.  One count pass, a scan of the counts, then tiles of rows
+// a part of the next stage (P <= SUB_PARTS parts, P a power of two) is a run
+// of SUB_PARTS / P groups, and the host scatters nothing.  One count pass, a scan of the counts, then tiles of rows
 // scattered with one atomic reservation per group and tile.
 constexpr uint32_t SUB_PARTS = 256;
 constexpr uint32_t SUB_TILE = 4096;
@@ -220,12 +219,29 @@ int partition_table(amj_ctx *ctx, const HostTable &X, int kc, uint32_t P, Parts 
         return AMJ_OK;
     }
     if (X.sub_col == kc && P <= SUB_PARTS && X.sub.size() == SUB_PARTS) {
-        // grouped on the device already: part p is the union of its groups
-        for (uint32_t g = 0; g < SUB_PARTS; g++)
+        // grouped on the device already: part p is SUB_PARTS / P consecutive
+        // groups.  The groups of one block lie one after another in every
+        // column, so they make one piece: a part is then one copy a column
+        // and block.  (Parts of every P-th group were one copy a column and
+        // group: 26.7K copies of 5.8 us for 4 tables of 2^24 rows in 8 parts,
+        // most of the join's time.)
+        for (uint32_t g = 0; g < SUB_PARTS; g++) {
+            const uint32_t p = (uint32_t)((uint64_t)g * P / SUB_PARTS);
+            std::vector<Piece> &parts = out->part[p];
             for (const Piece &pc : X.sub[g]) {
-                out->part[g & (P - 1)].push_back(pc);
-                out->rows[g & (P - 1)] += pc.n;
+                out->rows[p] += pc.n;
+                bool joined = false;
+                for (Piece &o : parts) {
+                    bool next = true;
+                    for (size_t c = 0; c < X.attrs.size() && next; c++) next = o.col[c] + o.n == pc.col[c];
+                    if (!next) continue;
+                    o.n += pc.n;
+                    joined = true;
+                    break;
+                }
+                if (!joined) parts.push_back(pc);
             }
+        }
         for (uint32_t p = 0; p < P; p++) out->max_rows = std::max(out->max_rows, out->rows[p]);
         return AMJ_OK;
     }
