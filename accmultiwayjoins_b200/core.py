@@ -336,21 +336,19 @@ class Context:
 
     def _result(self, res: L.amj_result, materialize: bool) -> Result:
         cols = None
-        if materialize:
-            k = res.num_attrs
-            rows = int(res.rows)
-            cols = []
-            for a in range(k):
-                if rows:
-                    cols.append(np.ctypeslib.as_array(res.cols[a], shape=(rows,)).copy())
-                else:
-                    cols.append(np.zeros(0, np.int32))
-        out = Result(count=int(res.count), checksum=int(res.checksum), num_attrs=int(res.num_attrs),
-                     build_ms=float(res.build_ms), probe_ms=float(res.probe_ms), total_ms=float(res.total_ms),
-                     stats={STAT_NAMES[i]: int(res.stats[i]) for i in range(len(STAT_NAMES))},
-                     kernel_ms=tuple(float(res.kernel_ms[i]) for i in range(4)), columns=cols)
-        L.load().amj_result_release(C.byref(res))
-        return out
+        try:
+            if materialize:
+                k = res.num_attrs
+                cols = [np.empty(int(res.rows), np.int32) for _ in range(k)]
+                if res.rows:
+                    dst = (C.POINTER(C.c_int32) * k)(*[c.ctypes.data_as(C.POINTER(C.c_int32)) for c in cols])
+                    L.check(L.load().amj_result_copy_host(C.byref(res), dst), "result_copy_host")
+            return Result(count=int(res.count), checksum=int(res.checksum), num_attrs=int(res.num_attrs),
+                          build_ms=float(res.build_ms), probe_ms=float(res.probe_ms), total_ms=float(res.total_ms),
+                          stats={STAT_NAMES[i]: int(res.stats[i]) for i in range(len(STAT_NAMES))},
+                          kernel_ms=tuple(float(res.kernel_ms[i]) for i in range(4)), columns=cols)
+        finally:
+            L.load().amj_result_release(C.byref(res))
 
     def amhj(self, query_type, relations: Sequence[Relation], ooc: int = 0, ws: int = 0, dro: int = 0,
              fib: int = 0, materialize: bool = False, reorder: bool = True, degree_order: bool = True,

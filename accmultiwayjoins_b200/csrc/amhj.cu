@@ -240,24 +240,33 @@ static int alloc_cols(amj_ctx *ctx, int k, uint64_t rows, int32_t **cols) {
 
 int finish_result_columns(amj_ctx *ctx, amj_result *res, int flags) {
     if (!(flags & AMJ_F_HOST_RESULT) || res->on_host) return AMJ_OK;
+    auto *o = static_cast<ResultOwner *>(res->priv);
+    if (!o) return fail(AMJ_EINVAL, "result: columns without an owner");
+    // all columns in one pinned block of the context's pool
+    void *block = nullptr;
+    size_t size = 0;
+    const size_t col = (size_t)(res->rows ? res->rows : 1) * sizeof(int32_t), stride = (col + 255) / 256 * 256;
+    AMJ_TRY(result_block_get(ctx, stride * res->num_attrs, &block, &size));
     int32_t *host[AMJ_MAX_ATTRS] = {};
-    for (int a = 0; a < res->num_attrs; a++) {
+    cudaError_t e = cudaSuccess;
+    for (int a = 0; a < (int)res->num_attrs && e == cudaSuccess; a++) {
         if (!res->cols[a]) continue;
-        if (cudaMallocHost((void **)&host[a], (res->rows ? res->rows : 1) * sizeof(int32_t)) != cudaSuccess) {
-            (void)cudaGetLastError();
-            for (int b = 0; b < a; b++) cudaFreeHost(host[b]);
-            return fail(AMJ_ENOMEM, "result: pinned host allocation failed");
-        }
-        if (res->rows)
-            AMJ_CUDA_TRY(cudaMemcpyAsync(host[a], res->cols[a], res->rows * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                         ctx->stream));
+        host[a] = reinterpret_cast<int32_t *>(static_cast<char *>(block) + a * stride);
+        if (res->rows) e = cudaMemcpyAsync(host[a], res->cols[a], col, cudaMemcpyDeviceToHost, ctx->stream);
     }
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    for (int a = 0; a < res->num_attrs; a++) {
+    const cudaError_t es = cudaStreamSynchronize(ctx->stream);   // also before the block can go back
+    if (e == cudaSuccess) e = es;
+    if (e != cudaSuccess) {
+        result_block_put(ctx, block, size);
+        return cuda_fail(e, "result: copy to host memory");
+    }
+    for (int a = 0; a < (int)res->num_attrs; a++) {
         if (!res->cols[a]) continue;
         dev_free(ctx, res->cols[a]);
         res->cols[a] = host[a];
     }
+    o->host_block = block;
+    o->host_bytes = size;
     res->on_host = 1;
     return AMJ_OK;
 }

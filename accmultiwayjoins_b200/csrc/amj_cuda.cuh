@@ -173,6 +173,7 @@ struct amj_ctx {
     void *c4_mtx = nullptr;                // 4-clique triangle matrices, kept across calls (grow-only)
     uint64_t c4_mtx_words = 0;
     void *pinned_cache = nullptr;          // pinned host blocks of out-of-core stages, kept across calls
+    void *result_pool = nullptr;           // pinned blocks of host results, kept across calls
 };
 
 struct amj_rel {
@@ -196,6 +197,14 @@ int dev_alloc(amj_ctx *ctx, void **p, size_t bytes);
 void dev_free(amj_ctx *ctx, void *p);
 // Free the pinned host blocks the context keeps for out-of-core stages.
 void pinned_cache_release(amj_ctx *ctx);
+
+// Pinned host blocks for materialised results.  Released blocks stay with the
+// context, up to RESULT_POOL_MAX bytes, for the next result (pinning costs
+// about 0.4 ms a megabyte); amj_ctx_trim and the context's end free them.
+// Results may be released by any thread.
+constexpr size_t RESULT_POOL_MAX = 256ull << 20;
+int result_block_get(amj_ctx *ctx, size_t bytes, void **p, size_t *size);
+void result_block_put(amj_ctx *ctx, void *p, size_t size);
 
 template <typename T>
 struct DBuf {

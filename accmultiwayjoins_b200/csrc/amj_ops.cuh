@@ -5,6 +5,8 @@
 
 struct ResultOwner {
     amj_ctx *ctx = nullptr;
+    void *host_block = nullptr;   // pinned block of all host columns, back to the context's pool on release
+    size_t host_bytes = 0;
 };
 
 namespace amj {

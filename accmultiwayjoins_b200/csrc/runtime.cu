@@ -8,11 +8,15 @@
 // come back as status codes with a per-thread message.
 #include "amj_cuda.cuh"
 
+#include <omp.h>
+
+#include <algorithm>
 #include <atomic>
 #include "amj_ops.cuh"
 
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 
 namespace amj {
@@ -53,6 +57,56 @@ int read_back(amj_ctx *ctx, void *dst, const void *d_src, size_t bytes) {
     AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     std::memcpy(dst, ctx->h_small, bytes);
     return AMJ_OK;
+}
+
+struct ResultPool {
+    std::mutex mu;
+    std::multimap<size_t, void *> blocks;   // by size
+    size_t bytes = 0;
+};
+
+int result_block_get(amj_ctx *ctx, size_t bytes, void **p, size_t *size) {
+    const size_t want = (std::max<size_t>(bytes, 1) + 65535) / 65536 * 65536;
+    auto *pool = static_cast<ResultPool *>(ctx->result_pool);
+    {
+        std::lock_guard<std::mutex> lk(pool->mu);
+        auto it = pool->blocks.lower_bound(want);
+        if (it != pool->blocks.end() && it->first <= 2 * want + (1u << 20)) {
+            *size = it->first;
+            *p = it->second;
+            pool->bytes -= it->first;
+            pool->blocks.erase(it);
+            return AMJ_OK;
+        }
+    }
+    if (cudaMallocHost(p, want) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return fail(AMJ_ENOMEM, "result: pinned host allocation failed");
+    }
+    *size = want;
+    return AMJ_OK;
+}
+
+void result_block_put(amj_ctx *ctx, void *p, size_t size) {
+    auto *pool = static_cast<ResultPool *>(ctx->result_pool);
+    {
+        std::lock_guard<std::mutex> lk(pool->mu);
+        if (pool->bytes + size <= RESULT_POOL_MAX) {
+            pool->bytes += size;
+            pool->blocks.emplace(size, p);
+            return;
+        }
+    }
+    (void)cudaFreeHost(p);
+}
+
+static void result_pool_clear(amj_ctx *ctx) {
+    auto *pool = static_cast<ResultPool *>(ctx->result_pool);
+    if (!pool) return;
+    std::lock_guard<std::mutex> lk(pool->mu);
+    for (auto &b : pool->blocks) (void)cudaFreeHost(b.second);
+    pool->blocks.clear();
+    pool->bytes = 0;
 }
 
 int status_reset(amj_ctx *ctx) {
@@ -140,6 +194,7 @@ extern "C" int amj_ctx_create(int device, const amj_opts *opts, amj_ctx **out) {
     AMJ_CUDA_TRY(cudaSetDevice(device));
     auto *c = new amj_ctx();
     c->device = device;
+    c->result_pool = new ResultPool();
     if (opts) c->opts = *opts;
     if (c->opts.block_size <= 0) c->opts.block_size = 256;
     if (c->opts.load_factor <= 0.f || c->opts.load_factor >= 1.f) c->opts.load_factor = 0.5f;
@@ -197,6 +252,8 @@ extern "C" void amj_ctx_destroy(amj_ctx *c) {
     if (c->h_status) (void)cudaFreeHost(c->h_status);
     if (c->c4_mtx) (void)cudaFree(c->c4_mtx);
     amj::pinned_cache_release(c);
+    result_pool_clear(c);
+    delete static_cast<ResultPool *>(c->result_pool);
     if (c->own_stream && c->stream) (void)cudaStreamDestroy(c->stream);
     (void)cudaGetLastError();
     delete c;
@@ -228,6 +285,7 @@ extern "C" int amj_ctx_trim(amj_ctx *c) {
     AMJ_CUDA_TRY(cudaSetDevice(c->device));
     AMJ_CUDA_TRY(cudaStreamSynchronize(c->stream));
     amj::pinned_cache_release(c);
+    result_pool_clear(c);
     if (c->c4_mtx) {
         AMJ_CUDA_TRY(cudaFree(c->c4_mtx));
         c->c4_mtx = nullptr;
@@ -318,6 +376,25 @@ void result_init(amj_result *res, int k) {
 }
 }  // namespace amj
 
+// Copies on the host cores: a large result's cost is the first touch of the
+// caller's fresh pages, which one thread does at 3 GB/s or less.
+extern "C" int amj_result_copy_host(const amj_result *res, int32_t *const *dst) {
+    if (!res || (res->rows && !dst)) return fail(AMJ_EINVAL, "result_copy_host: null argument");
+    if (!res->rows) return AMJ_OK;
+    if (!res->on_host) return fail(AMJ_EINVAL, "result_copy_host: the columns are on the device");
+    for (int a = 0; a < (int)res->num_attrs; a++)
+        if (!res->cols[a] || !dst[a]) return fail(AMJ_EINVAL, "result_copy_host: null column");
+    constexpr uint64_t CHUNK = 1u << 18;   // values
+    const uint64_t per = (res->rows + CHUNK - 1) / CHUNK, n = per * res->num_attrs;
+    const int threads = (int)std::min<uint64_t>(n, (uint64_t)omp_get_max_threads());
+#pragma omp parallel for schedule(dynamic, 1) num_threads(threads) if (threads > 1)
+    for (long long i = 0; i < (long long)n; i++) {
+        const uint64_t a = (uint64_t)i / per, lo = (uint64_t)i % per * CHUNK;
+        std::memcpy(dst[a] + lo, res->cols[a] + lo, std::min<uint64_t>(CHUNK, res->rows - lo) * sizeof(int32_t));
+    }
+    return AMJ_OK;
+}
+
 extern "C" void amj_result_release(amj_result *res) {
     if (!res) return;
     auto *o = (ResultOwner *)res->priv;
@@ -325,9 +402,11 @@ extern "C" void amj_result_release(amj_result *res) {
         if (o->ctx) (void)cudaSetDevice(o->ctx->device);
         for (int a = 0; a < AMJ_MAX_ATTRS; a++) {
             if (!res->cols[a]) continue;
+            if (res->on_host && o->host_block) continue;   // columns of the block below
             if (res->on_host) (void)cudaFreeHost(res->cols[a]);
             else if (o->ctx) dev_free(o->ctx, res->cols[a]);
         }
+        if (o->host_block) result_block_put(o->ctx, o->host_block, o->host_bytes);
         if (o->ctx && !res->on_host) (void)cudaStreamSynchronize(o->ctx->stream);
         delete o;
     }

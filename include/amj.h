@@ -225,6 +225,9 @@ int  amj_lftj_execute(amj_ctx *ctx, amj_rel *const *rels, int nrels,
 int  amj_lftj_execute_ordered(amj_ctx *ctx, amj_rel *const *rels, int nrels, int algo, int ooc, int ws,
                               int flags, const uint32_t *attr_order, int k, amj_result *out);
 
+/* copy the rows of a host result (AMJ_F_HOST_RESULT) into num_attrs arrays of
+ * res->rows values each, on the host cores */
+int  amj_result_copy_host(const amj_result *res, int32_t *const *dst);
 void amj_result_release(amj_result *res);
 
 /* ---- batched AMHJ: many queries, one build pass, one persistent probe launch ----

@@ -1277,3 +1277,25 @@ def test_clique4_matrix_order_by_ids(n, p):
             assert (m.count, m.checksum) == (got.count, got.checksum)
             assert np.all(a[:, :-1] < a[:, 1:]) and len(np.unique(a, axis=0)) == len(a) == got.count
             assert data.checksum(m.columns) == got.checksum
+
+
+@pytest.mark.parametrize("rows", [0, 1, 63, 64, 65537, 300_001])
+def test_host_results_reuse_blocks(rows):
+    """Materialised results of changing sizes through one context: the pinned
+    blocks come from the context's pool, and earlier results stay as they were."""
+    import gc
+    with Context(0) as ctx:
+        kept = []
+        for n in (rows, 1000, rows, 2 * rows + 1):
+            fact = [data.uniform(n, 0, 50, n + 1)]
+            dim = [data.permutation(50, 2), data.uniform(50, 0, 1 << 30, 3)]
+            r = ctx.amhj("NORMAL", [ctx.relation(fact, [0]), ctx.relation(dim, [0, 1])], materialize=True)
+            lookup = np.empty(50, np.int32)
+            lookup[dim[0]] = dim[1]
+            kept.append((r.columns, [fact[0], lookup[fact[0]]]))
+            assert r.count == n and data.checksum(r.columns) == r.checksum
+            gc.collect()
+        ctx.trim()
+    for got, want in kept:
+        assert all(np.array_equal(g, w) for g, w in zip(got, want))
+        assert all(g.flags.writeable and g.dtype == np.int32 for g in got)
