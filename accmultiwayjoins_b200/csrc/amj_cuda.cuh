@@ -266,5 +266,9 @@ enum SortKeyKind : int {
 // stable.  Ping-pongs between d_a and d_b; *result points at the sorted copy.
 int radix_sort_u64(amj_ctx *ctx, uint64_t *d_a, uint64_t *d_b, uint64_t n, int key_kind, int lo_bit,
                    int hi_bit, uint64_t **result);
+// The items (keys[i] << 32 | i) of n >= 1 keys, stably sorted by the low `bits`
+// (>= 1) bits of the key, into d_a or d_b (*result).
+int radix_sort_positions_u32(amj_ctx *ctx, const uint32_t *keys, uint64_t *d_a, uint64_t *d_b, uint64_t n, int bits,
+                             uint64_t **result);
 
 }  // namespace amj

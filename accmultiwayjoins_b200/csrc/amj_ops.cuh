@@ -77,10 +77,12 @@ constexpr uint64_t TRIE_LEVEL1_PAD = 4;
 // vmax >= 0: every value of both columns lies in [0, vmax] (no min/max pass)
 int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, Trie2 *out,
                 bool distinct = false, int32_t vmax = -1);
-// The distinct 2-level trie of a degree-ranked copy: every value in [0, nv)
-// and each row's first value below its second (rows bucketed by counting,
-// each row sorted on its own; the radix-sort build where a row is too long).
-int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, uint64_t nv, Trie2 *out);
+// The distinct 2-level trie of the degree-ranked copy of the edges (c0, c1):
+// every vertex renamed to its rank (below nv), edges from the lower to the
+// higher rank.  Rows bucketed by counting, each row sorted on its own; the
+// radix-sort build where a row is too long.  Level 0 holds every rank.
+int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, const int32_t *rank,
+                       uint64_t nv, Trie2 *out);
 
 // time between two events recorded on the context stream (ms)
 double event_ms(cudaEvent_t a, cudaEvent_t b);
@@ -90,11 +92,9 @@ double event_ms(cudaEvent_t a, cudaEvent_t b);
 int degree_ordered_copy(amj_ctx *ctx, const int32_t *c0, const int32_t *c1, uint64_t n, DBuf<int32_t> *ns,
                         DBuf<int32_t> *nd, bool *oriented);
 
-// The same copy with every vertex renamed to its rank in (degree, id) order:
-// edges (rank lo, rank hi), *inv[rank] = the vertex id, *nv ranks.
-int degree_ranked_copy(amj_ctx *ctx, const int32_t *c0, const int32_t *c1, uint64_t n, DBuf<int32_t> *ns,
-                       DBuf<int32_t> *nd, DBuf<int32_t> *inv, uint64_t *nv, bool *oriented);
-// The ranks alone: *rank[id] and *inv[rank] over ids 0..*nv-1 (when oriented).
+// Ranks of the vertices in order of their degrees (about: degree_bin in
+// graph_order.cu) when every edge has 0 <= c0 < c1 (*oriented): *rank[id] and
+// *inv[rank] over ids 0..*nv-1.
 int degree_ranks(amj_ctx *ctx, const int32_t *c0, const int32_t *c1, uint64_t n, DBuf<int32_t> *rank,
                  DBuf<int32_t> *inv, uint64_t *nv, bool *oriented);
 // The level-1 entries of a degree-ranked trie grouped by b (a stable sort).

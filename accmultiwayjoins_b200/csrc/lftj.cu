@@ -724,8 +724,7 @@ int lftj_tri_matrices(amj_ctx *ctx, const Trie2 &R, const uint64_t *wedge, const
         AMJ_CUDA_TRY(cudaGetLastError());
     }
     AMJ_TRY(scan_exclusive_u64(ctx, moff->p, moff->p, nv + 1, nullptr));
-    AMJ_CUDA_TRY(cudaMemcpyAsync(words, moff->p + nv, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    AMJ_TRY(read_back(ctx, words, moff->p + nv, sizeof(uint64_t)));
     if (*words > max_words) return fail(AMJ_ENOMEM, "LFTJ 4-clique: the triangle matrices do not fit");
     // the matrices live in one buffer the context keeps between calls (they
     // are the largest allocation of the query; allocating them anew every
@@ -781,12 +780,6 @@ int lftj_tri_matrices(amj_ctx *ctx, const Trie2 &R, const uint64_t *wedge, const
     return AMJ_OK;
 }
 
-// (b << 32 | entry) for every level-1 entry (a, b) of R
-__global__ void wedge_keys_kernel(const int32_t *__restrict__ data1, uint64_t n, uint64_t *__restrict__ keys) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        keys[i] = ((uint64_t)(uint32_t)data1[i] << 32) | i;
-}
-
 // The level-1 entries of a degree-ranked trie grouped by b: a stable sort
 // of (b << 32 | entry) on the rank bits of b.
 int build_wedges(amj_ctx *ctx, const Trie2 &R, uint64_t nv, DBuf<uint64_t> *out) {
@@ -796,14 +789,11 @@ int build_wedges(amj_ctx *ctx, const Trie2 &R, uint64_t nv, DBuf<uint64_t> *out)
     AMJ_TRY(out->alloc(ctx, n ? n : 1));
     if (n == 0) return AMJ_OK;
     AMJ_TRY(other.alloc(ctx, n));
-    note_launch(ctx);
-    wedge_keys_kernel<<<(unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)ctx->num_sms * 16), 256, 0,
-                        ctx->stream>>>(R.data1.p, n, out->p);
-    AMJ_CUDA_TRY(cudaGetLastError());
     int bits = 1;
     while (bits < 32 && (nv - 1) >> bits) bits++;
     uint64_t *sorted = nullptr;
-    AMJ_TRY(radix_sort_u64(ctx, out->p, other.p, n, SK_IDENT, 32, 32 + bits, &sorted));
+    AMJ_TRY(radix_sort_positions_u32(ctx, reinterpret_cast<const uint32_t *>(R.data1.p), out->p, other.p, n, bits,
+                                     &sorted));
     if (sorted != out->p) std::swap(*out, other);   // the sorted buffer becomes the result
     return AMJ_OK;
 }
@@ -1181,8 +1171,7 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
             AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)cand.p, (uint64_t *)cand.p, A.r_n,
                                        (uint64_t *)cand.p + A.r_n));
             unsigned long long total = 0;
-            AMJ_CUDA_TRY(cudaMemcpyAsync(&total, cand.p + A.r_n, sizeof(total), cudaMemcpyDeviceToHost, ctx->stream));
-            AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            AMJ_TRY(read_back(ctx, &total, cand.p + A.r_n, sizeof(total)));
             if (total) {
                 int per_sm = 0;
                 AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -1204,8 +1193,7 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
         }
     }
     LftjCounters h{};
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&h, ctr.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    AMJ_TRY(read_back(ctx, &h, ctr.p, sizeof(h)));
     *count = h.count;
     *checksum = h.checksum;
     if (written) *written = write ? (h.out_cursor < out_cap ? h.out_cursor : out_cap) : 0;

@@ -64,11 +64,11 @@ static int build_ranked_trie(amj_ctx *ctx, const amj_rel *r, Trie2 *t, DBuf<int3
     if (r->where == AMJ_MEM_HOST_STREAMED) return fail(AMJ_EUNSUPPORTED, "LFTJ: relations must be on the device");
     const bool swap = r->attrs[0] > r->attrs[1];
     const int32_t *c0 = r->d_cols[swap ? 1 : 0], *c1 = r->d_cols[swap ? 0 : 1];
-    DBuf<int32_t> ns, nd;
+    DBuf<int32_t> rank;
     bool oriented = false;
-    AMJ_TRY(degree_ranked_copy(ctx, c0, c1, r->n, &ns, &nd, inv, nv, &oriented));
+    AMJ_TRY(degree_ranks(ctx, c0, c1, r->n, &rank, inv, nv, &oriented));
     if (!oriented) return build_trie2(ctx, c0, c1, r->n, t, true);
-    AMJ_TRY(build_trie2_ranked(ctx, ns.p, nd.p, r->n, *nv, t));
+    AMJ_TRY(build_trie2_ranked(ctx, c0, c1, r->n, rank.p, *nv, t));
     if (wedges) AMJ_TRY(build_wedges(ctx, *t, *nv, wedges));
     return AMJ_OK;
 }

@@ -545,8 +545,7 @@ static int trie_max_children(amj_ctx *ctx, const Trie2 &T, uint64_t *maxc) {
                           ctx->stream>>>(T.off0.p, T.len0, m.p);
     AMJ_CUDA_TRY(cudaGetLastError());
     unsigned long long h = 0;
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&h, m.p, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    AMJ_TRY(read_back(ctx, &h, m.p, sizeof(h)));
     *maxc = h;
     return AMJ_OK;
 }
@@ -640,8 +639,7 @@ int lftj_clique4_matrix(amj_ctx *ctx, const Trie2 &T, const int32_t *inv, const 
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[1], ctx->stream));
     C4Counters h;
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&h, ctr.p, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    AMJ_TRY(read_back(ctx, &h, ctr.p, sizeof(h)));
     if (kernel_ms) *kernel_ms += event_ms(ctx->kev[0], ctx->kev[1]);
     *count = h.count;
     *checksum = h.checksum;

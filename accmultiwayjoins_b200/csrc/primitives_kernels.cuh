@@ -143,7 +143,16 @@ __device__ __forceinline__ uint64_t sort_key(uint64_t it) {
     return hash_pair((int32_t)(uint32_t)it, (int32_t)(uint32_t)(it >> 32));
 }
 
-template <int KK>
+// item idx of the input; IN32: the input is an array of 32-bit keys and the item
+// (key << 32 | idx), so that the first pass of a sort of keys with their
+// positions reads the keys and not items written out before
+template <bool IN32>
+__device__ __forceinline__ uint64_t rs_item(const uint64_t *__restrict__ in, uint64_t idx) {
+    if (IN32) return (uint64_t)reinterpret_cast<const uint32_t *>(in)[idx] << 32 | idx;
+    return in[idx];
+}
+
+template <int KK, bool IN32 = false>
 __global__ __launch_bounds__(RS_THREADS) void rs_upsweep_kernel(const uint64_t *__restrict__ in, uint32_t n,
                                                                  int shift, int bits,
                                                                  uint32_t *__restrict__ counts,
@@ -158,7 +167,7 @@ __global__ __launch_bounds__(RS_THREADS) void rs_upsweep_kernel(const uint64_t *
     for (int r = 0; r < RS_IPT; r++) {
         uint64_t idx = base + (uint64_t)r * 32 + lane;
         if (idx < n) {
-            uint32_t d = (uint32_t)(sort_key<KK>(in[idx]) >> shift) & dmask;
+            uint32_t d = (uint32_t)(sort_key<KK>(rs_item<IN32>(in, idx)) >> shift) & dmask;
             atomicAdd(&h[warp][d], 1u);
         }
     }
@@ -171,7 +180,7 @@ __global__ __launch_bounds__(RS_THREADS) void rs_upsweep_kernel(const uint64_t *
     }
 }
 
-template <int KK>
+template <int KK, bool IN32 = false>
 __global__ __launch_bounds__(RS_THREADS, 3) void rs_downsweep_kernel(const uint64_t *__restrict__ in,
                                                                    uint64_t *__restrict__ out, uint32_t n,
                                                                    int shift, int bits,
@@ -196,7 +205,7 @@ __global__ __launch_bounds__(RS_THREADS, 3) void rs_downsweep_kernel(const uint6
 #pragma unroll
     for (int r = 0; r < RS_IPT; r++) {
         const uint64_t idx = base + (uint64_t)r * 32 + lane;
-        it[r] = idx < n ? in[idx] : 0ull;
+        it[r] = idx < n ? rs_item<IN32>(in, idx) : 0ull;
     }
 #pragma unroll
     for (int r = 0; r < RS_IPT; r++) {

@@ -224,9 +224,14 @@ int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t
 
 // ---- 2-level tries of a degree-ranked copy: rows by counting ----
 // Every value lies in [0, nv) and every row's first value is below its
-// second, so the rows can be bucketed by their first value directly: a count
-// per value, a scan into row starts, and one scatter of the second values
-// into their rows, then each row sorted on its own.  After the degree
+// second, so the rows can be bucketed by their first value directly: one pass
+// ranks the edges, counts them per value and keeps each edge's place in its
+// row, a scan gives the row starts, one pass writes the second values to start
+// + place, then each row is sorted on its own.  Level 0 lists every rank, so
+// nothing is compacted and one host read (repeated rows, longest row) ends the
+// build: 26 device operations and 3 host reads a triangle query of 64K edges
+// instead of 49 and 6 (435 to 276 us), 1.42 instead of 1.80 ms of builds on C2.
+// After the degree
 // ranking a row holds the higher-ranked neighbours of one vertex, at most
 // sqrt(2 n) of them, and most rows hold a few: a warp sorts a row of up to
 // 32 values in registers (a bitonic network over shuffles) and up to
@@ -238,28 +243,61 @@ constexpr uint32_t RK_WARP_MAX = 1024;
 constexpr uint32_t RK_BLOCK_MAX = 8192;
 constexpr int RK_SORT_WARPS = 8;
 
-__global__ void rk_count_kernel(const int32_t *__restrict__ c0, uint64_t n, uint32_t *__restrict__ cnt) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        atomicAdd(&cnt[c0[i]], 1u);
-}
-
-__global__ void rk_max_kernel(const uint32_t *__restrict__ cnt, uint64_t nv, unsigned int *__restrict__ mx) {
-    uint32_t m = 0;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x)
-        m = max(m, cnt[v]);
+// Ranked edges (the lower rank first), the count of every lower rank, each
+// edge's place among those of its lower rank (the value its atomic returned),
+// and the longest row.  Four edges a thread, so that the dependent lookups of
+// one overlap those of the others.
+__global__ __launch_bounds__(256) void rk_edges_kernel(const int32_t *__restrict__ s, const int32_t *__restrict__ d,
+                                                       uint64_t n, const int32_t *__restrict__ rank,
+                                                       uint32_t *__restrict__ cnt, int32_t *__restrict__ lo,
+                                                       int32_t *__restrict__ hi, uint32_t *__restrict__ place,
+                                                       unsigned int *__restrict__ longest) {
+    const uint64_t i0 = blockIdx.x * 1024ull + threadIdx.x;
+    int32_t u[4], v[4];
+    uint32_t p[4], m = 0;
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(AMJ_FULL_MASK, m, d));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(mx, m);
+    for (int k = 0; k < 4; k++) {
+        const uint64_t i = i0 + k * 256;
+        if (i < n) {
+            u[k] = rank[s[i]];
+            v[k] = rank[d[i]];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (i0 + k * 256 < n) p[k] = atomicAdd(&cnt[min(u[k], v[k])], 1u);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint64_t i = i0 + k * 256;
+        if (i < n) {
+            lo[i] = min(u[k], v[k]);
+            hi[i] = max(u[k], v[k]);
+            place[i] = p[k];
+            m = max(m, p[k] + 1);
+        }
+    }
+    m = __reduce_max_sync(AMJ_FULL_MASK, m);
+    if ((threadIdx.x & 31) == 0 && m > ld_volatile_u32(longest)) atomicMax(longest, m);
 }
 
-// fill[] starts at zero: the row of value c0[i] gets c1[i] at its next free slot
-__global__ void rk_scatter_kernel(const int32_t *__restrict__ c0, const int32_t *__restrict__ c1, uint64_t n,
-                                  const uint32_t *__restrict__ start, uint32_t *__restrict__ fill,
-                                  int32_t *__restrict__ data1) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const int32_t v = c0[i];
-        data1[start[v] + atomicAdd(&fill[v], 1u)] = c1[i];
+__global__ __launch_bounds__(256) void rk_scatter_kernel(const int32_t *__restrict__ lo, const int32_t *__restrict__ hi,
+                                                         const uint32_t *__restrict__ place, uint64_t n,
+                                                         const uint32_t *__restrict__ start,
+                                                         int32_t *__restrict__ data1) {
+    const uint64_t i0 = blockIdx.x * 1024ull + threadIdx.x;
+    uint32_t p[4];
+    int32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const uint64_t i = i0 + k * 256;
+        if (i < n) {
+            p[k] = start[lo[i]] + place[i];
+            v[k] = hi[i];
+        }
     }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (i0 + k * 256 < n) data1[p[k]] = v[k];
 }
 
 // ascending bitonic sort of the pow2-sized x[0, m) by the threads t of a
@@ -292,7 +330,7 @@ __device__ __forceinline__ uint32_t rk_distinct(const int32_t *x, uint32_t len, 
 // row v = data1[s, s + len), 32 (E / 2) < len <= 32 E: sorted in place, its
 // level-0 value into src1, its number of distinct values into uniq[v]
 template <int E>
-__device__ __forceinline__ void rk_warp_row(int32_t *__restrict__ data1, int32_t *__restrict__ src1,
+__device__ __forceinline__ uint32_t rk_warp_row(int32_t *__restrict__ data1, int32_t *__restrict__ src1,
                                             uint32_t *__restrict__ uniq, uint32_t s, uint32_t len, uint64_t v,
                                             uint32_t lane) {
     int32_t x[E];
@@ -317,6 +355,7 @@ __device__ __forceinline__ void rk_warp_row(int32_t *__restrict__ data1, int32_t
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) u += __shfl_xor_sync(AMJ_FULL_MASK, u, d);
     if (lane == 0) uniq[v] = u;
+    return u;
 }
 
 // One warp a row, the row's values in registers (rows of up to RK_WARP_MAX);
@@ -326,7 +365,12 @@ __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(con
                                                                            int32_t *__restrict__ src1,
                                                                            uint32_t *__restrict__ uniq,
                                                                            uint32_t *__restrict__ longs,
-                                                                           unsigned int *__restrict__ nlong) {
+                                                                           unsigned int *__restrict__ nlong,
+                                                                           unsigned long long *__restrict__ distinct) {
+    __shared__ uint32_t usum;
+    if (threadIdx.x == 0) usum = 0;
+    __syncthreads();
+    uint32_t u = 0;   // distinct values of this warp's rows
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t warps = (uint64_t)gridDim.x * RK_SORT_WARPS;
     for (uint64_t v = blockIdx.x * (uint64_t)RK_SORT_WARPS + w; v < nv; v += warps) {
@@ -334,23 +378,27 @@ __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(con
         if (len <= 1) {
             if (len == 1 && lane == 0) src1[s] = (int32_t)v;
             if (lane == 0) uniq[v] = len;
+            u += len;
         } else if (len <= 32) {
-            rk_warp_row<1>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<1>(data1, src1, uniq, s, len, v, lane);
         } else if (len <= 64) {
-            rk_warp_row<2>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<2>(data1, src1, uniq, s, len, v, lane);
         } else if (len <= 128) {
-            rk_warp_row<4>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<4>(data1, src1, uniq, s, len, v, lane);
         } else if (len <= 256) {
-            rk_warp_row<8>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<8>(data1, src1, uniq, s, len, v, lane);
         } else if (len <= 512) {
-            rk_warp_row<16>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<16>(data1, src1, uniq, s, len, v, lane);
         } else if (len <= RK_WARP_MAX) {
-            rk_warp_row<32>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<32>(data1, src1, uniq, s, len, v, lane);
         } else if (lane == 0) {
             longs[atomicAdd(nlong, 1u)] = (uint32_t)v;
             uniq[v] = 0;
         }
     }
+    if (lane == 0) atomicAdd(&usum, u);
+    __syncthreads();
+    if (threadIdx.x == 0 && usum) atomicAdd(distinct, (unsigned long long)usum);
 }
 
 // One block a listed row (RK_WARP_MAX < length <= RK_BLOCK_MAX); the blocks
@@ -359,12 +407,14 @@ __global__ __launch_bounds__(512) void rk_sort_long_kernel(const uint32_t *__res
                                                            int32_t *__restrict__ data1, int32_t *__restrict__ src1,
                                                            uint32_t *__restrict__ uniq,
                                                            const uint32_t *__restrict__ longs,
-                                                           const unsigned int *__restrict__ nlong) {
+                                                           const unsigned int *__restrict__ nlong,
+                                                           unsigned long long *__restrict__ distinct) {
     __shared__ int32_t x[RK_BLOCK_MAX];
     __shared__ uint32_t usum;
     const uint32_t t = threadIdx.x, nt = blockDim.x;
     for (uint32_t r = blockIdx.x; r < *nlong; r += gridDim.x) {
         const uint32_t v = longs[r], s = start[v], len = start[v + 1] - s;
+        if (len > RK_BLOCK_MAX) continue;   // the host takes the radix build
         uint32_t m = 64;
         while (m < len) m <<= 1;
         if (t == 0) usum = 0;
@@ -378,7 +428,10 @@ __global__ __launch_bounds__(512) void rk_sort_long_kernel(const uint32_t *__res
             src1[s + i] = (int32_t)v;
         }
         __syncthreads();
-        if (t == 0) uniq[v] = usum;
+        if (t == 0) {
+            uniq[v] = usum;
+            atomicAdd(distinct, (unsigned long long)usum);
+        }
         __syncthreads();
     }
 }
@@ -406,107 +459,97 @@ __global__ void rk_compact_kernel(const uint32_t *__restrict__ start, const uint
     }
 }
 
-// level 0 (the values with children) and the dense row pointers
-__global__ void rk_level0_kernel(const uint32_t *__restrict__ ustart, const uint32_t *__restrict__ pos, uint64_t nv,
-                                 int32_t *__restrict__ data0, uint64_t *__restrict__ off0,
-                                 uint64_t *__restrict__ rowptr, uint64_t len0) {
+// level 0 (every rank) and the row pointers
+__global__ void rk_level0_kernel(const uint32_t *__restrict__ start, uint64_t nv, int32_t *__restrict__ data0,
+                                 uint64_t *__restrict__ rowptr) {
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v <= nv; v += (uint64_t)gridDim.x * blockDim.x) {
-        rowptr[v] = ustart[v];
-        if (v == nv) {
-            off0[len0] = ustart[nv];
-        } else if (ustart[v + 1] > ustart[v]) {
-            data0[pos[v]] = (int32_t)v;
-            off0[pos[v]] = ustart[v];
-        }
+        rowptr[v] = start[v];
+        if (v < nv) data0[v] = (int32_t)v;
     }
 }
 
-// 1 for the values with a row (every row keeps a value after deduplication)
-__global__ void rk_nonempty_kernel(const uint32_t *__restrict__ start, uint64_t nv, uint32_t *__restrict__ flag) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < nv; v += (uint64_t)gridDim.x * blockDim.x)
-        flag[v] = start[v + 1] > start[v] ? 1u : 0u;
-}
-
-int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, uint64_t nv, Trie2 *out) {
-    if (n == 0 || nv == 0 || nv >= (1ull << 31) || n >= (1ull << 32) - 4096)
-        return build_trie2(ctx, d_c0, d_c1, n, out, true, nv ? (int32_t)(nv - 1) : -1);
-    // per-value row lengths, the longest, the row starts, and the values with
-    // children (level 0) numbered by a scan of their flags
-    DBuf<uint32_t> start, fill, flag;
-    DBuf<unsigned int> ctr;   // [0] longest row, [1] rows listed for the block kernel
-    AMJ_TRY(start.alloc(ctx, nv + 1));
-    AMJ_TRY(fill.alloc(ctx, nv));
-    AMJ_TRY(flag.alloc(ctx, nv + 1));
-    AMJ_TRY(ctr.alloc(ctx, 2));
-    AMJ_CUDA_TRY(cudaMemsetAsync(start.p, 0, (nv + 1) * sizeof(uint32_t), ctx->stream));
-    AMJ_CUDA_TRY(cudaMemsetAsync(ctr.p, 0, 2 * sizeof(unsigned int), ctx->stream));
+int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, const int32_t *rank,
+                       uint64_t nv, Trie2 *out) {
+    if (n == 0 || nv == 0) return build_trie2(ctx, d_c0, d_c1, n, out, true, -1);
+    // ranked edges with their places in their rows; a scan of the counts
+    DBuf<int32_t> lo, hi;
+    DBuf<uint32_t> start, place;
+    struct Ctr {
+        unsigned int longest, nlong;   // longest row; rows listed for the block kernel
+        unsigned long long distinct;
+    };
+    AMJ_TRY(lo.alloc(ctx, n));
+    AMJ_TRY(hi.alloc(ctx, n));
+    AMJ_TRY(place.alloc(ctx, n));
+    // row starts, then the counters (8-byte aligned)
+    const uint64_t ctr_at = (nv + 2) / 2 * 2;
+    AMJ_TRY(start.alloc(ctx, ctr_at + sizeof(Ctr) / sizeof(uint32_t)));
+    Ctr *ctr = reinterpret_cast<Ctr *>(start.p + ctr_at);
+    AMJ_CUDA_TRY(cudaMemsetAsync(start.p, 0, ctr_at * sizeof(uint32_t) + sizeof(Ctr), ctx->stream));
+    const uint64_t tiles = (n + 1023) / 1024;
     note_launch(ctx);
-    rk_count_kernel<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(d_c0, n, start.p);
+    rk_edges_kernel<<<(unsigned)tiles, 256, 0, ctx->stream>>>(d_c0, d_c1, n, rank, start.p, lo.p, hi.p, place.p,
+                                                              &ctr->longest);
     AMJ_CUDA_TRY(cudaGetLastError());
-    note_launch(ctx);
-    rk_max_kernel<<<grid_for(ctx, nv), 256, 0, ctx->stream>>>(start.p, nv, ctr.p);
-    AMJ_CUDA_TRY(cudaGetLastError());
+    if (nv >= (1ull << 31) || n >= (1ull << 32) - 4096)
+        return build_trie2(ctx, lo.p, hi.p, n, out, true, (int32_t)(nv - 1));
     AMJ_TRY(scan_exclusive_u32(ctx, start.p, start.p, nv + 1, nullptr));
-    note_launch(ctx);
-    rk_nonempty_kernel<<<grid_for(ctx, nv), 256, 0, ctx->stream>>>(start.p, nv, flag.p);
-    AMJ_CUDA_TRY(cudaGetLastError());
-    AMJ_TRY(scan_exclusive_u32(ctx, flag.p, flag.p, nv, flag.p + nv));
-    uint32_t h[2] = {0, 0};   // longest row, values with children
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&h[0], ctr.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&h[1], flag.p + nv, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    const uint32_t longest = h[0], len0 = h[1];
-    if (longest > RK_BLOCK_MAX) return build_trie2(ctx, d_c0, d_c1, n, out, true, (int32_t)(nv - 1));
     // the rows, each sorted, with their distinct counts
     AMJ_TRY(out->data1.alloc(ctx, n + TRIE_LEVEL1_PAD));
     AMJ_TRY(out->src1.alloc(ctx, n));
     DBuf<uint32_t> uniq, longs;
     AMJ_TRY(uniq.alloc(ctx, nv + 1));
     AMJ_TRY(longs.alloc(ctx, std::max<uint64_t>(1, n / (RK_WARP_MAX + 1) + 1)));
-    AMJ_CUDA_TRY(cudaMemsetAsync(fill.p, 0, nv * sizeof(uint32_t), ctx->stream));
     note_launch(ctx);
-    rk_scatter_kernel<<<grid_for(ctx, n), 256, 0, ctx->stream>>>(d_c0, d_c1, n, start.p, fill.p, out->data1.p);
+    rk_scatter_kernel<<<(unsigned)tiles, 256, 0, ctx->stream>>>(lo.p, hi.p, place.p, n, start.p, out->data1.p);
     AMJ_CUDA_TRY(cudaGetLastError());
     const unsigned gs = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((nv + RK_SORT_WARPS - 1) / RK_SORT_WARPS,
                                                                            (uint64_t)ctx->num_sms * 8));
     note_launch(ctx);
     rk_sort_rows_kernel<<<gs, RK_SORT_WARPS * 32, 0, ctx->stream>>>(start.p, nv, out->data1.p, out->src1.p, uniq.p,
-                                                                    longs.p, ctr.p + 1);
+                                                                    longs.p, &ctr->nlong, &ctr->distinct);
     AMJ_CUDA_TRY(cudaGetLastError());
-    if (longest > RK_WARP_MAX) {
+    // no row of n edges in rank order is longer than sqrt(2 n) unless edges repeat
+    if (n > RK_WARP_MAX) {
         note_launch(ctx);
         rk_sort_long_kernel<<<ctx->num_sms, 512, 0, ctx->stream>>>(start.p, out->data1.p, out->src1.p, uniq.p,
-                                                                   longs.p, ctr.p + 1);
+                                                                   longs.p, &ctr->nlong, &ctr->distinct);
         AMJ_CUDA_TRY(cudaGetLastError());
     }
-    // distinct rows: scan the distinct counts; a compaction when some differ
-    uint32_t h_total = 0;
-    AMJ_TRY(scan_exclusive_u32(ctx, uniq.p, uniq.p, nv + 1, nullptr));
-    AMJ_CUDA_TRY(cudaMemcpyAsync(&h_total, uniq.p + nv, sizeof(h_total), cudaMemcpyDeviceToHost, ctx->stream));
-    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    if (h_total != n) {
-        DBuf<int32_t> d1, s1;
-        AMJ_TRY(d1.alloc(ctx, (uint64_t)h_total + TRIE_LEVEL1_PAD));
-        AMJ_TRY(s1.alloc(ctx, h_total ? h_total : 1));
-        note_launch(ctx);
-        rk_compact_kernel<<<grid_for(ctx, nv * 32), 256, 0, ctx->stream>>>(start.p, uniq.p, nv, out->data1.p, d1.p,
-                                                                            s1.p);
-        AMJ_CUDA_TRY(cudaGetLastError());
-        out->data1 = std::move(d1);
-        out->src1 = std::move(s1);
-    }
-    out->len1 = h_total;
-    // level 0 and the dense row pointers (a row with values keeps at least one)
-    out->len0 = len0;
-    AMJ_TRY(out->data0.alloc(ctx, len0 ? len0 : 1));
-    AMJ_TRY(out->off0.alloc(ctx, (uint64_t)len0 + 1));
-    AMJ_TRY(out->rowptr.alloc(ctx, nv + 1));
+    // level 0 and the row pointers, unless rows repeat or are too long
+    out->len0 = nv;
     out->rp_min = 0;
     out->rp_count = nv;
+    AMJ_TRY(out->data0.alloc(ctx, nv));
+    AMJ_TRY(out->rowptr.alloc(ctx, nv + 1));
+    out->off0.release();
+    out->off0.ctx = nullptr;   // a view: the row pointers of every rank
+    out->off0.p = out->rowptr.p;
+    out->off0.n = nv + 1;
     note_launch(ctx);
-    rk_level0_kernel<<<grid_for(ctx, nv + 1), 256, 0, ctx->stream>>>(uniq.p, flag.p, nv, out->data0.p, out->off0.p,
-                                                                     out->rowptr.p, len0);
+    rk_level0_kernel<<<grid_for(ctx, nv + 1), 256, 0, ctx->stream>>>(start.p, nv, out->data0.p, out->rowptr.p);
     AMJ_CUDA_TRY(cudaGetLastError());
+    Ctr h{};
+    AMJ_TRY(read_back(ctx, &h, ctr, sizeof(h)));
+    if (h.longest > RK_BLOCK_MAX) {
+        *out = Trie2();
+        return build_trie2(ctx, lo.p, hi.p, n, out, true, (int32_t)(nv - 1));
+    }
+    out->len1 = h.distinct;
+    if (h.distinct == n) return AMJ_OK;
+    // repeated rows: the distinct values of every row, compacted
+    AMJ_CUDA_TRY(cudaMemsetAsync(uniq.p + nv, 0, sizeof(uint32_t), ctx->stream));
+    AMJ_TRY(scan_exclusive_u32(ctx, uniq.p, uniq.p, nv + 1, nullptr));
+    DBuf<int32_t> d1, s1;
+    AMJ_TRY(d1.alloc(ctx, h.distinct + TRIE_LEVEL1_PAD));
+    AMJ_TRY(s1.alloc(ctx, h.distinct ? h.distinct : 1));
+    note_launch(ctx);
+    rk_compact_kernel<<<grid_for(ctx, nv * 32), 256, 0, ctx->stream>>>(start.p, uniq.p, nv, out->data1.p, d1.p, s1.p);
+    note_launch(ctx);
+    rk_level0_kernel<<<grid_for(ctx, nv + 1), 256, 0, ctx->stream>>>(uniq.p, nv, out->data0.p, out->rowptr.p);
+    AMJ_CUDA_TRY(cudaGetLastError());
+    out->data1 = std::move(d1);
+    out->src1 = std::move(s1);
     return AMJ_OK;
 }
 

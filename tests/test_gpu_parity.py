@@ -1299,3 +1299,28 @@ def test_host_results_reuse_blocks(rows):
     for got, want in kept:
         assert all(np.array_equal(g, w) for g, w in zip(got, want))
         assert all(g.flags.writeable and g.dtype == np.int32 for g in got)
+
+
+@pytest.mark.parametrize("degree", [0, 1, 1022, 1023, 1024, 1055, 1056, 5000])
+def test_degree_rank_bins(ctx, degree):
+    """Hubs whose degrees fall in and around the first linear and logarithmic
+    degree bins, tied and not, repeated rows among the edges."""
+    hubs = 6
+    leaves = 40 + degree
+    rng = np.random.default_rng(degree)
+    s, d = [], []
+    for h in range(hubs):
+        pick = rng.permutation(leaves)[:degree + (h % 3) - 1 if degree else 0]
+        s.append(np.full(len(pick), h))
+        d.append(hubs + pick)
+    u, v = np.triu_indices(hubs, 1)
+    s, d = np.concatenate(s + [u]).astype(np.int32), np.concatenate(d + [v]).astype(np.int32)
+    x, y = data.rmat(10, 6000, 0.57, 0.19, 0.19, 3)
+    x, y = x + hubs, y + hubs
+    s, d = np.concatenate([s, x, x[:50]]), np.concatenate([d, y, y[:50]])
+    e = ctx.relation([s, d], [0, 1])
+    us = np.unique(np.stack([s, d], 1), axis=0)
+    want = O.triangle(us[:, 0].copy(), us[:, 1].copy())
+    for algo in ("DFS", "BFS"):
+        r = ctx.lftj([e], algo=algo)
+        assert (r.count, r.checksum) == want
