@@ -73,7 +73,10 @@ struct TriArgs {
     unsigned long long *cursor_r; // claim cursor of the wedge kernel
     int bfs_wedge;                // BFS over one degree-ordered relation (R = S = T): the
                                   // candidates of entry (a, b) are T(a)'s values after b
-    const struct RankId *hid;     // wedge kernel: id and first hash step of every rank
+    const struct RankId *hid;     // wedge kernel, BFS wedges: id and first hash step of every rank
+    const uint32_t *hub_mtx;      // BFS wedges: row b - hub_base has bit c - hub_base for every edge (b, c)
+    int32_t hub_base;             // of the ranks from hub_base on; null: no matrix
+    uint32_t hub_words;           // words a row
 };
 
 // The vertex id of a rank and the first step of the tuple hash over it,
@@ -929,10 +932,32 @@ __global__ void lftj_tri_bfs_count_kernel(const __grid_constant__ TriArgs A, uns
     }
 }
 
+// ---- hub matrix of the breadth-first wedges ----
+// A candidate c of the edge (a, b) is looked up among b's children.  Ranks put
+// the hubs last and c > b, so for nearly every candidate both are hubs: the
+// edges among the top HUB_RANKS ranks are kept as a bit matrix (32 MB, which
+// L2 holds), and the lookup is one load instead of a binary search of six to
+// nine dependent ones.  Lower b are searched as before.  The matrix is built
+// from BFS_HUB_MIN candidates on: clearing and filling it takes up to 20 us.
+// R-MAT, 2M edges (HUB_FIGURES).
+constexpr uint64_t HUB_RANKS = 16384;
+constexpr uint64_t BFS_HUB_MIN = 1ull << 20;
+
+__global__ void hub_matrix_kernel(const int32_t *__restrict__ src, const int32_t *__restrict__ dst, uint64_t n,
+                                  int32_t base, uint32_t words, uint32_t *__restrict__ mtx) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const int32_t b = src[i];
+        if (b < base) continue;   // dst > src in rank order
+        const uint32_t c = (uint32_t)(dst[i] - base);
+        atomicOr(&mtx[(uint64_t)(uint32_t)(b - base) * words + (c >> 5)], 1u << (c & 31));
+    }
+}
+
 constexpr int BFS_TILE = 2048;
 constexpr int BFS_THREADS = 256;
 constexpr int BFS_SMEM_ENTRIES = 2048;
 constexpr int BFS_RUN = BFS_TILE / BFS_THREADS;   // consecutive candidates per thread
+static_assert(BFS_RUN < 32, "a run's hits are one mask");
 
 __device__ __forceinline__ uint64_t upper_bound_u64(const unsigned long long *a, uint64_t lo, uint64_t hi,
                                                     unsigned long long v) {
@@ -944,24 +969,31 @@ __device__ __forceinline__ uint64_t upper_bound_u64(const unsigned long long *a,
     return lo;
 }
 
+// first[t] = the entry that owns the first candidate of tile t.  One pass over
+// the entries; searched by one thread of every tile (two binary searches over
+// all entries) the tiles waited for it most of their time.
+__global__ void bfs_tile_first_kernel(const unsigned long long *__restrict__ offs, uint64_t n,
+                                      uint32_t *__restrict__ first) {
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < n; e += (uint64_t)gridDim.x * blockDim.x) {
+        const unsigned long long lo = offs[e], hi = offs[e + 1];
+        for (unsigned long long t = (lo + BFS_TILE - 1) / BFS_TILE; t * BFS_TILE < hi; t++) first[t] = (uint32_t)e;
+    }
+}
+
 template <bool WRITE>
 __global__ __launch_bounds__(BFS_THREADS) void lftj_tri_bfs_expand_kernel(const __grid_constant__ TriArgs A,
                                                                           const unsigned long long *__restrict__ offs,
+                                                                          const uint32_t *__restrict__ tile_first,
                                                                           unsigned long long total) {
     __shared__ unsigned long long s_off[BFS_SMEM_ENTRIES + 1];
-    __shared__ uint64_t s_e0, s_e1;
     unsigned long long cnt = 0, chk = 0;
     const int lane = threadIdx.x & 31;
     for (unsigned long long tile = blockIdx.x * (unsigned long long)BFS_TILE; tile < total;
          tile += (unsigned long long)gridDim.x * BFS_TILE) {
         const unsigned long long tend = (tile + BFS_TILE < total) ? tile + BFS_TILE : total;
-        if (threadIdx.x == 0) {
-            // entries owning candidates tile .. tend-1: offs[e] <= t < offs[e+1]
-            s_e0 = upper_bound_u64(offs, 0, A.r_n, tile) - 1;
-            s_e1 = upper_bound_u64(offs, 0, A.r_n, tend - 1) - 1;
-        }
-        __syncthreads();
-        const uint64_t e0 = s_e0, e1 = s_e1;
+        // entries owning candidates tile .. tend-1, or one past them
+        const uint64_t e0 = tile_first[tile / BFS_TILE];
+        const uint64_t e1 = tend < total ? tile_first[tile / BFS_TILE + 1] : A.r_n - 1;
         const uint64_t ne = e1 - e0 + 1;
         const bool in_smem = ne <= BFS_SMEM_ENTRIES;
         if (in_smem)
@@ -976,8 +1008,9 @@ __global__ __launch_bounds__(BFS_THREADS) void lftj_tri_bfs_expand_kernel(const 
         int32_t a = 0, b = 0, xa = 0, xb = 0;
         uint64_t hab = 0;
         bool s_short = false;
-        for (unsigned long long t = t0; t < t1; t++) {
-            if (e == ~0ull || t >= nxt) {
+        const uint32_t *hub_row = nullptr;   // b's row of the hub matrix
+        for (unsigned long long t = t0; t < t1;) {
+            {
                 if (e == ~0ull) {
                     if (in_smem) {
                         uint64_t lo = 0, hi = ne;
@@ -1003,25 +1036,65 @@ __global__ __launch_bounds__(BFS_THREADS) void lftj_tri_bfs_expand_kernel(const 
                 // expand the shorter list, search the longer (wedge form:
                 // expand T(a) after b, search S(b))
                 s_short = !A.bfs_wedge && (eb - sb) <= (ea - ta);
-                xa = A.inv ? A.inv[a] : a;
-                xb = A.inv ? A.inv[b] : b;
-                hab = amj_hash_step(amj_hash_step(AMJ_CHECKSUM_SEED, xa), xb);
+                if (A.inv) {
+                    // ids in increasing order, and the prefix of the smaller
+                    const RankId ra = A.hid[a], rb = A.hid[b];
+                    const bool alo = ra.id < rb.id;
+                    xa = alo ? ra.id : rb.id;
+                    xb = alo ? rb.id : ra.id;
+                    hab = alo ? ra.h1 : rb.h1;
+                    hub_row = A.hub_mtx && b >= A.hub_base
+                                  ? A.hub_mtx + (uint64_t)(uint32_t)(b - A.hub_base) * A.hub_words
+                                  : nullptr;
+                } else {
+                    xa = a;
+                    xb = b;
+                    hab = amj_hash_step(amj_hash_step(AMJ_CHECKSUM_SEED, xa), xb);
+                }
             }
-            const unsigned long long k = t - cur;
-            const int32_t c = s_short ? A.S.data1[sb + k]
-                                      : A.T.data1[(A.bfs_wedge ? A.r_lo + e + 1 : ta) + k];
-            const int32_t *hay = s_short ? A.T.data1 : A.S.data1;
-            uint64_t lo = s_short ? ta : sb, hi = s_short ? ea : eb;
-            while (lo < hi) {
-                uint64_t mid = (lo + hi) >> 1;
-                if (hay[mid] < c) lo = mid + 1;
-                else hi = mid;
+            // this edge's part of the run: membership of its candidates first
+            // (all loads in flight together), then the hits
+            const uint32_t len = (uint32_t)((nxt < t1 ? nxt : t1) - t);
+            const int32_t *cand = (s_short ? A.S.data1 + sb : A.T.data1 + (A.bfs_wedge ? A.r_lo + e + 1 : ta)) + (t - cur);
+            t += len;
+            uint32_t hits = 0;
+            if (hub_row) {
+                uint32_t x[BFS_RUN], w[BFS_RUN];
+#pragma unroll
+                for (int k = 0; k < BFS_RUN; k++) x[k] = (uint32_t)k < len ? (uint32_t)(cand[k] - A.hub_base) : 0u;
+#pragma unroll
+                for (int k = 0; k < BFS_RUN; k++) w[k] = hub_row[x[k] >> 5];
+#pragma unroll
+                for (int k = 0; k < BFS_RUN; k++) hits |= ((w[k] >> (x[k] & 31)) & 1u) << k;
+                hits &= (1u << len) - 1u;
+            } else {
+                const int32_t *hay = s_short ? A.T.data1 : A.S.data1;
+                for (uint32_t k = 0; k < len; k++) {
+                    const int32_t c = cand[k];
+                    uint64_t lo = s_short ? ta : sb, hi = s_short ? ea : eb;
+                    while (lo < hi) {
+                        uint64_t mid = (lo + hi) >> 1;
+                        if (hay[mid] < c) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    if (lo < (s_short ? ea : eb) && hay[lo] == c) hits |= 1u << k;
+                }
             }
-            const bool found = lo < (s_short ? ea : eb) && hay[lo] == c;
-            if (found) {
-                const int32_t xc = A.inv ? A.inv[c] : c;
-                cnt++;
-                chk += tri_chk(A, hab, xa, xb, xc);
+            cnt += __popc(hits);
+            while (hits) {
+                const int32_t c = cand[__ffs(hits) - 1];
+                hits &= hits - 1;
+                int32_t xc = c;
+                if (A.inv) {
+                    // the triangle (xc, xa, xb) in increasing order, hashed
+                    // from the prefix of its smallest id
+                    const RankId r = A.hid[c];
+                    xc = r.id;
+                    const bool first = xc < xa;
+                    chk += amj_hash_step(amj_hash_step(first ? r.h1 : hab, first ? xa : min(xc, xb)), max(xc, xb));
+                } else {
+                    chk += tri_chk(A, hab, xa, xb, xc);
+                }
                 if (WRITE) {
                     const unsigned long long p = atomicAdd(A.out_cursor, 1ull);
                     if (p < A.out_cap) tri_store(A, p, xa, xb, xc);
@@ -1172,6 +1245,27 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
                                        (uint64_t *)cand.p + A.r_n));
             unsigned long long total = 0;
             AMJ_TRY(read_back(ctx, &total, cand.p + A.r_n, sizeof(total)));
+            DBuf<uint32_t> hubs;
+            if (total && inv) {
+                AMJ_TRY(hid.alloc(ctx, nv));
+                note_launch(ctx);
+                rank_ids_kernel<<<(unsigned)std::min<uint64_t>((nv + 255) / 256, (uint64_t)ctx->num_sms * 16), 256,
+                                  0, ctx->stream>>>(inv, nv, hid.p);
+                AMJ_CUDA_TRY(cudaGetLastError());
+                A.hid = hid.p;
+            }
+            if (total >= BFS_HUB_MIN && A.bfs_wedge) {
+                const uint64_t k = std::min<uint64_t>(nv, HUB_RANKS);
+                A.hub_base = (int32_t)(nv - k);
+                A.hub_words = (uint32_t)((k + 31) / 32);
+                AMJ_TRY(hubs.alloc(ctx, k * A.hub_words));
+                AMJ_CUDA_TRY(cudaMemsetAsync(hubs.p, 0, k * A.hub_words * sizeof(uint32_t), ctx->stream));
+                note_launch(ctx);
+                hub_matrix_kernel<<<g1, 256, 0, ctx->stream>>>(R.src1.p, R.data1.p, R.len1, A.hub_base, A.hub_words,
+                                                               hubs.p);
+                AMJ_CUDA_TRY(cudaGetLastError());
+                A.hub_mtx = hubs.p;
+            }
             if (total) {
                 int per_sm = 0;
                 AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
@@ -1179,13 +1273,18 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
                     BFS_THREADS, 0));
                 if (per_sm < 1) per_sm = 1;
                 const uint64_t tiles = (total + BFS_TILE - 1) / BFS_TILE;
+                DBuf<uint32_t> first;
+                AMJ_TRY(first.alloc(ctx, tiles));
+                note_launch(ctx);
+                bfs_tile_first_kernel<<<g1, 256, 0, ctx->stream>>>(cand.p, A.r_n, first.p);
+                AMJ_CUDA_TRY(cudaGetLastError());
                 const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx->num_sms * per_sm);
                 note_launch(ctx);
                 AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[2], ctx->stream));
                 if (write)
-                    lftj_tri_bfs_expand_kernel<true><<<grid, BFS_THREADS, 0, ctx->stream>>>(A, cand.p, total);
+                    lftj_tri_bfs_expand_kernel<true><<<grid, BFS_THREADS, 0, ctx->stream>>>(A, cand.p, first.p, total);
                 else
-                    lftj_tri_bfs_expand_kernel<false><<<grid, BFS_THREADS, 0, ctx->stream>>>(A, cand.p, total);
+                    lftj_tri_bfs_expand_kernel<false><<<grid, BFS_THREADS, 0, ctx->stream>>>(A, cand.p, first.p, total);
                 AMJ_CUDA_TRY(cudaGetLastError());
                 AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[3], ctx->stream));
                 timed[1] = true;
