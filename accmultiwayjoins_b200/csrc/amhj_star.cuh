@@ -122,7 +122,32 @@ __global__ __launch_bounds__(256) void amhj_star_kernel(const __grid_constant__ 
     }
 }
 
-// ---- the canonical star, count mode: one 32-byte bucket head a lookup ----
+// A block's counts and checksums added to the totals: one atomic a block, since
+// the flat kernels run in many short blocks and the totals are two addresses
+// (one a warp cost 0.3 ms at 37K blocks).
+__device__ __forceinline__ void flat_totals(unsigned long long cnt, unsigned long long chk, unsigned long long *count,
+                                            unsigned long long *checksum) {
+    __shared__ unsigned long long c[8], h[8];
+    cnt = warp_sum(cnt);
+    chk = warp_sum(chk);
+    if ((threadIdx.x & 31) == 0) {
+        c[threadIdx.x >> 5] = cnt;
+        h[threadIdx.x >> 5] = chk;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; i++) {
+            cnt += c[i];
+            chk += h[i];
+        }
+        if (cnt) {
+            atomicAdd(count, cnt);
+            atomicAdd(checksum, chk);
+        }
+    }
+}
+
+// ---- the canonical star, count mode: one bucket head a lookup ----
 // The shape of the reference's star benchmarks: probe F(0..L-1) and, for
 // each key attribute c, one level D_c(c, L + c) of (key, payload) looked up
 // by c.  The tuple is then (F's row, the payloads in key order), so every
@@ -130,18 +155,14 @@ __global__ __launch_bounds__(256) void amhj_star_kernel(const __grid_constant__ 
 // registers (the general kernel above indexes an attribute array at run time,
 // a local-memory array, and loops over the levels).
 //
-// A probe of random lookups is bound by the L1's tag lookups, one for every
-// distinct line a warp's load touches: the general kernel makes four per
-// level (two bucket bounds, a key, a payload).  Before the probe every bucket
-// of a level gets a 32-byte head, one sector: its bounds and its first
-// HEAD_ROWS rows (key, payload), read by one 256-bit load.  Dimension
-// buckets hold one or two rows (keys unique, floorPow2(rows) buckets), so a
-// lookup is that one load.  A row whose buckets all hold at most
-// HEAD_ROWS rows, one of them with the key, is one tuple, hashed from
-// the keys' shared prefix.  Other rows count their matches per level from
-// the bounds and enumerate the product (an odometer over the levels, the
-// last fastest); products above STAR_MAX_PRODUCT are listed for the DFS
-// kernel as above.
+// Before the probe every bucket of a level gets a head that holds its first
+// rows (key, payload), so that a lookup is one load: the general kernel makes
+// four per level (two bucket bounds, a key, a payload).  Dimension buckets
+// hold one or two rows (keys unique, floorPow2(rows) buckets).  A row whose
+// lookups each find one match in the heads is one tuple, hashed from the keys'
+// shared prefix.  Other rows count their matches per level from the bounds and
+// enumerate the product (an odometer over the levels, the last fastest);
+// products above STAR_MAX_PRODUCT are listed for the DFS kernel as above.
 // A star (star_canon) or chain (chain_canon) plan with its levels in key
 // order: star level c is keyed by attribute c, chain level d by d + 1.
 struct CanonPlan {
@@ -202,8 +223,63 @@ __global__ void bucket_heads_kernel(const __grid_constant__ CanonPlan S, const _
     }
 }
 
+// A dimension bucket rarely holds more than two rows, and a lookup costs the L1
+// by the bytes each lane loads (0.90 to 0.92 ms for 240 M lookups of 32-byte heads
+// whatever the skew of the foreign keys, 1.11 ms as two 16-byte loads).  So the
+// star reads 16-byte heads by one 128-bit load: two (key, payload) rows, of
+// twice as many buckets (one more key bit), which take the same memory and
+// overflow as rarely as three rows of a 32-byte head.  A free row holds a key
+// of the neighbouring bucket, which no lookup here asks for; a bucket of more
+// rows holds such a key with payload 1 in its first row.
+// 60M-row star over 1M / 200K / 100K / 10K rows, Zipf(1.1) and uniform keys: 0.66
+// and 0.81 ms (0.90 and 0.92 with 32-byte heads).
+struct __align__(16) StarHead {
+    int32_t k0, p0, k1, p1;
+};
+static_assert(sizeof(StarHead) == 16 && 2 * sizeof(StarHead) == sizeof(BucketHead), "two star heads a bucket");
+// Blocks per SM: one lookup in flight a thread wants all of them (one dimension,
+// 50M rows: 0.30 ms with four blocks, 0.20 with eight), four run out of registers.
+constexpr int star_blocks(int L) { return L == 1 ? 8 : L == 2 ? 7 : 6; }
+constexpr uint32_t STAR_HEAD_SCAN = 8;   // longer index buckets are taken as overflowing
+
+// the heads of level blockIdx.y: index bucket h holds the rows of h and h + nb
+__global__ void star_heads_kernel(const __grid_constant__ CanonPlan S, const __grid_constant__ HeadOut H) {
+    const int c = blockIdx.y;
+    const uint32_t nb = S.nb[c];
+    const uint32_t *bp = S.bp[c];
+    StarHead *out = reinterpret_cast<StarHead *>(H.p[c]);
+    for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < nb; h += gridDim.x * blockDim.x) {
+        const uint32_t s = bp[h], n = bp[h + 1] - s;
+        // first of the two halves, then the other
+        StarHead o[2];
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+            const int32_t none = (int32_t)((h + x * nb) ^ 1u);
+            o[x] = StarHead{none, 0, none, 0};
+            uint32_t m = 0;
+            if (n <= STAR_HEAD_SCAN) {
+                for (uint32_t i = 0; i < n; i++) {
+                    const int32_t k = S.key[c][s + i];
+                    if ((((uint32_t)k & nb) != 0) != (x != 0)) continue;
+                    const int32_t p = S.pay[c][s + i];
+                    if (m == 0) {
+                        o[x].k0 = k;
+                        o[x].p0 = p;
+                    } else {
+                        o[x].k1 = k;
+                        o[x].p1 = p;
+                    }
+                    m++;
+                }
+            }
+            if (n > STAR_HEAD_SCAN || m > 2) o[x] = StarHead{none, 1, none, 0};
+            out[h + x * nb] = o[x];
+        }
+    }
+}
+
 template <int L>
-__global__ __launch_bounds__(256, 4) void amhj_star_canon_kernel(const __grid_constant__ CanonPlan S,
+__global__ __launch_bounds__(256, star_blocks(L)) void amhj_star_canon_kernel(const __grid_constant__ CanonPlan S,
                                                               unsigned long long *count, unsigned long long *checksum,
                                                               uint32_t *over, unsigned int *nover) {
     unsigned long long cnt = 0, chk = 0;
@@ -212,25 +288,21 @@ __global__ __launch_bounds__(256, 4) void amhj_star_canon_kernel(const __grid_co
         int32_t k[L];
 #pragma unroll
         for (int c = 0; c < L; c++) k[c] = __ldcs(S.fact[c] + r);
-        uint32_t w[L][8];
+        int4 w[L];
 #pragma unroll
-        for (int c = 0; c < L; c++) load_head(S.head[c] + ((uint32_t)k[c] & S.mask[c]), w[c]);
-        bool one = true;
+        for (int c = 0; c < L; c++)
+            w[c] = __ldg(reinterpret_cast<const int4 *>(S.head[c]) + ((uint32_t)k[c] & (2 * S.nb[c] - 1)));
+        bool one = true, empty = false;
         int32_t pay[L];
 #pragma unroll
         for (int c = 0; c < L; c++) {
-            const uint32_t n = w[c][1] - w[c][0];
-            uint32_t nm = 0;
-            int32_t p = 0;
-#pragma unroll
-            for (int i = 0; i < HEAD_ROWS; i++) {
-                const bool m = (uint32_t)i < n && (int32_t)w[c][2 + 2 * i] == k[c];
-                nm += m ? 1u : 0u;
-                p = m ? (int32_t)w[c][3 + 2 * i] : p;
-            }
-            one &= (n <= (uint32_t)HEAD_ROWS) & (nm == 1u);
-            pay[c] = p;
+            const bool m0 = w[c].x == k[c], m1 = w[c].z == k[c];
+            const uint32_t free_key = ((uint32_t)k[c] & (2 * S.nb[c] - 1)) ^ 1u;
+            one &= m0 != m1;
+            empty |= !m0 && !m1 && !((uint32_t)w[c].x == free_key && w[c].y != 0);
+            pay[c] = m0 ? w[c].y : w[c].w;
         }
+        if (empty) continue;   // a dimension without the key
         uint64_t hk = AMJ_CHECKSUM_SEED;
 #pragma unroll
         for (int c = 0; c < L; c++) hk = amj_hash_step(hk, k[c]);
@@ -246,9 +318,10 @@ __global__ __launch_bounds__(256, 4) void amhj_star_canon_kernel(const __grid_co
         uint64_t prod = 1;
 #pragma unroll
         for (int c = 0; c < L; c++) {
-            e[c] = w[c][1];
+            const uint32_t b = (uint32_t)k[c] & S.mask[c];
+            e[c] = S.bp[c][b + 1];
             uint32_t nm = 0, f = e[c];
-            for (uint32_t i = w[c][0]; i < e[c]; i++)
+            for (uint32_t i = S.bp[c][b]; i < e[c]; i++)
                 if (S.key[c][i] == k[c]) {
                     if (nm == 0) f = i;
                     nm++;
@@ -287,12 +360,7 @@ __global__ __launch_bounds__(256, 4) void amhj_star_canon_kernel(const __grid_co
             if (carry) break;
         }
     }
-    cnt = warp_sum(cnt);
-    chk = warp_sum(chk);
-    if ((threadIdx.x & 31) == 0 && cnt) {
-        atomicAdd(count, cnt);
-        atomicAdd(checksum, chk);
-    }
+    flat_totals(cnt, chk, count, checksum);   // 256-thread blocks
 }
 
 // ---- the canonical chain, count mode: a depth-first walk in registers ----
@@ -383,12 +451,7 @@ __global__ __launch_bounds__(256, L <= 3 ? 4 : 2) void amhj_chain_canon_kernel(c
             over[atomicAdd(nover, 1u)] = (uint32_t)(r - S.row_lo);
         }
     }
-    cnt = warp_sum(cnt);
-    chk = warp_sum(chk);
-    if ((threadIdx.x & 31) == 0 && cnt) {
-        atomicAdd(count, cnt);
-        atomicAdd(checksum, chk);
-    }
+    flat_totals(cnt, chk, count, checksum);   // 256-thread blocks
 }
 
 // ---- materialised star joins (two flat passes) ----

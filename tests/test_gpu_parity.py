@@ -1324,3 +1324,34 @@ def test_degree_rank_bins(ctx, degree):
     for algo in ("DFS", "BFS"):
         r = ctx.lftj([e], algo=algo)
         assert (r.count, r.checksum) == want
+
+
+@pytest.mark.parametrize("copies", [1, 2, 3, 9])
+@pytest.mark.parametrize("dims", [1, 2, 3, 4])
+@pytest.mark.parametrize("keys", ["dense", "sparse", "one"])
+def test_star_heads(dims, copies, keys):
+    """Star counts around the two rows of a head and the rows scanned for it:
+    unique and repeated dimension keys, keys without a partner, negative and
+    sparse keys, a dimension of a single bucket."""
+    n = 3000
+    m = 1 if keys == "one" else 64
+    base = {"dense": np.arange(m), "sparse": np.arange(m) * 1024 * 7 - 200_000, "one": np.array([5])}[keys]
+    rng = np.random.default_rng(dims * 10 + copies)
+    rels, fact = [], []
+    for j in range(dims):
+        rep = copies if j == 0 else 1 + (j % 2)
+        if keys == "dense":      # only some keys repeat
+            k = np.concatenate([base, np.repeat(base[:5], rep - 1)])
+        else:
+            k = np.repeat(base, rep)
+        k = rng.permutation(k).astype(np.int32)
+        rels.append(([k, data.uniform(len(k), -(1 << 31), 1 << 31, 20 + j)], [j, dims + j]))
+        miss = base[0] - 1 - np.arange(8)
+        fact.append(rng.choice(np.concatenate([base, base, base, miss]), n).astype(np.int32))
+    q = [(fact, list(range(dims)))] + rels
+    want = O.mhj(q)
+    with Context(0) as ctx:
+        rs = rels_on(ctx, q)
+        for plan in ("multiway", "frontier"):
+            got = ctx.amhj("NORMAL", rs, plan=plan)
+            assert (got.count, got.checksum) == want
