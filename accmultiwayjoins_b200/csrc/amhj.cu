@@ -126,6 +126,8 @@ int compile_plan(int query_type, amj_rel *const *rels, int nrels, int flags, Hos
 struct ExecScratch {
     std::map<IndexKey, HashIndex> indexes;
     DBuf<char> index_block;      // memory of the indexes built together
+    void *zeroed = nullptr;      // zeroed bytes of that block, for one pass
+    cudaEvent_t begin = nullptr; // recorded before the passes
     cudaEvent_t end = nullptr;   // to be recorded behind the last launch, when a pass knows it is the last
     bool ended = false;
     DBuf<ProbeState> st;
@@ -293,10 +295,6 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     P.row_lo = row_lo;
     P.row_hi = row_hi;
     const uint64_t rows = row_hi - row_lo;
-    struct Ctr {
-        unsigned long long count, checksum;
-        unsigned int nover, pad;
-    };
     const unsigned g = (unsigned)std::min<uint64_t>((rows + 255) / 256, (uint64_t)ctx->num_sms * 8);
     CanonPlan S{};
     int canon = star_canon(P, S);
@@ -328,10 +326,20 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
         canon = 0;
     }
     BucketHead *heads = reinterpret_cast<BucketHead *>(work.p);
-    Ctr *ctr = reinterpret_cast<Ctr *>(heads + nheads);
+    FlatCtr *ctr = reinterpret_cast<FlatCtr *>(heads + nheads);
+    FlatCtr *host = static_cast<FlatCtr *>(ctx->h_small);
     uint32_t *over = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(ctr) + 256);
-    AMJ_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(Ctr), ctx->stream));
-    AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[0], ctx->stream));
+    static_assert(sizeof(FlatCtr) <= BUCKET_ZEROED && sizeof(FlatCtr) <= READ_BACK_MAX, "the counters' places");
+    if (X.zeroed) {
+        ctr = static_cast<FlatCtr *>(X.zeroed);   // cleared with the bucket counts
+        X.zeroed = nullptr;
+    } else {
+        AMJ_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(FlatCtr), ctx->stream));
+    }
+    // a query of one pass is timed by its own events: each costs the stream a
+    // few microseconds
+    const cudaEvent_t kb = X.begin ? X.begin : ctx->kev[0], ke = X.end ? X.end : ctx->kev[1];
+    if (!X.begin) AMJ_CUDA_TRY(cudaEventRecord(kb, ctx->stream));
     if (canon) {
         HeadOut H{};
         size_t at = 0;
@@ -353,26 +361,25 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     note_launch(ctx);
     if (chain) {
         switch (canon) {
-        case 1: amhj_chain_canon_kernel<1><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-        case 2: amhj_chain_canon_kernel<2><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-        case 3: amhj_chain_canon_kernel<3><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-        case 4: amhj_chain_canon_kernel<4><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-        case 5: amhj_chain_canon_kernel<5><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-        default: amhj_chain_canon_kernel<6><<<g ? g : 1, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover);
+        case 1: amhj_chain_canon_kernel<1><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+        case 2: amhj_chain_canon_kernel<2><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+        case 3: amhj_chain_canon_kernel<3><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+        case 4: amhj_chain_canon_kernel<4><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+        case 5: amhj_chain_canon_kernel<5><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+        default: amhj_chain_canon_kernel<6><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over);
         }
     } else switch (canon) {
-    case 1: amhj_star_canon_kernel<1><<<gs, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-    case 2: amhj_star_canon_kernel<2><<<gs, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-    case 3: amhj_star_canon_kernel<3><<<gs, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-    case 4: amhj_star_canon_kernel<4><<<gs, 256, 0, ctx->stream>>>(S, &ctr->count, &ctr->checksum, over, &ctr->nover); break;
-    default: amhj_star_kernel<<<g ? g : 1, 256, 0, ctx->stream>>>(P, &ctr->count, &ctr->checksum, over, &ctr->nover);
+    case 1: amhj_star_canon_kernel<1><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+    case 2: amhj_star_canon_kernel<2><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+    case 3: amhj_star_canon_kernel<3><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+    case 4: amhj_star_canon_kernel<4><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
+    default: amhj_star_kernel<<<g ? g : 1, 256, 0, ctx->stream>>>(P, ctr, host, over);
     }
     AMJ_CUDA_TRY(cudaGetLastError());
-    AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[1], ctx->stream));
-    if (X.end) AMJ_CUDA_TRY(cudaEventRecord(X.end, ctx->stream));
-    Ctr h{};
-    AMJ_TRY(read_back(ctx, &h, ctr, sizeof(h)));
-    res->kernel_ms[0] += event_ms(ctx->kev[0], ctx->kev[1]);
+    AMJ_CUDA_TRY(cudaEventRecord(ke, ctx->stream));
+    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    const FlatCtr h = *host;   // written by the kernel's last block
+    res->kernel_ms[0] += event_ms(kb, ke);
     pr->count = h.count;
     pr->checksum = h.checksum;
     X.ended = X.end && h.nover == 0;
@@ -1148,7 +1155,7 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         }
         lvix[l] = &it->second;
     }
-    AMJ_TRY(build_bucket_indexes(ctx, specs, nspecs, &X.index_block));
+    AMJ_TRY(build_bucket_indexes(ctx, specs, nspecs, &X.index_block, &X.zeroed));
     AMJ_CUDA_TRY(cudaEventRecord(e1, ctx->stream));
 
     // ---- probe plan
@@ -1222,6 +1229,7 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         }
     } else {
         PassResult pr;
+        X.begin = e1;
         X.end = e2;
         rc = run_passes(ctx, PL, X, use_ws, dro != 0, materialize, 0, hp.probe->n, &pr, out, !(flags & AMJ_F_FRONTIER));
         if (rc == AMJ_OK) {

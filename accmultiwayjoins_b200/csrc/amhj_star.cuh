@@ -35,9 +35,46 @@ inline bool star_eligible(const ProbePlan &P) {
     return true;
 }
 
+// Totals of a flat kernel, and the rows it listed.
+struct FlatCtr {
+    unsigned long long count, checksum;
+    unsigned int nover, done;   // listed rows; blocks that have ended
+};
+
+// A block's count and checksum added to the totals: one atomic a block, since
+// the flat kernels run in many short blocks and the totals are two addresses
+// (one a warp cost 0.3 ms at 37K blocks).  The last block writes the totals to
+// pinned host memory, which saves the query a copy.  256-thread blocks.
+__device__ __forceinline__ void flat_totals(unsigned long long cnt, unsigned long long chk, FlatCtr *ctr, FlatCtr *host) {
+    __shared__ unsigned long long c[8], h[8];
+    cnt = warp_sum(cnt);
+    chk = warp_sum(chk);
+    if ((threadIdx.x & 31) == 0) {
+        c[threadIdx.x >> 5] = cnt;
+        h[threadIdx.x >> 5] = chk;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int i = 1; i < 8; i++) {
+            cnt += c[i];
+            chk += h[i];
+        }
+        if (cnt) {
+            atomicAdd(&ctr->count, cnt);
+            atomicAdd(&ctr->checksum, chk);
+        }
+        __threadfence();
+        if (atomicAdd(&ctr->done, 1u) == gridDim.x - 1) {
+            host->count = atomicAdd(&ctr->count, 0ull);
+            host->checksum = atomicAdd(&ctr->checksum, 0ull);
+            host->nover = atomicAdd(&ctr->nover, 0u);
+            __threadfence_system();
+        }
+    }
+}
+
 __global__ __launch_bounds__(256) void amhj_star_kernel(const __grid_constant__ ProbePlan P,
-                                                        unsigned long long *count, unsigned long long *checksum,
-                                                        uint32_t *over, unsigned int *nover) {
+                                                        FlatCtr *ctr, FlatCtr *host, uint32_t *over) {
     unsigned long long cnt = 0, chk = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t r = P.row_lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < P.row_hi; r += stride) {
@@ -70,7 +107,7 @@ __global__ __launch_bounds__(256) void amhj_star_kernel(const __grid_constant__ 
         }
         if (prod == 0) continue;
         if (prod > STAR_MAX_PRODUCT) {
-            over[atomicAdd(nover, 1u)] = (uint32_t)(r - P.row_lo);
+            over[atomicAdd(&ctr->nover, 1u)] = (uint32_t)(r - P.row_lo);
             continue;
         }
         if (prod == 1) {   // unique keys in every level: one tuple
@@ -114,37 +151,7 @@ __global__ __launch_bounds__(256) void amhj_star_kernel(const __grid_constant__ 
             if (l < 0) break;
         }
     }
-    cnt = warp_sum(cnt);
-    chk = warp_sum(chk);
-    if ((threadIdx.x & 31) == 0 && cnt) {
-        atomicAdd(count, cnt);
-        atomicAdd(checksum, chk);
-    }
-}
-
-// A block's counts and checksums added to the totals: one atomic a block, since
-// the flat kernels run in many short blocks and the totals are two addresses
-// (one a warp cost 0.3 ms at 37K blocks).
-__device__ __forceinline__ void flat_totals(unsigned long long cnt, unsigned long long chk, unsigned long long *count,
-                                            unsigned long long *checksum) {
-    __shared__ unsigned long long c[8], h[8];
-    cnt = warp_sum(cnt);
-    chk = warp_sum(chk);
-    if ((threadIdx.x & 31) == 0) {
-        c[threadIdx.x >> 5] = cnt;
-        h[threadIdx.x >> 5] = chk;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < 8; i++) {
-            cnt += c[i];
-            chk += h[i];
-        }
-        if (cnt) {
-            atomicAdd(count, cnt);
-            atomicAdd(checksum, chk);
-        }
-    }
+    flat_totals(cnt, chk, ctr, host);
 }
 
 // ---- the canonical star, count mode: one bucket head a lookup ----
@@ -280,8 +287,7 @@ __global__ void star_heads_kernel(const __grid_constant__ CanonPlan S, const __g
 
 template <int L>
 __global__ __launch_bounds__(256, star_blocks(L)) void amhj_star_canon_kernel(const __grid_constant__ CanonPlan S,
-                                                              unsigned long long *count, unsigned long long *checksum,
-                                                              uint32_t *over, unsigned int *nover) {
+                                                              FlatCtr *ctr, FlatCtr *host, uint32_t *over) {
     unsigned long long cnt = 0, chk = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t r = S.row_lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < S.row_hi; r += stride) {
@@ -331,7 +337,7 @@ __global__ __launch_bounds__(256, star_blocks(L)) void amhj_star_canon_kernel(co
         }
         if (prod == 0) continue;
         if (prod > STAR_MAX_PRODUCT) {
-            over[atomicAdd(nover, 1u)] = (uint32_t)(r - S.row_lo);
+            over[atomicAdd(&ctr->nover, 1u)] = (uint32_t)(r - S.row_lo);
             continue;
         }
         uint32_t pos[L];
@@ -360,7 +366,7 @@ __global__ __launch_bounds__(256, star_blocks(L)) void amhj_star_canon_kernel(co
             if (carry) break;
         }
     }
-    flat_totals(cnt, chk, count, checksum);   // 256-thread blocks
+    flat_totals(cnt, chk, ctr, host);
 }
 
 // ---- the canonical chain, count mode: a depth-first walk in registers ----
@@ -435,8 +441,7 @@ __device__ __forceinline__ bool chain_walk(const CanonPlan &S, int32_t key, uint
 // their per-level state in two blocks' worth of registers
 template <int L>
 __global__ __launch_bounds__(256, L <= 3 ? 4 : 2) void amhj_chain_canon_kernel(const __grid_constant__ CanonPlan S,
-                                                               unsigned long long *count, unsigned long long *checksum,
-                                                               uint32_t *over, unsigned int *nover) {
+                                                               FlatCtr *ctr, FlatCtr *host, uint32_t *over) {
     unsigned long long cnt = 0, chk = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t r = S.row_lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < S.row_hi; r += stride) {
@@ -448,10 +453,10 @@ __global__ __launch_bounds__(256, L <= 3 ? 4 : 2) void amhj_chain_canon_kernel(c
             cnt += rc;
             chk += rchk;
         } else {
-            over[atomicAdd(nover, 1u)] = (uint32_t)(r - S.row_lo);
+            over[atomicAdd(&ctr->nover, 1u)] = (uint32_t)(r - S.row_lo);
         }
     }
-    flat_totals(cnt, chk, count, checksum);   // 256-thread blocks
+    flat_totals(cnt, chk, ctr, host);
 }
 
 // ---- materialised star joins (two flat passes) ----

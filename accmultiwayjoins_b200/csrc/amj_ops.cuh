@@ -51,8 +51,10 @@ struct BucketSpec {
 constexpr uint64_t BUCKET_COUNT_MAX = 1ull << 23;   // rows of an index that the counting build takes
 constexpr int BUCKET_BUILD_MAX = 8;                 // indexes of one build_bucket_indexes call
 // Bucket indexes of up to BUCKET_COUNT_MAX rows each, all built by one set of
-// launches in one block of memory, which `block` owns.
-int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<char> *block);
+// launches in one block of memory, which `block` owns.  *zeroed (optional)
+// gets BUCKET_ZEROED zeroed bytes of the block (null when count is 0).
+constexpr size_t BUCKET_ZEROED = 64;
+int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<char> *block, void **zeroed = nullptr);
 
 int build_hash_index(amj_ctx *ctx, const int32_t *const *d_cols, int ncols, uint64_t n, int layout,
                      int key_mode, float load_factor, HashIndex *out);

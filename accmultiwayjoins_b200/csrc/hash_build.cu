@@ -193,7 +193,8 @@ __global__ void bucket_scatter_kernel(const __grid_constant__ BucketJobs A) {
     }
 }
 
-int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<char> *block) {
+int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<char> *block, void **zeroed) {
+    if (zeroed) *zeroed = nullptr;
     if (count <= 0) return AMJ_OK;
     if (count > BUCKET_BUILD_MAX) return fail(AMJ_EINVAL, "bucket indexes: too many at once");
     uint64_t rows = 0, buckets = 0, nmax = 0;
@@ -217,12 +218,14 @@ int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<
         ncols = std::max(ncols, sp.ncols);
     }
     auto round = [](uint64_t b) { return (b + 255) / 256 * 256; };
-    const uint64_t ptr_bytes = round((buckets + 1) * sizeof(uint32_t));
+    const uint64_t zero_at = ((buckets + 1) * sizeof(uint32_t) + 15) / 16 * 16, zero_bytes = zero_at + BUCKET_ZEROED;
+    const uint64_t ptr_bytes = round(zero_bytes);
     const uint64_t col_bytes = round(std::max<uint64_t>(rows, 1) * sizeof(int32_t));
     AMJ_TRY(block->alloc(ctx, ptr_bytes + ncols * col_bytes));
     DBuf<uint32_t> place;
     AMJ_TRY(place.alloc(ctx, rows));
     A.counts = reinterpret_cast<uint32_t *>(block->p);
+    if (zeroed) *zeroed = block->p + zero_at;
     A.place = place.p;
     for (int c = 0; c < ncols; c++) A.out[c] = reinterpret_cast<int32_t *>(block->p + ptr_bytes + c * col_bytes);
     for (int t = 0; t < count; t++) {
@@ -240,7 +243,7 @@ int build_bucket_indexes(amj_ctx *ctx, const BucketSpec *specs, int count, DBuf<
             ix.cols[c].n = specs[t].n;
         }
     }
-    AMJ_CUDA_TRY(cudaMemsetAsync(A.counts, 0, (buckets + 1) * sizeof(uint32_t), ctx->stream));
+    AMJ_CUDA_TRY(cudaMemsetAsync(A.counts, 0, zero_bytes, ctx->stream));
     if (!rows) return AMJ_OK;
     const dim3 grid(grid_for(ctx, nmax), count);
     note_launch(ctx);
