@@ -70,6 +70,7 @@ struct Trie2 {
     DBuf<uint64_t> rowptr;     // dense child offsets for values rp_min .. rp_min+rp_count-1 (+1 end entry)
     int32_t rp_min = 0;
     uint64_t rp_count = 0;     // 0 when no dense array was built
+    uint64_t range1 = 0;       // level 1's values span at most this many (0: not known)
 };
 
 // Level 1 of a built 2-level trie has TRIE_LEVEL1_PAD spare values after its
@@ -79,6 +80,17 @@ constexpr uint64_t TRIE_LEVEL1_PAD = 4;
 // vmax >= 0: every value of both columns lies in [0, vmax] (no min/max pass)
 int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, Trie2 *out,
                 bool distinct = false, int32_t vmax = -1);
+// The distinct 2-level tries of up to TRIE_JOBS_MAX relations, built together in
+// memory that `block` owns; level 0 lists every value of the first column's
+// range.  *built is false, and nothing is built, where a range is not dense, a
+// row is too long, rows repeat or a relation is empty.
+constexpr int TRIE_JOBS_MAX = 3;
+struct TrieCols {
+    const int32_t *c0, *c1;
+    uint64_t n;
+};
+int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf<char> *block, bool *built);
+
 // The distinct 2-level trie of the degree-ranked copy of the edges (c0, c1):
 // every vertex renamed to its rank (below nv), edges from the lower to the
 // higher rank.  Rows bucketed by counting, each row sorted on its own; the

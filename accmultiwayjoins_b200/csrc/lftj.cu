@@ -54,7 +54,8 @@ struct TriArgs {
     TrieRef R;
     uint64_t r_lo, r_hi;          // R level-1 slice handled by this launch
     unsigned long long *cursor0;  // claim cursor of the bitmap kernel over heavy_list
-    const uint32_t *heavy_list;   // R's level-0 indexes of the heavy vertices
+    const uint64_t *heavy_list;   // parts of the heavy vertices: R's level-0 index << 32 | part
+    uint32_t heavy_part;          // R-children a part
     const unsigned long long *heavy_n;
     uint32_t heavy_deg;           // 0: no bitmap kernel
     uint32_t bitmap_bits;
@@ -138,38 +139,48 @@ __device__ __forceinline__ bool heavy_vertex(const TriArgs &A, uint64_t r_deg, u
     return sp > 0 && sp <= (int64_t)A.bitmap_bits;
 }
 
-// R's level-0 indexes of the vertices the bitmap kernel owns, in any order
-__global__ void heavy_list_kernel(const __grid_constant__ TriArgs A, uint32_t *list, unsigned long long *n) {
+// The parts of the vertices the bitmap kernel owns, in any order: heavy_part
+// R-children each, so that a hub's are shared by several blocks.
+__global__ void heavy_list_kernel(const __grid_constant__ TriArgs A, uint64_t *list, unsigned long long *n) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < A.R.len0;
          i += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t rs = A.R.off0[i], re = A.R.off0[i + 1];
-        if ((rs > A.r_lo ? rs : A.r_lo) >= (re < A.r_hi ? re : A.r_hi)) continue;
+        const uint64_t es = rs > A.r_lo ? rs : A.r_lo, ee = re < A.r_hi ? re : A.r_hi;
+        if (es >= ee) continue;
         uint64_t ta, ea;
         child_range(A.T, A.R.data0[i], ta, ea);
         int32_t lo;
         uint32_t span;
-        if (heavy_vertex(A, re - rs, ta, ea, lo, span)) list[atomicAdd(n, 1ull)] = (uint32_t)i;
+        if (!heavy_vertex(A, re - rs, ta, ea, lo, span)) continue;
+        const uint32_t parts = (uint32_t)((ee - es + A.heavy_part - 1) / A.heavy_part);
+        const unsigned long long at = atomicAdd(n, (unsigned long long)parts);
+        for (uint32_t p = 0; p < parts; p++) list[at + p] = i << 32 | p;
     }
 }
 
-constexpr int BM_THREADS = 1024;
 constexpr int BM_UNROLL = 8;
 constexpr uint32_t BM_SEG = 1024;   // values of one child list per warp work item
 
-// Bitmap kernel: one block per heavy vertex a at a time.  The children of a
-// in T are set in a shared-memory bitmap (one bit per value in their span,
-// up to 2^20 values = 128 KB); then the children lists of every b in a's
-// R-children are streamed through the block, 1024 edges per batch, with a
-// block scan over their lengths so every thread takes one candidate c per
-// step (load-balanced, coalesced) and tests bit c.  Each child list is read
-// once per (a,b) and tested with one shared-memory load, instead of a
-// galloping search per needle window.
-template <bool WRITE>
-__global__ __launch_bounds__(BM_THREADS, 1) void lftj_tri_bitmap_kernel(const __grid_constant__ TriArgs A) {
+// Bitmap kernel: one block per part of a heavy vertex a at a time.  The
+// children of a in T are set in a shared-memory bitmap (one bit per value in
+// their span, up to 2^20 values = 128 KB); then the children lists of every b
+// among the part's R-children are cut into segments that the block's warps
+// claim and stream, one value c a lane and step, and bit c is tested.  Each
+// child list is read once per (a,b) and tested with one shared-memory load,
+// instead of a galloping search per needle window.
+// A part is a chain of short phases (bits, scan, segments, clearing) with
+// block barriers between them, so an SM wants several: where T's values span
+// at most BM_SMALL_BITS, eight blocks of 256 threads with a bitmap of that
+// span run per SM, else one block of 1024 threads.  1M-edge R-MAT relations:
+// BM_FIGURES.
+constexpr uint32_t BM_SMALL_BITS = 1u << 17;
+
+template <bool WRITE, int BM_THREADS>
+__global__ __launch_bounds__(BM_THREADS, BM_THREADS == 256 ? 8 : 1) void lftj_tri_bitmap_kernel(const __grid_constant__ TriArgs A) {
     extern __shared__ __align__(16) unsigned char bm_smem[];
     const uint32_t words = (A.bitmap_bits + 31) / 32;
     uint32_t *bits = (uint32_t *)bm_smem;
-    unsigned long long *pre = (unsigned long long *)(bm_smem + (size_t)words * 4);  // inclusive
+    unsigned long long *pre = (unsigned long long *)(bm_smem + ((size_t)words * 4 + 15) / 16 * 16);  // inclusive
     unsigned long long *hab = pre + BM_THREADS;
     uint32_t *sbeg = (uint32_t *)(hab + BM_THREADS);
     int32_t *bval = (int32_t *)(sbeg + BM_THREADS);
@@ -188,12 +199,14 @@ __global__ __launch_bounds__(BM_THREADS, 1) void lftj_tri_bitmap_kernel(const __
             s_i = x < *A.heavy_n ? A.heavy_list[x] : ~0ull;
         }
         __syncthreads();
-        const unsigned long long i = s_i;
+        const unsigned long long item = s_i;
         __syncthreads();
-        if (i >= A.R.len0) break;
+        if (item == ~0ull) break;
+        const uint64_t i = item >> 32;
         const uint64_t rs = A.R.off0[i], re = A.R.off0[i + 1];
-        const uint64_t es = rs > A.r_lo ? rs : A.r_lo, ee = re < A.r_hi ? re : A.r_hi;
-        if (es >= ee) continue;
+        const uint64_t es = (rs > A.r_lo ? rs : A.r_lo) + (item & 0xffffffffu) * A.heavy_part;
+        uint64_t ee = re < A.r_hi ? re : A.r_hi;
+        if (ee > es + A.heavy_part) ee = es + A.heavy_part;
         const int32_t a = A.R.data0[i];
         uint64_t ta, ea;
         child_range(A.T, a, ta, ea);
@@ -228,10 +241,10 @@ __global__ __launch_bounds__(BM_THREADS, 1) void lftj_tri_bitmap_kernel(const __
             if (warp == 0) {
                 unsigned long long w = lane < BM_THREADS / 32 ? s_wsum[lane] : 0ull;
                 unsigned long long wi = warp_inclusive_scan(w, lane);
-                s_wsum[lane] = wi - w;
+                if (lane < BM_THREADS / 32) s_wsum[lane] = wi - w;
                 uint32_t sw = lane < BM_THREADS / 32 ? s_ssum[lane] : 0u;
                 uint32_t swi = warp_inclusive_scan(sw, lane);
-                s_ssum[lane] = swi - sw;
+                if (lane < BM_THREADS / 32) s_ssum[lane] = swi - sw;
                 if (lane == 31) s_ssum[BM_THREADS / 32] = swi;
             }
             __syncthreads();
@@ -1147,7 +1160,7 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
     A.checksum = &ctr.p->checksum;
     A.out_cursor = &ctr.p->out_cursor;
     A.cursor0 = &ctr.p->cursor0;
-    DBuf<uint32_t> heavy;
+    DBuf<uint64_t> heavy;
     DBuf<RankId> hid;
     A.cursor_r = &ctr.p->cursor_r;
     const bool write = out != nullptr;
@@ -1192,23 +1205,31 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
                 timed[0] = true;
             }
             if (rest && heavy_deg) {
-                // the bitmap kernel takes the heavy vertices; its shared memory: bitmap + 1024 x 24 B
-                const uint32_t bits_max = 1u << 20;
-                const size_t smem = (size_t)bits_max / 8 + (size_t)BM_THREADS * (8 + 8 + 4 + 4 + 4);
+                // the bitmap kernel takes the heavy vertices; its shared memory:
+                // the bitmap and 28 B a thread
+                const bool small = T.range1 && T.range1 <= BM_SMALL_BITS;
+                const int threads = small ? 256 : 1024;
+                const uint32_t bits_max = small ? (uint32_t)((T.range1 + 31) / 32 * 32) : 1u << 20;
+                const size_t smem = ((size_t)bits_max / 8 + 15) / 16 * 16 + (size_t)threads * (8 + 8 + 4 + 4 + 4);
                 if (smem <= (size_t)ctx->max_smem_optin && R.len0) {
                     A.heavy_deg = heavy_deg;
                     A.bitmap_bits = bits_max;
-                    AMJ_TRY(heavy.alloc(ctx, R.len0));
+                    A.heavy_part = (uint32_t)threads;
+                    // every heavy vertex has a part that is not full, at most one a heavy_deg R-children
+                    AMJ_TRY(heavy.alloc(ctx, A.r_n / A.heavy_part + std::min<uint64_t>(R.len0, A.r_n) + 1));
                     A.heavy_list = heavy.p;
                     A.heavy_n = &ctr.p->heavy_n;
                     note_launch(ctx);
                     heavy_list_kernel<<<(unsigned)std::min<uint64_t>((R.len0 + 255) / 256, (uint64_t)ctx->num_sms * 8), 256, 0,
                                         ctx->stream>>>(A, heavy.p, &ctr.p->heavy_n);
                     AMJ_CUDA_TRY(cudaGetLastError());
-                    auto kb = write ? lftj_tri_bitmap_kernel<true> : lftj_tri_bitmap_kernel<false>;
+                    auto kb = small ? (write ? lftj_tri_bitmap_kernel<true, 256> : lftj_tri_bitmap_kernel<false, 256>)
+                                    : (write ? lftj_tri_bitmap_kernel<true, 1024> : lftj_tri_bitmap_kernel<false, 1024>);
                     AMJ_CUDA_TRY(cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                    int per_sm = 0;
+                    AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kb, threads, smem));
                     note_launch(ctx);
-                    kb<<<(unsigned)ctx->num_sms, BM_THREADS, smem, ctx->stream>>>(A);
+                    kb<<<(unsigned)(ctx->num_sms * std::max(per_sm, 1)), threads, smem, ctx->stream>>>(A);
                     AMJ_CUDA_TRY(cudaGetLastError());
                     timed[0] = true;
                 }

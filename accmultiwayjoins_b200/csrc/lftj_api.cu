@@ -76,13 +76,6 @@ static int build_ranked_trie(amj_ctx *ctx, const amj_rel *r, Trie2 *t, DBuf<int3
 
 using namespace amj;
 
-static int build_rel_trie(amj_ctx *ctx, const amj_rel *r, Trie2 *t) {
-    if (r->ncols != 2) return fail(AMJ_EUNSUPPORTED, "LFTJ: relations must have two columns");
-    if (r->where == AMJ_MEM_HOST_STREAMED) return fail(AMJ_EUNSUPPORTED, "LFTJ: relations must be on the device");
-    const bool swap = r->attrs[0] > r->attrs[1];
-    return build_trie2(ctx, r->d_cols[swap ? 1 : 0], r->d_cols[swap ? 0 : 1], r->n, t, true);
-}
-
 // The 4-clique over one edge relation (AMJ_F_CLIQUE4): a count pass, then
 // with AMJ_F_MATERIALIZE a write pass into exactly allocated columns.  With
 // matrices_only the query runs only where the triangle matrices apply;
@@ -361,6 +354,7 @@ static int lftj_execute_impl(amj_ctx *ctx, amj_rel *const *rels, int nrels, int 
     result_init(out, 3);
     AMJ_CUDA_TRY(cudaEventRecord(ctx->ev[0], ctx->stream));
 
+    DBuf<char> trie_block;   // memory of tries built together
     Trie2 tries[3];
     const Trie2 *R = nullptr, *S = nullptr, *T = nullptr;
     int sorted_out = 0;
@@ -383,16 +377,24 @@ static int lftj_execute_impl(amj_ctx *ctx, amj_rel *const *rels, int nrels, int 
         }
         R = S = T = &tries[0];
     } else {
+        TrieCols cols[3];
         for (int i = 0; i < 3; i++) {
             if (rels[i]->ncols != 2) return fail(AMJ_EUNSUPPORTED, "LFTJ: relations must have two columns");
+            if (rels[i]->where == AMJ_MEM_HOST_STREAMED)
+                return fail(AMJ_EUNSUPPORTED, "LFTJ: relations must be on the device");
             const uint32_t lo = std::min(rels[i]->attrs[0], rels[i]->attrs[1]);
             const uint32_t hi = std::max(rels[i]->attrs[0], rels[i]->attrs[1]);
             const Trie2 **slot = (lo == 0 && hi == 1) ? &R : (lo == 1 && hi == 2) ? &S : (lo == 0 && hi == 2) ? &T : nullptr;
             if (!slot || *slot)
                 return fail(AMJ_EUNSUPPORTED, "LFTJ: three relations must carry attributes (0,1), (1,2) and (0,2)");
-            AMJ_TRY(build_rel_trie(ctx, rels[i], &tries[i]));
             *slot = &tries[i];
+            const bool swap = rels[i]->attrs[0] > rels[i]->attrs[1];
+            cols[i] = TrieCols{rels[i]->d_cols[swap ? 1 : 0], rels[i]->d_cols[swap ? 0 : 1], rels[i]->n};
         }
+        bool built = false;
+        AMJ_TRY(build_tries2(ctx, cols, 3, tries, &trie_block, &built));
+        for (int i = 0; i < 3 && !built; i++)
+            AMJ_TRY(build_trie2(ctx, cols[i].c0, cols[i].c1, cols[i].n, &tries[i], true));
     }
     return triangle_run(ctx, *R, *S, *T, algo, ws, flags, sorted_out, nv ? inv.p : nullptr, wedges.p, nv, out);
 }

@@ -148,6 +148,7 @@ int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t
     }
     const uint32_t min0 = h_mm[0], min1 = h_mm[2];
     const int bits0 = bits_for(h_mm[1] - min0), bits1 = bits_for(h_mm[3] - min1);
+    out->range1 = (uint64_t)(h_mm[3] - min1) + 1;
 
     DBuf<uint64_t> a, b;
     AMJ_TRY(a.alloc(ctx, n));
@@ -234,13 +235,12 @@ int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t
 // After the degree
 // ranking a row holds the higher-ranked neighbours of one vertex, at most
 // sqrt(2 n) of them, and most rows hold a few: a warp sorts a row of up to
-// 32 values in registers (a bitonic network over shuffles) and up to
-// RK_WARP_MAX in its shared-memory slice; a block sorts the longer rows, up to
-// RK_BLOCK_MAX.  A graph with a longer row takes the radix-sort build.
+// RK_WARP_MAX values in registers (a bitonic network over shuffles); a block
+// sorts the longer rows, up to RK_BLOCK_MAX, in shared memory.  A graph with a longer row takes the radix-sort build.
 // Repeated rows (adjacent after the sort) are dropped by a compaction pass
 // when there are any.
 constexpr uint32_t RK_WARP_MAX = 1024;
-constexpr uint32_t RK_BLOCK_MAX = 8192;
+constexpr uint32_t RK_BLOCK_MAX = 32768;   // 128 KB of shared memory
 constexpr int RK_SORT_WARPS = 8;
 
 // Ranked edges (the lower rank first), the count of every lower rank, each
@@ -332,7 +332,7 @@ __device__ __forceinline__ uint32_t rk_distinct(const int32_t *x, uint32_t len, 
 template <int E>
 __device__ __forceinline__ uint32_t rk_warp_row(int32_t *__restrict__ data1, int32_t *__restrict__ src1,
                                             uint32_t *__restrict__ uniq, uint32_t s, uint32_t len, uint64_t v,
-                                            uint32_t lane) {
+                                            int32_t value, uint32_t lane) {
     int32_t x[E];
 #pragma unroll
     for (int e = 0; e < E; e++) {
@@ -349,7 +349,7 @@ __device__ __forceinline__ uint32_t rk_warp_row(int32_t *__restrict__ data1, int
             const int32_t before = e ? x[e - 1] : prev;
             u += (i == 0 || x[e] != before) ? 1u : 0u;
             data1[s + i] = x[e];
-            src1[s + i] = (int32_t)v;
+            src1[s + i] = value;
         }
     }
 #pragma unroll
@@ -361,6 +361,7 @@ __device__ __forceinline__ uint32_t rk_warp_row(int32_t *__restrict__ data1, int
 // One warp a row, the row's values in registers (rows of up to RK_WARP_MAX);
 // longer rows are listed for the block kernel.
 __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(const uint32_t *__restrict__ start,
+                                                                           const int32_t *__restrict__ values,
                                                                            uint64_t nv, int32_t *__restrict__ data1,
                                                                            int32_t *__restrict__ src1,
                                                                            uint32_t *__restrict__ uniq,
@@ -375,22 +376,23 @@ __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(con
     const uint64_t warps = (uint64_t)gridDim.x * RK_SORT_WARPS;
     for (uint64_t v = blockIdx.x * (uint64_t)RK_SORT_WARPS + w; v < nv; v += warps) {
         const uint32_t s = start[v], len = start[v + 1] - s;
+        const int32_t value = values ? values[v] : (int32_t)v;
         if (len <= 1) {
-            if (len == 1 && lane == 0) src1[s] = (int32_t)v;
+            if (len == 1 && lane == 0) src1[s] = value;
             if (lane == 0) uniq[v] = len;
             u += len;
         } else if (len <= 32) {
-            u += rk_warp_row<1>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<1>(data1, src1, uniq, s, len, v, value, lane);
         } else if (len <= 64) {
-            u += rk_warp_row<2>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<2>(data1, src1, uniq, s, len, v, value, lane);
         } else if (len <= 128) {
-            u += rk_warp_row<4>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<4>(data1, src1, uniq, s, len, v, value, lane);
         } else if (len <= 256) {
-            u += rk_warp_row<8>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<8>(data1, src1, uniq, s, len, v, value, lane);
         } else if (len <= 512) {
-            u += rk_warp_row<16>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<16>(data1, src1, uniq, s, len, v, value, lane);
         } else if (len <= RK_WARP_MAX) {
-            u += rk_warp_row<32>(data1, src1, uniq, s, len, v, lane);
+            u += rk_warp_row<32>(data1, src1, uniq, s, len, v, value, lane);
         } else if (lane == 0) {
             longs[atomicAdd(nlong, 1u)] = (uint32_t)v;
             uniq[v] = 0;
@@ -403,13 +405,14 @@ __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(con
 
 // One block a listed row (RK_WARP_MAX < length <= RK_BLOCK_MAX); the blocks
 // take the list's rows in turn
-__global__ __launch_bounds__(512) void rk_sort_long_kernel(const uint32_t *__restrict__ start,
+__global__ __launch_bounds__(1024) void rk_sort_long_kernel(const uint32_t *__restrict__ start,
+                                                           const int32_t *__restrict__ values,
                                                            int32_t *__restrict__ data1, int32_t *__restrict__ src1,
                                                            uint32_t *__restrict__ uniq,
                                                            const uint32_t *__restrict__ longs,
                                                            const unsigned int *__restrict__ nlong,
                                                            unsigned long long *__restrict__ distinct) {
-    __shared__ int32_t x[RK_BLOCK_MAX];
+    extern __shared__ int32_t x[];   // RK_BLOCK_MAX values
     __shared__ uint32_t usum;
     const uint32_t t = threadIdx.x, nt = blockDim.x;
     for (uint32_t r = blockIdx.x; r < *nlong; r += gridDim.x) {
@@ -425,7 +428,7 @@ __global__ __launch_bounds__(512) void rk_sort_long_kernel(const uint32_t *__res
         if (u) atomicAdd(&usum, u);
         for (uint32_t i = t; i < len; i += nt) {
             data1[s + i] = x[i];
-            src1[s + i] = (int32_t)v;
+            src1[s + i] = values ? values[v] : (int32_t)v;
         }
         __syncthreads();
         if (t == 0) {
@@ -434,6 +437,18 @@ __global__ __launch_bounds__(512) void rk_sort_long_kernel(const uint32_t *__res
         }
         __syncthreads();
     }
+}
+
+static int launch_sort_long(amj_ctx *ctx, const uint32_t *start, const int32_t *values, int32_t *data1, int32_t *src1,
+                            uint32_t *uniq, const uint32_t *longs, const unsigned int *nlong,
+                            unsigned long long *distinct) {
+    constexpr size_t smem = RK_BLOCK_MAX * sizeof(int32_t);
+    AMJ_CUDA_TRY(cudaFuncSetAttribute(rk_sort_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    note_launch(ctx);
+    rk_sort_long_kernel<<<ctx->num_sms, 1024, smem, ctx->stream>>>(start, values, data1, src1, uniq, longs, nlong,
+                                                                   distinct);
+    AMJ_CUDA_TRY(cudaGetLastError());
+    return AMJ_OK;
 }
 
 // repeated rows present: row v's distinct values move to ustart[v] (a warp a row)
@@ -506,15 +521,13 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
     const unsigned gs = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((nv + RK_SORT_WARPS - 1) / RK_SORT_WARPS,
                                                                            (uint64_t)ctx->num_sms * 8));
     note_launch(ctx);
-    rk_sort_rows_kernel<<<gs, RK_SORT_WARPS * 32, 0, ctx->stream>>>(start.p, nv, out->data1.p, out->src1.p, uniq.p,
+    rk_sort_rows_kernel<<<gs, RK_SORT_WARPS * 32, 0, ctx->stream>>>(start.p, nullptr, nv, out->data1.p, out->src1.p, uniq.p,
                                                                     longs.p, &ctr->nlong, &ctr->distinct);
     AMJ_CUDA_TRY(cudaGetLastError());
     // no row of n edges in rank order is longer than sqrt(2 n) unless edges repeat
     if (n > RK_WARP_MAX) {
-        note_launch(ctx);
-        rk_sort_long_kernel<<<ctx->num_sms, 512, 0, ctx->stream>>>(start.p, out->data1.p, out->src1.p, uniq.p,
-                                                                   longs.p, &ctr->nlong, &ctr->distinct);
-        AMJ_CUDA_TRY(cudaGetLastError());
+        AMJ_TRY(launch_sort_long(ctx, start.p, nullptr, out->data1.p, out->src1.p, uniq.p, longs.p, &ctr->nlong,
+                                 &ctr->distinct));
     }
     // level 0 and the row pointers, unless rows repeat or are too long
     out->len0 = nv;
@@ -550,6 +563,190 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
     AMJ_CUDA_TRY(cudaGetLastError());
     out->data1 = std::move(d1);
     out->src1 = std::move(s1);
+    return AMJ_OK;
+}
+
+// ---- 2-level tries of several relations, rows by counting ----
+// The tries of a triangle query's relations, built together as the ranked trie
+// is: counts per first-column value with each row's place, one scan, one move,
+// one sort of all rows, so that the query has ten launches and two host reads
+// for its builds instead of some hundred and nine (RST_FIGURES).  Level 0 lists every
+// value of the first column's range, which has to be dense (at most 4 n + 4096
+// values); with wider ranges, rows above RK_BLOCK_MAX or repeated rows *built
+// stays false and the caller builds the tries one by one.
+struct TrieJob {
+    const int32_t *c0, *c1;
+    uint32_t n, nrows;   // edges; values of the first column's range
+    uint32_t row0, e0;   // first row and first edge in the shared arrays
+    uint32_t min0;       // least first value (sign flipped)
+    uint64_t *rowptr;
+};
+struct TrieJobs {
+    TrieJob j[TRIE_JOBS_MAX];
+};
+
+// least and greatest value of both columns: mm[0..3] of a relation = ~min0, max0,
+// ~min1, max1, sign flipped (zeros are neutral); one set of atomics a block
+__global__ __launch_bounds__(256) void tries_minmax_kernel(const __grid_constant__ TrieJobs A,
+                                                           uint32_t *__restrict__ mm) {
+    const TrieJob &J = A.j[blockIdx.y];
+    uint32_t m[4] = {0, 0, 0, 0};
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < J.n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t a = (uint32_t)J.c0[i] ^ 0x80000000u, b = (uint32_t)J.c1[i] ^ 0x80000000u;
+        m[0] = max(m[0], ~a);
+        m[1] = max(m[1], a);
+        m[2] = max(m[2], ~b);
+        m[3] = max(m[3], b);
+    }
+    __shared__ uint32_t s[4][8];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        m[k] = __reduce_max_sync(AMJ_FULL_MASK, m[k]);
+        if ((threadIdx.x & 31) == 0) s[k][threadIdx.x >> 5] = m[k];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        uint32_t x = 0;
+        for (int w = 0; w < 8; w++) x = max(x, s[threadIdx.x][w]);
+        atomicMax(&mm[4 * blockIdx.y + threadIdx.x], x);
+    }
+}
+
+__global__ __launch_bounds__(256) void tries_count_kernel(const __grid_constant__ TrieJobs A, uint32_t *__restrict__ cnt,
+                                                          uint32_t *__restrict__ place) {
+    const TrieJob &J = A.j[blockIdx.y];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += gridDim.x * blockDim.x)
+        place[J.e0 + i] = atomicAdd(&cnt[J.row0 + (((uint32_t)J.c0[i] ^ 0x80000000u) - J.min0)], 1u);
+}
+
+__global__ __launch_bounds__(256) void tries_scatter_kernel(const __grid_constant__ TrieJobs A,
+                                                            const uint32_t *__restrict__ start,
+                                                            const uint32_t *__restrict__ place,
+                                                            int32_t *__restrict__ data1) {
+    const TrieJob &J = A.j[blockIdx.y];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += gridDim.x * blockDim.x)
+        data1[start[J.row0 + (((uint32_t)J.c0[i] ^ 0x80000000u) - J.min0)] + place[J.e0 + i]] = J.c1[i];
+}
+
+// level-0 values and row pointers (within the relation's own entries), and the
+// longest row
+__global__ __launch_bounds__(256) void tries_level0_kernel(const __grid_constant__ TrieJobs A,
+                                                           const uint32_t *__restrict__ start,
+                                                           int32_t *__restrict__ data0,
+                                                           unsigned int *__restrict__ longest) {
+    const TrieJob &J = A.j[blockIdx.y];
+    uint32_t m = 0;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v <= J.nrows; v += gridDim.x * blockDim.x) {
+        const uint32_t s = start[J.row0 + v];
+        J.rowptr[v] = s - J.e0;
+        if (v < J.nrows) {
+            data0[J.row0 + v] = (int32_t)((J.min0 + v) ^ 0x80000000u);
+            m = max(m, start[J.row0 + v + 1] - s);
+        }
+    }
+    m = __reduce_max_sync(AMJ_FULL_MASK, m);
+    if ((threadIdx.x & 31) == 0 && m > ld_volatile_u32(longest)) atomicMax(longest, m);
+}
+
+int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf<char> *block, bool *built) {
+    *built = false;
+    if (count < 1 || count > TRIE_JOBS_MAX) return fail(AMJ_EINVAL, "tries: bad count");
+    TrieJobs A{};
+    uint64_t n = 0, nmax = 0;
+    for (int t = 0; t < count; t++) {
+        if (cols[t].n == 0) return AMJ_OK;
+        A.j[t].c0 = cols[t].c0;
+        A.j[t].c1 = cols[t].c1;
+        n += cols[t].n;
+        nmax = std::max(nmax, cols[t].n);
+        if (n >= (1ull << 31)) return AMJ_OK;
+        A.j[t].n = (uint32_t)cols[t].n;
+        A.j[t].e0 = (uint32_t)(n - cols[t].n);
+    }
+    struct Ctr {
+        uint32_t mm[4 * TRIE_JOBS_MAX];
+        unsigned int longest, nlong;
+        unsigned long long distinct;
+    } h;
+    DBuf<Ctr> ctr;
+    AMJ_TRY(ctr.alloc(ctx, 1));
+    AMJ_CUDA_TRY(cudaMemsetAsync(ctr.p, 0, sizeof(Ctr), ctx->stream));
+    const unsigned gx = (unsigned)std::min<uint64_t>((nmax + 255) / 256, (uint64_t)ctx->num_sms * 8);
+    note_launch(ctx);
+    tries_minmax_kernel<<<dim3((unsigned)std::min<uint64_t>(gx, (uint64_t)ctx->num_sms * 2), count), 256, 0,
+                          ctx->stream>>>(A, ctr.p->mm);
+    AMJ_CUDA_TRY(cudaGetLastError());
+    AMJ_TRY(read_back(ctx, &h, ctr.p, sizeof(h)));
+    uint64_t rows = 0;
+    for (int t = 0; t < count; t++) {
+        const uint32_t mn = ~h.mm[4 * t], mx = h.mm[4 * t + 1];
+        out[t].range1 = (uint64_t)(h.mm[4 * t + 3] - ~h.mm[4 * t + 2]) + 1;
+        const uint64_t range = (uint64_t)(mx - mn) + 1;
+        if (range > 4 * cols[t].n + 4096) return AMJ_OK;
+        A.j[t].min0 = mn;
+        A.j[t].nrows = (uint32_t)range;
+        A.j[t].row0 = (uint32_t)rows;
+        rows += range;
+        if (rows >= (1ull << 31)) return AMJ_OK;
+    }
+    // the tries' arrays in one block, the scratch in another
+    auto round = [](uint64_t b) { return (b + 255) / 256 * 256; };
+    const uint64_t b_data1 = round((n + TRIE_LEVEL1_PAD) * 4), b_src1 = round(n * 4), b_data0 = round(rows * 4);
+    uint64_t b_rp = 0;
+    for (int t = 0; t < count; t++) b_rp += round(((uint64_t)A.j[t].nrows + 1) * 8);
+    AMJ_TRY(block->alloc(ctx, b_data1 + b_src1 + b_data0 + b_rp));
+    char *at = block->p;
+    int32_t *data1 = reinterpret_cast<int32_t *>(at), *src1 = reinterpret_cast<int32_t *>(at + b_data1);
+    int32_t *data0 = reinterpret_cast<int32_t *>(at + b_data1 + b_src1);
+    at += b_data1 + b_src1 + b_data0;
+    for (int t = 0; t < count; t++) {
+        A.j[t].rowptr = reinterpret_cast<uint64_t *>(at);
+        at += round(((uint64_t)A.j[t].nrows + 1) * 8);
+    }
+    DBuf<uint32_t> start, place, uniq, longs;
+    AMJ_TRY(start.alloc(ctx, rows + 1));
+    AMJ_TRY(place.alloc(ctx, n));
+    AMJ_TRY(uniq.alloc(ctx, rows));
+    AMJ_TRY(longs.alloc(ctx, n / (RK_WARP_MAX + 1) + 1));
+    AMJ_CUDA_TRY(cudaMemsetAsync(start.p, 0, (rows + 1) * sizeof(uint32_t), ctx->stream));
+    const dim3 grid(gx, count);
+    note_launch(ctx);
+    tries_count_kernel<<<grid, 256, 0, ctx->stream>>>(A, start.p, place.p);
+    AMJ_CUDA_TRY(cudaGetLastError());
+    AMJ_TRY(scan_exclusive_u32(ctx, start.p, start.p, rows + 1, nullptr));
+    note_launch(ctx);
+    tries_scatter_kernel<<<grid, 256, 0, ctx->stream>>>(A, start.p, place.p, data1);
+    note_launch(ctx);
+    tries_level0_kernel<<<grid, 256, 0, ctx->stream>>>(A, start.p, data0, &ctr.p->longest);
+    AMJ_CUDA_TRY(cudaGetLastError());
+    const unsigned gs = (unsigned)std::min<uint64_t>((rows + RK_SORT_WARPS - 1) / RK_SORT_WARPS,
+                                                     (uint64_t)ctx->num_sms * 8);
+    note_launch(ctx);
+    rk_sort_rows_kernel<<<gs, RK_SORT_WARPS * 32, 0, ctx->stream>>>(start.p, data0, rows, data1, src1, uniq.p, longs.p,
+                                                                    &ctr.p->nlong, &ctr.p->distinct);
+    AMJ_CUDA_TRY(cudaGetLastError());
+    if (nmax > RK_WARP_MAX)
+        AMJ_TRY(launch_sort_long(ctx, start.p, data0, data1, src1, uniq.p, longs.p, &ctr.p->nlong, &ctr.p->distinct));
+    AMJ_TRY(read_back(ctx, &h, ctr.p, sizeof(h)));
+    if (h.longest > RK_BLOCK_MAX || h.distinct != n) return AMJ_OK;
+    for (int t = 0; t < count; t++) {
+        // views of the block: no context, so they free nothing
+        Trie2 &o = out[t];
+        const TrieJob &J = A.j[t];
+        o.len0 = J.nrows;
+        o.len1 = J.n;
+        o.data1.p = data1 + J.e0;
+        o.data1.n = J.n;
+        o.src1.p = src1 + J.e0;
+        o.src1.n = J.n;
+        o.data0.p = data0 + J.row0;
+        o.data0.n = J.nrows;
+        o.off0.p = o.rowptr.p = J.rowptr;
+        o.off0.n = o.rowptr.n = (uint64_t)J.nrows + 1;
+        o.rp_min = (int32_t)(J.min0 ^ 0x80000000u);
+        o.rp_count = J.nrows;
+    }
+    *built = true;
     return AMJ_OK;
 }
 
