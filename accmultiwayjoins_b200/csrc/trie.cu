@@ -240,7 +240,7 @@ int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t
 // Repeated rows (adjacent after the sort) are dropped by a compaction pass
 // when there are any.
 constexpr uint32_t RK_WARP_MAX = 1024;
-constexpr uint32_t RK_BLOCK_MAX = 32768;   // 128 KB of shared memory
+constexpr uint32_t RK_BLOCK_MAX = 32768;   // 132 KB of shared memory, padded
 constexpr int RK_SORT_WARPS = 8;
 
 // Ranked edges (the lower rank first), the count of every lower rank, each
@@ -298,33 +298,6 @@ __global__ __launch_bounds__(256) void rk_scatter_kernel(const int32_t *__restri
 #pragma unroll
     for (int k = 0; k < 4; k++)
         if (i0 + k * 256 < n) data1[p[k]] = v[k];
-}
-
-// ascending bitonic sort of the pow2-sized x[0, m) by the threads t of a
-// group of nt, with sync() between stages
-template <class Sync>
-__device__ __forceinline__ void rk_bitonic(int32_t *x, uint32_t m, uint32_t t, uint32_t nt, Sync &&sync) {
-    for (uint32_t k = 2; k <= m; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = t; i < m; i += nt) {
-                const uint32_t p = i ^ j;
-                if (p > i) {
-                    const int32_t a = x[i], b = x[p];
-                    if ((a > b) == ((i & k) == 0)) {
-                        x[i] = b;
-                        x[p] = a;
-                    }
-                }
-            }
-            sync();
-        }
-}
-
-// distinct values of the sorted row x[0, len) (shared memory), counted by a group
-__device__ __forceinline__ uint32_t rk_distinct(const int32_t *x, uint32_t len, uint32_t t, uint32_t nt) {
-    uint32_t u = 0;
-    for (uint32_t i = t; i < len; i += nt) u += (i == 0 || x[i] != x[i - 1]) ? 1u : 0u;
-    return u;
 }
 
 // row v = data1[s, s + len), 32 (E / 2) < len <= 32 E: sorted in place, its
@@ -403,33 +376,86 @@ __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(con
     if (threadIdx.x == 0 && usum) atomicAdd(distinct, (unsigned long long)usum);
 }
 
+// A row of up to 1024 E values sorted by a block of 1024 threads in shared
+// memory: E warps sort 1024 values each in registers, then the runs are merged
+// pairwise, each thread placing E consecutive values of the result (its start
+// in the two runs by the merge path's binary search).  Values sit one word in
+// 33 apart, so that a lane's consecutive values fall in different banks.  (A
+// bitonic network over shared memory took 316 us for the long rows of three
+// 1M-edge R-MAT relations, this 76 us.)
+__device__ __forceinline__ uint32_t rk_pad(uint32_t i) { return i + (i >> 5); }
+
+template <int E>
+__device__ __forceinline__ void rk_block_sort(int32_t *x, const int32_t *__restrict__ row, uint32_t len) {
+    const uint32_t t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (w < E) {
+        int32_t v[32];
+#pragma unroll
+        for (int e = 0; e < 32; e++) {
+            const uint32_t i = w * 1024 + e * 32 + lane;
+            v[e] = i < len ? row[i] : INT32_MAX;
+        }
+        warp_bitonic_sort<32>(v, lane);
+#pragma unroll
+        for (int e = 0; e < 32; e++) x[rk_pad(w * 1024 + lane * 32 + e)] = v[e];
+    }
+    __syncthreads();
+    for (uint32_t width = 1024; width < 1024u * E; width *= 2) {
+        const uint32_t out0 = t * E, base = out0 / (2 * width) * (2 * width), diag = out0 - base;
+        const uint32_t A = base, B = base + width;
+        uint32_t lo = diag > width ? diag - width : 0, hi = min(diag, width);
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (x[rk_pad(A + mid)] <= x[rk_pad(B + diag - 1 - mid)]) lo = mid + 1;
+            else hi = mid;
+        }
+        uint32_t i = lo, j = diag - lo;
+        int32_t v[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const bool a = j >= width || (i < width && x[rk_pad(A + i)] <= x[rk_pad(B + j)]);
+            v[e] = a ? x[rk_pad(A + i)] : x[rk_pad(B + j)];
+            i += a ? 1u : 0u;
+            j += a ? 0u : 1u;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < E; e++) x[rk_pad(out0 + e)] = v[e];
+        __syncthreads();
+    }
+}
+
 // One block a listed row (RK_WARP_MAX < length <= RK_BLOCK_MAX); the blocks
 // take the list's rows in turn
 __global__ __launch_bounds__(1024) void rk_sort_long_kernel(const uint32_t *__restrict__ start,
-                                                           const int32_t *__restrict__ values,
-                                                           int32_t *__restrict__ data1, int32_t *__restrict__ src1,
-                                                           uint32_t *__restrict__ uniq,
-                                                           const uint32_t *__restrict__ longs,
-                                                           const unsigned int *__restrict__ nlong,
-                                                           unsigned long long *__restrict__ distinct) {
-    extern __shared__ int32_t x[];   // RK_BLOCK_MAX values
+                                                            const int32_t *__restrict__ values,
+                                                            int32_t *__restrict__ data1, int32_t *__restrict__ src1,
+                                                            uint32_t *__restrict__ uniq,
+                                                            const uint32_t *__restrict__ longs,
+                                                            const unsigned int *__restrict__ nlong,
+                                                            unsigned long long *__restrict__ distinct) {
+    extern __shared__ int32_t x[];   // RK_BLOCK_MAX values, padded
     __shared__ uint32_t usum;
     const uint32_t t = threadIdx.x, nt = blockDim.x;
     for (uint32_t r = blockIdx.x; r < *nlong; r += gridDim.x) {
         const uint32_t v = longs[r], s = start[v], len = start[v + 1] - s;
         if (len > RK_BLOCK_MAX) continue;   // the host takes the radix build
-        uint32_t m = 64;
-        while (m < len) m <<= 1;
         if (t == 0) usum = 0;
-        for (uint32_t i = t; i < m; i += nt) x[i] = i < len ? data1[s + i] : INT32_MAX;
-        __syncthreads();
-        rk_bitonic(x, m, t, nt, [] { __syncthreads(); });
-        const uint32_t u = rk_distinct(x, len, t, nt);
-        if (u) atomicAdd(&usum, u);
+        if (len <= 2048) rk_block_sort<2>(x, data1 + s, len);
+        else if (len <= 4096) rk_block_sort<4>(x, data1 + s, len);
+        else if (len <= 8192) rk_block_sort<8>(x, data1 + s, len);
+        else if (len <= 16384) rk_block_sort<16>(x, data1 + s, len);
+        else rk_block_sort<32>(x, data1 + s, len);
+        const int32_t value = values ? values[v] : (int32_t)v;
+        uint32_t u = 0;
         for (uint32_t i = t; i < len; i += nt) {
-            data1[s + i] = x[i];
-            src1[s + i] = values ? values[v] : (int32_t)v;
+            const int32_t y = x[rk_pad(i)];
+            u += (i == 0 || y != x[rk_pad(i - 1)]) ? 1u : 0u;
+            data1[s + i] = y;
+            src1[s + i] = value;
         }
+        u = warp_sum(u);
+        if ((t & 31) == 0 && u) atomicAdd(&usum, u);
         __syncthreads();
         if (t == 0) {
             uniq[v] = usum;
@@ -442,7 +468,7 @@ __global__ __launch_bounds__(1024) void rk_sort_long_kernel(const uint32_t *__re
 static int launch_sort_long(amj_ctx *ctx, const uint32_t *start, const int32_t *values, int32_t *data1, int32_t *src1,
                             uint32_t *uniq, const uint32_t *longs, const unsigned int *nlong,
                             unsigned long long *distinct) {
-    constexpr size_t smem = RK_BLOCK_MAX * sizeof(int32_t);
+    constexpr size_t smem = (RK_BLOCK_MAX + RK_BLOCK_MAX / 32) * sizeof(int32_t);
     AMJ_CUDA_TRY(cudaFuncSetAttribute(rk_sort_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     note_launch(ctx);
     rk_sort_long_kernel<<<ctx->num_sms, 1024, smem, ctx->stream>>>(start, values, data1, src1, uniq, longs, nlong,
@@ -524,8 +550,11 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
     rk_sort_rows_kernel<<<gs, RK_SORT_WARPS * 32, 0, ctx->stream>>>(start.p, nullptr, nv, out->data1.p, out->src1.p, uniq.p,
                                                                     longs.p, &ctr->nlong, &ctr->distinct);
     AMJ_CUDA_TRY(cudaGetLastError());
-    // no row of n edges in rank order is longer than sqrt(2 n) unless edges repeat
-    if (n > RK_WARP_MAX) {
+    // in rank order a row holds about sqrt(2 n) values at most unless edges
+    // repeat: small relations launch the block sort only when they turn out to
+    // need it
+    const bool long_rows = n >= (1u << 18);
+    if (long_rows) {
         AMJ_TRY(launch_sort_long(ctx, start.p, nullptr, out->data1.p, out->src1.p, uniq.p, longs.p, &ctr->nlong,
                                  &ctr->distinct));
     }
@@ -544,6 +573,11 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
     AMJ_CUDA_TRY(cudaGetLastError());
     Ctr h{};
     AMJ_TRY(read_back(ctx, &h, ctr, sizeof(h)));
+    if (!long_rows && h.nlong && h.longest <= RK_BLOCK_MAX) {
+        AMJ_TRY(launch_sort_long(ctx, start.p, nullptr, out->data1.p, out->src1.p, uniq.p, longs.p, &ctr->nlong,
+                                 &ctr->distinct));
+        AMJ_TRY(read_back(ctx, &h, ctr, sizeof(h)));
+    }
     if (h.longest > RK_BLOCK_MAX) {
         *out = Trie2();
         return build_trie2(ctx, lo.p, hi.p, n, out, true, (int32_t)(nv - 1));
@@ -570,7 +604,8 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
 // The tries of a triangle query's relations, built together as the ranked trie
 // is: counts per first-column value with each row's place, one scan, one move,
 // one sort of all rows, so that the query has ten launches and two host reads
-// for its builds instead of some hundred and nine (RST_FIGURES).  Level 0 lists every
+// for its builds instead of some hundred and nine (three relations of 1M edges:
+// 1.03 ms one by one, 0.36 ms together).  Level 0 lists every
 // value of the first column's range, which has to be dense (at most 4 n + 4096
 // values); with wider ranges, rows above RK_BLOCK_MAX or repeated rows *built
 // stays false and the caller builds the tries one by one.
@@ -612,11 +647,41 @@ __global__ __launch_bounds__(256) void tries_minmax_kernel(const __grid_constant
     }
 }
 
+// One tile of edges a block.  The first TRIES_SMEM_ROWS rows, where generators
+// and real graphs put their hubs, are counted in shared memory and reach the
+// global count once a block: a hub's atomics do not queue on one address (3M
+// edges of three R-MAT relations: 106 us with global counts only, 37 us now).
+constexpr uint32_t TRIES_SMEM_ROWS = 4096;
+constexpr int TRIES_PER_THREAD = 16;
+
 __global__ __launch_bounds__(256) void tries_count_kernel(const __grid_constant__ TrieJobs A, uint32_t *__restrict__ cnt,
                                                           uint32_t *__restrict__ place) {
+    __shared__ uint32_t h[TRIES_SMEM_ROWS];
     const TrieJob &J = A.j[blockIdx.y];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < J.n; i += gridDim.x * blockDim.x)
-        place[J.e0 + i] = atomicAdd(&cnt[J.row0 + (((uint32_t)J.c0[i] ^ 0x80000000u) - J.min0)], 1u);
+    const uint32_t i0 = blockIdx.x * (256u * TRIES_PER_THREAD);
+    if (i0 >= J.n) return;
+    for (uint32_t i = threadIdx.x; i < TRIES_SMEM_ROWS; i += 256) h[i] = 0;
+    __syncthreads();
+    uint32_t row[TRIES_PER_THREAD], p[TRIES_PER_THREAD];
+#pragma unroll
+    for (int k = 0; k < TRIES_PER_THREAD; k++) {
+        const uint32_t i = i0 + k * 256 + threadIdx.x;
+        row[k] = i < J.n ? ((uint32_t)J.c0[i] ^ 0x80000000u) - J.min0 : 0xffffffffu;
+    }
+#pragma unroll
+    for (int k = 0; k < TRIES_PER_THREAD; k++) {
+        if (row[k] < TRIES_SMEM_ROWS) p[k] = atomicAdd(&h[row[k]], 1u);
+        else if (row[k] != 0xffffffffu) p[k] = atomicAdd(&cnt[J.row0 + row[k]], 1u);
+    }
+    __syncthreads();
+    // h[row] becomes the block's first place in the row
+    for (uint32_t i = threadIdx.x; i < TRIES_SMEM_ROWS; i += 256)
+        if (h[i]) h[i] = atomicAdd(&cnt[J.row0 + i], h[i]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < TRIES_PER_THREAD; k++)
+        if (row[k] != 0xffffffffu)
+            place[J.e0 + i0 + k * 256 + threadIdx.x] = p[k] + (row[k] < TRIES_SMEM_ROWS ? h[row[k]] : 0u);
 }
 
 __global__ __launch_bounds__(256) void tries_scatter_kernel(const __grid_constant__ TrieJobs A,
@@ -711,7 +776,8 @@ int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf
     AMJ_CUDA_TRY(cudaMemsetAsync(start.p, 0, (rows + 1) * sizeof(uint32_t), ctx->stream));
     const dim3 grid(gx, count);
     note_launch(ctx);
-    tries_count_kernel<<<grid, 256, 0, ctx->stream>>>(A, start.p, place.p);
+    tries_count_kernel<<<dim3((unsigned)((nmax + 256 * TRIES_PER_THREAD - 1) / (256 * TRIES_PER_THREAD)), count), 256, 0,
+                         ctx->stream>>>(A, start.p, place.p);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(scan_exclusive_u32(ctx, start.p, start.p, rows + 1, nullptr));
     note_launch(ctx);

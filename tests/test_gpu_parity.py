@@ -1355,3 +1355,30 @@ def test_star_heads(dims, copies, keys):
         for plan in ("multiway", "frontier"):
             got = ctx.amhj("NORMAL", rs, plan=plan)
             assert (got.count, got.checksum) == want
+
+
+@pytest.mark.parametrize("deg", [1024, 1025, 2048, 2049, 8193, 32768, 32769])
+@pytest.mark.parametrize("shape", ["three", "repeated"])
+def test_trie_rows_around_the_block_sort(ctx, deg, shape):
+    """Rows at the limits of the warp sort, of each block sort and past the
+    longest: hubs of three relations (small negative and large values), and a
+    self-join whose hub row is long because its edges repeat."""
+    rng = np.random.default_rng(deg)
+    if shape == "three":
+        hub = rng.permutation(np.arange(-(1 << 30), -(1 << 30) + 3 * deg, 3)[:deg])
+        x, y = data.rmat(7, 600, 0.57, 0.19, 0.19, deg)
+        r = (np.concatenate([np.full(40, -5), x]), np.concatenate([np.arange(40), y]))
+        s_ = (np.concatenate([np.full(deg, 3), x]), np.concatenate([hub, y]))
+        t = (np.concatenate([np.full(deg, -5), x]), np.concatenate([hub, y]))
+        rels = [([a.astype(np.int32), b.astype(np.int32)], at) for (a, b), at in ((r, [0, 1]), (s_, [1, 2]), (t, [0, 2]))]
+        rels = [([c[0][p], c[1][p]], at) for c, at in rels for p in [rng.permutation(len(c[0]))]]
+        uniq = [([u[:, 0].copy(), u[:, 1].copy()], at) for (c, at) in rels for u in [np.unique(np.stack(c, 1), axis=0)]]
+        want = O.mhj(uniq)
+        got = ctx.lftj(rels_on(ctx, rels))
+        assert want[0] > deg
+    else:
+        s, d = data.rmat(8, 3000, 0.57, 0.19, 0.19, deg)
+        want = O.triangle(s, d)
+        s, d = np.concatenate([s, np.repeat(s[:1], deg)]), np.concatenate([d, np.repeat(d[:1], deg)])
+        got = ctx.lftj([ctx.relation([s, d], [0, 1])])
+    assert (got.count, got.checksum) == want
