@@ -288,7 +288,8 @@ static int run_passes(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws, bo
 
 // Count mode of a star or canonical chain plan (amhj_star.cuh): the flat
 // kernel, then the DFS kernel over the rows that were too much work for one
-// thread (a star's match product, a chain walk's bucket rows).
+// thread (a star's match product, a chain's bucket rows) and over a chain's
+// matches that were.
 static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws, uint64_t row_lo, uint64_t row_hi,
                           PassResult *pr, amj_result *res) {
     ProbePlan &P = PL.P;
@@ -318,9 +319,12 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
         nheads = 0;
     }
     // one block: the heads (read by 256-bit loads, which need 32-byte
-    // alignment), the counters, the list of rows left for the DFS kernel
+    // alignment), the counters, the list of rows left for the DFS kernel and,
+    // for a chain of two or more levels, that of matches left for it
     DBuf<char> work;
-    AMJ_TRY(work.alloc(ctx, nheads * sizeof(BucketHead) + 256 + std::max<uint64_t>(rows, 1) * sizeof(uint32_t)));
+    const uint64_t over_bytes = (std::max<uint64_t>(rows, 1) * sizeof(uint32_t) + 255) / 256 * 256;
+    const uint32_t pair_cap = chain && canon > 1 ? (uint32_t)std::min<uint64_t>(rows, 1u << 24) : 0u;
+    AMJ_TRY(work.alloc(ctx, nheads * sizeof(BucketHead) + 256 + over_bytes + (uint64_t)pair_cap * sizeof(uint2)));
     if (reinterpret_cast<uintptr_t>(work.p) % alignof(BucketHead) != 0 && canon) {
         if (chain) return run_passes(ctx, PL, X, ws, false, false, row_lo, row_hi, pr, res, false);
         canon = 0;
@@ -329,6 +333,7 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     FlatCtr *ctr = reinterpret_cast<FlatCtr *>(heads + nheads);
     FlatCtr *host = static_cast<FlatCtr *>(ctx->h_small);
     uint32_t *over = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(ctr) + 256);
+    uint2 *pairs = reinterpret_cast<uint2 *>(reinterpret_cast<char *>(over) + over_bytes);
     static_assert(sizeof(FlatCtr) <= BUCKET_ZEROED && sizeof(FlatCtr) <= READ_BACK_MAX, "the counters' places");
     if (X.zeroed) {
         ctr = static_cast<FlatCtr *>(X.zeroed);   // cleared with the bucket counts
@@ -361,12 +366,12 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     note_launch(ctx);
     if (chain) {
         switch (canon) {
-        case 1: amhj_chain_canon_kernel<1><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
-        case 2: amhj_chain_canon_kernel<2><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
-        case 3: amhj_chain_canon_kernel<3><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
-        case 4: amhj_chain_canon_kernel<4><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
-        case 5: amhj_chain_canon_kernel<5><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
-        default: amhj_chain_canon_kernel<6><<<g ? g : 1, 256, 0, ctx->stream>>>(S, ctr, host, over);
+        case 1: amhj_chain_canon_kernel<1><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over, pairs, pair_cap); break;
+        case 2: amhj_chain_canon_kernel<2><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over, pairs, pair_cap); break;
+        case 3: amhj_chain_canon_kernel<3><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over, pairs, pair_cap); break;
+        case 4: amhj_chain_canon_kernel<4><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over, pairs, pair_cap); break;
+        case 5: amhj_chain_canon_kernel<5><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over, pairs, pair_cap); break;
+        default: amhj_chain_canon_kernel<6><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over, pairs, pair_cap);
         }
     } else switch (canon) {
     case 1: amhj_star_canon_kernel<1><<<gs, 256, 0, ctx->stream>>>(S, ctr, host, over); break;
@@ -382,7 +387,35 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     res->kernel_ms[0] += event_ms(kb, ke);
     pr->count = h.count;
     pr->checksum = h.checksum;
-    X.ended = X.end && h.nover == 0;
+    X.ended = X.end && h.nover == 0 && h.npair == 0;
+    // more matches than the list holds: the whole query by the DFS kernel
+    if (h.npair > pair_cap) return run_passes(ctx, PL, X, true, false, false, row_lo, row_hi, pr, res, false);
+    if (h.npair) {
+        // the listed matches, joined with the levels after the first (below:
+        // with work sharing, as the listed rows)
+        DBuf<int32_t> c;
+        AMJ_TRY(c.alloc(ctx, 3 * (uint64_t)h.npair));
+        int32_t *c0 = c.p, *c1 = c0 + h.npair, *c2 = c1 + h.npair;
+        note_launch(ctx);
+        chain_gather_kernel<<<(unsigned)std::min<uint64_t>((h.npair + 255) / 256, (uint64_t)ctx->num_sms * 8), 256, 0,
+                              ctx->stream>>>(S, pairs, h.npair, c0, c1, c2);
+        AMJ_CUDA_TRY(cudaGetLastError());
+        ProbeLaunch sub = PL;
+        sub.P.L = (int8_t)(P.L - 1);
+        for (int l = 0; l < sub.P.L; l++) sub.P.lv[l] = P.lv[l + 1];
+        sub.P.probe_ncols = 3;
+        int32_t *cols[3] = {c0, c1, c2};
+        for (int a = 0; a < 3; a++) {
+            sub.P.probe_col[a] = cols[a];
+            sub.P.probe_attr[a] = (int8_t)a;
+        }
+        sub.P.warp_bytes = (uint32_t)sub.P.L * sub.P.depth_bytes;
+        plan_inline(sub.P);
+        PassResult rest;
+        AMJ_TRY(run_passes(ctx, sub, X, true, false, false, 0, h.npair, &rest, res, false));
+        pr->count += rest.count;
+        pr->checksum += rest.checksum;
+    }
     if (h.nover == 0) return AMJ_OK;
     // the listed rows, gathered into a probe relation of their own
     std::vector<DBuf<int32_t>> cols(P.probe_ncols);

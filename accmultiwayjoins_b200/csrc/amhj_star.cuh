@@ -39,6 +39,7 @@ inline bool star_eligible(const ProbePlan &P) {
 struct FlatCtr {
     unsigned long long count, checksum;
     unsigned int nover, done;   // listed rows; blocks that have ended
+    unsigned int npair, pad;    // chain: listed matches
 };
 
 // A block's count and checksum added to the totals: one atomic a block, since
@@ -68,6 +69,7 @@ __device__ __forceinline__ void flat_totals(unsigned long long cnt, unsigned lon
             host->count = atomicAdd(&ctr->count, 0ull);
             host->checksum = atomicAdd(&ctr->checksum, 0ull);
             host->nover = atomicAdd(&ctr->nover, 0u);
+            host->npair = atomicAdd(&ctr->npair, 0u);
             __threadfence_system();
         }
     }
@@ -369,15 +371,23 @@ __global__ __launch_bounds__(256, star_blocks(L)) void amhj_star_canon_kernel(co
     flat_totals(cnt, chk, ctr, host);
 }
 
-// ---- the canonical chain, count mode: a depth-first walk in registers ----
+// ---- the canonical chain, count mode: bucket rows handed out to lanes ----
 // The shape of the reference's chain benchmarks: probe R0(0, 1) and levels
 // R_d(d + 1, d + 2), level d looked up by the payload of level d - 1 (by
-// attribute 1 at d = 0).  One thread walks one probe row's matches depth
-// first, each level's lookup one bucket head (its bounds and first rows) and
-// the tuple hash extended by one step a level, so a tuple costs one step at
-// the last level.  A row whose walk would scan more than CHAIN_ROW_BUDGET
-// bucket rows (skewed keys) drops what it counted and is listed for the DFS
-// kernel, which shares such work across warps.
+// attribute 1 at d = 0).  A warp looks up 32 probe rows, one a lane, stages the
+// bucket heads (bounds and first rows) in shared memory and hands the buckets'
+// rows out one a lane; with two levels the matches' buckets are handed out the
+// same way, with more each lane walks its match's further levels depth first, a
+// head a lookup.  The tuple hash is extended by one step a level, so a tuple
+// costs one step at the last level.
+// Bound by instructions: a walk of a probe row a lane kept 8.7 of 32 lanes
+// active, since the rows' walks differ in length.  Measured, 3 x 1M rows,
+// 14.6 M tuples: 165 us so, 126 with the first level handed out, 100 with
+// both (and six blocks an SM).  Two or four matches a lane at a time, for more
+// loads in flight: 129 and 164 us.
+// A probe row whose first bucket, or a match whose further levels, hold more
+// than CHAIN_ROW_BUDGET bucket rows (skewed keys) count nothing and are listed
+// for the DFS kernel, which shares such work across warps.
 constexpr uint32_t CHAIN_ROW_BUDGET = 128;
 
 // L when plan P has the canonical chain shape (filling S but the heads), else 0
@@ -389,7 +399,7 @@ inline int chain_canon(const ProbePlan &P, CanonPlan &S) {
     for (int l = 0; l < L; l++) {
         const LevelDesc &lv = P.lv[l];
         const int d = lv.key_attr[0] - 1;
-        if (d < 0 || d >= L || seen[d] || lv.layout != AMJ_LAYOUT_BUCKET || lv.key_mode != KEY_SINGLE ||
+        if (d != l || seen[d] || lv.layout != AMJ_LAYOUT_BUCKET || lv.key_mode != KEY_SINGLE ||
             lv.cmp_mask != 1u || lv.ncols != 2 || lv.attr[0] != d + 1 || lv.attr[1] != d + 2)
             return 0;
         seen[d] = true;
@@ -437,26 +447,128 @@ __device__ __forceinline__ bool chain_walk(const CanonPlan &S, int32_t key, uint
     return true;
 }
 
-// four blocks per SM (64 registers) up to three levels; deeper walks keep
-// their per-level state in two blocks' worth of registers
+// rows of up to 32 buckets, waiting to be handed out
+struct ChainStage {
+    unsigned long long hv[32];           // hash of the partial tuple
+    int4 ent[32];                        // rows before the bucket's, bucket start, key, probe row
+    int2 kp[HEAD_ROWS][32];              // the bucket's first rows
+};
+
+// The whole warp: lane's bucket of level d (head w, n rows, possibly none) was
+// looked up by `key` from a partial tuple of hash hv; f(hit, row, payload, hash)
+// is called by all lanes together, a bucket row a lane.
+template <class F>
+__device__ __forceinline__ void chain_spread(const CanonPlan &S, int d, ChainStage &W, int lane, uint32_t n,
+                                             const uint32_t (&w)[8], int32_t key, unsigned long long hv, uint32_t row,
+                                             F &&f) {
+    const unsigned lt = lanemask_lt(), le = lt | (1u << lane);
+    const uint32_t incl = warp_inclusive_scan(n, lane), excl = incl - n;
+    const uint32_t tot = __shfl_sync(AMJ_FULL_MASK, incl, 31);
+    const unsigned live = __ballot_sync(AMJ_FULL_MASK, n > 0);
+    if (n) {
+        const int at = __popc(live & lt);
+        W.hv[at] = hv;
+        W.ent[at] = make_int4((int)excl, (int)w[0], key, (int)row);
+#pragma unroll
+        for (int i = 0; i < HEAD_ROWS; i++) W.kp[i][at] = make_int2((int)w[2 + 2 * i], (int)w[3 + 2 * i]);
+    }
+    __syncwarp();
+    int before = -1;   // buckets begun before this step, minus one
+    for (uint32_t j0 = 0; j0 < tot; j0 += 32) {
+        const unsigned begun = __reduce_or_sync(AMJ_FULL_MASK, n && excl - j0 < 32u ? 1u << (excl - j0) : 0u);
+        const int o = before + __popc(begun & le);
+        before += __popc(begun);
+        const uint32_t j = j0 + lane;
+        int2 kv = make_int2(0, 0);
+        int4 e = make_int4(0, 0, 1, 0);
+        if (j < tot) {
+            e = W.ent[o];
+            const uint32_t i = j - (uint32_t)e.x;
+            if (i < (uint32_t)HEAD_ROWS) kv = W.kp[i][o];
+            else kv = make_int2(S.key[d][(uint32_t)e.y + i], S.pay[d][(uint32_t)e.y + i]);
+        }
+        const bool hit = j < tot && kv.x == e.z;
+        f(hit, (uint32_t)e.w, kv.y, hit ? amj_hash_step(W.hv[o], kv.y) : 0ull);
+    }
+    __syncwarp();
+}
+
+// six blocks per SM (40 registers) up to two levels (1M rows: 100 us; four blocks
+// 116, eight 120), four (64 registers) at three; deeper walks keep their
+// per-level state in two blocks' worth of registers
 template <int L>
-__global__ __launch_bounds__(256, L <= 3 ? 4 : 2) void amhj_chain_canon_kernel(const __grid_constant__ CanonPlan S,
-                                                               FlatCtr *ctr, FlatCtr *host, uint32_t *over) {
+__global__ __launch_bounds__(256, L <= 2 ? 6 : L <= 3 ? 4 : 2) void amhj_chain_canon_kernel(
+    const __grid_constant__ CanonPlan S, FlatCtr *ctr, FlatCtr *host, uint32_t *over, uint2 *pairs,
+    uint32_t pair_cap) {
+    __shared__ ChainStage smem[L == 2 ? 2 : 1][8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     unsigned long long cnt = 0, chk = 0;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t r = S.row_lo + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < S.row_hi; r += stride) {
-        const int32_t a0 = __ldcs(S.fact[0] + r), a1 = __ldcs(S.fact[1] + r);
-        const uint64_t h = amj_hash_step(amj_hash_step(AMJ_CHECKSUM_SEED, a0), a1);
-        unsigned long long rc = 0, rchk = 0;
-        uint32_t budget = CHAIN_ROW_BUDGET;
-        if (chain_walk<0, L>(S, a1, h, rc, rchk, budget)) {
-            cnt += rc;
-            chk += rchk;
-        } else {
-            over[atomicAdd(&ctr->nover, 1u)] = (uint32_t)(r - S.row_lo);
+    // a match whose walk is too long for a lane
+    auto list = [&](uint32_t row, int32_t v) {
+        if (*(volatile unsigned int *)&ctr->npair > pair_cap) return;   // so that the count cannot wrap
+        const uint32_t at = atomicAdd(&ctr->npair, 1u);
+        if (at < pair_cap) pairs[at] = make_uint2(row, (uint32_t)v);
+    };
+    for (uint64_t base = S.row_lo + blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < S.row_hi;
+         base += stride) {
+        const uint64_t r = base + lane;
+        uint32_t n = 0, w[8] = {};
+        int32_t a0 = 0, a1 = 0;
+        if (r < S.row_hi) {
+            a0 = __ldcs(S.fact[0] + r);
+            a1 = __ldcs(S.fact[1] + r);
+            load_head(S.head[0] + ((uint32_t)a1 & S.mask[0]), w);
+            n = w[1] - w[0];
+            if (n > CHAIN_ROW_BUDGET) {
+                over[atomicAdd(&ctr->nover, 1u)] = (uint32_t)(r - S.row_lo);
+                n = 0;
+            }
         }
+        chain_spread(S, 0, smem[0][wid], lane, n, w, a1, amj_hash_step(amj_hash_step(AMJ_CHECKSUM_SEED, a0), a1),
+                     (uint32_t)(r - S.row_lo), [&](bool hit, uint32_t row, int32_t v, unsigned long long h) {
+            if constexpr (L == 1) {
+                cnt += hit;
+                chk += h;
+            } else if constexpr (L == 2) {
+                uint32_t n1 = 0, w1[8] = {};
+                if (hit) {
+                    load_head(S.head[1] + ((uint32_t)v & S.mask[1]), w1);
+                    n1 = w1[1] - w1[0];
+                    if (n1 > CHAIN_ROW_BUDGET) {
+                        list(row, v);
+                        n1 = 0;
+                    }
+                }
+                chain_spread(S, 1, smem[1][wid], lane, n1, w1, v, h, 0,
+                             [&](bool hit1, uint32_t, int32_t, unsigned long long h1) {
+                    cnt += hit1;
+                    chk += h1;
+                });
+            } else if (hit) {
+                unsigned long long rc = 0, rchk = 0;
+                uint32_t budget = CHAIN_ROW_BUDGET;
+                if (chain_walk<1, L>(S, v, h, rc, rchk, budget)) {
+                    cnt += rc;
+                    chk += rchk;
+                } else {
+                    list(row, v);
+                }
+            }
+        });
     }
     flat_totals(cnt, chk, ctr, host);
+}
+
+// the listed matches as a probe relation (0, 1, 2) of the remaining levels
+__global__ void chain_gather_kernel(const __grid_constant__ CanonPlan S, const uint2 *__restrict__ pairs, uint32_t n,
+                                    int32_t *__restrict__ c0, int32_t *__restrict__ c1, int32_t *__restrict__ c2) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 p = pairs[i];
+        c0[i] = S.fact[0][S.row_lo + p.x];
+        c1[i] = S.fact[1][S.row_lo + p.x];
+        c2[i] = (int32_t)p.y;
+    }
 }
 
 // ---- materialised star joins (two flat passes) ----

@@ -408,6 +408,32 @@ def test_amhj_chain_flat_walk_and_listed_rows(ctx, nlev):
     assert (got.count, got.checksum) == O.mhj(other)
 
 
+@pytest.mark.parametrize("nlev", [2, 3])
+@pytest.mark.parametrize("nprobe", [1, 31, 32, 300])
+@pytest.mark.parametrize("hot", [1, 2, 400])
+def test_amhj_chain_listed_matches(ctx, nlev, nprobe, hot):
+    """A chain's matches whose next bucket is longer than a lane walks (more
+    than 128 rows) are listed and joined from level 1 on: a few of them, or
+    more than the list holds (as many as the probe has rows), which joins the
+    query by the DFS kernel; buckets of 128 rows are still walked."""
+    rng = np.random.Generator(np.random.PCG64(70 + nlev))
+    rels = [([np.arange(nprobe, dtype=np.int32), rng.integers(0, 40, nprobe).astype(np.int32)], [0, 1])]
+    rels.append(([rng.integers(0, 40, 1600).astype(np.int32), rng.integers(0, 402, 1600).astype(np.int32)], [1, 2]))
+    heavy = np.repeat(np.arange(hot), 129 if hot < 400 else 130)
+    keys = np.concatenate([heavy, np.repeat(np.arange(400, 402), 128), rng.integers(hot, 400, 300) if hot < 400 else
+                           heavy[:0]]).astype(np.int32)
+    rels.append(([keys, rng.integers(0, 4000, len(keys)).astype(np.int32)], [2, 3]))
+    if nlev == 3:
+        rels.append(([rng.integers(0, 4000, 2000).astype(np.int32), rng.integers(0, 9, 2000).astype(np.int32)], [3, 4]))
+    want = O.mhj(rels)
+    hs = [ctx.relation(c, a) for c, a in rels]
+    for ws in (0, 1):
+        got = ctx.amhj("NORMAL", hs, ws=ws)
+        assert (got.count, got.checksum) == want, ws
+    got = ctx.amhj("NORMAL", hs, plan="frontier")
+    assert (got.count, got.checksum) == want
+
+
 @pytest.mark.parametrize("qt", ["TRI", "FOUR"])
 @pytest.mark.parametrize("reorder", [True, False])
 @pytest.mark.parametrize("degree_order", [True, False])
