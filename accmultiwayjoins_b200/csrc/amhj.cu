@@ -259,7 +259,7 @@ int finish_result_columns(amj_ctx *ctx, amj_result *res, int flags) {
     const cudaError_t es = cudaStreamSynchronize(ctx->stream);   // also before the block can go back
     if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) {
-        result_block_put(ctx, block, size);
+        result_block_put(*ctx->result_pool, block, size);
         return cuda_fail(e, "result: copy to host memory");
     }
     for (int a = 0; a < (int)res->num_attrs; a++) {
@@ -268,6 +268,7 @@ int finish_result_columns(amj_ctx *ctx, amj_result *res, int flags) {
         res->cols[a] = host[a];
     }
     o->host_block = block;
+    o->host_pool = ctx->result_pool;
     o->host_bytes = size;
     res->on_host = 1;
     return AMJ_OK;

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 #include "amj.h"
@@ -12,6 +13,8 @@
 #define AMJ_FULL_MASK 0xffffffffu
 
 namespace amj {
+
+struct ResultPool;   // runtime.cu
 
 int cuda_fail(cudaError_t e, const char *what);
 
@@ -173,7 +176,7 @@ struct amj_ctx {
     void *c4_mtx = nullptr;                // 4-clique triangle matrices, kept across calls (grow-only)
     uint64_t c4_mtx_words = 0;
     void *pinned_cache = nullptr;          // pinned host blocks of out-of-core stages, kept across calls
-    void *result_pool = nullptr;           // pinned blocks of host results, kept across calls
+    std::shared_ptr<amj::ResultPool> result_pool;   // pinned blocks of host results, kept across calls
 };
 
 struct amj_rel {
@@ -204,7 +207,7 @@ void pinned_cache_release(amj_ctx *ctx);
 // Results may be released by any thread.
 constexpr size_t RESULT_POOL_MAX = 256ull << 20;
 int result_block_get(amj_ctx *ctx, size_t bytes, void **p, size_t *size);
-void result_block_put(amj_ctx *ctx, void *p, size_t size);
+void result_block_put(ResultPool &pool, void *p, size_t size) noexcept;
 
 template <typename T>
 struct DBuf {

@@ -5,7 +5,10 @@
 
 struct ResultOwner {
     amj_ctx *ctx = nullptr;
-    void *host_block = nullptr;   // pinned block of all host columns, back to the context's pool on release
+    // pinned block of all host columns, back to the context's pool on release
+    // (a result may outlive its context, whose pool then keeps no block)
+    void *host_block = nullptr;
+    std::shared_ptr<amj::ResultPool> host_pool;
     size_t host_bytes = 0;
 };
 

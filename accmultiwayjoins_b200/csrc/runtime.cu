@@ -62,12 +62,15 @@ int read_back(amj_ctx *ctx, void *dst, const void *d_src, size_t bytes) {
 struct ResultPool {
     std::mutex mu;
     std::multimap<size_t, void *> blocks;   // by size
-    size_t bytes = 0;
+    size_t bytes = 0, limit = RESULT_POOL_MAX;   // limit 0: the context is gone
+    ~ResultPool() {
+        for (auto &b : blocks) (void)cudaFreeHost(b.second);
+    }
 };
 
 int result_block_get(amj_ctx *ctx, size_t bytes, void **p, size_t *size) {
     const size_t want = (std::max<size_t>(bytes, 1) + 65535) / 65536 * 65536;
-    auto *pool = static_cast<ResultPool *>(ctx->result_pool);
+    ResultPool *pool = ctx->result_pool.get();
     {
         std::lock_guard<std::mutex> lk(pool->mu);
         auto it = pool->blocks.lower_bound(want);
@@ -87,23 +90,24 @@ int result_block_get(amj_ctx *ctx, size_t bytes, void **p, size_t *size) {
     return AMJ_OK;
 }
 
-void result_block_put(amj_ctx *ctx, void *p, size_t size) {
-    auto *pool = static_cast<ResultPool *>(ctx->result_pool);
-    {
-        std::lock_guard<std::mutex> lk(pool->mu);
-        if (pool->bytes + size <= RESULT_POOL_MAX) {
-            pool->bytes += size;
-            pool->blocks.emplace(size, p);
+void result_block_put(ResultPool &pool, void *p, size_t size) noexcept {
+    try {
+        std::lock_guard<std::mutex> lk(pool.mu);
+        if (pool.bytes + size <= pool.limit) {
+            pool.blocks.emplace(size, p);
+            pool.bytes += size;
             return;
         }
+    } catch (...) {   // no memory for the entry: give the block back
     }
     (void)cudaFreeHost(p);
 }
 
-static void result_pool_clear(amj_ctx *ctx) {
-    auto *pool = static_cast<ResultPool *>(ctx->result_pool);
+static void result_pool_clear(amj_ctx *ctx, bool closing = false) {
+    ResultPool *pool = ctx->result_pool.get();
     if (!pool) return;
     std::lock_guard<std::mutex> lk(pool->mu);
+    if (closing) pool->limit = 0;
     for (auto &b : pool->blocks) (void)cudaFreeHost(b.second);
     pool->blocks.clear();
     pool->bytes = 0;
@@ -194,7 +198,7 @@ extern "C" int amj_ctx_create(int device, const amj_opts *opts, amj_ctx **out) {
     AMJ_CUDA_TRY(cudaSetDevice(device));
     auto *c = new amj_ctx();
     c->device = device;
-    c->result_pool = new ResultPool();
+    c->result_pool = std::make_shared<ResultPool>();
     if (opts) c->opts = *opts;
     if (c->opts.block_size <= 0) c->opts.block_size = 256;
     if (c->opts.load_factor <= 0.f || c->opts.load_factor >= 1.f) c->opts.load_factor = 0.5f;
@@ -252,8 +256,7 @@ extern "C" void amj_ctx_destroy(amj_ctx *c) {
     if (c->h_status) (void)cudaFreeHost(c->h_status);
     if (c->c4_mtx) (void)cudaFree(c->c4_mtx);
     amj::pinned_cache_release(c);
-    result_pool_clear(c);
-    delete static_cast<ResultPool *>(c->result_pool);
+    result_pool_clear(c, true);
     if (c->own_stream && c->stream) (void)cudaStreamDestroy(c->stream);
     (void)cudaGetLastError();
     delete c;
@@ -399,14 +402,14 @@ extern "C" void amj_result_release(amj_result *res) {
     if (!res) return;
     auto *o = (ResultOwner *)res->priv;
     if (o) {
-        if (o->ctx) (void)cudaSetDevice(o->ctx->device);
+        if (o->ctx && !res->on_host) (void)cudaSetDevice(o->ctx->device);
         for (int a = 0; a < AMJ_MAX_ATTRS; a++) {
             if (!res->cols[a]) continue;
             if (res->on_host && o->host_block) continue;   // columns of the block below
             if (res->on_host) (void)cudaFreeHost(res->cols[a]);
             else if (o->ctx) dev_free(o->ctx, res->cols[a]);
         }
-        if (o->host_block) result_block_put(o->ctx, o->host_block, o->host_bytes);
+        if (o->host_block) result_block_put(*o->host_pool, o->host_block, o->host_bytes);
         if (o->ctx && !res->on_host) (void)cudaStreamSynchronize(o->ctx->stream);
         delete o;
     }

@@ -1327,6 +1327,27 @@ def test_host_results_reuse_blocks(rows):
         assert all(g.flags.writeable and g.dtype == np.int32 for g in got)
 
 
+def test_host_result_outlives_its_context():
+    """A host result released after its context: its block goes back to the
+    driver, not to the context's pool."""
+    import ctypes as C
+    from accmultiwayjoins_b200 import _lib as L
+    ctx = Context(0)
+    fact, dim = [data.uniform(5000, 0, 50, 1)], [data.permutation(50, 2), data.uniform(50, 0, 1 << 30, 3)]
+    rels = [ctx.relation(fact, [0]), ctx.relation(dim, [0, 1])]
+    arr = (C.c_void_p * 2)(*[r.handle for r in rels])
+    res = L.amj_result()
+    L.check(L.load().amj_amhj_execute(ctx.handle, L.AMJ_QUERY_NORMAL, arr, 2, 0, 0, 0, 0,
+                                      L.AMJ_F_MATERIALIZE | L.AMJ_F_HOST_RESULT, C.byref(res)), "amhj_execute")
+    ctx.close()
+    cols = [np.empty(5000, np.int32) for _ in range(2)]
+    dst = (C.POINTER(C.c_int32) * 2)(*[c.ctypes.data_as(C.POINTER(C.c_int32)) for c in cols])
+    L.check(L.load().amj_result_copy_host(C.byref(res), dst), "result_copy_host")
+    assert res.rows == 5000 and data.checksum(cols) == int(res.checksum)
+    L.load().amj_result_release(C.byref(res))
+    assert not res.priv and res.rows == 0
+
+
 @pytest.mark.parametrize("degree", [0, 1, 1022, 1023, 1024, 1055, 1056, 5000])
 def test_degree_rank_bins(ctx, degree):
     """Hubs whose degrees fall in and around the first linear and logarithmic
