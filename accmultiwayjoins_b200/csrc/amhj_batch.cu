@@ -355,6 +355,7 @@ struct amj_batch {
     DBuf<unsigned long long> tri_base, tri_ctr, tri_first;
     DBuf<TriHeadJob> tri_jobs;
     DBuf<BucketHead> tri_heads;
+    DBuf<uint32_t> tri_bits;
     uint32_t ntri = 0, ntri_jobs = 0;
     uint64_t ntri_heads = 0;
     unsigned tri_grid = 0;
@@ -403,6 +404,7 @@ struct amj_batch {
         tri_first.release();
         tri_jobs.release();
         tri_heads.release();
+        tri_bits.release();
         q_count.release();
         q_checksum.release();
         st.release();
@@ -651,6 +653,7 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
         }
         if (total * sizeof(BucketHead) <= ctx->device_mem / 8) {
             AMJ_TRY(ensure(ctx, b->tri_heads, total));
+            AMJ_TRY(ensure(ctx, b->tri_bits, total));
             AMJ_TRY(ensure(ctx, b->tri_jobs, hj.size()));
             AMJ_TRY(ensure(ctx, b->tri_first, first.size()));
             if (reinterpret_cast<uintptr_t>(b->tri_heads.p) % alignof(BucketHead) == 0) {
@@ -662,7 +665,10 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
                 b->ntri_jobs = (uint32_t)hj.size();
                 b->ntri_heads = total;
                 for (uint32_t q = 0; q < nq; q++)
-                    if (hplans[q].tri) hplans[q].tri_heads = b->tri_heads.p + first_of[where[level_job[q][1]]];
+                    if (hplans[q].tri) {
+                        hplans[q].tri_heads = b->tri_heads.p + first_of[where[level_job[q][1]]];
+                        hplans[q].tri_bits = b->tri_bits.p + first_of[where[level_job[q][1]]];
+                    }
             }
         }
     }
@@ -770,7 +776,7 @@ static int batch_record(amj_batch *b, bool capturing) {
         note_launch(ctx);
         batch_tri_heads_kernel<<<batch_grid_for(ctx, b->ntri_heads), 256, 0, s>>>(b->tri_jobs.p, b->tri_first.p,
                                                                                   b->ntri_jobs, b->ntri_heads,
-                                                                                  b->tri_heads.p);
+                                                                                  b->tri_heads.p, b->tri_bits.p);
         AMJ_CUDA_TRY(cudaGetLastError());
     }
     AMJ_TRY(mark(b->ev[1], s, capturing));

@@ -105,6 +105,7 @@ struct alignas(16) ProbePlan {
     uint32_t fib_suffix_attrs;             // attributes the cached tuples provide
     int32_t fib_level;                     // -1: off
     const BucketHead *tri_heads;           // tri: heads of the pair index (null: not built)
+    const uint32_t *tri_bits;              // tri: a word of pair hashes' high bits a bucket (with tri_heads)
 };
 static_assert(sizeof(ProbePlan) % 16 == 0, "plans are copied as 16-byte words");
 

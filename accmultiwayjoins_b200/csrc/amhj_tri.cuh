@@ -13,13 +13,18 @@
 // A unit is TRI_CHUNK candidates.  A warp loads the rows of its unit 32 at a
 // time, one a lane, and hands out their candidates one a lane: the lane whose
 // row starts at a candidate marks it in a 32-bit word, so the owner of a
-// candidate is a population count and not a search.  The filter is one 32-byte
-// bucket head (two bounds and three rows) instead of two bounds and then the
-// rows' columns.  There is no frontier, no task and no wait: every candidate
-// is one filter lookup.  Bound by the random sectors of the heads.
+// candidate is a population count and not a search.  Most candidates close no
+// triangle (107 M of 697 M do), so a word a bucket, with a bit for each row's pair
+// hash, turns them down first: 4 bytes a candidate, which the L1 and L2 hold.
+// Those that pass wait in a ring until 32 of them look up their bucket's head (two
+// bounds and three rows, 32 bytes) together.  There is no frontier, no task and
+// no wait on another warp.  Bound by the latency of the dependent loads and by
+// instructions (half of the issue slots before the bits).
 // Measured, 54 triangle queries of 10K to 1M edges, 107 M triangles: the probe
-// takes 7.3 ms; through the frontier DFS, with b's list alone and the pair
-// filter's bounds and columns read one by one, it took 40.2 ms.
+// takes 5.2 ms; 7.2 with a head lookup a candidate (6.8 to 8.8 with 16-byte heads
+// of twice as many buckets); 40.2 through the frontier DFS, with b's list alone and
+// the pair filter's bounds and columns read one by one.  Two candidates a
+// lane and step: 5.2.
 #pragma once
 #include "amhj_kernel.cuh"
 
@@ -58,9 +63,13 @@ struct TriLaunch {
 struct TriWarp {
     unsigned long long hab[32];   // hash prefix of (a, b)
     int4 ent[32];                 // list start minus the candidates before it, key, other vertex
+    // candidates that passed the filter's bits, a ring of 64
+    unsigned long long qhab[64];
+    int4 q[64];                   // other vertex, candidate, pair hash
 };
 
-__global__ __launch_bounds__(TRI_THREADS) void batch_tri_kernel(const TriLaunch T) {
+// six blocks an SM (four, five, eight: 5.5, 5.4, 5.4 ms)
+__global__ __launch_bounds__(TRI_THREADS, 6) void batch_tri_kernel(const TriLaunch T) {
     __shared__ TriWarp smem[TRI_WARPS];
     const int lane = threadIdx.x & 31;
     TriWarp &W = smem[threadIdx.x >> 5];
@@ -68,7 +77,41 @@ __global__ __launch_bounds__(TRI_THREADS) void batch_tri_kernel(const TriLaunch 
     const unsigned long long total = T.tri_base[T.nq];
     unsigned long long cnt = 0, chk = 0;
     int cur = -1;
+    uint32_t qh = 0, qn = 0;   // the ring's first entry and their number
+    // look up the ring's first n <= 32 entries in the current query's filter
+    auto drain = [&](uint32_t n) {
+        if ((uint32_t)lane < n) {
+            const ProbePlan &P = T.plans[cur];
+            const LevelDesc &fl = P.lv[1];
+            const int4 x = W.q[(qh + lane) & 63];
+            const uint32_t h = (uint32_t)x.z & fl.mask;
+            uint32_t m = 0, rs, re;
+            if (P.tri_heads) {
+                uint32_t w[8];
+                load_head(P.tri_heads + h, w);
+                rs = w[0];
+                re = w[1];
+                const uint32_t k = re - rs;
+#pragma unroll
+                for (int i = 0; i < HEAD_ROWS; i++)
+                    m += ((uint32_t)i < k && (int32_t)w[2 + 2 * i] == x.x && (int32_t)w[3 + 2 * i] == x.y) ? 1u : 0u;
+                rs = k > (uint32_t)HEAD_ROWS ? rs + HEAD_ROWS : re;
+            } else {
+                rs = fl.buc_ptrs[h];
+                re = fl.buc_ptrs[h + 1];
+            }
+            for (; rs < re; rs++) m += (fl.col[0][rs] == x.x && fl.col[1][rs] == x.y) ? 1u : 0u;
+            if (m) {
+                cnt += m;
+                chk += m * amj_hash_step(W.qhab[(qh + lane) & 63], x.y);
+            }
+        }
+        __syncwarp();
+        qh += n;
+        qn -= n;
+    };
     auto flush = [&]() {
+        if (qn) drain(qn);
         const unsigned long long c = warp_sum(cnt), h = warp_sum(chk);
         if (lane == 0 && cur >= 0 && c) {
             atomicAdd(&T.q_count[cur], c);
@@ -94,8 +137,8 @@ __global__ __launch_bounds__(TRI_THREADS) void batch_tri_kernel(const TriLaunch 
         const uint64_t rlo = warp_row_of(E, rows, g0, lane), rhi = warp_row_of(E, rows, g1 - 1, lane) + 1;
         const int32_t *ca = tri_col(P, 0), *cb = tri_col(P, 1);
         const int32_t *key0 = P.lv[0].col[0], *val0 = P.lv[0].col[1];
-        const LevelDesc &fl = P.lv[1];
-        const BucketHead *heads = P.tri_heads;
+        const uint32_t *bits = P.tri_bits;
+        const uint32_t mask1 = P.lv[1].mask;
         for (uint64_t r0 = rlo; r0 < rhi; r0 += 32) {
             const uint64_t r = r0 + lane;
             uint32_t sz = 0, s = 0;
@@ -129,32 +172,26 @@ __global__ __launch_bounds__(TRI_THREADS) void batch_tri_kernel(const TriLaunch 
                 const int o = before + __popc(starts & le);
                 before += __popc(starts);
                 const uint32_t j = j0 + lane;
-                if (j >= tot) continue;
-                const int4 e = W.ent[o];
-                const uint32_t slot = (uint32_t)e.x + j;
-                const int32_t c = val0[slot];
-                if (key0[slot] != e.y) continue;
-                const uint32_t h = hash_pair(e.z, c) & fl.mask;
-                uint32_t m = 0, rs, re;
-                if (heads) {
-                    uint32_t w[8];
-                    load_head(heads + h, w);
-                    rs = w[0];
-                    re = w[1];
-                    const uint32_t n = re - rs;
-#pragma unroll
-                    for (int i = 0; i < HEAD_ROWS; i++)
-                        m += ((uint32_t)i < n && (int32_t)w[2 + 2 * i] == e.z && (int32_t)w[3 + 2 * i] == c) ? 1u : 0u;
-                    rs += HEAD_ROWS;
-                } else {
-                    rs = fl.buc_ptrs[h];
-                    re = fl.buc_ptrs[h + 1];
+                bool hit = false;
+                int4 e = make_int4(0, 0, 0, 0);
+                int32_t c = 0;
+                uint32_t h = 0;
+                if (j < tot) {
+                    e = W.ent[o];
+                    const uint32_t slot = (uint32_t)e.x + j;
+                    c = val0[slot];
+                    h = hash_pair(e.z, c);
+                    hit = key0[slot] == e.y && (!bits || ((__ldg(bits + (h & mask1)) >> (h >> 27)) & 1u));
                 }
-                for (; rs < re; rs++) m += (fl.col[0][rs] == e.z && fl.col[1][rs] == c) ? 1u : 0u;
-                if (m) {
-                    cnt += m;
-                    chk += m * amj_hash_step(W.hab[o], c);
+                const unsigned hits = __ballot_sync(AMJ_FULL_MASK, hit);
+                if (hit) {
+                    const uint32_t at = (qh + qn + __popc(hits & lt)) & 63;
+                    W.q[at] = make_int4(e.z, c, (int)h, 0);
+                    W.qhab[at] = W.hab[o];
                 }
+                __syncwarp();
+                qn += __popc(hits);
+                if (qn >= 32) drain(32);
             }
         }
     }
@@ -169,7 +206,8 @@ struct TriHeadJob {
 };
 
 __global__ void batch_tri_heads_kernel(const TriHeadJob *__restrict__ jobs, const unsigned long long *__restrict__ first,
-                                       uint32_t njobs, uint64_t total, BucketHead *__restrict__ heads) {
+                                       uint32_t njobs, uint64_t total, BucketHead *__restrict__ heads,
+                                       uint32_t *__restrict__ bits) {
     for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t lo = 0, hi = njobs;
         while (hi - lo > 1) {
@@ -189,6 +227,9 @@ __global__ void batch_tri_heads_kernel(const TriHeadJob *__restrict__ jobs, cons
             o.kp[2 * i + 1] = in ? J.c1[o.s + i] : 0;
         }
         heads[t] = o;
+        uint32_t w = 0;
+        for (uint32_t i = o.s; i < o.e && w != ~0u; i++) w |= 1u << (hash_pair(J.c0[i], J.c1[i]) >> 27);
+        bits[t] = w;
     }
 }
 
