@@ -11,7 +11,7 @@
 // exceeds STAR_MAX_PRODUCT (a skewed dimension) is listed instead and joined
 // afterwards by the DFS kernel, which shares such work across warps.
 // Count mode only; bucket layout only.  Stars and chains in the numbering of
-// the reference's benchmarks also have register kernels over 32-byte bucket
+// the reference's benchmarks also have kernels over 16- and 32-byte bucket
 // heads (amhj_star_canon_kernel, amhj_chain_canon_kernel, below), and
 // materialised stars two flat passes (star_rowcount_kernel,
 // star_write_kernel).
