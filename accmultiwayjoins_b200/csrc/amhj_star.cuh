@@ -66,6 +66,7 @@ __device__ __forceinline__ void flat_totals(unsigned long long cnt, unsigned lon
         }
         __threadfence();
         if (atomicAdd(&ctr->done, 1u) == gridDim.x - 1) {
+            __threadfence();   // the other blocks' sums before the reads below
             host->count = atomicAdd(&ctr->count, 0ull);
             host->checksum = atomicAdd(&ctr->checksum, 0ull);
             host->nover = atomicAdd(&ctr->nover, 0u);
