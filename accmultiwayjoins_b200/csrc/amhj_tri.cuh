@@ -198,6 +198,11 @@ __global__ __launch_bounds__(TRI_THREADS, 6) void batch_tri_kernel(const TriLaun
     flush();
 }
 
+// Rows of a bucket that its filter word is made of; longer buckets get a word of
+// ones.  One thread reads them one by one: an edge repeated a million times
+// kept it (and the batch) busy for 89 ms.
+constexpr uint32_t TRI_BITS_ROWS = 64;
+
 // heads of the pair indexes of the triangle queries
 struct TriHeadJob {
     const uint32_t *bp;
@@ -227,7 +232,9 @@ __global__ void batch_tri_heads_kernel(const TriHeadJob *__restrict__ jobs, cons
             o.kp[2 * i + 1] = in ? J.c1[o.s + i] : 0;
         }
         heads[t] = o;
-        uint32_t w = 0;
+        // a long bucket's word would have nearly every bit set, or its rows are
+        // copies of one pair, which never set them all: it turns nothing down
+        uint32_t w = o.e - o.s > TRI_BITS_ROWS ? ~0u : 0u;
         for (uint32_t i = o.s; i < o.e && w != ~0u; i++) w |= 1u << (hash_pair(J.c0[i], J.c1[i]) >> 27);
         bits[t] = w;
     }
