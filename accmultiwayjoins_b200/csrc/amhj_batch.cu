@@ -73,12 +73,13 @@ struct TileOwner {
     bool whole;       // every row of the tile is its
 };
 
+template <uint32_t TILE = BATCH_TILE>
 __device__ __forceinline__ TileOwner tile_owner(const unsigned long long *__restrict__ base, uint32_t n,
                                                 unsigned long long r0) {
     __shared__ TileOwner t;
     if (threadIdx.x == 0) {
         t.first = find_last_le(base, n, r0);
-        t.whole = t.first + 1 >= n || base[t.first + 1] >= r0 + BATCH_TILE;
+        t.whole = t.first + 1 >= n || base[t.first + 1] >= r0 + TILE;
     }
     __syncthreads();
     return t;
@@ -219,13 +220,18 @@ __global__ void batch_oa_insert_kernel(const BatchJob *__restrict__ jobs, const 
     }
 }
 
-// level-0 candidate counts of every query's probe rows; sizes[rows] = 0
+// Level-0 candidate counts of every query's probe rows; sizes[rows] = 0.  RPT
+// rows a thread: four over bucket indexes, whose counts are two loads; one over
+// open addressing, where a hub's count is a long scan, and a thread with four of
+// them, or a larger block, keeps the launch waiting (four triangle queries of
+// 2^17 edges: 1.33 ms with four, 0.62 with one).
+template <int RPT>
 __global__ __launch_bounds__(256) void batch_l0_sizes_kernel(const ProbePlan *__restrict__ plans,
                                                              const unsigned long long *__restrict__ qrow, uint32_t nq,
                                                              uint64_t rows, unsigned long long *__restrict__ sizes) {
-    const uint64_t r0 = blockIdx.x * (uint64_t)BATCH_TILE;
-    const TileOwner own = tile_owner(qrow, nq, r0);
-    for (int k = 0; k < 4; k++) {
+    const uint64_t r0 = blockIdx.x * (uint64_t)(256 * RPT);
+    const TileOwner own = tile_owner<256 * RPT>(qrow, nq, r0);
+    for (int k = 0; k < RPT; k++) {
         const uint64_t r = r0 + k * 256 + threadIdx.x;
         if (r > rows) return;
         if (r == rows) {
@@ -338,6 +344,7 @@ struct amj_batch {
     int sort_bits = 0, ncols_max = 1;
     uint32_t block = 256, warp_stride = 0;
     bool weighted = false;   // some query has inlined filter levels
+    void (*kern)(const BatchLaunch) = nullptr;   // the probe kernel
     unsigned grid = 0;
     size_t smem = 0;
     DBuf<BatchJob> d_jobs;
@@ -448,15 +455,13 @@ int normalize_batch_opts(const amj_batch_opts *in, amj_batch_opts *o) {
     return AMJ_OK;
 }
 
-template <int T, bool WT>
-static int batch_kernel_setup(amj_ctx *ctx, size_t smem, unsigned *grid) {
-    auto kern = amhj_batch_kernel<T, WT>;
-    AMJ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int per_sm = 0;
-    AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem));
-    if (per_sm < 1) return fail(AMJ_EUNSUPPORTED, "batch: probe frontier does not fit in shared memory");
-    *grid = (unsigned)(ctx->num_sms * per_sm);
-    return AMJ_OK;
+// the probe kernel of a batch (batch_min_blocks)
+using BatchKernel = void (*)(const BatchLaunch);
+
+template <int T>
+static BatchKernel batch_kernel_of(bool weighted, bool open_addr) {
+    if (!weighted) return amhj_batch_kernel<T, false, false>;
+    return open_addr ? amhj_batch_kernel<T, true, true> : amhj_batch_kernel<T, true, false>;
 }
 
 static unsigned batch_tiles(uint64_t rows) { return (unsigned)((rows + BATCH_TILE - 1) / BATCH_TILE); }
@@ -686,15 +691,14 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     if (b->smem > (size_t)ctx->max_smem_optin) return fail(AMJ_EUNSUPPORTED, "batch: frontier exceeds shared memory");
     b->weighted = false;
     for (const ProbePlan &P : hplans) b->weighted |= P.has_inl != 0 && !P.tri;
-    if (b->weighted) {
-        if (b->block == 128) AMJ_TRY((batch_kernel_setup<128, true>(ctx, b->smem, &b->grid)));
-        else if (b->block == 256) AMJ_TRY((batch_kernel_setup<256, true>(ctx, b->smem, &b->grid)));
-        else AMJ_TRY((batch_kernel_setup<512, true>(ctx, b->smem, &b->grid)));
-    } else {
-        if (b->block == 128) AMJ_TRY((batch_kernel_setup<128, false>(ctx, b->smem, &b->grid)));
-        else if (b->block == 256) AMJ_TRY((batch_kernel_setup<256, false>(ctx, b->smem, &b->grid)));
-        else AMJ_TRY((batch_kernel_setup<512, false>(ctx, b->smem, &b->grid)));
-    }
+    b->kern = b->block == 128   ? batch_kernel_of<128>(b->weighted, b->oa_rows > 0)
+              : b->block == 256 ? batch_kernel_of<256>(b->weighted, b->oa_rows > 0)
+                                : batch_kernel_of<512>(b->weighted, b->oa_rows > 0);
+    AMJ_CUDA_TRY(cudaFuncSetAttribute(b->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
+    int per_sm = 0;
+    AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->kern, (int)b->block, b->smem));
+    if (per_sm < 1) return fail(AMJ_EUNSUPPORTED, "batch: probe frontier does not fit in shared memory");
+    b->grid = (unsigned)(ctx->num_sms * per_sm);
     int tri_per_sm = 0;
     AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tri_per_sm, batch_tri_kernel, TRI_THREADS, 0));
     b->tri_grid = (unsigned)(ctx->num_sms * std::max(tri_per_sm, 1));
@@ -782,8 +786,12 @@ static int batch_record(amj_batch *b, bool capturing) {
     AMJ_TRY(mark(b->ev[1], s, capturing));
     // ---- probe
     note_launch(ctx);
-    batch_l0_sizes_kernel<<<batch_tiles(b->probe_rows + 1), 256, 0, s>>>(b->plans.p, b->qrow.p, nq,
-                                                                                b->probe_rows, b->sizes.p);
+    if (b->oa_rows)
+        batch_l0_sizes_kernel<1><<<(unsigned)(b->probe_rows / 256 + 1), 256, 0, s>>>(b->plans.p, b->qrow.p, nq,
+                                                                                    b->probe_rows, b->sizes.p);
+    else
+        batch_l0_sizes_kernel<4><<<batch_tiles(b->probe_rows + 1), 256, 0, s>>>(b->plans.p, b->qrow.p, nq,
+                                                                               b->probe_rows, b->sizes.p);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)b->sizes.p, (uint64_t *)b->l0.p, b->probe_rows + 1, nullptr));
     note_launch(ctx);
@@ -822,15 +830,7 @@ static int batch_record(amj_batch *b, bool capturing) {
     L.spin_limit_ns = (uint64_t)ctx->opts.spin_limit_ms * 1000000ull;
     L.warp_stride = b->warp_stride;
     note_launch(ctx);
-    if (b->weighted) {
-        if (b->block == 128) amhj_batch_kernel<128, true><<<b->grid, 128, b->smem, s>>>(L);
-        else if (b->block == 256) amhj_batch_kernel<256, true><<<b->grid, 256, b->smem, s>>>(L);
-        else amhj_batch_kernel<512, true><<<b->grid, 512, b->smem, s>>>(L);
-    } else {
-        if (b->block == 128) amhj_batch_kernel<128, false><<<b->grid, 128, b->smem, s>>>(L);
-        else if (b->block == 256) amhj_batch_kernel<256, false><<<b->grid, 256, b->smem, s>>>(L);
-        else amhj_batch_kernel<512, false><<<b->grid, 512, b->smem, s>>>(L);
-    }
+    b->kern<<<b->grid, b->block, b->smem, s>>>(L);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(mark(b->ev[2], s, capturing));
     b->launches_per_run = ctx->launches - l0;

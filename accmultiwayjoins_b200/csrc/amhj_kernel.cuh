@@ -734,8 +734,19 @@ __device__ __forceinline__ void batch_flush(const BatchLaunch &B, int q, ProbeAc
     acc.cnt = acc.chk = 0;
 }
 
-template <int THREADS, bool WT>
-__global__ __launch_bounds__(THREADS) void amhj_batch_kernel(const __grid_constant__ BatchLaunch B) {
+// Blocks per SM.  The compiler's own choice moves between 64 and 80 registers
+// with every change to the code, and neither is always better: a fourth block
+// of 256 threads hides more latency but takes its frontiers (up to 53 KB) from
+// the L1.  Batches over bucket indexes are faster with three (9M-row chain
+// beside four small queries 1.14 ms, 1.40 with four; two FOUR queries of 2^16
+// edges 3.64 ms and 3.81), weighted ones over open addressing (OA) with four
+// (two FOUR queries 11.0 ms, 11.7 with three; four triangle queries 6.1 and 6.4).
+constexpr int batch_min_blocks(int threads, bool wt, bool oa) {
+    return threads == 128 ? 7 : threads == 512 ? 2 : wt && oa ? 4 : 3;
+}
+
+template <int THREADS, bool WT, bool OA>
+__global__ __launch_bounds__(THREADS, batch_min_blocks(THREADS, WT, OA)) void amhj_batch_kernel(const __grid_constant__ BatchLaunch B) {
     extern __shared__ __align__(16) char smem[];
     const int lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();
