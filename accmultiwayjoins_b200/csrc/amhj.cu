@@ -521,7 +521,7 @@ static int run_passes(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws, bo
         AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)l0.p, (uint64_t *)l0.p, rows, (uint64_t *)l0.p + rows));
         unsigned long long total = 0;
         AMJ_TRY(read_back(ctx, &total, l0.p + rows, sizeof(total)));
-        P.l0_chunk = l0_chunk_for(total, (uint64_t)ctx->num_sms * 32);
+        P.l0_chunk = l0_chunk_for(total, (uint64_t)ctx->num_sms * 32, l0_deep(P));
         nchunks = (total + P.l0_chunk - 1) / P.l0_chunk;
         if (nchunks > 0xffffffffull) return fail(AMJ_EUNSUPPORTED, "AMHJ: 2^42 or more level-0 candidates in one slice");
         P.lbs = 1;

@@ -16,8 +16,8 @@
 //          open-addressing layout inserts every row into its table's slot
 //          range in one kernel.
 //  probe   level-0 candidate counts of every query's probe rows, one prefix
-//          array over all of them, units of 1024 level-0 candidates per query,
-//          and amhj_batch_kernel over the whole unit space plus the shared
+//          array over all of them, units of 64 to 1024 level-0 candidates per
+//          query, and amhj_batch_kernel over the whole unit space plus the shared
 //          work-sharing queue.  Triangle queries have units and a kernel of
 //          their own (amhj_tri.cuh).  Counts and checksums land in per-query
 //          slots.
@@ -253,8 +253,8 @@ __global__ __launch_bounds__(256) void batch_l0_sizes_kernel(const ProbePlan *__
 
 // First unit of every query: unit_base[q] counts the units of the queries
 // before q (none for a triangle query), tri_base[q] the units of TRI_CHUNK
-// candidates of the triangle queries before q.  units[0] = all units, units[1]
-// = level-0 candidates per unit (l0_chunk_for); one block
+// candidates of the triangle queries before q.  units[0] = all units, units[1 +
+// l0_deep(plan)] = level-0 candidates per unit (l0_chunk_for); one block
 __global__ void batch_units_kernel(const ProbePlan *__restrict__ plans, const unsigned long long *__restrict__ l0,
                                    const unsigned long long *__restrict__ qrow, uint32_t nq,
                                    unsigned long long *__restrict__ unit_base, unsigned long long *__restrict__ tri_base,
@@ -270,14 +270,14 @@ __global__ void batch_units_kernel(const ProbePlan *__restrict__ plans, const un
         if (!plans[q].tri) mine += l0[qrow[q + 1]] - l0[qrow[q]];
     if (mine) atomicAdd(&cand, mine);
     __syncthreads();
-    const uint32_t chunk = l0_chunk_for(cand, warps);
+    const uint32_t chunk[2] = {l0_chunk_for(cand, warps, false), l0_chunk_for(cand, warps, true)};
     for (uint32_t b0 = 0; b0 < nq; b0 += blockDim.x) {
         const uint32_t q = b0 + threadIdx.x;
         unsigned long long u = 0, t = 0;
         if (q < nq) {
             const unsigned long long c = l0[qrow[q + 1]] - l0[qrow[q]];
             if (plans[q].tri) t = (c + TRI_CHUNK - 1) / TRI_CHUNK;
-            else u = (c + chunk - 1) / chunk;
+            else u = (c + chunk[l0_deep(plans[q])] - 1) / chunk[l0_deep(plans[q])];
         }
         const unsigned long long uincl = warp_inclusive_scan(u, lane), tincl = warp_inclusive_scan(t, lane);
         if (lane == 31) {
@@ -306,7 +306,8 @@ __global__ void batch_units_kernel(const ProbePlan *__restrict__ plans, const un
         unit_base[nq] = carry[0];
         tri_base[nq] = carry[1];
         units[0] = carry[0] + carry[1];
-        units[1] = chunk;
+        units[1] = chunk[0];
+        units[2] = chunk[1];
     }
 }
 
@@ -358,7 +359,7 @@ struct amj_batch {
     DBuf<ProbePlan> plans;
     DBuf<unsigned long long> qrow, sizes, l0, unit_base, q_count, q_checksum;
     // triangle queries (amhj_tri.cuh): first units; [0] unit counter, [1] units of
-    // the whole batch, [2] level-0 candidates per unit; and the heads of their pair indexes
+    // the whole batch, [2], [3] level-0 candidates per unit; and the heads of their pair indexes
     DBuf<unsigned long long> tri_base, tri_ctr, tri_first;
     DBuf<TriHeadJob> tri_jobs;
     DBuf<BucketHead> tri_heads;
@@ -598,7 +599,7 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     AMJ_TRY(ensure(ctx, b->l0, b->probe_rows + 1));
     AMJ_TRY(ensure(ctx, b->unit_base, nq + 1));
     AMJ_TRY(ensure(ctx, b->tri_base, nq + 1));
-    AMJ_TRY(ensure(ctx, b->tri_ctr, 3));
+    AMJ_TRY(ensure(ctx, b->tri_ctr, 4));
     AMJ_TRY(ensure(ctx, b->q_count, nq));
     AMJ_TRY(ensure(ctx, b->q_checksum, nq));
     AMJ_TRY(ensure(ctx, b->plans, nq));
@@ -795,7 +796,7 @@ static int batch_record(amj_batch *b, bool capturing) {
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(scan_exclusive_u64(ctx, (const uint64_t *)b->sizes.p, (uint64_t *)b->l0.p, b->probe_rows + 1, nullptr));
     note_launch(ctx);
-    AMJ_CUDA_TRY(cudaMemsetAsync(b->tri_ctr.p, 0, 3 * sizeof(unsigned long long), s));
+    AMJ_CUDA_TRY(cudaMemsetAsync(b->tri_ctr.p, 0, 4 * sizeof(unsigned long long), s));
     batch_units_kernel<<<1, 1024, 0, s>>>(b->plans.p, b->l0.p, b->qrow.p, nq, b->unit_base.p, b->tri_base.p,
                                           b->tri_ctr.p + 1, b->grid * (b->block / 32));
     AMJ_CUDA_TRY(cudaGetLastError());

@@ -156,12 +156,22 @@ __device__ __forceinline__ uint64_t warp_row_of(const unsigned long long *E, uin
 // took 24.6 ms in units of 1024 and 7.1 ms in units of 64.  Units shrink down to L0_CHUNK_MIN
 // until every warp gets L0_UNITS_PER_WARP of them; a unit costs two searches
 // for its rows, which the largest size makes negligible on large inputs.
+// Where level 0 is the last to have a frontier (two relations, triangles with
+// their filter inline) a unit's work is its candidates, and four units a warp
+// even it out; more only cost searches.  Hash-plan triangles, 2^19 edges at
+// scale 15: 1.69 ms so (1, 2 or 8 a warp the same), 1.76 with 16, 2.19 with 64;
+// 2^17 edges written out 4.5, 5.3 and 6.4 ms.
 constexpr uint32_t L0_CHUNK_MAX = 1024, L0_CHUNK_MIN = 64;
 constexpr uint32_t L0_UNITS_PER_WARP = 64;
+constexpr uint32_t L0_UNITS_PER_WARP_FLAT = 4;
 
-__host__ __device__ inline uint32_t l0_chunk_for(unsigned long long candidates, unsigned long long warps) {
+// whether plan P has a frontier level after level 0
+__host__ __device__ inline bool l0_deep(const ProbePlan &P) { return P.next_lv[0] < P.L; }
+
+__host__ __device__ inline uint32_t l0_chunk_for(unsigned long long candidates, unsigned long long warps, bool deep) {
+    const uint32_t units = deep ? L0_UNITS_PER_WARP : L0_UNITS_PER_WARP_FLAT;
     uint32_t c = L0_CHUNK_MAX;
-    while (c > L0_CHUNK_MIN && candidates / c < L0_UNITS_PER_WARP * warps) c >>= 1;
+    while (c > L0_CHUNK_MIN && candidates / c < units * warps) c >>= 1;
     return c;
 }
 
@@ -713,7 +723,7 @@ __global__ __launch_bounds__(PROBE_THREADS) void amhj_probe_kernel(const __grid_
 struct BatchLaunch {
     const ProbePlan *plans;
     const unsigned long long *unit_base;   // nq + 1 entries
-    const unsigned long long *l0_chunk;    // level-0 candidates per unit of this run
+    const unsigned long long *l0_chunk;    // level-0 candidates per unit of this run: [l0_deep(plan)]
     unsigned long long *q_count;
     unsigned long long *q_checksum;
     WsQueue Q;
@@ -754,7 +764,6 @@ __global__ __launch_bounds__(THREADS, batch_min_blocks(THREADS, WT, OA)) void am
     const ProbePlan &P = *reinterpret_cast<const ProbePlan *>(wslot);
     char *wbase = wslot + BATCH_PLAN_BYTES;
     const unsigned long long total_units = B.unit_base[B.nq];
-    const uint32_t chunk = (uint32_t)*B.l0_chunk;
     ProbeAcc acc;
     UnitOut u;
     L0Chunk ch;
@@ -791,10 +800,12 @@ __global__ __launch_bounds__(THREADS, batch_min_blocks(THREADS, WT, OA)) void am
                 int4 *dst = reinterpret_cast<int4 *>(wslot);
                 for (uint32_t i = lane; i < sizeof(ProbePlan) / 16; i += 32) dst[i] = src[i];
                 __syncwarp();
+                if (lane == 0) reinterpret_cast<ProbePlan *>(wslot)->l0_chunk = (uint32_t)B.l0_chunk[l0_deep(P)];
+                __syncwarp();
                 cur = q;
             }
             if (!task) {
-                l0_chunk_setup(P, chunk, b - B.unit_base[q], lane, ch);
+                l0_chunk_setup(P, P.l0_chunk, b - B.unit_base[q], lane, ch);
             } else {
                 depth = load_task<PM_COUNT, true>(P, B.Q, wbase, tslot, lane);
             }

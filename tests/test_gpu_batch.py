@@ -257,3 +257,20 @@ def test_batch_triangles_through_repeated_edges(copies):
         b.submit("TRI", [ctx.relation([s, d], [0, 1])])
         r = b.run()
         assert (r.counts[0], r.checksums[0]) == O.triangle(s, d)
+
+
+def test_batch_units_of_queries_without_a_second_frontier():
+    """Triangles over open addressing end at their first level (the filter is
+    inline): their units shrink to give each warp a few of them, not the many
+    that even out the trees below a chain's level 0."""
+    s, d = data.rmat(12, 1 << 16, 0.57, 0.19, 0.19, 5)
+    chain = data.chain_relations(20_000, 1 << 12, 3, seed=2)
+    with Context(0) as ctx, ctx.batch() as b:
+        b.submit("TRI", [ctx.relation([s, d], [0, 1])])
+        flat = b.run(layout="oa")
+        assert (flat.counts[0], flat.checksums[0]) == O.triangle(s, d)
+        assert 4000 <= flat.units <= 8 * 148 * 32 + 1   # with 64 a warp over 100 thousand
+        b.submit("NORMAL", [ctx.relation(c, a) for c, a in chain])
+        both = b.run(layout="oa")
+        assert both.units - flat.units > 1000
+        assert list(zip(both.counts, both.checksums)) == [(flat.counts[0], flat.checksums[0]), O.mhj(chain)]
