@@ -366,6 +366,7 @@ struct amj_batch {
     DBuf<uint32_t> tri_bits;
     uint32_t ntri = 0, ntri_jobs = 0;
     uint64_t ntri_heads = 0;
+    bool no_heads = false;     // these queries run without heads: there was no room for them
     unsigned tri_grid = 0;
     DBuf<ProbeState> st;
     DBuf<Task> tasks;
@@ -474,6 +475,64 @@ static int ensure(amj_ctx *ctx, DBuf<T> &buf, size_t n) {
     if (buf.p && buf.n >= n) return AMJ_OK;
     buf.release();
     return buf.alloc(ctx, n);
+}
+
+// Give the triangle queries' heads back and plan without them.
+static void batch_drop_heads(amj_batch *b, std::vector<ProbePlan> &hplans) {
+    b->tri_heads.release();
+    b->tri_bits.release();
+    b->ntri_jobs = 0;
+    b->ntri_heads = 0;
+    for (ProbePlan &P : hplans) {
+        P.tri_heads = nullptr;
+        P.tri_bits = nullptr;
+    }
+}
+
+// The pair indexes of the triangle queries get bucket heads and filter words (36 B
+// a bucket) while these take at most an eighth of the device's memory and stay
+// within the context's memory budget, where it has one; a server's lanes, which
+// admit requests by batch_estimate_bytes, go without.  AMJ_ENOMEM: there is no
+// room for them.
+static int batch_tri_heads_prepare(amj_batch *b, std::vector<ProbePlan> &hplans, const std::vector<int> &where,
+                                   const std::vector<std::vector<int>> &level_job) {
+    amj_ctx *ctx = b->ctx;
+    b->ntri_jobs = 0;
+    b->ntri_heads = 0;
+    if (!b->ntri || ctx->iprov) return AMJ_OK;
+    uint64_t total = 0;
+    std::map<int, uint64_t> first_of;   // job -> first head
+    std::vector<TriHeadJob> hj;
+    std::vector<unsigned long long> first;
+    for (size_t q = 0; q < hplans.size(); q++) {
+        if (!hplans[q].tri) continue;
+        const int job = where[level_job[q][1]];
+        if (!first_of.emplace(job, total).second) continue;
+        const LevelDesc &lv = hplans[q].lv[1];
+        hj.push_back(TriHeadJob{lv.buc_ptrs, lv.col[0], lv.col[1], total});
+        first.push_back(total);
+        total += (uint64_t)lv.mask + 1;
+    }
+    const uint64_t bytes = total * (sizeof(BucketHead) + sizeof(uint32_t));
+    if (bytes > ctx->device_mem / 8 || (ctx->opts.mem_budget && bytes > ctx->opts.mem_budget)) return AMJ_OK;
+    AMJ_TRY(ensure(ctx, b->tri_heads, total));
+    AMJ_TRY(ensure(ctx, b->tri_bits, total));
+    AMJ_TRY(ensure(ctx, b->tri_jobs, hj.size()));
+    AMJ_TRY(ensure(ctx, b->tri_first, first.size()));
+    if (reinterpret_cast<uintptr_t>(b->tri_heads.p) % alignof(BucketHead) != 0) return AMJ_OK;
+    AMJ_CUDA_TRY(cudaMemcpyAsync(b->tri_jobs.p, hj.data(), hj.size() * sizeof(TriHeadJob), cudaMemcpyHostToDevice,
+                                 ctx->stream));
+    AMJ_CUDA_TRY(cudaMemcpyAsync(b->tri_first.p, first.data(), first.size() * sizeof(unsigned long long),
+                                 cudaMemcpyHostToDevice, ctx->stream));
+    AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));   // the host arrays end here
+    b->ntri_jobs = (uint32_t)hj.size();
+    b->ntri_heads = total;
+    for (size_t q = 0; q < hplans.size(); q++)
+        if (hplans[q].tri) {
+            hplans[q].tri_heads = b->tri_heads.p + first_of[where[level_job[q][1]]];
+            hplans[q].tri_bits = b->tri_bits.p + first_of[where[level_job[q][1]]];
+        }
+    return AMJ_OK;
 }
 
 static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
@@ -638,52 +697,18 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
         if (P.tri) b->ntri++;
         else max_warp_bytes = std::max(max_warp_bytes, P.warp_bytes);
     }
-    // the pair indexes of the triangle queries get bucket heads (32 B a bucket)
-    // while these take at most an eighth of the device's memory; a server's
-    // lanes, which admit requests by batch_estimate_bytes, go without
-    b->ntri_jobs = 0;
-    b->ntri_heads = 0;
-    if (b->ntri && !ctx->iprov) {
-        uint64_t total = 0;
-        std::map<int, uint64_t> first_of;   // job -> first head
-        std::vector<TriHeadJob> hj;
-        std::vector<unsigned long long> first;
-        for (uint32_t q = 0; q < nq; q++) {
-            if (!hplans[q].tri) continue;
-            const int job = where[level_job[q][1]];
-            if (!first_of.emplace(job, total).second) continue;
-            const LevelDesc &lv = hplans[q].lv[1];
-            hj.push_back(TriHeadJob{lv.buc_ptrs, lv.col[0], lv.col[1], total});
-            first.push_back(total);
-            total += (uint64_t)lv.mask + 1;
-        }
-        if (total * sizeof(BucketHead) <= ctx->device_mem / 8) {
-            AMJ_TRY(ensure(ctx, b->tri_heads, total));
-            AMJ_TRY(ensure(ctx, b->tri_bits, total));
-            AMJ_TRY(ensure(ctx, b->tri_jobs, hj.size()));
-            AMJ_TRY(ensure(ctx, b->tri_first, first.size()));
-            if (reinterpret_cast<uintptr_t>(b->tri_heads.p) % alignof(BucketHead) == 0) {
-                AMJ_CUDA_TRY(cudaMemcpyAsync(b->tri_jobs.p, hj.data(), hj.size() * sizeof(TriHeadJob),
-                                             cudaMemcpyHostToDevice, ctx->stream));
-                AMJ_CUDA_TRY(cudaMemcpyAsync(b->tri_first.p, first.data(), first.size() * sizeof(unsigned long long),
-                                             cudaMemcpyHostToDevice, ctx->stream));
-                AMJ_CUDA_TRY(cudaStreamSynchronize(ctx->stream));   // the host arrays end here
-                b->ntri_jobs = (uint32_t)hj.size();
-                b->ntri_heads = total;
-                for (uint32_t q = 0; q < nq; q++)
-                    if (hplans[q].tri) {
-                        hplans[q].tri_heads = b->tri_heads.p + first_of[where[level_job[q][1]]];
-                        hplans[q].tri_bits = b->tri_bits.p + first_of[where[level_job[q][1]]];
-                    }
-            }
-        }
-    }
-    AMJ_CUDA_TRY(cudaMemcpyAsync(b->plans.p, hplans.data(), nq * sizeof(ProbePlan), cudaMemcpyHostToDevice,
-                                 ctx->stream));
     b->task_cap = hplans[0].task_cap;
     AMJ_TRY(ensure(ctx, b->st, 1));
     AMJ_TRY(ensure(ctx, b->tasks, b->task_cap));
     AMJ_TRY(ensure(ctx, b->ready, b->task_cap));
+
+    // what the batch can do without comes last: on a full device it runs
+    // without heads
+    const int hrc = b->no_heads ? (int)AMJ_ENOMEM : batch_tri_heads_prepare(b, hplans, where, level_job);
+    if (hrc == AMJ_ENOMEM) batch_drop_heads(b, hplans);
+    else AMJ_TRY(hrc);
+    AMJ_CUDA_TRY(cudaMemcpyAsync(b->plans.p, hplans.data(), nq * sizeof(ProbePlan), cudaMemcpyHostToDevice,
+                                 ctx->stream));
 
     // ---- probe launch shape
     b->block = (uint32_t)o.block_size;
@@ -843,10 +868,7 @@ static bool same_opts(const amj_batch_opts &a, const amj_batch_opts &b) {
            a.task_chunk == b.task_chunk && a.grid_blocks == b.grid_blocks;
 }
 
-// Enqueue one run on the context stream: the device sequence (replayed
-// graph or eager launches), then the results into pinned host memory and the
-// completion event.  Returns without waiting.
-int batch_launch(amj_batch *b, const amj_batch_opts &o) {
+static int batch_launch_once(amj_batch *b, const amj_batch_opts &o) {
     amj_ctx *ctx = b->ctx;
     AMJ_CUDA_TRY(cudaSetDevice(ctx->device));
     if (!b->prepared || !same_opts(o, b->popts)) AMJ_TRY(batch_prepare(b, o));
@@ -872,12 +894,12 @@ int batch_launch(amj_batch *b, const amj_batch_opts &o) {
                 if (g) cudaGraphDestroy(g);
                 return rc;
             }
-            if (ce != cudaSuccess) return fail(AMJ_ECUDA, std::string("batch: graph capture: ") + cudaGetErrorString(ce));
+            if (ce != cudaSuccess) return cuda_fail(ce, "batch: graph capture");
             b->graph = g;
             const cudaError_t ie = cudaGraphInstantiate(&b->exec, g, 0);
             if (ie != cudaSuccess) {
                 b->drop_graph();
-                return fail(AMJ_ECUDA, std::string("batch: graph instantiate: ") + cudaGetErrorString(ie));
+                return cuda_fail(ie, "batch: graph instantiate");
             }
         }
         AMJ_CUDA_TRY(cudaGraphLaunch(b->exec, ctx->stream));
@@ -896,10 +918,25 @@ int batch_launch(amj_batch *b, const amj_batch_opts &o) {
     return AMJ_OK;
 }
 
+// Enqueue one run on the context stream: the device sequence (replayed
+// graph or eager launches), then the results into pinned host memory and the
+// completion event.  Returns without waiting.  A run whose own scratch no
+// longer fits beside the triangle queries' heads is enqueued again without them.
+int batch_launch(amj_batch *b, const amj_batch_opts &o) {
+    int rc = batch_launch_once(b, o);
+    if (rc == AMJ_ENOMEM && b->ntri_heads) {
+        b->invalidate();
+        b->no_heads = true;
+        rc = batch_launch_once(b, o);
+    }
+    return rc;
+}
+
 // drop the submitted queries, keep the buffers for the next ones
 void batch_clear(amj_batch *b) {
     b->invalidate();
     b->qs.clear();
+    b->no_heads = false;
 }
 
 // whether the last launched run has completed (no waiting)

@@ -116,7 +116,9 @@ typedef struct amj_opts {
     uint32_t spin_limit_ms;    /* bound on every device-side wait (0: 5000)       */
     uint64_t task_capacity;    /* work-sharing queue capacity in tasks (0: 1<<22) */
     uint64_t ooc_slice_rows;   /* ooc probe slice rows (0: derived from budget)   */
-    uint64_t mem_budget;       /* device bytes the ooc planner may use (0: free/2) */
+    uint64_t mem_budget;       /* device bytes the ooc planner may use (0: free/2); where
+                                  set, also a bound on the heads that a batch builds for
+                                  its triangle queries (it runs without them above it)  */
     uint32_t lftj_heavy_degree; /* ALFTJ ws=1: children count from which a vertex is
                                    joined by the block-wide bitmap kernel (0: 32)  */
     float    dro_headroom;     /* DRO output estimate multiplier (0: 1.05)        */
