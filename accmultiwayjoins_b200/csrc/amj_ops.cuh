@@ -76,23 +76,26 @@ struct Trie2 {
     uint64_t range1 = 0;       // level 1's values span at most this many (0: not known)
 };
 
-// Level 1 of a built 2-level trie has TRIE_LEVEL1_PAD spare values after its
-// last one, so kernels may read it in aligned 16-byte quads.
+// Level 1 of a trie of build_trie2 or build_trie2_ranked has TRIE_LEVEL1_PAD spare
+// values after its last one, so kernels may read it in aligned 16-byte quads.
 constexpr uint64_t TRIE_LEVEL1_PAD = 4;
+// mm_known: least and greatest values of both columns with their signs flipped,
+// where the caller has them;
 // distinct: drop repeated rows (the set semantics of the leapfrog triejoin);
 // vmax >= 0: every value of both columns lies in [0, vmax] (no min/max pass)
 int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, Trie2 *out,
-                bool distinct = false, int32_t vmax = -1);
-// The distinct 2-level tries of up to TRIE_JOBS_MAX relations, built together in
-// memory that `block` owns; level 0 lists every value of the first column's
-// range.  *built is false, and nothing is built, where a range is not dense, a
-// row is too long, rows repeat or a relation is empty.
+                bool distinct = false, int32_t vmax = -1, const uint32_t *mm_known = nullptr);
+// The distinct 2-level tries of up to TRIE_JOBS_MAX relations, built together where
+// their rows can be bucketed by counting (trie.cu), the others as build_trie2
+// builds them.  `block` owns memory of the tries; level 0 of a trie built
+// with others lists every value of the first column's range, and its level 1 may
+// start at any value of an array: no aligned groups of four, no spare values.
 constexpr int TRIE_JOBS_MAX = 3;
 struct TrieCols {
     const int32_t *c0, *c1;
     uint64_t n;
 };
-int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf<char> *block, bool *built);
+int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf<char> *block);
 
 // The distinct 2-level trie of the degree-ranked copy of the edges (c0, c1):
 // every vertex renamed to its rank (below nv), edges from the lower to the

@@ -391,10 +391,7 @@ static int lftj_execute_impl(amj_ctx *ctx, amj_rel *const *rels, int nrels, int 
             const bool swap = rels[i]->attrs[0] > rels[i]->attrs[1];
             cols[i] = TrieCols{rels[i]->d_cols[swap ? 1 : 0], rels[i]->d_cols[swap ? 0 : 1], rels[i]->n};
         }
-        bool built = false;
-        AMJ_TRY(build_tries2(ctx, cols, 3, tries, &trie_block, &built));
-        for (int i = 0; i < 3 && !built; i++)
-            AMJ_TRY(build_trie2(ctx, cols[i].c0, cols[i].c1, cols[i].n, &tries[i], true));
+        AMJ_TRY(build_tries2(ctx, cols, 3, tries, &trie_block));
     }
     return triangle_run(ctx, *R, *S, *T, algo, ws, flags, sorted_out, nv ? inv.p : nullptr, wedges.p, nv, out);
 }

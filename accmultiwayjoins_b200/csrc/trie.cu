@@ -119,7 +119,7 @@ static int bits_for(uint32_t range) {
 }
 
 int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t n, Trie2 *out, bool distinct,
-                int32_t vmax) {
+                int32_t vmax, const uint32_t *mm_known) {
     if (n >= (1ull << 32) - 4096) return fail(AMJ_EUNSUPPORTED, "trie build: 2^32 or more rows");
     out->len1 = n;
     if (n == 0) {
@@ -131,7 +131,9 @@ int build_trie2(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, uint64_t
         return AMJ_OK;
     }
     uint32_t h_mm[4];   // flipped min / max of both columns
-    if (vmax >= 0) {
+    if (mm_known) {
+        std::memcpy(h_mm, mm_known, sizeof(h_mm));
+    } else if (vmax >= 0) {
         // the caller knows every value lies in [0, vmax]
         h_mm[0] = h_mm[2] = 0x80000000u;
         h_mm[1] = h_mm[3] = (uint32_t)vmax ^ 0x80000000u;
@@ -331,6 +333,14 @@ __device__ __forceinline__ uint32_t rk_warp_row(int32_t *__restrict__ data1, int
     return u;
 }
 
+// The rows of one trie, or of several end to end: distinct values are counted for
+// each trie.  row[p] is the first row of trie p > 0.
+struct RowParts {
+    uint32_t row[TRIE_JOBS_MAX] = {0, 0xffffffffu, 0xffffffffu};
+    __device__ __forceinline__ int of(uint64_t v) const { return (v >= row[1] ? 1 : 0) + (v >= row[2] ? 1 : 0); }
+};
+static_assert(TRIE_JOBS_MAX == 3, "RowParts::of");
+
 // One warp a row, the row's values in registers (rows of up to RK_WARP_MAX);
 // longer rows are listed for the block kernel.
 __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(const uint32_t *__restrict__ start,
@@ -340,16 +350,24 @@ __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(con
                                                                            uint32_t *__restrict__ uniq,
                                                                            uint32_t *__restrict__ longs,
                                                                            unsigned int *__restrict__ nlong,
+                                                                           const RowParts parts,
                                                                            unsigned long long *__restrict__ distinct) {
-    __shared__ uint32_t usum;
-    if (threadIdx.x == 0) usum = 0;
+    __shared__ uint32_t usum[TRIE_JOBS_MAX];
+    if (threadIdx.x < TRIE_JOBS_MAX) usum[threadIdx.x] = 0;
     __syncthreads();
-    uint32_t u = 0;   // distinct values of this warp's rows
+    uint32_t u = 0;   // distinct values of this warp's rows of the current part
+    int part = 0;
     const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint64_t warps = (uint64_t)gridDim.x * RK_SORT_WARPS;
     for (uint64_t v = blockIdx.x * (uint64_t)RK_SORT_WARPS + w; v < nv; v += warps) {
         const uint32_t s = start[v], len = start[v + 1] - s;
         const int32_t value = values ? values[v] : (int32_t)v;
+        const int p = parts.of(v);
+        if (p != part) {
+            if (lane == 0) atomicAdd(&usum[part], u);
+            u = 0;
+            part = p;
+        }
         if (len <= 1) {
             if (len == 1 && lane == 0) src1[s] = value;
             if (lane == 0) uniq[v] = len;
@@ -371,9 +389,10 @@ __global__ __launch_bounds__(RK_SORT_WARPS * 32, 4) void rk_sort_rows_kernel(con
             uniq[v] = 0;
         }
     }
-    if (lane == 0) atomicAdd(&usum, u);
+    if (lane == 0) atomicAdd(&usum[part], u);
     __syncthreads();
-    if (threadIdx.x == 0 && usum) atomicAdd(distinct, (unsigned long long)usum);
+    if (threadIdx.x < TRIE_JOBS_MAX && usum[threadIdx.x])
+        atomicAdd(&distinct[threadIdx.x], (unsigned long long)usum[threadIdx.x]);
 }
 
 // A row of up to 1024 E values sorted by a block of 1024 threads in shared
@@ -433,6 +452,7 @@ __global__ __launch_bounds__(1024) void rk_sort_long_kernel(const uint32_t *__re
                                                             uint32_t *__restrict__ uniq,
                                                             const uint32_t *__restrict__ longs,
                                                             const unsigned int *__restrict__ nlong,
+                                                            const RowParts parts,
                                                             unsigned long long *__restrict__ distinct) {
     extern __shared__ int32_t x[];   // RK_BLOCK_MAX values, padded
     __shared__ uint32_t usum;
@@ -459,27 +479,28 @@ __global__ __launch_bounds__(1024) void rk_sort_long_kernel(const uint32_t *__re
         __syncthreads();
         if (t == 0) {
             uniq[v] = usum;
-            atomicAdd(distinct, (unsigned long long)usum);
+            atomicAdd(&distinct[parts.of(v)], (unsigned long long)usum);
         }
         __syncthreads();
     }
 }
 
 static int launch_sort_long(amj_ctx *ctx, const uint32_t *start, const int32_t *values, int32_t *data1, int32_t *src1,
-                            uint32_t *uniq, const uint32_t *longs, const unsigned int *nlong,
+                            uint32_t *uniq, const uint32_t *longs, const unsigned int *nlong, const RowParts &parts,
                             unsigned long long *distinct) {
     constexpr size_t smem = (RK_BLOCK_MAX + RK_BLOCK_MAX / 32) * sizeof(int32_t);
     AMJ_CUDA_TRY(cudaFuncSetAttribute(rk_sort_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     note_launch(ctx);
     rk_sort_long_kernel<<<ctx->num_sms, 1024, smem, ctx->stream>>>(start, values, data1, src1, uniq, longs, nlong,
-                                                                   distinct);
+                                                                   parts, distinct);
     AMJ_CUDA_TRY(cudaGetLastError());
     return AMJ_OK;
 }
 
 // repeated rows present: row v's distinct values move to ustart[v] (a warp a row)
 __global__ void rk_compact_kernel(const uint32_t *__restrict__ start, const uint32_t *__restrict__ ustart,
-                                  uint64_t nv, const int32_t *__restrict__ data1, int32_t *__restrict__ out1,
+                                  const int32_t *__restrict__ values, uint64_t nv,
+                                  const int32_t *__restrict__ data1, int32_t *__restrict__ out1,
                                   int32_t *__restrict__ outsrc) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -493,7 +514,7 @@ __global__ void rk_compact_kernel(const uint32_t *__restrict__ start, const uint
             if (keep) {
                 const uint32_t o = at + __popc(b & ((1u << lane) - 1u));
                 out1[o] = data1[s + i];
-                outsrc[o] = (int32_t)v;
+                outsrc[o] = values ? values[v] : (int32_t)v;
             }
             at += __popc(b);
         }
@@ -517,8 +538,9 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
     DBuf<uint32_t> start, place;
     struct Ctr {
         unsigned int longest, nlong;   // longest row; rows listed for the block kernel
-        unsigned long long distinct;
+        unsigned long long distinct[TRIE_JOBS_MAX];
     };
+    const RowParts one;
     AMJ_TRY(lo.alloc(ctx, n));
     AMJ_TRY(hi.alloc(ctx, n));
     AMJ_TRY(place.alloc(ctx, n));
@@ -548,7 +570,7 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
                                                                            (uint64_t)ctx->num_sms * 8));
     note_launch(ctx);
     rk_sort_rows_kernel<<<gs, RK_SORT_WARPS * 32, 0, ctx->stream>>>(start.p, nullptr, nv, out->data1.p, out->src1.p, uniq.p,
-                                                                    longs.p, &ctr->nlong, &ctr->distinct);
+                                                                    longs.p, &ctr->nlong, one, ctr->distinct);
     AMJ_CUDA_TRY(cudaGetLastError());
     // in rank order a row holds about sqrt(2 n) values at most unless edges
     // repeat: small relations launch the block sort only when they turn out to
@@ -556,7 +578,7 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
     const bool long_rows = n >= (1u << 18);
     if (long_rows) {
         AMJ_TRY(launch_sort_long(ctx, start.p, nullptr, out->data1.p, out->src1.p, uniq.p, longs.p, &ctr->nlong,
-                                 &ctr->distinct));
+                                 one, ctr->distinct));
     }
     // level 0 and the row pointers, unless rows repeat or are too long
     out->len0 = nv;
@@ -575,23 +597,24 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
     AMJ_TRY(read_back(ctx, &h, ctr, sizeof(h)));
     if (!long_rows && h.nlong && h.longest <= RK_BLOCK_MAX) {
         AMJ_TRY(launch_sort_long(ctx, start.p, nullptr, out->data1.p, out->src1.p, uniq.p, longs.p, &ctr->nlong,
-                                 &ctr->distinct));
+                                 one, ctr->distinct));
         AMJ_TRY(read_back(ctx, &h, ctr, sizeof(h)));
     }
     if (h.longest > RK_BLOCK_MAX) {
         *out = Trie2();
         return build_trie2(ctx, lo.p, hi.p, n, out, true, (int32_t)(nv - 1));
     }
-    out->len1 = h.distinct;
-    if (h.distinct == n) return AMJ_OK;
+    out->len1 = h.distinct[0];
+    if (h.distinct[0] == n) return AMJ_OK;
     // repeated rows: the distinct values of every row, compacted
     AMJ_CUDA_TRY(cudaMemsetAsync(uniq.p + nv, 0, sizeof(uint32_t), ctx->stream));
     AMJ_TRY(scan_exclusive_u32(ctx, uniq.p, uniq.p, nv + 1, nullptr));
     DBuf<int32_t> d1, s1;
-    AMJ_TRY(d1.alloc(ctx, h.distinct + TRIE_LEVEL1_PAD));
-    AMJ_TRY(s1.alloc(ctx, h.distinct ? h.distinct : 1));
+    AMJ_TRY(d1.alloc(ctx, h.distinct[0] + TRIE_LEVEL1_PAD));
+    AMJ_TRY(s1.alloc(ctx, h.distinct[0] ? h.distinct[0] : 1));
     note_launch(ctx);
-    rk_compact_kernel<<<grid_for(ctx, nv * 32), 256, 0, ctx->stream>>>(start.p, uniq.p, nv, out->data1.p, d1.p, s1.p);
+    rk_compact_kernel<<<grid_for(ctx, nv * 32), 256, 0, ctx->stream>>>(start.p, uniq.p, nullptr, nv, out->data1.p, d1.p,
+                                                                       s1.p);
     note_launch(ctx);
     rk_level0_kernel<<<grid_for(ctx, nv + 1), 256, 0, ctx->stream>>>(uniq.p, nv, out->data0.p, out->rowptr.p);
     AMJ_CUDA_TRY(cudaGetLastError());
@@ -607,8 +630,10 @@ int build_trie2_ranked(amj_ctx *ctx, const int32_t *d_c0, const int32_t *d_c1, u
 // for its builds instead of some hundred and nine (three relations of 1M edges:
 // 1.03 ms one by one, 0.36 ms together).  Level 0 lists every
 // value of the first column's range, which has to be dense (at most 4 n + 4096
-// values); with wider ranges, rows above RK_BLOCK_MAX or repeated rows *built
-// stays false and the caller builds the tries one by one.
+// values).  Repeated rows are dropped by a compaction of the relations that have
+// some (1.05 to 1.41 ms with one repeated row in each of three 1M-edge relations; 2.11 ms
+// when one sent all of them to the radix sort).  A relation with a wider range, or with a row above
+// RK_BLOCK_MAX, is built alone.
 struct TrieJob {
     const int32_t *c0, *c1;
     uint32_t n, nrows;   // edges; values of the first column's range
@@ -694,7 +719,7 @@ __global__ __launch_bounds__(256) void tries_scatter_kernel(const __grid_constan
 }
 
 // level-0 values and row pointers (within the relation's own entries), and the
-// longest row
+// longest row of every relation
 __global__ __launch_bounds__(256) void tries_level0_kernel(const __grid_constant__ TrieJobs A,
                                                            const uint32_t *__restrict__ start,
                                                            int32_t *__restrict__ data0,
@@ -710,63 +735,90 @@ __global__ __launch_bounds__(256) void tries_level0_kernel(const __grid_constant
         }
     }
     m = __reduce_max_sync(AMJ_FULL_MASK, m);
-    if ((threadIdx.x & 31) == 0 && m > ld_volatile_u32(longest)) atomicMax(longest, m);
+    __shared__ uint32_t wm[8];
+    if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; w++) m = max(m, wm[w]);
+        if (m > ld_volatile_u32(longest + blockIdx.y)) atomicMax(longest + blockIdx.y, m);
+    }
 }
 
-int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf<char> *block, bool *built) {
-    *built = false;
-    if (count < 1 || count > TRIE_JOBS_MAX) return fail(AMJ_EINVAL, "tries: bad count");
+// the row pointers of a relation whose repeated rows were dropped
+__global__ void tries_rowptr_kernel(const uint32_t *__restrict__ ustart, uint64_t nrows, uint64_t len1,
+                                    uint64_t *__restrict__ rowptr) {
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v <= nrows; v += (uint64_t)gridDim.x * blockDim.x)
+        rowptr[v] = v < nrows ? ustart[v] : len1;
+}
+
+// The tries of the relations whose rows can be bucketed by counting; *alone gets a
+// bit for every other one.  mm[t]: least and greatest values of its columns,
+// sign flipped, as build_trie2 takes them (of relations with rows).
+static int build_tries2_joint(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf<char> *block,
+                              uint32_t (*mm)[4], bool *mm_read, uint32_t *alone) {
+    *alone = (1u << count) - 1;
     TrieJobs A{};
-    uint64_t n = 0, nmax = 0;
-    for (int t = 0; t < count; t++) {
-        if (cols[t].n == 0) return AMJ_OK;
-        A.j[t].c0 = cols[t].c0;
-        A.j[t].c1 = cols[t].c1;
-        n += cols[t].n;
-        nmax = std::max(nmax, cols[t].n);
-        if (n >= (1ull << 31)) return AMJ_OK;
-        A.j[t].n = (uint32_t)cols[t].n;
-        A.j[t].e0 = (uint32_t)(n - cols[t].n);
-    }
     struct Ctr {
         uint32_t mm[4 * TRIE_JOBS_MAX];
-        unsigned int longest, nlong;
-        unsigned long long distinct;
+        unsigned int longest[TRIE_JOBS_MAX], nlong;
+        unsigned long long distinct[TRIE_JOBS_MAX];
     } h;
+    uint64_t nmax = 0, n = 0;
+    for (int t = 0; t < count; t++) {
+        if (cols[t].n >= (1ull << 31)) return AMJ_OK;
+        A.j[t].c0 = cols[t].c0;
+        A.j[t].c1 = cols[t].c1;
+        A.j[t].n = (uint32_t)cols[t].n;
+        nmax = std::max(nmax, cols[t].n);
+    }
+    if (!nmax) return AMJ_OK;
     DBuf<Ctr> ctr;
     AMJ_TRY(ctr.alloc(ctx, 1));
     AMJ_CUDA_TRY(cudaMemsetAsync(ctr.p, 0, sizeof(Ctr), ctx->stream));
-    const unsigned gx = (unsigned)std::min<uint64_t>((nmax + 255) / 256, (uint64_t)ctx->num_sms * 8);
     note_launch(ctx);
-    tries_minmax_kernel<<<dim3((unsigned)std::min<uint64_t>(gx, (uint64_t)ctx->num_sms * 2), count), 256, 0,
+    tries_minmax_kernel<<<dim3((unsigned)std::min<uint64_t>((nmax + 255) / 256, (uint64_t)ctx->num_sms * 2), count), 256, 0,
                           ctx->stream>>>(A, ctr.p->mm);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(read_back(ctx, &h, ctr.p, sizeof(h)));
+    // the relations built together: job j of A is relation rel[j]
+    int rel[TRIE_JOBS_MAX], jobs = 0;
     uint64_t rows = 0;
+    nmax = 0;
     for (int t = 0; t < count; t++) {
-        const uint32_t mn = ~h.mm[4 * t], mx = h.mm[4 * t + 1];
-        out[t].range1 = (uint64_t)(h.mm[4 * t + 3] - ~h.mm[4 * t + 2]) + 1;
-        const uint64_t range = (uint64_t)(mx - mn) + 1;
-        if (range > 4 * cols[t].n + 4096) return AMJ_OK;
-        A.j[t].min0 = mn;
-        A.j[t].nrows = (uint32_t)range;
-        A.j[t].row0 = (uint32_t)rows;
+        if (!cols[t].n) continue;
+        for (int k = 0; k < 4; k++) mm[t][k] = k & 1 ? h.mm[4 * t + k] : ~h.mm[4 * t + k];
+        const uint64_t range = (uint64_t)(mm[t][1] - mm[t][0]) + 1;
+        if (range > 4 * cols[t].n + 4096 || rows + range >= (1ull << 31) || n + cols[t].n >= (1ull << 31)) continue;
+        TrieJob &J = A.j[jobs];
+        J.c0 = cols[t].c0;
+        J.c1 = cols[t].c1;
+        J.n = (uint32_t)cols[t].n;
+        J.min0 = mm[t][0];
+        J.nrows = (uint32_t)range;
+        J.row0 = (uint32_t)rows;
+        J.e0 = (uint32_t)n;
         rows += range;
-        if (rows >= (1ull << 31)) return AMJ_OK;
+        n += cols[t].n;
+        nmax = std::max(nmax, cols[t].n);
+        rel[jobs++] = t;
     }
+    *mm_read = true;
+    if (!jobs) return AMJ_OK;
     // the tries' arrays in one block, the scratch in another
     auto round = [](uint64_t b) { return (b + 255) / 256 * 256; };
     const uint64_t b_data1 = round((n + TRIE_LEVEL1_PAD) * 4), b_src1 = round(n * 4), b_data0 = round(rows * 4);
     uint64_t b_rp = 0;
-    for (int t = 0; t < count; t++) b_rp += round(((uint64_t)A.j[t].nrows + 1) * 8);
+    for (int j = 0; j < jobs; j++) b_rp += round(((uint64_t)A.j[j].nrows + 1) * 8);
     AMJ_TRY(block->alloc(ctx, b_data1 + b_src1 + b_data0 + b_rp));
     char *at = block->p;
     int32_t *data1 = reinterpret_cast<int32_t *>(at), *src1 = reinterpret_cast<int32_t *>(at + b_data1);
     int32_t *data0 = reinterpret_cast<int32_t *>(at + b_data1 + b_src1);
     at += b_data1 + b_src1 + b_data0;
-    for (int t = 0; t < count; t++) {
-        A.j[t].rowptr = reinterpret_cast<uint64_t *>(at);
-        at += round(((uint64_t)A.j[t].nrows + 1) * 8);
+    RowParts parts;
+    for (int j = 0; j < jobs; j++) {
+        parts.row[j] = A.j[j].row0;
+        A.j[j].rowptr = reinterpret_cast<uint64_t *>(at);
+        at += round(((uint64_t)A.j[j].nrows + 1) * 8);
     }
     DBuf<uint32_t> start, place, uniq, longs;
     AMJ_TRY(start.alloc(ctx, rows + 1));
@@ -774,46 +826,86 @@ int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf
     AMJ_TRY(uniq.alloc(ctx, rows));
     AMJ_TRY(longs.alloc(ctx, n / (RK_WARP_MAX + 1) + 1));
     AMJ_CUDA_TRY(cudaMemsetAsync(start.p, 0, (rows + 1) * sizeof(uint32_t), ctx->stream));
-    const dim3 grid(gx, count);
+    const dim3 grid((unsigned)std::min<uint64_t>((nmax + 255) / 256, (uint64_t)ctx->num_sms * 8), jobs);
     note_launch(ctx);
-    tries_count_kernel<<<dim3((unsigned)((nmax + 256 * TRIES_PER_THREAD - 1) / (256 * TRIES_PER_THREAD)), count), 256, 0,
+    tries_count_kernel<<<dim3((unsigned)((nmax + 256 * TRIES_PER_THREAD - 1) / (256 * TRIES_PER_THREAD)), jobs), 256, 0,
                          ctx->stream>>>(A, start.p, place.p);
     AMJ_CUDA_TRY(cudaGetLastError());
     AMJ_TRY(scan_exclusive_u32(ctx, start.p, start.p, rows + 1, nullptr));
     note_launch(ctx);
     tries_scatter_kernel<<<grid, 256, 0, ctx->stream>>>(A, start.p, place.p, data1);
     note_launch(ctx);
-    tries_level0_kernel<<<grid, 256, 0, ctx->stream>>>(A, start.p, data0, &ctr.p->longest);
+    tries_level0_kernel<<<grid, 256, 0, ctx->stream>>>(A, start.p, data0, ctr.p->longest);
     AMJ_CUDA_TRY(cudaGetLastError());
     const unsigned gs = (unsigned)std::min<uint64_t>((rows + RK_SORT_WARPS - 1) / RK_SORT_WARPS,
                                                      (uint64_t)ctx->num_sms * 8);
     note_launch(ctx);
     rk_sort_rows_kernel<<<gs, RK_SORT_WARPS * 32, 0, ctx->stream>>>(start.p, data0, rows, data1, src1, uniq.p, longs.p,
-                                                                    &ctr.p->nlong, &ctr.p->distinct);
+                                                                    &ctr.p->nlong, parts, ctr.p->distinct);
     AMJ_CUDA_TRY(cudaGetLastError());
     if (nmax > RK_WARP_MAX)
-        AMJ_TRY(launch_sort_long(ctx, start.p, data0, data1, src1, uniq.p, longs.p, &ctr.p->nlong, &ctr.p->distinct));
+        AMJ_TRY(launch_sort_long(ctx, start.p, data0, data1, src1, uniq.p, longs.p, &ctr.p->nlong, parts,
+                                 ctr.p->distinct));
     AMJ_TRY(read_back(ctx, &h, ctr.p, sizeof(h)));
-    if (h.longest > RK_BLOCK_MAX || h.distinct != n) return AMJ_OK;
-    for (int t = 0; t < count; t++) {
-        // views of the block: no context, so they free nothing
-        Trie2 &o = out[t];
-        const TrieJob &J = A.j[t];
+    for (int j = 0; j < jobs; j++) {
+        Trie2 &o = out[rel[j]];
+        const TrieJob &J = A.j[j];
+        if (h.longest[j] > RK_BLOCK_MAX) continue;   // unsorted rows
+        const uint64_t len1 = h.distinct[j];
+        if (len1 == J.n) {
+            // views of the block: no context, so they free nothing
+            o.data1.p = data1 + J.e0;
+            o.data1.n = J.n;
+            o.src1.p = src1 + J.e0;
+            o.src1.n = J.n;
+        } else {
+            // repeated rows: the distinct values of every row, moved together
+            uint32_t *ustart = uniq.p + J.row0;
+            AMJ_TRY(o.data1.alloc(ctx, len1 + TRIE_LEVEL1_PAD));
+            AMJ_TRY(o.src1.alloc(ctx, len1));
+            AMJ_TRY(scan_exclusive_u32(ctx, ustart, ustart, J.nrows, nullptr));
+            note_launch(ctx);
+            rk_compact_kernel<<<grid_for(ctx, (uint64_t)J.nrows * 32), 256, 0, ctx->stream>>>(
+                start.p + J.row0, ustart, data0 + J.row0, J.nrows, data1, o.data1.p, o.src1.p);
+            note_launch(ctx);
+            tries_rowptr_kernel<<<grid_for(ctx, (uint64_t)J.nrows + 1), 256, 0, ctx->stream>>>(ustart, J.nrows, len1,
+                                                                                             J.rowptr);
+            AMJ_CUDA_TRY(cudaGetLastError());
+        }
         o.len0 = J.nrows;
-        o.len1 = J.n;
-        o.data1.p = data1 + J.e0;
-        o.data1.n = J.n;
-        o.src1.p = src1 + J.e0;
-        o.src1.n = J.n;
+        o.len1 = len1;
         o.data0.p = data0 + J.row0;
         o.data0.n = J.nrows;
         o.off0.p = o.rowptr.p = J.rowptr;
         o.off0.n = o.rowptr.n = (uint64_t)J.nrows + 1;
         o.rp_min = (int32_t)(J.min0 ^ 0x80000000u);
         o.rp_count = J.nrows;
+        o.range1 = (uint64_t)(mm[rel[j]][3] - mm[rel[j]][2]) + 1;
+        *alone &= ~(1u << rel[j]);
     }
-    *built = true;
     return AMJ_OK;
+}
+
+int build_tries2(amj_ctx *ctx, const TrieCols *cols, int count, Trie2 *out, DBuf<char> *block) {
+    if (count < 1 || count > TRIE_JOBS_MAX) return fail(AMJ_EINVAL, "tries: bad count");
+    uint32_t mm[TRIE_JOBS_MAX][4], alone = 0;
+    bool mm_read = false;
+    auto build_alone = [&](uint32_t which) {
+        for (int t = 0; t < count; t++)
+            if ((which >> t) & 1u)
+                AMJ_TRY(build_trie2(ctx, cols[t].c0, cols[t].c1, cols[t].n, &out[t], true, -1,
+                                    mm_read && cols[t].n ? mm[t] : nullptr));
+        return (int)AMJ_OK;
+    };
+    int rc = build_tries2_joint(ctx, cols, count, out, block, mm, &mm_read, &alone);
+    if (rc == AMJ_OK) rc = build_alone(alone);
+    if (rc == AMJ_ENOMEM) {
+        // one by one, beside nothing else
+        for (int t = 0; t < count; t++) out[t] = Trie2();
+        block->release();
+        rc = build_alone((1u << count) - 1);
+    }
+    return rc;
 }
 
 // ---- N-level tries ----
