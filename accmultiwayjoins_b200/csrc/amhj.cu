@@ -127,7 +127,7 @@ struct ExecScratch {
     std::map<IndexKey, HashIndex> indexes;
     DBuf<char> index_block;      // memory of the indexes built together
     void *zeroed = nullptr;      // zeroed bytes of that block, for one pass
-    cudaEvent_t begin = nullptr; // recorded before the passes
+    cudaEvent_t begin = nullptr; // to be recorded before the first launch of the passes
     cudaEvent_t end = nullptr;   // to be recorded behind the last launch, when a pass knows it is the last
     bool ended = false;
     DBuf<ProbeState> st;
@@ -210,6 +210,13 @@ static int ensure_state(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws) 
     PL.st = X.st.p;
     PL.tasks = X.tasks.p;
     PL.task_ready = X.ready.p;
+    return AMJ_OK;
+}
+
+// the probe phase begins, unless it has begun
+static int begin_probe(amj_ctx *ctx, ExecScratch &X) {
+    if (X.begin) AMJ_CUDA_TRY(cudaEventRecord(X.begin, ctx->stream));
+    X.begin = nullptr;
     return AMJ_OK;
 }
 
@@ -342,10 +349,12 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     } else {
         AMJ_CUDA_TRY(cudaMemsetAsync(ctr, 0, sizeof(FlatCtr), ctx->stream));
     }
-    // a query of one pass is timed by its own events: each costs the stream a
-    // few microseconds
+    // the kernels of a query of one pass are timed by the events of its probe
+    // phase, which begins here and ends with them: another pair of events costs
+    // the query two or three microseconds (10K-row chain: 80 us, then 83)
     const cudaEvent_t kb = X.begin ? X.begin : ctx->kev[0], ke = X.end ? X.end : ctx->kev[1];
-    if (!X.begin) AMJ_CUDA_TRY(cudaEventRecord(kb, ctx->stream));
+    X.begin = nullptr;
+    AMJ_CUDA_TRY(cudaEventRecord(kb, ctx->stream));
     if (canon) {
         HeadOut H{};
         size_t at = 0;
@@ -451,6 +460,7 @@ static int run_star_write(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, uint64_
     PL.P.row_lo = row_lo;
     PL.P.row_hi = row_hi;
     ProbePlan P = PL.P;
+    AMJ_TRY(begin_probe(ctx, X));
     const uint64_t rows = row_hi - row_lo;
     DBuf<unsigned long long> off, ctr;
     AMJ_TRY(off.alloc(ctx, rows + 1));
@@ -495,6 +505,7 @@ static int run_passes(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws, bo
         return run_flat_count(ctx, PL, X, ws, row_lo, row_hi, pr, res);
     if (materialize && !dro && allow_flat && star_eligible(PL.P))
         return run_star_write(ctx, PL, X, row_lo, row_hi, pr, res);
+    AMJ_TRY(begin_probe(ctx, X));
     AMJ_TRY(ensure_state(ctx, PL, X, ws));
     ProbePlan &P = PL.P;
     P.row_lo = row_lo;
@@ -1190,7 +1201,7 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         lvix[l] = &it->second;
     }
     AMJ_TRY(build_bucket_indexes(ctx, specs, nspecs, &X.index_block, &X.zeroed));
-    AMJ_CUDA_TRY(cudaEventRecord(e1, ctx->stream));
+    X.begin = e1;
 
     // ---- probe plan
     ProbeLaunch PL;
@@ -1201,7 +1212,10 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
     plan_inline(P);
     P.sort_out = sort_out ? 1 : 0;
     PL.status = ctx->d_status;
-    if (fib && !dro && hp.L >= 3) AMJ_TRY(build_fib(ctx, hp, lvix, PL, X, out));
+    if (fib && !dro && hp.L >= 3) {
+        AMJ_TRY(begin_probe(ctx, X));
+        AMJ_TRY(build_fib(ctx, hp, lvix, PL, X, out));
+    }
 
     int rc = AMJ_OK;
     if (hp.L == 0) {
@@ -1231,9 +1245,11 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
             out->rows = r->n;
         }
     } else if (ooc || hp.probe->where == AMJ_MEM_HOST_STREAMED) {
+        AMJ_TRY(begin_probe(ctx, X));
         rc = amhj_ooc_execute(ctx, PL, &X, hp.probe, use_ws, dro != 0, materialize, flags, out);
     } else if (flags & AMJ_F_THREAD_PER_ROW) {
         // the thread-per-row baseline (count only)
+        AMJ_TRY(begin_probe(ctx, X));
         if (materialize || !thread_row_eligible(P)) {
             rc = fail(AMJ_EUNSUPPORTED, "amhj_execute: the thread-per-row baseline counts over bucket indexes only");
         } else {
@@ -1263,7 +1279,6 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         }
     } else {
         PassResult pr;
-        X.begin = e1;
         X.end = e2;
         rc = run_passes(ctx, PL, X, use_ws, dro != 0, materialize, 0, hp.probe->n, &pr, out, !(flags & AMJ_F_FRONTIER));
         if (rc == AMJ_OK) {
@@ -1282,6 +1297,7 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         amj_result_release(out);
         return rc;
     }
+    AMJ_TRY(begin_probe(ctx, X));   // no pass
     if (!X.ended) {
         AMJ_CUDA_TRY(cudaEventRecord(e2, ctx->stream));
         AMJ_CUDA_TRY(cudaEventSynchronize(e2));

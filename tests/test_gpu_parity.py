@@ -1429,3 +1429,17 @@ def test_trie_rows_around_the_block_sort(ctx, deg, shape):
         s, d = np.concatenate([s, np.repeat(s[:1], deg)]), np.concatenate([d, np.repeat(d[:1], deg)])
         got = ctx.lftj([ctx.relation([s, d], [0, 1])])
     assert (got.count, got.checksum) == want
+
+
+def test_kernel_time_of_a_flat_query_is_its_kernels(ctx):
+    """kernel_ms[0] of a query joined by the flat kernels leaves out what comes
+    between the builds and the kernels: the search for frequent keys (fib=1; no
+    key is frequent here, so the flat kernel runs after it)."""
+    rels = [([np.arange(20000, dtype=np.int32), data.permutation(20000, i)], [i, i + 1]) for i in range(4)]
+    hs = rels_on(ctx, rels)
+    for ws, fib in ((0, 0), (1, 1)):
+        runs = [ctx.amhj("NORMAL", hs, ws=ws, fib=fib) for _ in range(5)]
+        assert all((r.count, r.checksum) == O.mhj(rels) for r in runs)
+        assert all(0 < r.kernel_ms[0] <= r.probe_ms < r.total_ms and r.build_ms > 0 for r in runs)
+        if fib:
+            assert min(r.kernel_ms[0] / r.probe_ms for r in runs) < 0.5
