@@ -240,7 +240,8 @@ __global__ void bucket_heads_kernel(const __grid_constant__ CanonPlan S, const _
 // twice as many buckets (one more key bit), which take the same memory and
 // overflow as rarely as three rows of a 32-byte head.  A free row holds a key
 // of the neighbouring bucket, which no lookup here asks for; a bucket of more
-// rows holds such a key with payload 1 in its first row.
+// rows holds such keys with its index bucket's bounds as payloads, the first
+// raised by one so that it is not zero.
 // 60M-row star over 1M / 200K / 100K / 10K rows, Zipf(1.1) and uniform keys: 0.66
 // and 0.81 ms (0.90 and 0.92 with 32-byte heads).
 struct __align__(16) StarHead {
@@ -248,8 +249,15 @@ struct __align__(16) StarHead {
 };
 static_assert(sizeof(StarHead) == 16 && 2 * sizeof(StarHead) == sizeof(BucketHead), "two star heads a bucket");
 // Blocks per SM: one lookup in flight a thread wants all of them (one dimension,
-// 50M rows: 0.30 ms with four blocks, 0.20 with eight), four run out of registers.
-constexpr int star_blocks(int L) { return L == 1 ? 8 : L == 2 ? 7 : 6; }
+// 50M rows: 0.30 ms with four blocks, 0.20 with eight).  Two dimensions take five:
+// rows with several matches run out of registers with more (4M rows, 8 matches in
+// each: 2.49 ms with seven, 2.24 with five, 2.08 with four; one match in each, 8M
+// rows: 0.197, 0.204 and 0.209).
+constexpr int star_blocks(int L) { return L == 1 ? 8 : L == 2 ? 5 : 6; }
+// Dimensions up to which a row's overflowing buckets take their bounds from the
+// heads (one dimension, 3 rows a key: 0.32 to 0.28 ms); with four, keeping the
+// heads that long cost the rows with a key missing (0.32 to 0.37 ms).
+constexpr int STAR_HEAD_BOUNDS = 2;
 constexpr uint32_t STAR_HEAD_SCAN = 8;   // longer index buckets are taken as overflowing
 
 // the heads of level blockIdx.y: index bucket h holds the rows of h and h + nb
@@ -282,7 +290,7 @@ __global__ void star_heads_kernel(const __grid_constant__ CanonPlan S, const __g
                     m++;
                 }
             }
-            if (n > STAR_HEAD_SCAN || m > 2) o[x] = StarHead{none, 1, none, 0};
+            if (n > STAR_HEAD_SCAN || m > 2) o[x] = StarHead{none, (int32_t)(s + 1), none, (int32_t)(s + n)};
             out[h + x * nb] = o[x];
         }
     }
@@ -328,9 +336,16 @@ __global__ __launch_bounds__(256, star_blocks(L)) void amhj_star_canon_kernel(co
 #pragma unroll
         for (int c = 0; c < L; c++) {
             const uint32_t b = (uint32_t)k[c] & S.mask[c];
-            e[c] = S.bp[c][b + 1];
+            uint32_t s;
+            if (L <= STAR_HEAD_BOUNDS && (uint32_t)w[c].x == (((uint32_t)k[c] & (2 * S.nb[c] - 1)) ^ 1u) && w[c].y != 0) {
+                s = (uint32_t)w[c].y - 1;
+                e[c] = (uint32_t)w[c].w;
+            } else {
+                s = S.bp[c][b];
+                e[c] = S.bp[c][b + 1];
+            }
             uint32_t nm = 0, f = e[c];
-            for (uint32_t i = S.bp[c][b]; i < e[c]; i++)
+            for (uint32_t i = s; i < e[c]; i++)
                 if (S.key[c][i] == k[c]) {
                     if (nm == 0) f = i;
                     nm++;
