@@ -994,7 +994,11 @@ __global__ void bfs_tile_first_kernel(const unsigned long long *__restrict__ off
     }
 }
 
-template <bool WRITE>
+// HUBS: the launch has a hub matrix, and a thread takes all of an edge's
+// candidates in its run at once.  Without one it takes them one by one, so that
+// lanes whose edges have few candidates keep step with the others (R-MAT, 1M
+// edges as given: 1.27 ms, 1.56 with an edge at once).
+template <bool WRITE, bool HUBS>
 __global__ __launch_bounds__(BFS_THREADS) void lftj_tri_bfs_expand_kernel(const __grid_constant__ TriArgs A,
                                                                           const unsigned long long *__restrict__ offs,
                                                                           const uint32_t *__restrict__ tile_first,
@@ -1024,7 +1028,7 @@ __global__ __launch_bounds__(BFS_THREADS) void lftj_tri_bfs_expand_kernel(const 
         bool s_short = false;
         const uint32_t *hub_row = nullptr;   // b's row of the hub matrix
         for (unsigned long long t = t0; t < t1;) {
-            {
+            if (HUBS || e == ~0ull || t >= nxt) {
                 if (e == ~0ull) {
                     if (in_smem) {
                         uint64_t lo = 0, hi = ne;
@@ -1057,47 +1061,17 @@ __global__ __launch_bounds__(BFS_THREADS) void lftj_tri_bfs_expand_kernel(const 
                     xa = alo ? ra.id : rb.id;
                     xb = alo ? rb.id : ra.id;
                     hab = alo ? ra.h1 : rb.h1;
-                    hub_row = A.hub_mtx && b >= A.hub_base
-                                  ? A.hub_mtx + (uint64_t)(uint32_t)(b - A.hub_base) * A.hub_words
-                                  : nullptr;
+                    if (HUBS)
+                        hub_row = b >= A.hub_base ? A.hub_mtx + (uint64_t)(uint32_t)(b - A.hub_base) * A.hub_words
+                                                  : nullptr;
                 } else {
                     xa = a;
                     xb = b;
                     hab = amj_hash_step(amj_hash_step(AMJ_CHECKSUM_SEED, xa), xb);
                 }
             }
-            // this edge's part of the run: membership of its candidates first
-            // (all loads in flight together), then the hits
-            const uint32_t len = (uint32_t)((nxt < t1 ? nxt : t1) - t);
             const int32_t *cand = (s_short ? A.S.data1 + sb : A.T.data1 + (A.bfs_wedge ? A.r_lo + e + 1 : ta)) + (t - cur);
-            t += len;
-            uint32_t hits = 0;
-            if (hub_row) {
-                uint32_t x[BFS_RUN], w[BFS_RUN];
-#pragma unroll
-                for (int k = 0; k < BFS_RUN; k++) x[k] = (uint32_t)k < len ? (uint32_t)(cand[k] - A.hub_base) : 0u;
-#pragma unroll
-                for (int k = 0; k < BFS_RUN; k++) w[k] = hub_row[x[k] >> 5];
-#pragma unroll
-                for (int k = 0; k < BFS_RUN; k++) hits |= ((w[k] >> (x[k] & 31)) & 1u) << k;
-                hits &= (1u << len) - 1u;
-            } else {
-                const int32_t *hay = s_short ? A.T.data1 : A.S.data1;
-                for (uint32_t k = 0; k < len; k++) {
-                    const int32_t c = cand[k];
-                    uint64_t lo = s_short ? ta : sb, hi = s_short ? ea : eb;
-                    while (lo < hi) {
-                        uint64_t mid = (lo + hi) >> 1;
-                        if (hay[mid] < c) lo = mid + 1;
-                        else hi = mid;
-                    }
-                    if (lo < (s_short ? ea : eb) && hay[lo] == c) hits |= 1u << k;
-                }
-            }
-            cnt += __popc(hits);
-            while (hits) {
-                const int32_t c = cand[__ffs(hits) - 1];
-                hits &= hits - 1;
+            auto emit = [&](int32_t c) {
                 int32_t xc = c;
                 if (A.inv) {
                     // the triangle (xc, xa, xb) in increasing order, hashed
@@ -1112,6 +1086,41 @@ __global__ __launch_bounds__(BFS_THREADS) void lftj_tri_bfs_expand_kernel(const 
                 if (WRITE) {
                     const unsigned long long p = atomicAdd(A.out_cursor, 1ull);
                     if (p < A.out_cap) tri_store(A, p, xa, xb, xc);
+                }
+            };
+            const uint32_t len = HUBS ? (uint32_t)((nxt < t1 ? nxt : t1) - t) : 1u;
+            t += len;
+            if (HUBS && hub_row) {
+                // membership of this edge's part of the run first (all loads in
+                // flight together), then the hits
+                uint32_t x[BFS_RUN], w[BFS_RUN], hits = 0;
+#pragma unroll
+                for (int k = 0; k < BFS_RUN; k++) x[k] = (uint32_t)k < len ? (uint32_t)(cand[k] - A.hub_base) : 0u;
+#pragma unroll
+                for (int k = 0; k < BFS_RUN; k++) w[k] = hub_row[x[k] >> 5];
+#pragma unroll
+                for (int k = 0; k < BFS_RUN; k++) hits |= ((w[k] >> (x[k] & 31)) & 1u) << k;
+                hits &= (1u << len) - 1u;
+                cnt += __popc(hits);
+                while (hits) {
+                    const int32_t c = cand[__ffs(hits) - 1];
+                    hits &= hits - 1;
+                    emit(c);
+                }
+            } else {
+                const int32_t *hay = s_short ? A.T.data1 : A.S.data1;
+                for (uint32_t k = 0; k < len; k++) {
+                    const int32_t c = cand[k];
+                    uint64_t lo = s_short ? ta : sb, hi = s_short ? ea : eb;
+                    while (lo < hi) {
+                        uint64_t mid = (lo + hi) >> 1;
+                        if (hay[mid] < c) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    if (lo < (s_short ? ea : eb) && hay[lo] == c) {
+                        cnt++;
+                        emit(c);
+                    }
                 }
             }
         }
@@ -1289,10 +1298,10 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
                 A.hub_mtx = hubs.p;
             }
             if (total) {
+                auto kern = A.hub_mtx ? (write ? lftj_tri_bfs_expand_kernel<true, true> : lftj_tri_bfs_expand_kernel<false, true>)
+                                      : (write ? lftj_tri_bfs_expand_kernel<true, false> : lftj_tri_bfs_expand_kernel<false, false>);
                 int per_sm = 0;
-                AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &per_sm, write ? lftj_tri_bfs_expand_kernel<true> : lftj_tri_bfs_expand_kernel<false>,
-                    BFS_THREADS, 0));
+                AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BFS_THREADS, 0));
                 if (per_sm < 1) per_sm = 1;
                 const uint64_t tiles = (total + BFS_TILE - 1) / BFS_TILE;
                 DBuf<uint32_t> first;
@@ -1303,10 +1312,7 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
                 const unsigned grid = (unsigned)std::min<uint64_t>(tiles, (uint64_t)ctx->num_sms * per_sm);
                 note_launch(ctx);
                 AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[2], ctx->stream));
-                if (write)
-                    lftj_tri_bfs_expand_kernel<true><<<grid, BFS_THREADS, 0, ctx->stream>>>(A, cand.p, first.p, total);
-                else
-                    lftj_tri_bfs_expand_kernel<false><<<grid, BFS_THREADS, 0, ctx->stream>>>(A, cand.p, first.p, total);
+                kern<<<grid, BFS_THREADS, 0, ctx->stream>>>(A, cand.p, first.p, total);
                 AMJ_CUDA_TRY(cudaGetLastError());
                 AMJ_CUDA_TRY(cudaEventRecord(ctx->kev[3], ctx->stream));
                 timed[1] = true;

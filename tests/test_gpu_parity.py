@@ -1443,3 +1443,27 @@ def test_kernel_time_of_a_flat_query_is_its_kernels(ctx):
         assert all(0 < r.kernel_ms[0] <= r.probe_ms < r.total_ms and r.build_ms > 0 for r in runs)
         if fib:
             assert min(r.kernel_ms[0] / r.probe_ms for r in runs) < 0.5
+
+
+@pytest.mark.parametrize("form", ["oriented", "as_given", "both_ways", "complete"])
+def test_lftj_bfs_written_out_with_and_without_hub_matrix(ctx, form):
+    """Breadth-first triangles written out, from enough candidates for the hub
+    matrix on (oriented relations joined in degree order) and by search only."""
+    if form == "complete":
+        s, d = (c.astype(np.int32) for c in np.triu_indices(200, 1))
+    else:
+        s, d = data.rmat(13, 1 << 17, 0.57, 0.19, 0.19, 9)
+    cnt, chk, want = O.triangle(s, d, tuples=True)
+    assert form != "complete" or cnt > 1 << 20
+    if form == "both_ways":
+        s, d = np.concatenate([s, d]), np.concatenate([d, s])
+    e = ctx.relation([s, d], [0, 1])
+    got = ctx.lftj([e], algo="BFS", materialize=True, degree_order=False if form == "as_given" else None)
+    same = ctx.lftj([e], algo="DFS", materialize=True)
+    assert (got.count, got.checksum) == (same.count, same.checksum)
+    assert data.checksum(got.columns) == got.checksum
+    rows = sorted_rows(got.columns)
+    assert np.array_equal(rows, sorted_rows(same.columns))
+    if form != "both_ways":
+        assert (got.count, got.checksum) == (cnt, chk)
+        assert np.array_equal(rows, sorted_rows(want))
