@@ -1289,13 +1289,17 @@ int lftj_triangle(amj_ctx *ctx, const Trie2 &R, const Trie2 &S, const Trie2 &T, 
                 const uint64_t k = std::min<uint64_t>(nv, HUB_RANKS);
                 A.hub_base = (int32_t)(nv - k);
                 A.hub_words = (uint32_t)((k + 31) / 32);
-                AMJ_TRY(hubs.alloc(ctx, k * A.hub_words));
-                AMJ_CUDA_TRY(cudaMemsetAsync(hubs.p, 0, k * A.hub_words * sizeof(uint32_t), ctx->stream));
-                note_launch(ctx);
-                hub_matrix_kernel<<<g1, 256, 0, ctx->stream>>>(R.src1.p, R.data1.p, R.len1, A.hub_base, A.hub_words,
-                                                               hubs.p);
-                AMJ_CUDA_TRY(cudaGetLastError());
-                A.hub_mtx = hubs.p;
+                // without room for it: search
+                const int rc = hubs.alloc(ctx, k * A.hub_words);
+                if (rc != AMJ_OK && rc != AMJ_ENOMEM) return rc;
+                if (rc == AMJ_OK) {
+                    AMJ_CUDA_TRY(cudaMemsetAsync(hubs.p, 0, k * A.hub_words * sizeof(uint32_t), ctx->stream));
+                    note_launch(ctx);
+                    hub_matrix_kernel<<<g1, 256, 0, ctx->stream>>>(R.src1.p, R.data1.p, R.len1, A.hub_base,
+                                                                   A.hub_words, hubs.p);
+                    AMJ_CUDA_TRY(cudaGetLastError());
+                    A.hub_mtx = hubs.p;
+                }
             }
             if (total) {
                 auto kern = A.hub_mtx ? (write ? lftj_tri_bfs_expand_kernel<true, true> : lftj_tri_bfs_expand_kernel<false, true>)

@@ -40,11 +40,12 @@ def scratch_of(call):
 
 
 @contextlib.contextmanager
-def device_with(free):
-    """The device filled up to `free` bytes."""
+def device_with(free, trim=True):
+    """The device filled up to `free` bytes (and the pool's unused blocks, unless they are given back first)."""
     import torch
     torch.cuda.synchronize()
-    pool_call("cudaMemPoolTrimTo", 0)
+    if trim:
+        pool_call("cudaMemPoolTrimTo", 0)
     torch.cuda.empty_cache()
     left = torch.cuda.mem_get_info()[0]
     assert left > free
@@ -107,3 +108,19 @@ def test_batch_triangles_with_and_without_heads(kind, n):
                 assert (r.counts[1], r.checksums[1]) == O.triangle(d, s)
             launches.append(r.launches)
     assert launches[1] == launches[0] - 1   # the heads' kernel
+
+
+def test_breadth_first_triangles_without_room_for_the_hub_matrix():
+    """A complete graph of 200 vertices with its ids spread over 20 thousand: 1.3
+    million candidates over 20 thousand edges, and a matrix of 32 MB."""
+    u, v = np.triu_indices(200, 1)
+    s, d = (u * 100).astype(np.int32), (v * 100).astype(np.int32)
+    want = O.triangle(s, d)
+    with Context(0) as ctx:
+        e = ctx.relation([s, d], [0, 1])
+        assert (lambda r: (r.count, r.checksum))(ctx.lftj([e], algo="BFS")) == want
+        pool_call("cudaMemPoolTrimTo", 0)
+        assert (lambda r: (r.count, r.checksum))(ctx.lftj([e], algo="DFS")) == want   # the pool's first block
+        with device_with(8 * MB, trim=False):
+            got = ctx.lftj([e], algo="BFS")
+            assert (got.count, got.checksum) == want
