@@ -332,7 +332,10 @@ static int run_flat_count(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws
     DBuf<char> work;
     const uint64_t over_bytes = (std::max<uint64_t>(rows, 1) * sizeof(uint32_t) + 255) / 256 * 256;
     const uint32_t pair_cap = chain && canon > 1 ? (uint32_t)std::min<uint64_t>(rows, 1u << 24) : 0u;
-    AMJ_TRY(work.alloc(ctx, nheads * sizeof(BucketHead) + 256 + over_bytes + (uint64_t)pair_cap * sizeof(uint2)));
+    const int rc = work.alloc(ctx, nheads * sizeof(BucketHead) + 256 + over_bytes + (uint64_t)pair_cap * sizeof(uint2));
+    if (rc == AMJ_ENOMEM)   // no room for the heads and lists: the DFS kernel needs neither
+        return run_passes(ctx, PL, X, ws, false, false, row_lo, row_hi, pr, res, false);
+    AMJ_TRY(rc);
     if (reinterpret_cast<uintptr_t>(work.p) % alignof(BucketHead) != 0 && canon) {
         if (chain) return run_passes(ctx, PL, X, ws, false, false, row_lo, row_hi, pr, res, false);
         canon = 0;

@@ -124,3 +124,24 @@ def test_breadth_first_triangles_without_room_for_the_hub_matrix():
         with device_with(8 * MB, trim=False):
             got = ctx.lftj([e], algo="BFS")
             assert (got.count, got.checksum) == want
+
+
+def result(r):
+    return r.count, r.checksum
+
+
+def test_chain_counts_without_room_for_heads_and_lists():
+    """8M probe rows and small build relations: the lists of what the flat
+    kernel leaves (12 bytes a probe row) are nearly all of the query's memory;
+    the frontier kernel joins it without them."""
+    n = 1 << 23
+    rels = [([data.uniform(n, 0, 4000, 1), data.uniform(n, 0, 4000, 2)], [0, 1])]
+    rels += [([data.uniform(1000, 0, 4000, 3 + i), data.uniform(1000, 0, 4000, 7 + i)], [1 + i, 2 + i]) for i in range(2)]
+    with Context(0) as ctx:
+        hs = [ctx.relation(c, at) for c, at in rels]
+        want = result(ctx.amhj("NORMAL", hs, plan="frontier"))
+        assert want[0] > 0
+        need, got = scratch_of(lambda: result(ctx.amhj("NORMAL", hs)))
+        assert got == want and need > 12 << 23
+        with device_with(need // 2):
+            assert result(ctx.amhj("NORMAL", hs)) == want
