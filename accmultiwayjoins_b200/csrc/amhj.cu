@@ -1203,7 +1203,16 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         }
         lvix[l] = &it->second;
     }
-    AMJ_TRY(build_bucket_indexes(ctx, specs, nspecs, &X.index_block, &X.zeroed));
+    int brc = build_bucket_indexes(ctx, specs, nspecs, &X.index_block, &X.zeroed);
+    if (brc == AMJ_ENOMEM && nspecs > 1) {
+        // one by one: each with its own columns only, and its own places at a time
+        X.index_block.release();
+        X.zeroed = nullptr;
+        brc = AMJ_OK;
+        for (int i = 0; i < nspecs && brc == AMJ_OK; i++)
+            brc = build_bucket_indexes(ctx, &specs[i], 1, &specs[i].out->block);
+    }
+    AMJ_TRY(brc);
     X.begin = e1;
 
     // ---- probe plan

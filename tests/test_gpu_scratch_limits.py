@@ -145,3 +145,20 @@ def test_chain_counts_without_room_for_heads_and_lists():
         assert got == want and need > 12 << 23
         with device_with(need // 2):
             assert result(ctx.amhj("NORMAL", hs)) == want
+
+
+def test_indexes_built_together_or_one_by_one():
+    """A wide small table beside a long narrow one: built together they share
+    columns as many and as long as any needs, built one by one they do not."""
+    n = 1 << 23
+    wide = [data.uniform(100, 0, 1 << 20, 3 + i) for i in range(4)]
+    rels = [([data.uniform(1000, 0, 100, 1), data.uniform(1000, 0, n, 2)], [0, 1]),
+            ([data.permutation(n, 8), data.uniform(n, 0, 1 << 20, 9)], [1, 2]), (wide, [0, 3, 4, 5])]
+    rels[2][0][0][:] = np.arange(100)
+    want = O.mhj(rels)
+    with Context(0) as ctx:
+        hs = [ctx.relation(c, at) for c, at in rels]
+        need, got = scratch_of(lambda: result(ctx.amhj("NORMAL", hs)))
+        assert got == want and want[0] == 1000 and need > 23 << 23   # 4 columns, bounds, places
+        with device_with(need - (5 << 23)):                          # 2 columns fewer: 8 bytes a row
+            assert result(ctx.amhj("NORMAL", hs)) == want
