@@ -203,8 +203,8 @@ static int ensure_state(amj_ctx *ctx, ProbeLaunch &PL, ExecScratch &X, bool ws) 
         AMJ_TRY(X.st.alloc(ctx, 1));
         AMJ_TRY(status_reset(ctx));
     }
-    if (ws && !X.tasks.p) {
-        AMJ_TRY(X.tasks.alloc(ctx, PL.P.task_cap));
+    if (ws && !X.ready.p) {
+        if (!X.tasks.p) AMJ_TRY(X.tasks.alloc(ctx, PL.P.task_cap));
         AMJ_TRY(X.ready.alloc(ctx, PL.P.task_cap));
     }
     PL.st = X.st.p;
@@ -240,7 +240,10 @@ static int alloc_cols(amj_ctx *ctx, int k, uint64_t rows, int32_t **cols) {
     for (int a = 0; a < k; a++) {
         int rc = dev_alloc(ctx, (void **)&cols[a], (rows ? rows : 1) * sizeof(int32_t));
         if (rc != AMJ_OK) {
-            for (int b = 0; b < a; b++) dev_free(ctx, cols[b]);
+            for (int b = 0; b < a; b++) {
+                dev_free(ctx, cols[b]);
+                cols[b] = nullptr;
+            }
             return rc;
         }
     }
@@ -824,16 +827,17 @@ static int build_fib(amj_ctx *ctx, const HostPlan &hp, const std::vector<const H
     PassResult sub;
     amj_result sub_res;   // its statistics are not the query's
     std::memset(&sub_res, 0, sizeof(sub_res));
-    AMJ_TRY(run_passes(ctx, SL, X, true, false, true, 0, K, &sub, &sub_res, false, FIB_MAX_ROWS));
+    const int rc = run_passes(ctx, SL, X, true, false, true, 0, K, &sub, &sub_res, false, FIB_MAX_ROWS);
     const uint64_t T = sub.count;
     const int k = hp.k;
-    std::vector<DBuf<int32_t>> tmp(k);   // own the pass's columns from here on
+    std::vector<DBuf<int32_t>> tmp(k);   // own the pass's columns, also those of a pass that failed
     int32_t *tcols[AMJ_MAX_ATTRS] = {};
     for (int at = 0; at < k; at++) {
         tmp[at].ctx = ctx;
         tmp[at].p = tcols[at] = sub.cols[at];
         tmp[at].n = T;
     }
+    AMJ_TRY(rc);
     if (T == 0 || T > FIB_MAX_ROWS) return AMJ_OK;
     // 3. group the suffix tuples by key: hash set of the keys, sort by cache index
     uint32_t slots = 512;
@@ -1293,6 +1297,8 @@ extern "C" int amj_amhj_execute(amj_ctx *ctx, int query_type, amj_rel *const *re
         PassResult pr;
         X.end = e2;
         rc = run_passes(ctx, PL, X, use_ws, dro != 0, materialize, 0, hp.probe->n, &pr, out, !(flags & AMJ_F_FRONTIER));
+        if (rc != AMJ_OK)
+            for (int a = 0; a < hp.k; a++) dev_free(ctx, pr.cols[a]);
         if (rc == AMJ_OK) {
             out->count = pr.count;
             out->checksum = pr.checksum;
