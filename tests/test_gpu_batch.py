@@ -274,3 +274,22 @@ def test_batch_units_of_queries_without_a_second_frontier():
         both = b.run(layout="oa")
         assert both.units - flat.units > 1000
         assert list(zip(both.counts, both.checksums)) == [(flat.counts[0], flat.checksums[0]), O.mhj(chain)]
+
+
+@pytest.mark.parametrize("beside", ["nothing", "star", "chain"])
+def test_batch_triangles_beside_other_queries(beside):
+    """Triangle queries alone, and beside a query of the other kernel: every
+    count and checksum, eager and replayed."""
+    edges = [data.rmat(9, 3000, 0.57, 0.19, 0.19, s) for s in (1, 2, 3)]
+    queries = [("TRI", [(list(e), [0, 1])], O.triangle(*e)) for e in edges]
+    star = [([data.uniform(100, 0, 50, 1)], [0]), ([data.permutation(50, 2), data.uniform(50, 0, 9, 3)], [0, 1])]
+    chain = data.chain_relations(4000, 600, 4, seed=5)
+    if beside != "nothing":
+        rels = star if beside == "star" else chain
+        queries.insert(1, ("NORMAL", rels, O.mhj(rels)))
+    with Context(0) as ctx, ctx.batch() as b:
+        for qt, rels, _ in queries:
+            b.submit(qt, [ctx.relation(c, a) for c, a in rels])
+        for graph in (False, True, True):
+            r = b.run(use_graph=graph)
+            assert list(zip(r.counts, r.checksums)) == [w for _, _, w in queries]

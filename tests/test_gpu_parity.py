@@ -1467,3 +1467,61 @@ def test_lftj_bfs_written_out_with_and_without_hub_matrix(ctx, form):
     if form != "both_ways":
         assert (got.count, got.checksum) == (cnt, chk)
         assert np.array_equal(rows, sorted_rows(want))
+
+
+@pytest.mark.parametrize("materialize", [False, True])
+@pytest.mark.parametrize("fib", [0, 1])
+@pytest.mark.parametrize("capacity", [1, 2, 7, 64])
+def test_work_sharing_with_a_full_queue(capacity, fib, materialize):
+    """Task queues that fill up at once, without direct output: ranges and parts
+    of frontiers that find no slot stay with their warp, some lanes of one
+    frontier push and others do not, and served ranges are split in half."""
+    n = 3000
+    rels = [([data.uniform(400, 0, 9, 1), data.uniform(400, 0, 40, 2)], [0, 1]),
+            ([data.zipf(n, 40, 1.1, 3), data.uniform(n, 0, 30, 4)], [1, 2]),
+            ([np.concatenate([np.arange(30), np.zeros(90, int), np.ones(60, int)]).astype(np.int32),
+              data.uniform(180, 0, 20, 5)], [2, 3]),
+            ([data.zipf(60, 20, 1.0, 6), data.uniform(60, 0, 9, 7)], [3, 4])]
+    want = O.mhj(rels)
+    assert want[0] > 200_000
+    with Context(0, task_chunk=32, task_capacity=capacity) as ctx:
+        got = ctx.amhj("NORMAL", rels_on(ctx, rels), ws=1, fib=fib, materialize=materialize, plan="frontier")
+        assert (got.count, got.checksum) == want
+        assert got.stats["tasks_pushed"] == got.stats["tasks_popped"] <= capacity * (2 if materialize else 1)
+        assert got.stats["tasks_pushed"] > 0
+        assert not fib or got.stats["fib_rows_served"] > 0
+        if materialize:
+            assert len(got.columns[0]) == want[0] and data.checksum(got.columns) == want[1]
+
+
+@pytest.mark.parametrize("capacity", [1, 2, 7, 64])
+@pytest.mark.parametrize("plan", ["multiway", "hash"])
+def test_weighted_work_sharing_with_a_full_queue(capacity, plan):
+    """FOUR by hash lookups: frontiers of weighted tuples and a queue that fills up."""
+    s, d = data.rmat(9, 9000, 0.6, 0.15, 0.15, 4)
+    want = O.four_clique(s, d)
+    with Context(0, task_chunk=32, task_capacity=capacity) as ctx:
+        e = ctx.relation([s, d], [0, 1])
+        got = ctx.amhj("FOUR", [e], ws=1, plan=plan, degree_order=False)
+        assert (got.count, got.checksum) == want
+        assert got.stats["tasks_pushed"] == got.stats["tasks_popped"] <= capacity
+
+
+def test_host_results_larger_than_the_pool(ctx):
+    """Results of 272 MB, more than the context keeps: one after another, with a
+    small one between them."""
+    n = 17_000_000
+    fact = [data.uniform(n, 0, 50, 1), data.uniform(n, 0, 60, 2)]
+    dims = [[data.permutation(m, 3), data.uniform(m, 0, 1 << 30, 4)] for m in (50, 60)]
+    looked_up = []
+    for f, (k, p) in zip(fact, dims):
+        t = np.empty(len(k), np.int32)
+        t[k] = p
+        looked_up.append(t[f])
+    for rows in (n, 1000, n):
+        hs = [ctx.relation([c[:rows].copy() for c in fact], [0, 1])]
+        hs += [ctx.relation(d, [i, 2 + i]) for i, d in enumerate(dims)]
+        r = ctx.amhj("NORMAL", hs, materialize=True)
+        assert r.count == rows
+        assert all(np.array_equal(g, w[:rows]) for g, w in zip(r.columns, fact + looked_up))
+    ctx.trim()
