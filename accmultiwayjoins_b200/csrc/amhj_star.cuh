@@ -411,14 +411,12 @@ inline int chain_canon(const ProbePlan &P, CanonPlan &S) {
     const int L = P.L;
     if (L < 1 || L + 2 > AMJ_MAX_ATTRS || P.probe_ncols != 2 || P.k != L + 2) return 0;
     if (P.has_inl || P.sort_out || P.fib_level >= 0 || P.probe_attr[0] != 0 || P.probe_attr[1] != 1) return 0;
-    bool seen[AMJ_MAX_BUILD_TABLES] = {};
     for (int l = 0; l < L; l++) {
         const LevelDesc &lv = P.lv[l];
         const int d = lv.key_attr[0] - 1;
-        if (d != l || seen[d] || lv.layout != AMJ_LAYOUT_BUCKET || lv.key_mode != KEY_SINGLE ||
+        if (d != l || lv.layout != AMJ_LAYOUT_BUCKET || lv.key_mode != KEY_SINGLE ||
             lv.cmp_mask != 1u || lv.ncols != 2 || lv.attr[0] != d + 1 || lv.attr[1] != d + 2)
             return 0;
-        seen[d] = true;
         S.key[d] = lv.col[0];
         S.pay[d] = lv.col[1];
         S.bp[d] = lv.buc_ptrs;
