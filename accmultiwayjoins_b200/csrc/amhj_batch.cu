@@ -461,9 +461,9 @@ int normalize_batch_opts(const amj_batch_opts *in, amj_batch_opts *o) {
 using BatchKernel = void (*)(const BatchLaunch);
 
 template <int T>
-static BatchKernel batch_kernel_of(bool weighted, bool open_addr) {
-    if (!weighted) return amhj_batch_kernel<T, false, false>;
-    return open_addr ? amhj_batch_kernel<T, true, true> : amhj_batch_kernel<T, true, false>;
+static BatchKernel batch_kernel_of(bool weighted, bool four_sm) {
+    if (four_sm) return weighted ? amhj_batch_kernel<T, true, true> : amhj_batch_kernel<T, false, true>;
+    return weighted ? amhj_batch_kernel<T, true, false> : amhj_batch_kernel<T, false, false>;
 }
 
 static unsigned batch_tiles(uint64_t rows) { return (unsigned)((rows + BATCH_TILE - 1) / BATCH_TILE); }
@@ -717,9 +717,10 @@ static int batch_prepare(amj_batch *b, const amj_batch_opts &o) {
     if (b->smem > (size_t)ctx->max_smem_optin) return fail(AMJ_EUNSUPPORTED, "batch: frontier exceeds shared memory");
     b->weighted = false;
     for (const ProbePlan &P : hplans) b->weighted |= P.has_inl != 0 && !P.tri;
-    b->kern = b->block == 128   ? batch_kernel_of<128>(b->weighted, b->oa_rows > 0)
-              : b->block == 256 ? batch_kernel_of<256>(b->weighted, b->oa_rows > 0)
-                                : batch_kernel_of<512>(b->weighted, b->oa_rows > 0);
+    const bool four_sm = o.grid_blocks > 0 || (b->weighted && b->oa_rows > 0);
+    b->kern = b->block == 128   ? batch_kernel_of<128>(b->weighted, four_sm)
+              : b->block == 256 ? batch_kernel_of<256>(b->weighted, four_sm)
+                                : batch_kernel_of<512>(b->weighted, four_sm);
     AMJ_CUDA_TRY(cudaFuncSetAttribute(b->kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem));
     int per_sm = 0;
     AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b->kern, (int)b->block, b->smem));

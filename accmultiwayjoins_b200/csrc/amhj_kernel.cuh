@@ -749,14 +749,17 @@ __device__ __forceinline__ void batch_flush(const BatchLaunch &B, int q, ProbeAc
 // of 256 threads hides more latency but takes its frontiers (up to 53 KB) from
 // the L1.  Batches over bucket indexes are faster with three (9M-row chain
 // beside four small queries 1.14 ms, 1.40 with four; two FOUR queries of 2^16
-// edges 3.64 ms and 3.81), weighted ones over open addressing (OA) with four
+// edges 3.64 ms and 3.81), weighted ones over open addressing with four
 // (two FOUR queries 11.0 ms, 11.7 with three; four triangle queries 6.1 and 6.4).
-constexpr int batch_min_blocks(int threads, bool wt, bool oa) {
-    return threads == 128 ? 7 : threads == 512 ? 2 : wt && oa ? 4 : 3;
+// FOUR_SM: at most 64 registers, so that blocks of four kernels fit an SM
+// together; taken by every batch on a share of the device (grid_blocks), whose
+// warps wait for blocks of their own kernel that others could keep out.
+constexpr int batch_min_blocks(int threads, bool four_sm) {
+    return four_sm ? 1024 / threads : threads == 128 ? 7 : threads == 512 ? 2 : 3;
 }
 
-template <int THREADS, bool WT, bool OA>
-__global__ __launch_bounds__(THREADS, batch_min_blocks(THREADS, WT, OA)) void amhj_batch_kernel(const __grid_constant__ BatchLaunch B) {
+template <int THREADS, bool WT, bool FOUR_SM>
+__global__ __launch_bounds__(THREADS, batch_min_blocks(THREADS, FOUR_SM)) void amhj_batch_kernel(const __grid_constant__ BatchLaunch B) {
     extern __shared__ __align__(16) char smem[];
     const int lane = threadIdx.x & 31;
     const unsigned lt = lanemask_lt();

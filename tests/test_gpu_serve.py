@@ -174,3 +174,32 @@ def test_server_rejects_bad_requests():
             srv.wait(12345)
         assert e.value.status == L.AMJ_EINVAL
         srv.close()
+
+
+@pytest.mark.parametrize("qt", ["NORMAL", "FOUR"])
+def test_batches_on_a_share_of_the_device_fit_four_to_an_sm(qt):
+    """The batch kernels of lanes and of an out-of-core lane wait for blocks of
+    their own, so blocks of four of them have to fit an SM together: at most 64
+    registers of 256 threads.  The launch's warps show in its units: the query
+    has candidates for 64 units of 128 a warp with three blocks an SM, but not
+    with four, and is then cut into units of 64."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = 1 << 20
+    rows = 55 * sms * 32 * 128 // n   # level-0 candidates a probe row, about
+    keys = n // rows
+    rng = np.random.default_rng(3)
+    with Context(0) as ctx, ctx.batch() as b:
+        chain = [[np.arange(n, dtype=np.int32), np.arange(n, dtype=np.int32) % keys],
+                 [np.arange(n, dtype=np.int32) % keys, rng.integers(0, 1 << 20, n).astype(np.int32)],
+                 [np.full(4, -1, np.int32), np.arange(4, dtype=np.int32)]]
+        b.submit("NORMAL", [ctx.relation(c, [i, i + 1]) for i, c in enumerate(chain)])
+        want = [(0, 0)]
+        if qt == "FOUR":
+            s, d = data.rmat(7, 700, 0.57, 0.19, 0.19, 1)
+            b.submit("FOUR", [ctx.relation([s, d], [0, 1])])
+            want.append(O.four_clique(s, d))
+        r = b.run(opts=b._opts(grid_blocks=4 * sms))
+        assert list(zip(r.counts, r.checksums)) == want
+        candidates = n * (n // keys)
+        assert candidates / 64 <= r.units <= candidates / 64 + 20_000
