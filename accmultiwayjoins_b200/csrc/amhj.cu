@@ -153,6 +153,7 @@ double event_ms(cudaEvent_t a, cudaEvent_t b) {
 template <int MODE, bool WS, bool WT>
 static int launch_probe_t(amj_ctx *ctx, const ProbeLaunch &PL, size_t smem) {
     auto kern = amhj_probe_kernel<MODE, WS, WT>;
+    if (WS && ctx->opts.max_blocks) kern = amhj_probe_four_sm_kernel<MODE, WT>;
     AMJ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     AMJ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, PROBE_THREADS, smem));

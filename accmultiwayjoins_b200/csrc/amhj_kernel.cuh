@@ -593,7 +593,7 @@ static __global__ void amhj_l0_sizes_kernel(const __grid_constant__ ProbePlan P,
 }
 
 template <int MODE, bool WS, bool WT>
-__global__ __launch_bounds__(PROBE_THREADS) void amhj_probe_kernel(const __grid_constant__ ProbeLaunch L) {
+__device__ __forceinline__ void probe_body(const ProbeLaunch &L) {
     extern __shared__ __align__(16) char smem[];
     const ProbePlan &P = L.P;
     const WsQueue Q{L.st, L.tasks, L.task_ready, L.status};
@@ -710,6 +710,20 @@ __global__ __launch_bounds__(PROBE_THREADS) void amhj_probe_kernel(const __grid_
         atomicAdd(&L.st->checksum, chk);
     }
     if (lane == 0 && fib) atomicAdd(&L.st->fib_rows, fib);
+}
+
+template <int MODE, bool WS, bool WT>
+__global__ __launch_bounds__(PROBE_THREADS) void amhj_probe_kernel(const __grid_constant__ ProbeLaunch L) {
+    probe_body<MODE, WS, WT>(L);
+}
+
+// The same held to 64 registers (of up to 80), for contexts that cap their blocks
+// (max_blocks): with work sharing its warps wait for blocks of their own, and
+// those have to fit beside the kernels of the other contexts.
+template <int MODE, bool WT>
+__global__ __launch_bounds__(PROBE_THREADS, 1024 / PROBE_THREADS) void amhj_probe_four_sm_kernel(
+    const __grid_constant__ ProbeLaunch L) {
+    probe_body<MODE, true, WT>(L);
 }
 
 // ------------------------------------------------------------- batched --

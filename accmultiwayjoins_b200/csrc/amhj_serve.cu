@@ -326,8 +326,9 @@ extern "C" int amj_server_create(amj_ctx *ctx, const amj_serve_opts *opts, amj_s
     // time; their idle warps wait for their own unstarted blocks, so all of
     // them must be resident together.  Each gets an equal share of four probe
     // blocks per SM: with the default 256-thread blocks (at most 64 registers
-    // a thread, frontiers of at most 61 KB for a batch of 8-attribute queries
-    // and 29 KB for an ooc chain) one block of each fits an SM together.
+    // a thread in the instances that a share of the device takes, frontiers of
+    // at most 61 KB for a batch of 8-attribute queries and 29 KB for an ooc
+    // chain) one block of each fits an SM together.
     int sms = 0;
     AMJ_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     const int kernels = s->opts.lanes + (s->opts.ooc_lane ? 1 : 0);

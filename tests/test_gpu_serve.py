@@ -203,3 +203,26 @@ def test_batches_on_a_share_of_the_device_fit_four_to_an_sm(qt):
         assert list(zip(r.counts, r.checksums)) == want
         candidates = n * (n // keys)
         assert candidates / 64 <= r.units <= candidates / 64 + 20_000
+
+
+@pytest.mark.parametrize("dro,materialize,fib", [(0, False, 0), (0, False, 1), (0, True, 0), (0, True, 1), (1, True, 0)])
+def test_work_sharing_on_a_share_of_the_device(dro, materialize, fib):
+    """Contexts that cap their blocks (max_blocks) take probe kernels held to 64
+    registers: the same counts, tuples and direct output, residual passes
+    included, and weighted plans."""
+    rels = data.chain_relations(3000, 300, 4, seed=7)
+    rels[2][0][0][:1500] = 5
+    cnt, chk, cols = O.mhj(rels, tuples=True)
+    s, d = data.rmat(8, 2500, 0.57, 0.19, 0.19, 2)
+    with Context(0, max_blocks=148, task_chunk=64, dro_headroom=0.5) as ctx:
+        r = ctx.amhj("NORMAL", [ctx.relation(c, a) for c, a in rels], ws=1, dro=dro, fib=fib, materialize=materialize,
+                     plan="frontier")
+        assert (r.count, r.checksum) == (cnt, chk) and r.stats["tasks_pushed"] > 0
+        if materialize:
+            assert len(r.columns[0]) == cnt and data.checksum(r.columns) == chk
+        if dro:
+            assert r.stats["residual_units"] > 0
+        e = ctx.relation([s, d], [0, 1])
+        for qt, want in (("TRI", O.triangle(s, d)), ("FOUR", O.four_clique(s, d))):
+            r = ctx.amhj(qt, [e], ws=1, dro=dro, materialize=materialize, plan="hash", degree_order=False)
+            assert (r.count, r.checksum) == want
