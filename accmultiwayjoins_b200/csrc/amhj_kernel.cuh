@@ -130,7 +130,8 @@ static __device__ int ws_acquire(const WsQueue &Q, uint32_t cap, uint64_t spin_l
 // split of single long ranges leaves frontiers of many ranges below twice the
 // task size, and trees of them below one unit or task, to one warp: 14 skewed
 // chains ended in a tail of 7.1 ms whatever the size of their units, 5.0 ms with
-// the sharing.
+// the sharing.  The line is not sharp: 64, 256 and 1024 take 0.71, 0.69 and 0.68 ms
+// on a skewed 4-way chain of 1M rows, and the same on batches of chains and stars.
 constexpr uint32_t WS_SHARE_MIN = 256;
 
 // last index r in [0, n) with E[r] <= g (E non-decreasing, E[0] <= g); warp-uniform call

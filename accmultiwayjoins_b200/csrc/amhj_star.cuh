@@ -252,7 +252,9 @@ static_assert(sizeof(StarHead) == 16 && 2 * sizeof(StarHead) == sizeof(BucketHea
 // 50M rows: 0.30 ms with four blocks, 0.20 with eight).  Two dimensions take five:
 // rows with several matches run out of registers with more (4M rows, 8 matches in
 // each: 2.49 ms with seven, 2.24 with five, 2.08 with four; one match in each, 8M
-// rows: 0.197, 0.204 and 0.209).
+// rows: 0.197, 0.204 and 0.209).  16M rows of three dimensions with four, five, six
+// and seven blocks: 0.361, 0.352, 0.347 and 0.380 ms; of four: 0.465, 0.451, 0.446,
+// 0.596.
 constexpr int star_blocks(int L) { return L == 1 ? 8 : L == 2 ? 5 : 6; }
 // Dimensions up to which a row's overflowing buckets take their bounds from the
 // heads (one dimension, 3 rows a key: 0.32 to 0.28 ms); with four, keeping the
@@ -508,8 +510,10 @@ __device__ __forceinline__ void chain_spread(const CanonPlan &S, int d, ChainSta
 }
 
 // six blocks per SM (40 registers) up to two levels (1M rows: 100 us; four blocks
-// 116, eight 120), four (64 registers) at three; deeper walks keep their
-// per-level state in two blocks' worth of registers
+// 116, eight 120), four (64 registers) at three (0.332 ms; 0.360 with six, 0.369
+// with three); deeper walks keep their per-level state in two blocks' worth of
+// registers (1M rows, four and five levels: 1.10 and 3.71 ms; three blocks measure
+// 0.83 and 2.90, four 0.73 and 3.40)
 template <int L>
 __global__ __launch_bounds__(256, L <= 2 ? 6 : L <= 3 ? 4 : 2) void amhj_chain_canon_kernel(
     const __grid_constant__ CanonPlan S, FlatCtr *ctr, FlatCtr *host, uint32_t *over, uint2 *pairs,

@@ -172,7 +172,10 @@ constexpr uint32_t BM_SEG = 1024;   // values of one child list per warp work it
 // block barriers between them, so an SM wants several: where T's values span
 // at most BM_SMALL_BITS, eight blocks of 256 threads with a bitmap of that
 // span run per SM, else one block of 1024 threads.  1M-edge R-MAT relations:
-// 0.49 ms, with one block per SM and vertex 0.97 ms.
+// 0.49 ms, with one block per SM and vertex 0.97 ms.  Whole queries by the small
+// and by the large form, three relations: 1M edges over 2^17 ids 0.97 and 1.13 ms,
+// over 2^18 0.96 and 1.13, 2M edges over 2^19 1.82 and 1.93, so that the line could
+// lie higher than it does.
 constexpr uint32_t BM_SMALL_BITS = 1u << 17;
 
 template <bool WRITE, int BM_THREADS>
@@ -951,7 +954,10 @@ __global__ void lftj_tri_bfs_count_kernel(const __grid_constant__ TriArgs A, uns
 // edges among the top HUB_RANKS ranks are kept as a bit matrix (32 MB, which
 // L2 holds), and the lookup is one load instead of a binary search of six to
 // nine dependent ones.  Lower b are searched as before.  The matrix is built
-// from BFS_HUB_MIN candidates on: clearing and filling it takes up to 20 us.
+// from BFS_HUB_MIN candidates on: clearing and filling it takes up to 20 us
+// (R-MAT as triangles, query with and without it: 2^17 edges 276 and 267 us, 2^18
+// 302 and 319, 2^19 369 and 439, 2^21 0.88 and 1.35 ms).  8192 or 32768 ranks:
+// 2^21 edges 0.96 and 0.88 ms, 2^19 372 and 399 us.
 // R-MAT, 2M edges: expand kernel 1637 to 938 us by the matrix, 882 us with a
 // thread's run tested together, 618 us with the tiles' owners found beforehand.
 constexpr uint64_t HUB_RANKS = 16384;

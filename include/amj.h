@@ -257,7 +257,7 @@ typedef struct amj_batch_stats {
     double   build_ms, probe_ms, total_ms;   /* device time of the run               */
     uint64_t launches;                       /* kernels in one run                   */
     uint64_t tasks_pushed, tasks_popped;     /* work-sharing tasks                   */
-    uint64_t units;                          /* level-0 units of 1024 candidates     */
+    uint64_t units;                          /* level-0 units, 64 to 1024 candidates */
     uint64_t build_rows, build_jobs;         /* rows indexed, distinct indexes       */
     int32_t  graph;                          /* 1: the run replayed a captured graph */
     int32_t  pad;
